@@ -1,16 +1,32 @@
 // tmk_march.cuh -- column-marching volume kernel.
 //
 // A warp owns 32 adjacent columns of a patch (28 updated columns plus a
-// 2-column halo on each side) and streams up a run of rows.  Per row it
-// computes the x predictor (each lane's neighbours read from the row's copy in
-// shared memory, which also holds the column one beyond the warp on either
-// side: the outermost slopes need them, and with them a 2-column halo is
-// enough for the 3-cell stencil of one update) and the y predictor
-// (a rolling window of rows in registers), the first-pass Riemann states,
-// the transverse corrections, the final Riemann states, the fluxes and the
-// conservative update -- the CTU sequence of LinElastPatchGodunov::computeWHalf
-// and LinElastPhysics::computeUpdate (srcLinElast/LinElastPatchGodunov.cpp:174-469)
-// -- emitting one updated row per step, three rows behind the loads.
+// 2-column halo on each side) and streams up a run of rows, emitting one
+// updated row per step: the CTU sequence of LinElastPatchGodunov::computeWHalf
+// and LinElastPhysics::computeUpdate (srcLinElast/LinElastPatchGodunov.cpp:174-469).
+//
+// The medium of a level is uniform, so past the limiters every stage is linear
+// with constant coefficients and is carried out on the characteristic values
+// that meet at a face instead of on states: for a wave pair (v, s) of
+// direction D and impedance Z,
+//   An = s + Z v + traced left-going delta    at the cell's lo face,
+//   Ap = s - Z v + traced right-going delta   at the cell's hi face
+// are all that RIEMANNF (srcLinElast/LinElastPhysicsF.ChF:601-765) reads of the
+// predicted states WM, WP of a cell.  The face state between cells i-1 and i is
+// s = (An_i + Ap_{i-1})/2, v = (An_i - Ap_{i-1})/(2Z), so the difference of the
+// two face states of a cell follows from the jumps
+//   jn = An_{i+1} - An_i,   jp = Ap_i - Ap_{i-1}
+// as ds = (jn + jp)/2, dv = (jn - jp)/(2Z).  The transverse term (GETADWDXF,
+// :791-901) of one direction moves the values An, Ap of the other one by
+// multiples of ds and dv, and the update (GETFLUXF, :265-353) is a multiple of
+// ds and dv of the moved values.  No predicted state, face state or flux is
+// formed (but the fluxes of coarse-fine faces, for the flux registers): a wave
+// pair takes 10 operations to trace, 4 for the jumps' sums and differences, 4
+// to correct, where states took about 60, and one or two values per pair are
+// exchanged between lanes and carried from row to row instead of all
+// components.  The stresses in An and Ap are taken relative to the scenario's
+// background, which every jump cancels: in FP32 their rounding is that of the
+// waves' amplitude, not of the 100 MPa they ride on.
 //
 // The state of the two fault sides is packed into one pair per component
 // (.x = side 1, .y = side 2; the y direction of side 2 is mirrored, rv = -1),
@@ -19,10 +35,8 @@
 //   in-plane  (vx vy sxx syy szz sxy): a P-wave pair, an S-wave pair and the
 //             two normal stresses tied to the P-wave stress by lam/(lam+2G);
 //   antiplane (vz sxz syz): an S-wave pair and one stress with zero speed.
-// The characteristic transforms, the PPM tracing (Colella & Woodward 1984
-// eq. 1.12, written as a*w_near + b*w_far with a = (1-s)^2, b = s^2 - s) and
-// the syntheses of srcLinElast/LinElastPhysicsF.ChF:359-555 are applied per
-// wave pair.
+// The PPM tracing is Colella & Woodward 1984 eq. 1.12, written as
+// a*w_near + b*w_far with a = (1-s)^2, b = s^2 - s.
 #pragma once
 #include "tmk_device.cuh"
 #include "tmk_kernels.cuh"
@@ -42,9 +56,10 @@ TMK_D float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 TMK_D float2 psub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 TMK_D double2 padd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 TMK_D double2 pmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
-TMK_D double2 pfma(double2 a, double2 b, double2 c) { return make_double2(a.x * b.x + c.x, a.y * b.y + c.y); }
+TMK_D double2 pfma(double2 a, double2 b, double2 c) { return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)); }
 TMK_D double2 psub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-template <typename P> TMK_D P pneg(P a) { return pmul(a, mk2(decltype(a.x)(-1), decltype(a.x)(-1))); }
+TMK_D float2 pneg(float2 a) { return pmul(a, make_float2(-1.f, -1.f)); }
+TMK_D double2 pneg(double2 a) { return make_double2(-a.x, -a.y); }
 
 TMK_D float2 shfl_up2(float2 v, int d) {
   return make_float2(__shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d));
@@ -98,79 +113,87 @@ template <int G, int D> TMK_HD constexpr bool live(int c) {
   return !((R::hasZc && (c == R::zc0 || c == R::zc1)) || (R::hasZf && c == R::zf));
 }
 
-// Packed constants of one direction.  A packed FP32x2 instruction takes a
-// constant operand straight from the parameter bank only when both halves are
-// the same scalar (a broadcast); a pair of two values has to be loaded into
-// registers at each use once the registers are full.  So every constant is
-// also kept as its side-1 scalar (the s* fields): in x, and for the constants
-// that do not change sign with the mirrored y direction of side 2, the
-// kernels build the pair from that scalar (kc, ke); only the y-direction
-// constants with rv (side 2 = -side 1) are used as pairs.
+// Wave pairs of a group: in-plane 0 = P, 1 = S; antiplane 0 = S.
+template <int G> constexpr int kWaves = G == 0 ? 2 : 1;
+template <int G> TMK_HD constexpr bool is_p(int w) { return G == 0 && w == 0; }
+template <int G, int D> TMK_HD constexpr int wave_v(int w) { return is_p<G>(w) ? Role<G, D>::vP : Role<G, D>::vS; }
+template <int G, int D> TMK_HD constexpr int wave_s(int w) { return is_p<G>(w) ? Role<G, D>::sP : Role<G, D>::sS; }
+
+// Constants of one direction D (E: the other one).  A packed FP32x2
+// instruction takes a constant operand straight from the parameter bank only
+// when both halves are the same scalar (a broadcast); a pair of two values has
+// to be loaded into registers.  The products of two constants that both carry
+// rv (side 2 = -side 1 in y) are the same on both sides, so only the ones with
+// a single rv are pairs: the impedances of y, the velocity terms.
 template <typename T>
 struct MK {
   using P = typename PairOf<T>::P;
-  P ZpE, ZsE;          // characteristic w = s +- ZE v (ZE = rv Z)
-  P nZpE, nZsE;        // -ZE
-  P hZpE, hZsE;        // synthesis v = (w- - w+) * rv/(2Z)
-  P half, r, nr;       // 1/2, lam/(lam+2G), -lam/(lam+2G)
-  P aP, bP, aS, bS;    // PPM tracing coefficients of the P and S speeds
-  P f_irho, f_l2g, f_lam, f_G;   // GETFLUXF: -rv * {1/rho, lam+2G, lam, G}
-  P a_irho, a_l2g, a_lam, a_G;   // GETADWDXF: -rv*scale * {...}
-  // side-1 scalars of the pairs above
-  T sZpE, sZsE, snZpE, snZsE, shZpE, shZsE, saP, sbP, saS, sbS;
-  T sf_irho, sf_l2g, sf_lam, sf_G, sa_irho, sa_l2g, sa_lam, sa_G;
-  TMK_HD void load(const DevParams& p, int D, double dtdx, double scale) {
-    const T s2 = (D == 1) ? T(-1) : T(1);       // rv of side 2
-    ZpE = mk2((T)p.Zp, (T)(s2 * p.Zp)); ZsE = mk2((T)p.Zs, (T)(s2 * p.Zs));
-    nZpE = mk2((T)-p.Zp, (T)(-s2 * p.Zp)); nZsE = mk2((T)-p.Zs, (T)(-s2 * p.Zs));
-    hZpE = mk2((T)(0.5 / p.Zp), (T)(s2 * 0.5 / p.Zp)); hZsE = mk2((T)(0.5 / p.Zs), (T)(s2 * 0.5 / p.Zs));
-    half = mk2(T(0.5), T(0.5));
-    const T rr = (T)(p.lam / (p.lam + 2.0 * p.G));
-    r = mk2(rr, rr);
-    nr = mk2(-rr, -rr);
+  P Zp, Zs, nZp, nZs;  // characteristics w = s +- Z v (rv Z)
+  T aP, bP, aS, bS;    // PPM tracing coefficients of the P and S speeds, halved (the deltas are kept doubled)
+  // transverse term of D on the characteristic values of E: the stress part
+  // from the differences jn - jp, the velocity part (times E's impedance) from
+  // the sums jn + jp
+  T c_lam, c_G;
+  P cvP, cvS, ncvP, ncvS;
+  // update: velocities from the sums, stresses from the differences
+  P e_v;
+  T e_l2g, e_lam, e_G;
+  // face states and GETFLUXF: v = (An - Ap) hZ, F = -rv * {1/rho, lam+2G, lam, G}
+  P hZp, hZs, f_irho, f_l2g, f_lam, f_G;
+  // per wave pair (P, in-plane S, antiplane S): the background's
+  // characteristic values, whose stress part is zero, and its stress
+  P bgn[3], bgp[3];
+  T s0[3];
+  TMK_HD void load(const DevParams& p, int D, double dtdx) {
+    const double s2 = (D == 1) ? -1.0 : 1.0;    // rv of side 2
+    auto two = [](double a, double b) { return mk2((T)a, (T)b); };
+    Zp = two(p.Zp, s2 * p.Zp); Zs = two(p.Zs, s2 * p.Zs);
+    nZp = two(-p.Zp, -s2 * p.Zp); nZs = two(-p.Zs, -s2 * p.Zs);
     const double sp = p.cp * dtdx, ss = p.cs * dtdx;
-    const T ap = (T)((1.0 - sp) * (1.0 - sp)), bp = (T)(sp * sp - sp);
-    const T as = (T)((1.0 - ss) * (1.0 - ss)), bs = (T)(ss * ss - ss);
-    aP = mk2(ap, ap); bP = mk2(bp, bp); aS = mk2(as, as); bS = mk2(bs, bs);
-    const double m1 = -1.0, m2 = -s2;
-    f_irho = mk2((T)(m1 / p.rho), (T)(m2 / p.rho));
-    f_l2g = mk2((T)(m1 * (p.lam + 2.0 * p.G)), (T)(m2 * (p.lam + 2.0 * p.G)));
-    f_lam = mk2((T)(m1 * p.lam), (T)(m2 * p.lam));
-    f_G = mk2((T)(m1 * p.G), (T)(m2 * p.G));
-    a_irho = mk2((T)(m1 * scale / p.rho), (T)(m2 * scale / p.rho));
-    a_l2g = mk2((T)(m1 * scale * (p.lam + 2.0 * p.G)), (T)(m2 * scale * (p.lam + 2.0 * p.G)));
-    a_lam = mk2((T)(m1 * scale * p.lam), (T)(m2 * scale * p.lam));
-    a_G = mk2((T)(m1 * scale * p.G), (T)(m2 * scale * p.G));
-    sZpE = ZpE.x; sZsE = ZsE.x; snZpE = nZpE.x; snZsE = nZsE.x; shZpE = hZpE.x; shZsE = hZsE.x;
-    saP = ap; sbP = bp; saS = as; sbS = bs;
-    sf_irho = f_irho.x; sf_l2g = f_l2g.x; sf_lam = f_lam.x; sf_G = f_G.x;
-    sa_irho = a_irho.x; sa_l2g = a_l2g.x; sa_lam = a_lam.x; sa_G = a_G.x;
+    aP = (T)(0.5 * (1.0 - sp) * (1.0 - sp)); bP = (T)(0.5 * (sp * sp - sp));
+    aS = (T)(0.5 * (1.0 - ss) * (1.0 - ss)); bS = (T)(0.5 * (ss * ss - ss));
+    const double l2g = p.lam + 2.0 * p.G;
+    c_lam = (T)(0.5 * dtdx * p.lam * (0.5 / p.Zp));
+    c_G = (T)(0.5 * dtdx * p.G * (0.5 / p.Zs));
+    // the velocity term carries the rv of y in both directions (D's or E's)
+    const double vP = p.Zp * (0.25 * dtdx / p.rho), vS = p.Zs * (0.25 * dtdx / p.rho);
+    cvP = two(vP, -vP); cvS = two(vS, -vS); ncvP = two(-vP, vP); ncvS = two(-vS, vS);
+    const double ev = 0.5 * dtdx / p.rho;
+    e_v = two(ev, s2 * ev);
+    e_l2g = (T)(dtdx * l2g * (0.5 / p.Zp)); e_lam = (T)(dtdx * p.lam * (0.5 / p.Zp));
+    e_G = (T)(dtdx * p.G * (0.5 / p.Zs));
+    hZp = two(0.5 / p.Zp, s2 * 0.5 / p.Zp); hZs = two(0.5 / p.Zs, s2 * 0.5 / p.Zs);
+    f_irho = two(-1.0 / p.rho, -s2 / p.rho);
+    f_l2g = two(-l2g, -s2 * l2g); f_lam = two(-p.lam, -s2 * p.lam); f_G = two(-p.G, -s2 * p.G);
+    const int v[3] = {D, 1 - D, 2}, s[3] = {3 + D, 6, 7 + D};
+    for (int w = 0; w < 3; ++w) {
+      const double Z = w == 0 ? p.Zp : p.Zs;
+      bgn[w] = two(Z * p.bg[v[w]], s2 * Z * p.bg[11 + v[w]]);
+      bgp[w] = two(-Z * p.bg[v[w]], -s2 * Z * p.bg[11 + v[w]]);
+      s0[w] = (T)p.bg[s[w]];            // both sides start from one background (tmk_context_create)
+    }
   }
 };
 
-// Constant `name` of direction D as a pair: in x a broadcast of its scalar,
-// in y the stored pair (side 2 = -side 1 for the constants carrying rv).
-template <int D, typename T>
-TMK_D typename PairOf<T>::P kc_(const typename PairOf<T>::P& pair, T s) {
-  if constexpr (D == 0) return mk2(s, s);
+// A constant of direction D that carries rv in y: in x a broadcast of one
+// scalar, in y the stored pair.
+template <int D, typename P> TMK_D P kpair(const P& pair) {
+  if constexpr (D == 0) return mk2(pair.x, pair.x);
   else return pair;
 }
-#define KC(name) kc_<D, T>(k.name, k.s##name)
-// a constant with the same value on both sides in either direction
-#define KE(name) mk2(k.s##name, k.s##name)
-#define KHALF mk2(T(0.5), T(0.5))
+template <typename T> TMK_D auto kall(T s) { return mk2(s, s); }
 
 // Everything the marching kernel needs that is uniform over a launch (all
 // patches of a level share the scenario, dt and dx).  Built on the host and
 // passed by value as a __grid_constant__ parameter, so the kernel reads the
-// constants from the parameter bank instead of holding ~90 of them in
-// registers through the row loop.
+// constants from the parameter bank instead of holding them in registers
+// through the row loop.
 template <typename T>
 struct MarchConst {
   using P = typename PairOf<T>::P;
   MK<T> kx, ky;
-  P bg[9];           // background of the evolving components (.x side 1, .y side 2)
   P sc;              // -dt/dx
+  T nbg[9];          // minus the background of the evolving components
   int plim, clim, lim, ppm;
   int xout_lo, xout_hi, yout_lo, yout_hi;
   void* stash[2];    // row-0 intermediates of the fault-row items, per component group
@@ -182,11 +205,10 @@ struct MarchConst {
   T pdt;
   int plastic;
   TMK_HD void load(const DevParams& p, double dt, double dx) {
-    const double dtdx = dt / dx;
-    kx.load(p, 0, dtdx, -(1.0 / 2.0) * dt / dx);
-    ky.load(p, 1, dtdx, -(1.0 / 2.0) * dt / dx);
-    for (int c = 0; c < 9; ++c) bg[c] = mk2((T)p.bg[c], (T)p.bg[11 + c]);
+    kx.load(p, 0, dt / dx);
+    ky.load(p, 1, dt / dx);
     sc = mk2((T)(-dt / dx), (T)(-dt / dx));
+    for (int c = 0; c < 9; ++c) nbg[c] = (T)-p.bg[c];
     plim = p.prim_lim != 0; clim = p.char_lim != 0; lim = plim || clim; ppm = p.order != 0;
     xout_lo = p.bc[0] == 0; xout_hi = p.bc[1] == 0; yout_lo = p.bc[2] == 0; yout_hi = p.bc[3] == 0;
     plastic = 0;
@@ -195,206 +217,195 @@ struct MarchConst {
   }
 };
 
-// ---- limiters on pairs (differences packed, the nonlinear part per half)
-TMK_D float copysg(float a, float b) { return copysignf(a, b); }
-TMK_D double copysg(double a, double b) { return copysign(a, b); }
+// ---- limiters.  On GB300 an FP64 instruction holds its pipe for 64 cycles a
+// warp, so the FP64 form's comparisons, signs and powers of two are done on the
+// bit patterns with integer instructions; magnitudes order as their patterns,
+// and a NaN is larger than every number, so a minimum drops it as fmin does.
+TMK_D unsigned long long mag64(double x) { return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull; }
+// min(|a|, |b|) with the sign of a
+TMK_D float clip_mag(float a, float b) { return copysignf(fminf(fabsf(a), fabsf(b)), a); }
+TMK_D double clip_mag(double a, double b) {
+  const unsigned long long ma = mag64(a), mb = mag64(b);
+  const unsigned long long m = ma < mb ? ma : mb;
+  return __longlong_as_double((long long)(m | ((unsigned long long)__double_as_longlong(a) & 0x8000000000000000ull)));
+}
+TMK_D float clip_mag(float a, float b, float c) { return copysignf(fminf(fminf(fabsf(a), fabsf(b)), fabsf(c)), a); }
+TMK_D double clip_mag(double a, double b, double c) {
+  const unsigned long long mb = mag64(b), mc = mag64(c);
+  const unsigned long long m = mb < mc ? mb : mc;
+  return clip_mag(a, __longlong_as_double((long long)m));
+}
+// x * 2^k for |k| <= 2
+template <int K> TMK_D double mul_pow2(double x) {
+  const int hi = __double2hiint(x);
+  const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
+  if (e - 3u < 2041u) return __hiloint2double(hi + (K << 20), __double2loint(x));   // normal before and after
+  return x == 0.0 ? x : x * (K == 1 ? 2.0 : 0.25);
+}
+TMK_D float2 quarter(float2 a) { return pmul(a, make_float2(0.25f, 0.25f)); }
+TMK_D double2 quarter(double2 a) { return make_double2(mul_pow2<-2>(a.x), mul_pow2<-2>(a.y)); }
+TMK_D float2 twice(float2 a) { return padd(a, a); }
+TMK_D double2 twice(double2 a) { return make_double2(mul_pow2<1>(a.x), mul_pow2<1>(a.y)); }
+// a b > 0 per half (both nonzero numbers of one sign)
+TMK_D void same_sign(float2 a, float2 b, bool& x, bool& y) {
+  const float2 p = pmul(a, b);
+  x = p.x > 0.f;
+  y = p.y > 0.f;
+}
+TMK_D bool same_sign1(double a, double b) {
+  const unsigned long long inf = 0x7ff0000000000000ull;
+  return (__double2hiint(a) ^ __double2hiint(b)) >= 0 && mag64(a) - 1 < inf && mag64(b) - 1 < inf;
+}
+TMK_D void same_sign(double2 a, double2 b, bool& x, bool& y) { x = same_sign1(a.x, b.x); y = same_sign1(a.y, b.y); }
 
-// van Leer: sign(dc) min(|dc|, 2|dl|, 2|dr|) when dl dr > 0, else 0 (dl2, dr2:
-// the doubled differences, exact; one three-input minimum)
-template <typename T> TMK_D T vl1(T dl2, T dr2, T dc, T prod) {
-  const T t = fmin(fmin(fabs(dc), fabs(dl2)), fabs(dr2));
-  return prod > T(0) ? copysg(t, dc) : T(0);
+// Limited slope of the middle value from the negated one-sided differences
+// nl = w_{i-1} - w_i and nr = w_i - w_{i+1} (at a domain edge the missing one
+// is given the other's value: the one-sided difference the reference uses):
+// minus half the van Leer slope, sign(dc) min(|dc|, 2|dl|, 2|dr|) when
+// dl dr > 0, else 0.  okx, oky: whether dl dr > 0.
+template <typename P> TMK_D P half_slope(P nl, P nr, bool limit, bool& okx, bool& oky) {
+  using T = decltype(nl.x);
+  const P q = quarter(padd(nl, nr));
+  okx = oky = true;
+  if (!limit) return q;
+  same_sign(nl, nr, okx, oky);
+  return mk2(okx ? clip_mag(q.x, nl.x, nr.x) : T(0), oky ? clip_mag(q.y, nl.y, nr.y) : T(0));
 }
 
-// Limited slope of the middle value.  A missing neighbour (outside the
-// domain) stands for the reflection 2 w0 - w_other, which makes the two
-// one-sided differences equal: the centred formula becomes the one-sided
-// difference the reference uses there.
-template <typename P> TMK_D P slope2(P wm, P w0, P wp, bool hasL, bool hasR, bool limit) {
-  using T = decltype(wm.x);
-  const P half = mk2(T(0.5), T(0.5));
-  P dl = psub(w0, wm), dr = psub(wp, w0);
-  if (!hasL) dl = dr;
-  if (!hasR) dr = dl;
-  const P dc = pmul(half, padd(dl, dr));
-  if (!limit) return dc;
-  const P prod = pmul(dl, dr);
-  const P dl2 = padd(dl, dl), dr2 = padd(dr, dr);
-  return mk2(vl1(dl2.x, dr2.x, dc.x, prod.x), vl1(dl2.y, dr2.y, dc.y, prod.y));
+// Twice the PPM delta (lo face value - w) of a cell from its negated
+// difference to the cell below and both cells' half slopes:
+// w_lo = (w_{i-1} + w_i)/2 - (s_i - s_{i-1})/6.
+template <typename T, typename P> TMK_D P delta_lo(P nl, P n_i, P n_im1) {
+  return pfma(psub(n_i, n_im1), kall(T(2.0 / 3.0)), nl);
 }
+// twice the hi delta from the next cell's: w_hi(i) = w_lo(i+1)
+template <typename T, typename P> TMK_D P delta_hi(P nr, P dlo_next) { return pfma(nr, kall(T(-2)), dlo_next); }
 
-// PPM limiter (Colella & Woodward 1984 eq. 1.10): both deltas zero at an
-// extremum, otherwise each clipped to twice the other's magnitude.
-template <typename T> TMK_D T clampabs(T v, T b) { return fmin(fmax(v, -fabs(b)), fabs(b)); }
+// PPM limiter (Colella & Woodward 1984 eq. 1.10) of the deltas m, p of a cell:
+// both zero at an extremum, otherwise each clipped to twice the other's
+// magnitude.  With slopes limited as above m is between -0.17 dl and -0.83 dl
+// and p between 0.17 dr and 0.83 dr, so m p < 0 exactly where dl dr > 0; the
+// caller has zeroed m elsewhere, which makes both results zero.
+template <typename P> TMK_D void limit_mono(P& m, P& p) {
+  const P m2 = twice(m), p2 = twice(p);
+  const P a = mk2(clip_mag(m.x, p2.x), clip_mag(m.y, p2.y));
+  p = mk2(clip_mag(p.x, m2.x), clip_mag(p.y, m2.y));
+  m = a;
+}
+// the same limiter for deltas of unknown sign (characteristic limiting)
 template <typename P> TMK_D void limit2(P& m, P& p) {
   using T = decltype(m.x);
-  const P two = mk2(T(2), T(2));
-  const P m2 = pmul(two, m), p2 = pmul(two, p), prod = pmul(m, p);
-  const T amx = clampabs(m.x, p2.x), apx = clampabs(p.x, m2.x);
-  const T amy = clampabs(m.y, p2.y), apy = clampabs(p.y, m2.y);
-  m.x = prod.x < T(0) ? amx : T(0); p.x = prod.x < T(0) ? apx : T(0);
-  m.y = prod.y < T(0) ? amy : T(0); p.y = prod.y < T(0) ? apy : T(0);
+  bool x, y;
+  same_sign(m, pneg(p), x, y);
+  m = mk2(x ? m.x : T(0), y ? m.y : T(0));
+  limit_mono(m, p);
 }
 
-// interior PPM face value between cells a (lower) and b: (a+b)/2 - (sb - sa)/6
-template <typename T, typename P> TMK_D P face2(P a, P b, P sa, P sb) {
-  const P h = mk2(T(0.5), T(0.5)), m6 = mk2(T(-1.0 / 6.0), T(-1.0 / 6.0));
-  return pfma(psub(sb, sa), m6, pmul(h, padd(a, b)));
-}
-
-// PPM normal predictor of a group in direction D from the unlimited face
-// deltas dm (lo face) and dp (hi face) of each component; WM, WP = w + traced.
+// The traced characteristic values of a cell in direction D (see the head of
+// the file) from its state w and its doubled deltas m (lo) and p (hi).
 template <int G, int D, typename T>
-TMK_D void predict(const MK<T>& k, const typename PairOf<T>::P* w, typename PairOf<T>::P* dm,
-                   typename PairOf<T>::P* dp, bool plim, bool clim, typename PairOf<T>::P* WM,
-                   typename PairOf<T>::P* WP) {
+TMK_D void trace(const MK<T>& k, const typename PairOf<T>::P* w, const typename PairOf<T>::P* m,
+                 const typename PairOf<T>::P* p, bool clim, typename PairOf<T>::P* An, typename PairOf<T>::P* Ap) {
   using P = typename PairOf<T>::P;
-  using R = Role<G, D>;
-  constexpr int N = Grp<G>::N;
-  if (plim) {
 #pragma unroll
-    for (int c = 0; c < N; ++c)
-      if (live<G, D>(c)) limit2(dm[c], dp[c]);
-  }
-  // S wave pair
-  {
-    P nm = pfma(KC(ZsE), dm[R::vS], dm[R::sS]), pm = pfma(KC(nZsE), dm[R::vS], dm[R::sS]);
-    P np = pfma(KC(ZsE), dp[R::vS], dp[R::sS]), pp = pfma(KC(nZsE), dp[R::vS], dp[R::sS]);
+  for (int q = 0; q < kWaves<G>; ++q) {
+    const int v = wave_v<G, D>(q), s = wave_s<G, D>(q);
+    const P Z = kpair<D>(is_p<G>(q) ? k.Zp : k.Zs), nZ = kpair<D>(is_p<G>(q) ? k.nZp : k.nZs);
+    const P a = kall(is_p<G>(q) ? k.aP : k.aS), b = kall(is_p<G>(q) ? k.bP : k.bS);
+    P nm = pfma(Z, m[v], m[s]), np = pfma(Z, p[v], p[s]);
+    P pm = pfma(nZ, m[v], m[s]), pp = pfma(nZ, p[v], p[s]);
     if (clim) { limit2(nm, np); limit2(pm, pp); }
-    P nmt = pfma(KE(aS), nm, pmul(KE(bS), np));       // w- traced to the lo face
-    P ppt = pfma(KE(aS), pp, pmul(KE(bS), pm));       // w+ traced to the hi face
-    WM[R::sS] = padd(w[R::sS], pmul(KHALF, padd(nmt, pm)));
-    WM[R::vS] = padd(w[R::vS], pmul(KC(hZsE), psub(nmt, pm)));
-    WP[R::sS] = padd(w[R::sS], pmul(KHALF, padd(np, ppt)));
-    WP[R::vS] = padd(w[R::vS], pmul(KC(hZsE), psub(np, ppt)));
+    An[q] = pfma(b, np, pfma(a, nm, pfma(Z, w[v], w[s])));
+    Ap[q] = pfma(b, pm, pfma(a, pp, pfma(nZ, w[v], w[s])));
   }
-  if constexpr (R::hasP) {
-    P nm = pfma(KC(ZpE), dm[R::vP], dm[R::sP]), pm = pfma(KC(nZpE), dm[R::vP], dm[R::sP]);
-    P np = pfma(KC(ZpE), dp[R::vP], dp[R::sP]), pp = pfma(KC(nZpE), dp[R::vP], dp[R::sP]);
-    if (clim) { limit2(nm, np); limit2(pm, pp); }
-    P nmt = pfma(KE(aP), nm, pmul(KE(bP), np));
-    P ppt = pfma(KE(aP), pp, pmul(KE(bP), pm));
-    P sPm = pmul(KHALF, padd(nmt, pm)), sPp = pmul(KHALF, padd(np, ppt));
-    WM[R::sP] = padd(w[R::sP], sPm);
-    WM[R::vP] = padd(w[R::vP], pmul(KC(hZpE), psub(nmt, pm)));
-    WP[R::sP] = padd(w[R::sP], sPp);
-    WP[R::vP] = padd(w[R::vP], pmul(KC(hZpE), psub(np, ppt)));
-  }
-  // the zero-speed components of direction D are not read (live<G, D>)
+}
+// the cell's own characteristic values (CTU: no delta)
+template <int G, int D, typename T>
+TMK_D void chars(const MK<T>& k, const typename PairOf<T>::P* w, typename PairOf<T>::P* An,
+                 typename PairOf<T>::P* Ap) {
 #pragma unroll
-  for (int c = 0; c < Grp<G>::N; ++c)
-    if (!live<G, D>(c)) { WM[c] = mk2(T(0), T(0)); WP[c] = mk2(T(0), T(0)); }
+  for (int q = 0; q < kWaves<G>; ++q) {
+    const int v = wave_v<G, D>(q), s = wave_s<G, D>(q);
+    An[q] = pfma(kpair<D>(is_p<G>(q) ? k.Zp : k.Zs), w[v], w[s]);
+    Ap[q] = pfma(kpair<D>(is_p<G>(q) ? k.nZp : k.nZs), w[v], w[s]);
+  }
 }
 
-// RIEMANNF for a group: L = state left of the face, Rt = right
-template <int G, int D, typename T>
-TMK_D void riem(const MK<T>& k, const typename PairOf<T>::P* L, const typename PairOf<T>::P* Rt,
-                typename PairOf<T>::P* g) {
-  using P = typename PairOf<T>::P;
-  using R = Role<G, D>;
-  {
-    P wpos = pfma(KC(nZsE), L[R::vS], L[R::sS]);
-    P wneg = pfma(KC(ZsE), Rt[R::vS], Rt[R::sS]);
-    g[R::sS] = pmul(KHALF, padd(wneg, wpos));
-    g[R::vS] = pmul(KC(hZsE), psub(wneg, wpos));
-  }
-  if constexpr (R::hasP) {
-    P wpos = pfma(KC(nZpE), L[R::vP], L[R::sP]);
-    P wneg = pfma(KC(ZpE), Rt[R::vP], Rt[R::sP]);
-    P s = pmul(KHALF, padd(wneg, wpos));
-    g[R::sP] = s;
-    g[R::vP] = pmul(KC(hZpE), psub(wneg, wpos));
-  }
-  // zero-speed components of the face state: not read (live<G, D>)
+// The characteristic value arriving from outside a domain edge
+// (LINELASTOUTBCF, LINELASTFREEBCF): the background's, or minus the one that
+// leaves the domain (of the whole stress: both are relative to s0).
+template <int G, typename T, typename P>
+TMK_D void edge_value(const MK<T>& k, const P* bg, bool outflow, const P* leaving, P* arriving) {
 #pragma unroll
-  for (int c = 0; c < Grp<G>::N; ++c)
-    if (!live<G, D>(c)) g[c] = mk2(decltype(L[0].x)(0), decltype(L[0].x)(0));
+  for (int q = 0; q < kWaves<G>; ++q) {
+    const int w = G == 0 ? q : 2;
+    arriving[q] = outflow ? bg[w] : pfma(kall(T(-2)), kall(k.s0[w]), pneg(leaving[q]));
+  }
 }
 
-// Background state of a group, read from the launch constants by group index.
-template <int G, typename P>
-struct BgView {
-  const P* all;   // the 9 evolving components
-  TMK_D P operator[](int c) const { return all[Grp<G>::glob(c)]; }
-};
+// sums and differences of the jumps
+template <int G, typename P> TMK_D void jumps(const P* jn, const P* jp, P* sum, P* dif) {
+#pragma unroll
+  for (int q = 0; q < kWaves<G>; ++q) { sum[q] = padd(jn[q], jp[q]); dif[q] = psub(jn[q], jp[q]); }
+}
 
-// LINELASTOUTBCF / LINELASTFREEBCF for a group.  lo: the inside state is the
-// cell above/right of the face; SHF keeps the reference's velocity-minus-stress form.
+// Transverse term of direction D with scale -1/2 dt/dx on the characteristic
+// values Bn, Bp of the other direction.  E's P pair takes the normal stress
+// from D's P wave (lam) and the velocity from D's S wave; E's S pair takes the
+// shear stress from D's S wave (G) and the velocity from D's P wave; the
+// antiplane stress of D does not enter E's wave.
 template <int G, int D, typename T>
-TMK_D void edge2(const MK<T>& k, bool lo, bool outflow, const typename PairOf<T>::P* Wi,
-                 const BgView<G, typename PairOf<T>::P>& bg, typename PairOf<T>::P* g) {
+TMK_D void correct(const MK<T>& k, const typename PairOf<T>::P* sum, const typename PairOf<T>::P* dif,
+                   typename PairOf<T>::P* Bn, typename PairOf<T>::P* Bp) {
+  if constexpr (G == 0) {
+    Bn[0] = pfma(k.cvP, sum[1], pfma(kall(k.c_lam), dif[0], Bn[0]));
+    Bp[0] = pfma(k.ncvP, sum[1], pfma(kall(k.c_lam), dif[0], Bp[0]));
+    Bn[1] = pfma(k.cvS, sum[0], pfma(kall(k.c_G), dif[1], Bn[1]));
+    Bp[1] = pfma(k.ncvS, sum[0], pfma(kall(k.c_G), dif[1], Bp[1]));
+  } else {
+    Bn[0] = pfma(k.cvS, sum[0], Bn[0]);
+    Bp[0] = pfma(k.ncvS, sum[0], Bp[0]);
+  }
+}
+
+// The conservative update's increments -dt/dx (F_hi - F_lo): the x part (D = 0)
+// starts them, the y part adds to them; the state is rounded once, when they
+// are added to it.
+template <int G, int D, typename T>
+TMK_D void add_update(const MK<T>& k, const typename PairOf<T>::P* sum, const typename PairOf<T>::P* dif,
+                      typename PairOf<T>::P* du) {
   using P = typename PairOf<T>::P;
   using R = Role<G, D>;
-  {
-    P wneg, wpos;
-    if (lo) {
-      wneg = pfma(KC(ZsE), Wi[R::vS], Wi[R::sS]);
-      wpos = outflow ? pfma(KC(nZsE), bg[R::vS], bg[R::sS]) : pneg(wneg);
-    } else {
-      wpos = pfma(KC(nZsE), Wi[R::vS], Wi[R::sS]);
-      wneg = outflow ? pfma(KC(ZsE), bg[R::vS], bg[R::sS]) : pneg(wpos);
+  auto acc = [&](int c, P a, P b) { du[c] = D == 0 ? pmul(a, b) : pfma(a, b, du[c]); };
+#pragma unroll
+  for (int q = 0; q < kWaves<G>; ++q) {
+    acc(wave_v<G, D>(q), kpair<D>(k.e_v), sum[q]);
+    acc(wave_s<G, D>(q), kall(is_p<G>(q) ? k.e_l2g : k.e_G), dif[q]);
+  }
+  if constexpr (R::hasP) {
+    acc(R::zc0, kall(k.e_lam), dif[0]);
+    acc(R::zc1, kall(k.e_lam), dif[0]);
+  }
+  if constexpr (R::hasZf && D == 0) du[R::zf] = mk2(T(0), T(0));
+}
+
+// GETFLUXF of the face state with characteristic values Bn, Bp
+template <int G, int D, typename T>
+TMK_D void face_flux(const MK<T>& k, const typename PairOf<T>::P* Bn, const typename PairOf<T>::P* Bp,
+                     typename PairOf<T>::P* F) {
+  using P = typename PairOf<T>::P;
+  using R = Role<G, D>;
+#pragma unroll
+  for (int q = 0; q < kWaves<G>; ++q) {
+    const P fs = pfma(kall(T(0.5)), padd(Bn[q], Bp[q]), kall(k.s0[G == 0 ? q : 2]));
+    const P fv = pmul(is_p<G>(q) ? k.hZp : k.hZs, psub(Bn[q], Bp[q]));
+    F[wave_v<G, D>(q)] = pmul(k.f_irho, fs);
+    F[wave_s<G, D>(q)] = pmul(is_p<G>(q) ? k.f_l2g : k.f_G, fv);
+    if constexpr (R::hasP) {
+      if (is_p<G>(q)) { F[R::zc0] = pmul(k.f_lam, fv); F[R::zc1] = F[R::zc0]; }
     }
-    g[R::sS] = pmul(KHALF, padd(wneg, wpos));
-    g[R::vS] = pmul(KC(hZsE), psub(wneg, wpos));
   }
-  if constexpr (R::hasP) {
-    P wneg, wpos;
-    if (lo) {
-      wneg = pfma(KC(ZpE), Wi[R::vP], Wi[R::sP]);
-      wpos = outflow ? pfma(KC(nZpE), bg[R::vP], bg[R::sP]) : pneg(wneg);
-    } else {
-      wpos = pfma(KC(nZpE), Wi[R::vP], Wi[R::sP]);
-      wneg = outflow ? pfma(KC(ZpE), bg[R::vP], bg[R::sP]) : pneg(wpos);
-    }
-    P s = pmul(KHALF, padd(wneg, wpos));
-    g[R::sP] = s;
-    g[R::vP] = pmul(KC(hZpE), psub(wneg, wpos));
-  }
-  // zero-speed components (the reference's SHF terms): not read (live<G, D>)
-#pragma unroll
-  for (int c = 0; c < Grp<G>::N; ++c)
-    if (!live<G, D>(c)) g[c] = mk2(T(0), T(0));
-}
-
-// GETFLUXF for a group
-template <int G, int D, typename T>
-TMK_D void flux2(const MK<T>& k, const typename PairOf<T>::P* g, typename PairOf<T>::P* F) {
-  using R = Role<G, D>;
-  F[R::vS] = pmul(KC(f_irho), g[R::sS]);
-  F[R::sS] = pmul(KC(f_G), g[R::vS]);
-  if constexpr (R::hasP) {
-    F[R::vP] = pmul(KC(f_irho), g[R::sP]);
-    F[R::sP] = pmul(KC(f_l2g), g[R::vP]);
-    F[R::zc0] = pmul(KC(f_lam), g[R::vP]);
-    F[R::zc1] = pmul(KC(f_lam), g[R::vP]);
-  }
-  if constexpr (R::hasZf) F[R::zf] = mk2(decltype(g[0].x)(0), decltype(g[0].x)(0));
-}
-
-// GETADWDXF increment from the face states at the hi (h) and lo (l) faces, added to q1 and q2
-template <int G, int D, typename T>
-TMK_D void adw2(const MK<T>& k, const typename PairOf<T>::P* h, const typename PairOf<T>::P* l,
-                typename PairOf<T>::P* q1, typename PairOf<T>::P* q2) {
-  using P = typename PairOf<T>::P;
-  using R = Role<G, D>;
-  {
-    P a = pmul(KC(a_irho), psub(h[R::sS], l[R::sS]));
-    q1[R::vS] = padd(q1[R::vS], a); q2[R::vS] = padd(q2[R::vS], a);
-    P b = pmul(KC(a_G), psub(h[R::vS], l[R::vS]));
-    q1[R::sS] = padd(q1[R::sS], b); q2[R::sS] = padd(q2[R::sS], b);
-  }
-  if constexpr (R::hasP) {
-    P a = pmul(KC(a_irho), psub(h[R::sP], l[R::sP]));
-    q1[R::vP] = padd(q1[R::vP], a); q2[R::vP] = padd(q2[R::vP], a);
-    P dv = psub(h[R::vP], l[R::vP]);
-    P b = pmul(KC(a_l2g), dv);
-    q1[R::sP] = padd(q1[R::sP], b); q2[R::sP] = padd(q2[R::sP], b);
-    // the targets are states of the other direction: their components that
-    // are zero-speed there are not read
-    P c = pmul(KC(a_lam), dv);
-    if constexpr (live<G, 1 - D>(R::zc0)) { q1[R::zc0] = padd(q1[R::zc0], c); q2[R::zc0] = padd(q2[R::zc0], c); }
-    if constexpr (live<G, 1 - D>(R::zc1)) { q1[R::zc1] = padd(q1[R::zc1], c); q2[R::zc1] = padd(q2[R::zc1], c); }
-  }
+  if constexpr (R::hasZf) F[R::zf] = mk2(T(0), T(0));
 }
 
 // ---------------------------------------------------------------- the kernel
@@ -404,50 +415,26 @@ TMK_D void adw2(const MK<T>& k, const typename PairOf<T>::P* h, const typename P
 // and keeps what it needs in stash slot fslot.
 // [cap0, cap0+ncap) are the item's entries in its group's capture list.
 struct MarchItem { int patch, x0, y0, y1, fslot, cap0, ncap; };
-// vectors a fault-row item keeps for its row 0 (x states, first-pass y face 1,
-// final y flux 1, old state)
-constexpr int MARCH_STASH_VECS = 5;
+// vectors of a group's N components' size that a fault-row item keeps for its
+// row 0: the traced x values (An, Ap), the first-pass and the final values at
+// y face 1 (An of row 1, Ap of row 0 each; two per wave pair, N = 3 pairs'
+// worth per component count of 6), the old state
+constexpr int MARCH_STASH_VECS = 3;
 
 constexpr int MARCH_COLS = 28;   // updated columns per warp
 constexpr int MARCH_HALO = 2;    // halo lanes on either side (lane l holds column x0 - 2 + l)
 constexpr int MARCH_WARPS = 4;   // warps per CTA
 
-// Per-row vectors a lane carries from row to row in shared memory rather than
-// registers: the x states of row q-1 (WMx, WPx), the first-pass y face q-1
-// (H1y), the final y flux q-1 (Fy), the old state of row q-1 (Wold), the
-// y-predicted and corrected states of row q-1 (WPy, WPcy), and the y slope
-// and lo-face value of row q (Sy, Fyf).  Each keeps only the components that
-// are read: the x states the components live in x, the y states and faces
-// those live in y.  The FP64 form keeps the last four in registers: in shared
-// memory its in-plane CTA would need 131 KB, one CTA per SM.
-enum MarchCarry { kWMx = 0, kWPx, kH1y, kFy, kWold, kWPy, kWPcy, kSy, kFyf, kNumCarry };
-template <int G>
-TMK_HD constexpr bool carry_needed(int v, int c) {
-  return (v == kWMx || v == kWPx) ? live<G, 0>(c) : (v == kFy || v == kWold) ? true : live<G, 1>(c);
-}
-template <typename T>
-TMK_HD constexpr bool carry_in_smem(int v) { return v < kWPy || sizeof(T) == 4; }
-// position of (vector v, component c) among the shared-memory slots of a lane
-template <typename T, int G>
-TMK_HD constexpr int carry_slot(int v, int c) {
-  int k = 0;
-  for (int vv = 0; vv < v; ++vv)
-    for (int cc = 0; cc < Grp<G>::N; ++cc) k += (carry_in_smem<T>(vv) && carry_needed<G>(vv, cc)) ? 1 : 0;
-  for (int cc = 0; cc < c; ++cc) k += carry_needed<G>(v, cc) ? 1 : 0;
-  return k;
-}
-template <typename T, int G>
-TMK_HD constexpr int carry_slots() { return carry_slot<T, G>(kNumCarry, 0); }
-// Rows q..q+2 of the rolling window plus the row in flight live in a per-warp
-// ring of shared memory filled by cp.async; slot = row & 3.  A ring row holds
-// MARCH_RW entries per component: the column left of lane 0, the warp's 32
-// columns, the column right of lane 31.
-constexpr int MARCH_RING = 4;
+// Rows q-1 (the old state of the row updated at step q) to q+2 of the rolling
+// window and the rows in flight live in a per-warp ring of shared memory
+// filled by cp.async; slot = row & 7.  A ring row holds MARCH_RW entries per
+// component: the column left of lane 0, the warp's 32 columns, the column
+// right of lane 31.  MARCH_AHEAD: the row requested at step q is q + AHEAD.
+constexpr int MARCH_RING = 8;
+constexpr int MARCH_AHEAD = 4;
 constexpr int MARCH_RW = 34;
 template <typename T, int G>
-constexpr size_t march_warp_pairs() {
-  return (size_t)carry_slots<T, G>() * 32 + (size_t)MARCH_RING * Grp<G>::N * MARCH_RW;
-}
+constexpr size_t march_warp_pairs() { return (size_t)MARCH_RING * Grp<G>::N * MARCH_RW; }
 template <typename T, int G>
 constexpr size_t march_smem_bytes() {
   return (size_t)MARCH_WARPS * march_warp_pairs<T, G>() * sizeof(typename PairOf<T>::P);
@@ -468,7 +455,8 @@ template <typename T> TMK_D void cp_async_elem(T* dst_smem, const T* src, unsign
                : "memory");
 }
 TMK_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-TMK_D void cp_async_wait_all_but_newest() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+// all but the newest K groups have landed
+template <int K> TMK_D void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(K) : "memory"); }
 
 // The inputs of a cell's plastic return the in-plane group does not hold: the
 // antiplane group's updated sxz, syz (stored by the antiplane kernel, which
@@ -521,11 +509,10 @@ TMK_D void store_cell(const PatchDev<T>& pp, const MarchConst<T>& mc, size_t o, 
 // level's flux-register capture buffer (flux registers of the AMR coupling).
 // Entry kinds: 0 the x face below the lane's column, 1 the one above, 2 the
 // y face below the row, 3 the one above; entries are sorted by row and the
-// loop is uniform over the warp.
-template <typename T, int G>
+// loop is uniform over the warp.  flux(kind, F) gives the fluxes of a face.
+template <typename T, int G, typename FluxOf>
 TMK_D void march_capture(const PatchDev<T>& pp, const MarchItem& it, const MarchConst<T>& mc, int row, int lane,
-                         const typename PairOf<T>::P* Fx, const typename PairOf<T>::P* Fxh,
-                         const typename PairOf<T>::P* Fylo, const typename PairOf<T>::P* Fyhi, int& cpos) {
+                         int& cpos, FluxOf flux) {
   using P = typename PairOf<T>::P;
   constexpr int N = Grp<G>::N;
   const int4* caps = mc.caps[G];
@@ -535,12 +522,13 @@ TMK_D void march_capture(const PatchDev<T>& pp, const MarchItem& it, const March
     if (e.x > row) break;
     ++cpos;
     if (e.x < row || e.z != lane) continue;   // rows left to the fault-row kernel, other lanes
+    P F[N];
+    flux(e.y, F);
 #pragma unroll
     for (int c = 0; c < N; ++c) {
-      const P v = e.y == 0 ? Fx[c] : e.y == 1 ? Fxh[c] : e.y == 2 ? Fylo[c] : Fyhi[c];
       const int g = Grp<G>::glob(c);
-      pp.cap[(size_t)e.w * 22 + g] = (double)v.x;
-      pp.cap[(size_t)e.w * 22 + 11 + g] = (double)v.y;
+      pp.cap[(size_t)e.w * 22 + g] = (double)F[c].x;
+      pp.cap[(size_t)e.w * 22 + 11 + g] = (double)F[c].y;
     }
   }
 }
@@ -560,10 +548,9 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
                                                                  const MarchItem* __restrict__ items, int nitems,
                                                                  const __grid_constant__ MarchConst<T> mc) {
   using P = typename PairOf<T>::P;
-  constexpr int N = Grp<G>::N;
+  constexpr int N = Grp<G>::N, NW = kWaves<G>;
   extern __shared__ __align__(16) unsigned char march_smem[];
-  P* const carry = reinterpret_cast<P*>(march_smem) + (size_t)(threadIdx.x >> 5) * march_warp_pairs<T, G>();
-  P* const ring = carry + carry_slots<T, G>() * 32;
+  P* const ring = reinterpret_cast<P*>(march_smem) + (size_t)(threadIdx.x >> 5) * march_warp_pairs<T, G>();
   const int wid = blockIdx.x * MARCH_WARPS + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   // a later kernel of the step may be scheduled now; every warp waits for the
@@ -588,40 +575,41 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   const bool ext_in = (lane == 0 || lane == 31) && x + dxe >= dlo0 && x + dxe <= dhi0 && x + dxe >= pp.alo0 &&
                       x + dxe <= ahi0;
   const int ext_pos = lane == 0 ? 0 : 33;
-  const bool inL = x - 1 >= dlo0, inR = x + 1 <= dhi0;
   constexpr bool kFixed = SCH == MARCH_SCH_PPM_PRIM;
   const bool plim = kFixed || mc.plim != 0, clim = !kFixed && mc.clim != 0, lim = kFixed || mc.lim != 0;
   const bool ppm = kFixed || mc.ppm != 0;
   const MK<T>& kx = mc.kx;
   const MK<T>& ky = mc.ky;
-  const P sc = mc.sc;
-  const BgView<G, P> bg{mc.bg};
-  const bool xout_lo = mc.xout_lo != 0, xout_hi = mc.xout_hi != 0, yout_lo = mc.yout_lo != 0,
-             yout_hi = mc.yout_hi != 0;
   const bool fault = pp.fault != 0;
   const bool defer0 = it.fslot >= 0;      // row 0 is finished by march_fault_row_kernel
   const bool col_valid = x >= it.x0 && x < it.x0 + MARCH_COLS && x >= pp.vlo0 && x <= pp.vhi0;
   const size_t plane = (size_t)pp.anx * pp.any;
-  // a lane of this warp holds a face on a domain x edge: the x Riemann solves
-  // are the interior ones for every lane, overwritten there by the edge
-  // condition; other warps (most) skip the edge code on a uniform branch
-  const bool warp_xedge = __any_sync(0xffffffffu, x == dlo0 || x == dhi0 + 1);
+  // a lane of this warp holds a cell on a domain x edge: every lane takes the
+  // interior differences and face values, overwritten there by the edge's;
+  // other warps (most) skip the edge code on a uniform branch
+  const bool edge_lo = x == dlo0, edge_hi = x == dhi0;
+  const bool warp_xedge = __any_sync(0xffffffffu, edge_lo || edge_hi);
+
+  const int q_s = max(it.y0 - 1, dlo1);
+  const int q_e = it.y1 + 1;
 
   auto load_row = [&](int y, P* w) {
     const bool ok = lane_in && y >= dlo1 && y <= dhi1;
     const size_t o = ok ? fab_idx(pp, 0, x, y) : 0;
 #pragma unroll
     for (int c = 0; c < N; ++c) {
+      if (!live<G, 1>(c)) { w[c] = mk2(T(0), T(0)); continue; }
       const int g = Grp<G>::glob(c);
       w[c] = ok ? mk2(pp.Uin[o + (size_t)g * plane], pp.Uin[o + (size_t)(11 + g) * plane]) : mk2(T(0), T(0));
     }
   };
   // row y into its ring slot: cp.async for cells in the domain, zeros
-  // elsewhere; the two outer columns only for the components live in x (the
-  // only ones whose neighbours are read)
+  // elsewhere (and for rows past the last one the item reads); the two outer
+  // columns only for the components live in x (the only ones whose neighbours
+  // are read)
   auto ring_row = [&](int y) -> P* { return ring + (size_t)((y & (MARCH_RING - 1)) * N) * MARCH_RW; };
   auto load_row_async = [&](int y) {
-    const bool yin = y >= dlo1 && y <= dhi1;
+    const bool yin = y >= dlo1 && y <= dhi1 && y <= q_e + 2;
     const bool ok = lane_in && yin;
     const size_t o = ok ? fab_idx(pp, 0, x, y) : 0;
     const unsigned nb = ok ? (unsigned)sizeof(T) : 0u;
@@ -636,7 +624,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
       cp_async_elem(d2 + 1, src + (size_t)(11 + g) * plane, nb);
     }
     if (lane == 0 || lane == 31) {      // the outer columns: own address -1 / +1 (oke implies ok)
-      const bool oke = ext_in && yin;
+      const bool oke = ext_in && ok;
       const unsigned nbe = oke ? (unsigned)sizeof(T) : 0u;
       const T* const srce = oke ? src + dxe : src;
       P* const dste = rowp + ext_pos;
@@ -651,250 +639,214 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
     }
     cp_async_commit();
   };
-  // the outer columns of row y, loaded directly (the rows staged before the loop)
-  auto store_ext_sync = [&](int y) {
-    if (lane == 0 || lane == 31) {
-      const bool oke = ext_in && y >= dlo1 && y <= dhi1;
-      const size_t oe = oke ? fab_idx(pp, 0, x + dxe, y) : 0;
-      P* de = ring_row(y) + ext_pos;
-#pragma unroll
-      for (int c = 0; c < N; ++c) {
-        if (!live<G, 0>(c)) continue;
-        const int g = Grp<G>::glob(c);
-        de[c * MARCH_RW] = oke ? mk2(pp.Uin[oe + (size_t)g * plane], pp.Uin[oe + (size_t)(11 + g) * plane])
-                               : mk2(T(0), T(0));
-      }
-    }
-  };
-  auto get_row = [&](int y, P* w) {
-    const P* src = ring_row(y) + lane + 1;
-#pragma unroll
-    for (int c = 0; c < N; ++c) w[c] = src[c * MARCH_RW];
-  };
 
-  // x-direction normal predictor of row w (its ring row: rw) and the
-  // first-pass x-face state on the lane's lo face (H1 lo) and hi face (H1 hi)
-  auto xrow = [&](const P* w, const P* rw, P* WM, P* WP, P* H1lo, P* H1hi) {
-    if (ppm) {
-      P dm[N], dp[N];
-#pragma unroll
-      for (int c = 0; c < N; ++c) {
-        if (!live<G, 0>(c)) { dm[c] = mk2(T(0), T(0)); dp[c] = dm[c]; continue; }
-        const P wl = rw[c * MARCH_RW + lane], wr = rw[c * MARCH_RW + lane + 2];
-        P s = slope2(wl, w[c], wr, inL, inR, lim);
-        P sl = shfl_up2(s, 1);
-        P flo = inL ? face2<T>(wl, w[c], sl, s) : pfma(mk2(T(-0.5), T(-0.5)), s, w[c]);
-        P fhi = shfl_dn2(flo, 1);
-        if (!inR) fhi = pfma(mk2(T(0.5), T(0.5)), s, w[c]);
-        dm[c] = psub(flo, w[c]);
-        dp[c] = psub(fhi, w[c]);
-      }
-      predict<G, 0, T>(kx, w, dm, dp, plim, clim, WM, WP);
-    } else {
-#pragma unroll
-      for (int c = 0; c < N; ++c) { WM[c] = w[c]; WP[c] = w[c]; }
-    }
-    P L[N];
-#pragma unroll
-    for (int c = 0; c < N; ++c) L[c] = live<G, 0>(c) ? shfl_up2(WP[c], 1) : mk2(T(0), T(0));
-    riem<G, 0, T>(kx, L, WM, H1lo);
-    if (warp_xedge) {                 // the domain-edge conditions, only in warps that reach an x edge
-      if (x == dlo0) edge2<G, 0, T>(kx, true, xout_lo, WM, bg, H1lo);
-      else if (x == dhi0 + 1) edge2<G, 0, T>(kx, false, xout_hi, L, bg, H1lo);
-    }
-#pragma unroll
-    for (int c = 0; c < N; ++c) H1hi[c] = live<G, 0>(c) ? shfl_dn2(H1lo[c], 1) : mk2(T(0), T(0));
-  };
-
-  const int q_s = max(it.y0 - 1, dlo1);
-  const int q_e = it.y1 + 1;
   int cpos = it.cap0;                     // next coarse-fine face to store
-  P rcar[kNumCarry - kWPy][N];     // the register-resident carries (FP64 form)
-  auto cput = [&](int v, const P* a) {
+  // carried from row to row: the half slopes and the lo deltas of row q (zeroed
+  // at extrema where the limiter zeroes them), the traced x values of row q-1,
+  // the traced and corrected y values of row q-1 (An, Ap) and their jump jp
+  P n4[N], dlo[N];
+  P Anx[NW], Apx[NW], Any[NW], Apy[NW], jpy[NW], Bny[NW], Bpy[NW], jpB[NW];
 #pragma unroll
-    for (int c = 0; c < N; ++c) {
-      if (!carry_needed<G>(v, c)) continue;
-      if (carry_in_smem<T>(v)) carry[carry_slot<T, G>(v, c) * 32 + lane] = a[c];
-      else rcar[v - kWPy][c] = a[c];
-    }
-  };
-  auto cget = [&](int v, P* a) {
-#pragma unroll
-    for (int c = 0; c < N; ++c)
-      a[c] = !carry_needed<G>(v, c) ? mk2(T(0), T(0))
-             : carry_in_smem<T>(v) ? carry[carry_slot<T, G>(v, c) * 32 + lane] : rcar[v - kWPy][c];
-  };
-  // rolling window of rows q, q+1, q+2 (ring slots); slope(q) and the lo-face value of row q carried
+  for (int w = 0; w < NW; ++w) {
+    Anx[w] = mk2(T(0), T(0)); Apx[w] = Anx[w]; Any[w] = Anx[w]; Apy[w] = Anx[w]; jpy[w] = Anx[w];
+    Bny[w] = Anx[w]; Bpy[w] = Anx[w]; jpB[w] = Anx[w];
+  }
   {
-    P Wa[N], Wb[N], W0[N], W1[N], W2[N], sy0[N], Fy0[N];
+#pragma unroll
+    for (int y = 0; y < MARCH_AHEAD; ++y) load_row_async(q_s + y);
+    P Wa[N], Wb[N];
     load_row(q_s - 2, Wa);
     load_row(q_s - 1, Wb);
-    load_row(q_s, W0);
-    load_row(q_s + 1, W1);
-    load_row(q_s + 2, W2);
-    {
-      P* r0 = ring_row(q_s) + lane + 1; P* r1 = ring_row(q_s + 1) + lane + 1; P* r2 = ring_row(q_s + 2) + lane + 1;
-#pragma unroll
-      for (int c = 0; c < N; ++c) { r0[c * MARCH_RW] = W0[c]; r1[c * MARCH_RW] = W1[c]; r2[c * MARCH_RW] = W2[c]; }
-      store_ext_sync(q_s);
-      store_ext_sync(q_s + 1);
-      store_ext_sync(q_s + 2);
-    }
-    const bool hl = q_s - 1 >= dlo1, hr = q_s + 1 <= dhi1;
+    cp_async_wait<MARCH_AHEAD - 2>();      // rows q_s, q_s + 1 have landed (a lane reads its own columns)
+    const bool hl = q_s - 1 >= dlo1, hll = q_s - 2 >= dlo1, hr = q_s + 1 <= dhi1;
+    const P* r0 = ring_row(q_s) + lane + 1;
+    const P* r1 = ring_row(q_s + 1) + lane + 1;
 #pragma unroll
     for (int c = 0; c < N; ++c) {
-      if (!live<G, 1>(c)) { sy0[c] = mk2(T(0), T(0)); Fy0[c] = sy0[c]; continue; }
-      sy0[c] = slope2(Wb[c], W0[c], W1[c], hl, hr, lim);
+      n4[c] = mk2(T(0), T(0)); dlo[c] = n4[c];
+      if (!live<G, 1>(c)) continue;
+      const P W0 = r0[c * MARCH_RW];
+      P nl = psub(Wb[c], W0), nr = psub(W0, r1[c * MARCH_RW]);
+      if (!hl) nl = nr;
+      if (!hr) nr = nl;
+      if (!hl && !hr) { nl = mk2(T(0), T(0)); nr = nl; }
+      bool okx, oky, ax, ay;
+      n4[c] = half_slope(nl, nr, lim, okx, oky);
       if (hl) {
-        P sm = slope2(Wa[c], Wb[c], W0[c], q_s - 2 >= dlo1, true, lim);
-        Fy0[c] = face2<T>(Wb[c], W0[c], sm, sy0[c]);
+        P na = psub(Wa[c], Wb[c]);
+        if (!hll) na = nl;
+        dlo[c] = delta_lo<T>(nl, n4[c], half_slope(na, nl, lim, ax, ay));
       } else {
-        Fy0[c] = pfma(mk2(T(-0.5), T(-0.5)), sy0[c], W0[c]);
+        dlo[c] = twice(n4[c]);
       }
+      if (plim) dlo[c] = mk2(okx ? dlo[c].x : T(0), oky ? dlo[c].y : T(0));
     }
-    cput(kSy, sy0);
-    cput(kFyf, Fy0);
   }
 
   for (int q = q_s; q <= q_e; ++q) {
-    const bool rowin = q <= dhi1;
-    load_row_async(q + 3);            // next row in flight while this one is computed
+    load_row_async(q + MARCH_AHEAD);  // rows in flight while this one is computed
     // fused plastic return: its other inputs for row q-1, stored at the end of
     // this iteration, requested now so that the row's work hides their latency
     P pin[3];
     if constexpr (PL) {
       if (col_valid && q - 1 >= it.y0 && q - 1 <= it.y1) plastic_inputs<T>(pp, fab_idx(pp, 0, x, q - 1), plane, pin);
     }
-    cp_async_wait_all_but_newest();   // rows up to q+2 have landed
-    __syncwarp();                     // ... every lane's copies, whose neighbours read them
-    P W0[N], W1[N], W2[N];
-    get_row(q, W0);
-    get_row(q + 1, W1);
-    get_row(q + 2, W2);
-    P WMy[N], WPy[N], WMcy[N], WPcy[N], WMx[N], WPx[N], H1lo[N], H1hi[N];
-    P sy1[N], Fy1[N];
-    if (rowin) {
-      // y predictor of row q
+    cp_async_wait<MARCH_AHEAD - 2>();     // rows up to q+2 have landed
+    __syncwarp();                         // ... every lane's copies, whose neighbours read them
+    P An_q[NW], Ap_q[NW], Bn_q[NW], Bp_q[NW], Anx_q[NW], Apx_q[NW];
+    if (q <= dhi1) {
+      const P* const rw = ring_row(q);
+      P W0[N], m[N], p[N];
+#pragma unroll
+      for (int c = 0; c < N; ++c) { W0[c] = rw[c * MARCH_RW + lane + 1]; m[c] = mk2(T(0), T(0)); p[c] = m[c]; }
+      // the cell's state relative to the background, for its characteristic values
+      P Wr[N];
+#pragma unroll
+      for (int c = 0; c < N; ++c) Wr[c] = padd(W0[c], kall(mc.nbg[Grp<G>::glob(c)]));
       if (ppm) {
-        const bool hl = true, hr = q + 2 <= dhi1;
-        P dm[N], dp[N], sy0[N], Fy0[N];
-        cget(kSy, sy0);
-        cget(kFyf, Fy0);
+        // y deltas of row q; slope and lo delta of row q+1
+        const P* const r1 = ring_row(q + 1) + lane + 1;
+        const P* const r2 = ring_row(q + 2) + lane + 1;
+        const bool has1 = q + 1 <= dhi1, has2 = q + 2 <= dhi1;
 #pragma unroll
         for (int c = 0; c < N; ++c) {
-          if (!live<G, 1>(c)) { sy1[c] = mk2(T(0), T(0)); Fy1[c] = sy1[c]; dm[c] = sy1[c]; dp[c] = sy1[c]; continue; }
-          sy1[c] = slope2(W0[c], W1[c], W2[c], hl, hr, lim);
-          Fy1[c] = (q + 1 <= dhi1) ? face2<T>(W0[c], W1[c], sy0[c], sy1[c])
-                                   : pfma(mk2(T(0.5), T(0.5)), sy0[c], W0[c]);
-          dm[c] = psub(Fy0[c], W0[c]);
-          dp[c] = psub(Fy1[c], W0[c]);
+          if (!live<G, 1>(c)) continue;
+          const P W1 = r1[c * MARCH_RW];
+          const P nl = psub(W0[c], W1);
+          P nr = psub(W1, r2[c * MARCH_RW]);
+          if (!has2) nr = nl;
+          bool okx, oky;
+          const P n1 = half_slope(nl, nr, lim, okx, oky);
+          P d1 = delta_lo<T>(nl, n1, n4[c]);
+          m[c] = dlo[c];
+          p[c] = delta_hi<T>(nl, d1);
+          if (!has1) p[c] = pneg(twice(n4[c]));
+          if (plim) {
+            limit_mono(m[c], p[c]);
+            d1 = mk2(okx ? d1.x : T(0), oky ? d1.y : T(0));
+          }
+          n4[c] = n1;
+          dlo[c] = d1;
         }
-        predict<G, 1, T>(ky, W0, dm, dp, plim, clim, WMy, WPy);
-        cput(kSy, sy1);
-        cput(kFyf, Fy1);
-      } else {
+        trace<G, 1, T>(ky, Wr, m, p, clim, An_q, Ap_q);
+        // x deltas
 #pragma unroll
-        for (int c = 0; c < N; ++c) { WMy[c] = W0[c]; WPy[c] = W0[c]; }
-      }
-      // x predictor of row q, first-pass x faces, corrected y states of row q
-      xrow(W0, ring_row(q), WMx, WPx, H1lo, H1hi);
-#pragma unroll
-      for (int c = 0; c < N; ++c) { WMcy[c] = WMy[c]; WPcy[c] = WPy[c]; }
-      adw2<G, 0, T>(kx, H1hi, H1lo, WMcy, WPcy);
-    }
-    // first-pass y face q (lo face of row q)
-    P H1y[N];
-    P WPy_p[N];
-    cget(kWPy, WPy_p);
-    const bool need_h1y = (q > q_s) || (q == dlo1);
-    if (need_h1y) {
-      if (q == dlo1) {
-        if (fault) {
-          // the fault kernel's first-pass face state: only row 0's transverse
-          // correction reads it, and row 0 of a fault patch is finished later
-#pragma unroll
-          for (int c = 0; c < N; ++c) H1y[c] = mk2(T(0), T(0));
-        } else {
-          edge2<G, 1, T>(ky, true, yout_lo, WMy, bg, H1y);
+        for (int c = 0; c < N; ++c) {
+          if (!live<G, 0>(c)) continue;
+          P nl = psub(rw[c * MARCH_RW + lane], W0[c]), nr = psub(W0[c], rw[c * MARCH_RW + lane + 2]);
+          if (warp_xedge) {
+            const P nl0 = nl;
+            if (edge_lo) nl = nr;
+            if (edge_hi) nr = edge_lo ? mk2(T(0), T(0)) : nl0;
+            if (edge_lo && edge_hi) nl = nr;
+          }
+          bool okx, oky;
+          const P n = half_slope(nl, nr, lim, okx, oky);
+          P d = delta_lo<T>(nl, n, shfl_up2(n, 1));
+          if (warp_xedge && edge_lo) d = twice(n);
+          p[c] = delta_hi<T>(nr, shfl_dn2(d, 1));
+          if (warp_xedge && edge_hi) p[c] = pneg(twice(n));
+          if (plim) {
+            d = mk2(okx ? d.x : T(0), oky ? d.y : T(0));
+            limit_mono(d, p[c]);
+          }
+          m[c] = d;
         }
-      } else if (!rowin) {
-        edge2<G, 1, T>(ky, false, yout_hi, WPy_p, bg, H1y);
+        trace<G, 0, T>(kx, Wr, m, p, clim, Anx_q, Apx_q);
       } else {
-        riem<G, 1, T>(ky, WPy_p, WMy, H1y);
+        chars<G, 1, T>(ky, Wr, An_q, Ap_q);
+        chars<G, 0, T>(kx, Wr, Anx_q, Apx_q);
       }
-    }
-    // final y face q
-    P Fy[N];
-    P WPcy_p[N];
-    cget(kWPcy, WPcy_p);
-    if (q >= it.y0) {
-      if (q == dlo1 && fault) {
+      // first-pass x faces of row q, corrected y values
+      P AnR[NW], ApL[NW], jn[NW], jp[NW], sum[NW], dif[NW];
 #pragma unroll
-        for (int c = 0; c < N; ++c) Fy[c] = mk2(T(0), T(0));   // the fault flux: row 0 is finished later
-      } else {
-        P g[N];
-        if (q == dlo1) edge2<G, 1, T>(ky, true, yout_lo, WMcy, bg, g);
-        else if (!rowin) edge2<G, 1, T>(ky, false, yout_hi, WPcy_p, bg, g);
-        else riem<G, 1, T>(ky, WPcy_p, WMcy, g);
-        flux2<G, 1, T>(ky, g, Fy);
-      }
-    }
-    // row q-1: transverse correction of its x states, final x faces, update;
-    // row 0 of a fault patch: keep what march_fault_row_kernel needs
-    if (defer0 && q - 1 == dlo1) {
-      P* st = reinterpret_cast<P*>(mc.stash[G]) + (size_t)it.fslot * MARCH_STASH_VECS * N * 32 + lane;
-      P a[N];
-      cget(kWMx, a);
-#pragma unroll
-      for (int c = 0; c < N; ++c) st[(0 * N + c) * 32] = a[c];
-      cget(kWPx, a);
-#pragma unroll
-      for (int c = 0; c < N; ++c) st[(1 * N + c) * 32] = a[c];
-#pragma unroll
-      for (int c = 0; c < N; ++c) { st[(2 * N + c) * 32] = H1y[c]; st[(3 * N + c) * 32] = Fy[c]; }
-      cget(kWold, a);
-#pragma unroll
-      for (int c = 0; c < N; ++c) st[(4 * N + c) * 32] = a[c];
-    } else if (q - 1 >= it.y0) {
-      P WMcx[N], WPcx[N];
-      {
-        P H1y_p[N];
-        cget(kWMx, WMcx);
-        cget(kWPx, WPcx);
-        cget(kH1y, H1y_p);
-        adw2<G, 1, T>(ky, H1y, H1y_p, WMcx, WPcx);
-      }
-      P L[N], g[N], Fx[N], Fxh[N];
-#pragma unroll
-      for (int c = 0; c < N; ++c) L[c] = live<G, 0>(c) ? shfl_up2(WPcx[c], 1) : mk2(T(0), T(0));
-      riem<G, 0, T>(kx, L, WMcx, g);
+      for (int w = 0; w < NW; ++w) { AnR[w] = shfl_dn2(Anx_q[w], 1); ApL[w] = shfl_up2(Apx_q[w], 1); }
       if (warp_xedge) {
-        if (x == dlo0) edge2<G, 0, T>(kx, true, xout_lo, WMcx, bg, g);
-        else if (x == dhi0 + 1) edge2<G, 0, T>(kx, false, xout_hi, L, bg, g);
+        if (edge_lo) edge_value<G>(kx, kx.bgp, mc.xout_lo != 0, Anx_q, ApL);
+        if (edge_hi) edge_value<G>(kx, kx.bgn, mc.xout_hi != 0, Apx_q, AnR);
       }
-      flux2<G, 0, T>(kx, g, Fx);
 #pragma unroll
-      for (int c = 0; c < N; ++c) Fxh[c] = shfl_dn2(Fx[c], 1);
-      const int yr = q - 1;
-      P Fy_p[N], Wold[N];
-      cget(kFy, Fy_p);
-      cget(kWold, Wold);
-      if (col_valid && yr <= it.y1) {
-        P u[N];
-#pragma unroll
-        for (int c = 0; c < N; ++c) u[c] = pfma(padd(psub(Fxh[c], Fx[c]), psub(Fy[c], Fy_p[c])), sc, Wold[c]);
-        store_cell<T, G, PL>(pp, mc, fab_idx(pp, 0, x, yr), plane, u, pin);
+      for (int w = 0; w < NW; ++w) {
+        jn[w] = psub(AnR[w], Anx_q[w]);
+        jp[w] = psub(Apx_q[w], ApL[w]);
+        Bn_q[w] = An_q[w];
+        Bp_q[w] = Ap_q[w];
       }
-      if (it.ncap && yr <= it.y1) march_capture<T, G>(pp, it, mc, yr, lane, Fx, Fxh, Fy_p, Fy, cpos);
+      jumps<G>(jn, jp, sum, dif);
+      correct<G, 0, T>(kx, sum, dif, Bn_q, Bp_q);
+    } else {
+      // past the domain's y-hi edge: the values arriving through it
+      edge_value<G>(ky, ky.bgn, mc.yout_hi != 0, Apy, An_q);
+      edge_value<G>(ky, ky.bgn, mc.yout_hi != 0, Bpy, Bn_q);
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        Ap_q[w] = mk2(T(0), T(0)); Bp_q[w] = Ap_q[w]; Anx_q[w] = Ap_q[w]; Apx_q[w] = Ap_q[w];
+      }
     }
-    // advance the window
-    cput(kWMx, WMx);
-    cput(kWPx, WPx);
-    cput(kH1y, H1y);
-    cput(kFy, Fy);
-    cput(kWold, W0);
-    cput(kWPy, WPy);
-    cput(kWPcy, WPcy);
+    const int yr = q - 1;
+    if (defer0 && yr == dlo1) {
+      // row 0 of a fault patch: keep what march_fault_row_kernel needs
+      P* st = reinterpret_cast<P*>(mc.stash[G]) + (size_t)it.fslot * MARCH_STASH_VECS * N * 32 + lane;
+      const P* wo = ring_row(yr) + lane + 1;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        st[(0 * NW + w) * 32] = Anx[w]; st[(1 * NW + w) * 32] = Apx[w];
+        st[(2 * NW + w) * 32] = An_q[w]; st[(3 * NW + w) * 32] = Apy[w];
+        st[(4 * NW + w) * 32] = Bn_q[w]; st[(5 * NW + w) * 32] = Bpy[w];
+      }
+#pragma unroll
+      for (int c = 0; c < N; ++c) st[(6 * NW + c) * 32] = wo[c * MARCH_RW];
+    } else if (yr >= it.y0) {
+      // row q-1: transverse correction of its x values, final x faces, update
+      P jn[NW], jp[NW], sum[NW], dif[NW], BnR[NW], BpL[NW], du[N], u[N];
+#pragma unroll
+      for (int w = 0; w < NW; ++w) jn[w] = psub(An_q[w], Any[w]);
+      jumps<G>(jn, jpy, sum, dif);
+      correct<G, 1, T>(ky, sum, dif, Anx, Apx);
+#pragma unroll
+      for (int w = 0; w < NW; ++w) { BnR[w] = shfl_dn2(Anx[w], 1); BpL[w] = shfl_up2(Apx[w], 1); }
+      if (warp_xedge) {
+        if (edge_lo) edge_value<G>(kx, kx.bgp, mc.xout_lo != 0, Anx, BpL);
+        if (edge_hi) edge_value<G>(kx, kx.bgn, mc.xout_hi != 0, Apx, BnR);
+      }
+#pragma unroll
+      for (int w = 0; w < NW; ++w) { jn[w] = psub(BnR[w], Anx[w]); jp[w] = psub(Apx[w], BpL[w]); }
+      jumps<G>(jn, jp, sum, dif);
+      add_update<G, 0, T>(kx, sum, dif, du);
+#pragma unroll
+      for (int w = 0; w < NW; ++w) jn[w] = psub(Bn_q[w], Bny[w]);
+      jumps<G>(jn, jpB, sum, dif);
+      add_update<G, 1, T>(ky, sum, dif, du);
+      const P* wo = ring_row(yr) + lane + 1;
+#pragma unroll
+      for (int c = 0; c < N; ++c) u[c] = padd(wo[c * MARCH_RW], du[c]);
+      if (col_valid && yr <= it.y1) store_cell<T, G, PL>(pp, mc, fab_idx(pp, 0, x, yr), plane, u, pin);
+      if (it.ncap && yr <= it.y1)
+        march_capture<T, G>(pp, it, mc, yr, lane, cpos, [&](int kind, P* F) {
+          if (kind == 0) face_flux<G, 0, T>(kx, Anx, BpL, F);
+          else if (kind == 1) face_flux<G, 0, T>(kx, BnR, Apx, F);
+          else if (kind == 3) face_flux<G, 1, T>(ky, Bn_q, Bpy, F);
+          else {
+            P below[NW];
+#pragma unroll
+            for (int w = 0; w < NW; ++w) below[w] = psub(Bpy[w], jpB[w]);
+            face_flux<G, 1, T>(ky, Bny, below, F);
+          }
+        });
+    }
+    // advance: the jumps over row q of the values from below (at the domain's
+    // y-lo edge those arriving through it; a fault patch's row 0 is finished later)
+    if (q == dlo1 && !fault) {
+      edge_value<G>(ky, ky.bgp, mc.yout_lo != 0, An_q, Apy);
+      edge_value<G>(ky, ky.bgp, mc.yout_lo != 0, Bn_q, Bpy);
+    }
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      jpy[w] = psub(Ap_q[w], Apy[w]);
+      jpB[w] = psub(Bp_q[w], Bpy[w]);
+      Any[w] = An_q[w]; Apy[w] = Ap_q[w]; Bny[w] = Bn_q[w]; Bpy[w] = Bp_q[w];
+      Anx[w] = Anx_q[w]; Apx[w] = Apx_q[w];
+    }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -902,21 +854,24 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
 
 // Row 0 of a fault-row strip of group G once the fault kernel has produced the
 // first-pass fault states and the fault-face fluxes: the transverse correction
-// of the row's x states, its final x faces and its update (the same steps as
-// the marching loop, with the stashed row-0 intermediates).
+// of the row's x values, its final x faces and its update (the same steps as
+// the marching loop, with the stashed row-0 values).
 template <typename T, int G>
 TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const MarchConst<T>& mc, int lane) {
   using P = typename PairOf<T>::P;
-  constexpr int N = Grp<G>::N;
+  constexpr int N = Grp<G>::N, NW = kWaves<G>;
   const int x = it.x0 - MARCH_HALO + lane;
   const int dlo0 = pp.dlo0, dhi0 = pp.dhi0, dlo1 = pp.dlo1;
   const P* st = reinterpret_cast<const P*>(mc.stash[G]) + (size_t)it.fslot * MARCH_STASH_VECS * N * 32 + lane;
-  P WMcx[N], WPcx[N], H1y1[N], Fy1[N], Wold[N], H1y0[N], Fy0[N];
+  P Bnx[NW], Bpx[NW], An1[NW], Ap0[NW], Bn1[NW], Bp0[NW], u[N], Fy0[N], Fy1[N];
 #pragma unroll
-  for (int c = 0; c < N; ++c) {
-    WMcx[c] = st[(0 * N + c) * 32]; WPcx[c] = st[(1 * N + c) * 32];
-    H1y1[c] = st[(2 * N + c) * 32]; Fy1[c] = st[(3 * N + c) * 32]; Wold[c] = st[(4 * N + c) * 32];
+  for (int w = 0; w < NW; ++w) {
+    Bnx[w] = st[(0 * NW + w) * 32]; Bpx[w] = st[(1 * NW + w) * 32];
+    An1[w] = st[(2 * NW + w) * 32]; Ap0[w] = st[(3 * NW + w) * 32];
+    Bn1[w] = st[(4 * NW + w) * 32]; Bp0[w] = st[(5 * NW + w) * 32];
   }
+#pragma unroll
+  for (int c = 0; c < N; ++c) u[c] = st[(6 * NW + c) * 32];
   const int fi1 = x - (pp.vlo0 - 1);
   const bool ok1 = fi1 >= 0 && fi1 < pp.nfirst && x >= dlo0 && x <= dhi0;
   const int nv = pp.vhi0 - pp.vlo0 + 1, fi2 = x - pp.vlo0;
@@ -924,31 +879,50 @@ TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const Ma
 #pragma unroll
   for (int c = 0; c < N; ++c) {
     const int g = Grp<G>::glob(c);
-    H1y0[c] = ok1 ? mk2((T)pp.first[(size_t)g * pp.nfirst + fi1], (T)pp.first[(size_t)(11 + g) * pp.nfirst + fi1])
-                  : mk2(T(0), T(0));
     Fy0[c] = ok2 ? mk2((T)pp.ffault[(size_t)g * nv + fi2], (T)pp.ffault[(size_t)(11 + g) * nv + fi2])
                  : mk2(T(0), T(0));
   }
-  adw2<G, 1, T>(mc.ky, H1y1, H1y0, WMcx, WPcx);
-  const BgView<G, P> bg{mc.bg};
-  P L[N], g[N], Fx[N], Fxh[N];
+  // y face 1 less the first-pass fault state, as the sums (2 ds) and
+  // differences (2 Z dv) of the jumps that the transverse term takes
+  P sum[NW], dif[NW], jn[NW], jp[NW], BnR[NW], BpL[NW];
 #pragma unroll
-  for (int c = 0; c < N; ++c) L[c] = live<G, 0>(c) ? shfl_up2(WPcx[c], 1) : mk2(T(0), T(0));
-  if (x == dlo0) edge2<G, 0, T>(mc.kx, true, mc.xout_lo != 0, WMcx, bg, g);
-  else if (x == dhi0 + 1) edge2<G, 0, T>(mc.kx, false, mc.xout_hi != 0, L, bg, g);
-  else riem<G, 0, T>(mc.kx, L, WMcx, g);
-  flux2<G, 0, T>(mc.kx, g, Fx);
+  for (int w = 0; w < NW; ++w) {
+    const int gv = Grp<G>::glob(wave_v<G, 1>(w)), gs = Grp<G>::glob(wave_s<G, 1>(w));
+    P v0 = mk2(T(0), T(0)), s0 = v0;
+    if (ok1) {
+      const double b = (double)mc.ky.s0[G == 0 ? w : 2];
+      v0 = mk2((T)pp.first[(size_t)gv * pp.nfirst + fi1], (T)pp.first[(size_t)(11 + gv) * pp.nfirst + fi1]);
+      s0 = mk2((T)(pp.first[(size_t)gs * pp.nfirst + fi1] - b), (T)(pp.first[(size_t)(11 + gs) * pp.nfirst + fi1] - b));
+    }
+    sum[w] = psub(padd(An1[w], Ap0[w]), padd(s0, s0));
+    dif[w] = pfma(is_p<G>(w) ? mc.ky.nZp : mc.ky.nZs, padd(v0, v0), psub(An1[w], Ap0[w]));
+  }
+  correct<G, 1, T>(mc.ky, sum, dif, Bnx, Bpx);
 #pragma unroll
-  for (int c = 0; c < N; ++c) Fxh[c] = shfl_dn2(Fx[c], 1);
+  for (int w = 0; w < NW; ++w) { BnR[w] = shfl_dn2(Bnx[w], 1); BpL[w] = shfl_up2(Bpx[w], 1); }
+  if (x == dlo0) edge_value<G>(mc.kx, mc.kx.bgp, mc.xout_lo != 0, Bnx, BpL);
+  if (x == dhi0) edge_value<G>(mc.kx, mc.kx.bgn, mc.xout_hi != 0, Bpx, BnR);
+  face_flux<G, 1, T>(mc.ky, Bn1, Bp0, Fy1);
   if (it.ncap) {
     int cpos = it.cap0;
-    march_capture<T, G>(pp, it, mc, dlo1, lane, Fx, Fxh, Fy0, Fy1, cpos);
+    march_capture<T, G>(pp, it, mc, dlo1, lane, cpos, [&](int kind, P* F) {
+      if (kind == 0) face_flux<G, 0, T>(mc.kx, Bnx, BpL, F);
+      else if (kind == 1) face_flux<G, 0, T>(mc.kx, BnR, Bpx, F);
+      else {
+#pragma unroll
+        for (int c = 0; c < N; ++c) F[c] = kind == 2 ? Fy0[c] : Fy1[c];
+      }
+    });
   }
   const bool col_valid = x >= it.x0 && x < it.x0 + MARCH_COLS && x >= pp.vlo0 && x <= pp.vhi0;
   if (col_valid) {
-    P u[N];
 #pragma unroll
-    for (int c = 0; c < N; ++c) u[c] = pfma(padd(psub(Fxh[c], Fx[c]), psub(Fy1[c], Fy0[c])), mc.sc, Wold[c]);
+    for (int w = 0; w < NW; ++w) { jn[w] = psub(BnR[w], Bnx[w]); jp[w] = psub(Bpx[w], BpL[w]); }
+    jumps<G>(jn, jp, sum, dif);
+    P du[N];
+    add_update<G, 0, T>(mc.kx, sum, dif, du);
+#pragma unroll
+    for (int c = 0; c < N; ++c) u[c] = padd(u[c], pfma(psub(Fy1[c], Fy0[c]), mc.sc, du[c]));
     const size_t plane = (size_t)pp.anx * pp.any, o = fab_idx(pp, 0, x, dlo1);
     P pin[3];
     if (mc.plastic) {
@@ -979,8 +953,5 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS) march_fault_row_kernel(const
   }
 }
 
-#undef KC
-#undef KE
-#undef KHALF
 
 }  // namespace tmk
