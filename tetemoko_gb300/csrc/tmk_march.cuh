@@ -53,13 +53,14 @@ TMK_HD double2 mk2(double a, double b) { return make_double2(a, b); }
 TMK_D float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 TMK_D float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 TMK_D float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-TMK_D float2 psub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+TMK_D float2 psub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 TMK_D double2 padd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 TMK_D double2 pmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
 TMK_D double2 pfma(double2 a, double2 b, double2 c) { return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)); }
 TMK_D double2 psub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 TMK_D float2 pneg(float2 a) { return pmul(a, make_float2(-1.f, -1.f)); }
-TMK_D double2 pneg(double2 a) { return make_double2(-a.x, -a.y); }
+TMK_D double flip(double a) { return __hiloint2double(__double2hiint(a) ^ 0x80000000, __double2loint(a)); }
+TMK_D double2 pneg(double2 a) { return make_double2(flip(a.x), flip(a.y)); }
 
 TMK_D float2 shfl_up2(float2 v, int d) {
   return make_float2(__shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d));
@@ -221,31 +222,41 @@ struct MarchConst {
 // warp, so the FP64 form's comparisons, signs and powers of two are done on the
 // bit patterns with integer instructions; magnitudes order as their patterns,
 // and a NaN is larger than every number, so a minimum drops it as fmin does.
-TMK_D unsigned long long mag64(double x) { return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull; }
+// (the masks act on the high word: a 64-bit one is turned back into an FP64
+// absolute value, which holds the FP64 pipe like a sum)
+TMK_D unsigned long long mag64(double x) {
+  unsigned long long m;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(m) : "r"(__double2loint(x)), "r"(__double2hiint(x) & 0x7fffffff));
+  return m;
+}
 // min(|a|, |b|) with the sign of a
 TMK_D float clip_mag(float a, float b) { return copysignf(fminf(fabsf(a), fabsf(b)), a); }
+TMK_D double with_sign(unsigned long long m, double a) {
+  return __hiloint2double((int)(m >> 32) | (__double2hiint(a) & 0x80000000), (int)m);
+}
 TMK_D double clip_mag(double a, double b) {
   const unsigned long long ma = mag64(a), mb = mag64(b);
-  const unsigned long long m = ma < mb ? ma : mb;
-  return __longlong_as_double((long long)(m | ((unsigned long long)__double_as_longlong(a) & 0x8000000000000000ull)));
+  return with_sign(ma < mb ? ma : mb, a);
 }
 TMK_D float clip_mag(float a, float b, float c) { return copysignf(fminf(fminf(fabsf(a), fabsf(b)), fabsf(c)), a); }
 TMK_D double clip_mag(double a, double b, double c) {
-  const unsigned long long mb = mag64(b), mc = mag64(c);
+  const unsigned long long ma = mag64(a), mb = mag64(b), mc = mag64(c);
   const unsigned long long m = mb < mc ? mb : mc;
-  return clip_mag(a, __longlong_as_double((long long)m));
+  return with_sign(ma < m ? ma : m, a);
 }
-// x * 2^k for |k| <= 2
+// x * 2^K by the exponent bits (|K| <= 3); zeros, denormals and numbers near
+// the overflow limit, which only serve as bounds here, are returned as they are
 template <int K> TMK_D double mul_pow2(double x) {
   const int hi = __double2hiint(x);
   const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-  if (e - 3u < 2041u) return __hiloint2double(hi + (K << 20), __double2loint(x));   // normal before and after
-  return x == 0.0 ? x : x * (K == 1 ? 2.0 : 0.25);
+  return __hiloint2double(e - 3u < 2040u ? hi + (K << 20) : hi, __double2loint(x));
 }
 TMK_D float2 quarter(float2 a) { return pmul(a, make_float2(0.25f, 0.25f)); }
 TMK_D double2 quarter(double2 a) { return make_double2(mul_pow2<-2>(a.x), mul_pow2<-2>(a.y)); }
 TMK_D float2 twice(float2 a) { return padd(a, a); }
 TMK_D double2 twice(double2 a) { return make_double2(mul_pow2<1>(a.x), mul_pow2<1>(a.y)); }
+TMK_D float2 eight_times(float2 a) { return pmul(a, make_float2(8.f, 8.f)); }
+TMK_D double2 eight_times(double2 a) { return make_double2(mul_pow2<3>(a.x), mul_pow2<3>(a.y)); }
 // a b > 0 per half (both nonzero numbers of one sign)
 TMK_D void same_sign(float2 a, float2 b, bool& x, bool& y) {
   const float2 p = pmul(a, b);
@@ -262,14 +273,14 @@ TMK_D void same_sign(double2 a, double2 b, bool& x, bool& y) { x = same_sign1(a.
 // nl = w_{i-1} - w_i and nr = w_i - w_{i+1} (at a domain edge the missing one
 // is given the other's value: the one-sided difference the reference uses):
 // minus half the van Leer slope, sign(dc) min(|dc|, 2|dl|, 2|dr|) when
-// dl dr > 0, else 0.  okx, oky: whether dl dr > 0.
-template <typename P> TMK_D P half_slope(P nl, P nr, bool limit, bool& okx, bool& oky) {
+// dl dr > 0, else 0.
+template <typename P> TMK_D P half_slope(P nl, P nr, bool limit) {
   using T = decltype(nl.x);
   const P q = quarter(padd(nl, nr));
-  okx = oky = true;
   if (!limit) return q;
-  same_sign(nl, nr, okx, oky);
-  return mk2(okx ? clip_mag(q.x, nl.x, nr.x) : T(0), oky ? clip_mag(q.y, nl.y, nr.y) : T(0));
+  bool x, y;
+  same_sign(nl, nr, x, y);
+  return mk2(x ? clip_mag(q.x, nl.x, nr.x) : T(0), y ? clip_mag(q.y, nl.y, nr.y) : T(0));
 }
 
 // Twice the PPM delta (lo face value - w) of a cell from its negated
@@ -281,15 +292,18 @@ template <typename T, typename P> TMK_D P delta_lo(P nl, P n_i, P n_im1) {
 // twice the hi delta from the next cell's: w_hi(i) = w_lo(i+1)
 template <typename T, typename P> TMK_D P delta_hi(P nr, P dlo_next) { return pfma(nr, kall(T(-2)), dlo_next); }
 
-// PPM limiter (Colella & Woodward 1984 eq. 1.10) of the deltas m, p of a cell:
-// both zero at an extremum, otherwise each clipped to twice the other's
-// magnitude.  With slopes limited as above m is between -0.17 dl and -0.83 dl
-// and p between 0.17 dr and 0.83 dr, so m p < 0 exactly where dl dr > 0; the
-// caller has zeroed m elsewhere, which makes both results zero.
-template <typename P> TMK_D void limit_mono(P& m, P& p) {
-  const P m2 = twice(m), p2 = twice(p);
-  const P a = mk2(clip_mag(m.x, p2.x), clip_mag(m.y, p2.y));
-  p = mk2(clip_mag(p.x, m2.x), clip_mag(p.y, m2.y));
+// PPM limiter (Colella & Woodward 1984 eq. 1.10) of the doubled deltas m, p of
+// a cell with half slope n: both zero at an extremum, otherwise each clipped to
+// twice the other's magnitude.  With slopes limited as above, m lies between
+// -0.17 and -0.83 of dl (doubled: twice that) and p between 0.17 and 0.83 of
+// dr, so m p < 0 exactly where dl dr > 0, that is where n is not zero; there
+// the clipped values stay below 2 * 1.66 min(|dl|, |dr|) <= 6.7 |n|, so the
+// further bound 8 |n| only acts where n is zero and makes both zero without a
+// test.
+template <typename P> TMK_D void limit_mono(P& m, P& p, P n) {
+  const P m2 = twice(m), p2 = twice(p), b = eight_times(n);
+  const P a = mk2(clip_mag(m.x, p2.x, b.x), clip_mag(m.y, p2.y, b.y));
+  p = mk2(clip_mag(p.x, m2.x, b.x), clip_mag(p.y, m2.y, b.y));
   m = a;
 }
 // the same limiter for deltas of unknown sign (characteristic limiting)
@@ -298,7 +312,10 @@ template <typename P> TMK_D void limit2(P& m, P& p) {
   bool x, y;
   same_sign(m, pneg(p), x, y);
   m = mk2(x ? m.x : T(0), y ? m.y : T(0));
-  limit_mono(m, p);
+  const P m2 = twice(m), p2 = twice(p);
+  const P a = mk2(clip_mag(m.x, p2.x), clip_mag(m.y, p2.y));
+  p = mk2(clip_mag(p.x, m2.x), clip_mag(p.y, m2.y));
+  m = a;
 }
 
 // The traced characteristic values of a cell in direction D (see the head of
@@ -447,12 +464,30 @@ template <typename T, int G> struct MarchMinBlocks {
   static constexpr int value = sizeof(T) == 4 ? ((G == 0) ? 3 : 5) : ((G == 0) ? 2 : 4);
 };
 
-// asynchronous copy of one element into shared memory (completion tracked per
-// thread); nbytes = sizeof(T), or 0: nothing is read and zeros are written
-template <typename T> TMK_D void cp_async_elem(T* dst_smem, const T* src, unsigned nbytes = sizeof(T)) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(sizeof(T)), "r"(nbytes)
+// asynchronous copy of one element to shared address dst + OFF (completion
+// tracked per thread); nbytes = sizeof(T), or 0: nothing is read and zeros are
+// written
+template <typename T, int OFF> TMK_D void cp_async_elem(unsigned dst, const T* src, unsigned nbytes) {
+  asm volatile("cp.async.ca.shared.global [%0 + %4], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(sizeof(T)), "r"(nbytes),
+               "n"(OFF)
                : "memory");
+}
+// component plane g of a FAB from the address in plane 0 (one 32 x 32 + 64-bit
+// multiply-add; the planes hold fewer than 2^32 cells)
+template <typename T> TMK_D T* plane_ptr(T* p0, unsigned plane, int g) {
+  return reinterpret_cast<T*>((unsigned long long)p0 + (unsigned long long)plane * (unsigned)(g * sizeof(T)));
+}
+// the cp.async copies of one lane's column of a ring row, components C...
+template <typename T, int G, int C, bool XONLY>
+TMK_D void cp_async_column(unsigned dst, const T* src, unsigned plane, unsigned nbytes) {
+  if constexpr (C < Grp<G>::N) {
+    if constexpr (!XONLY || live<G, 0>(C)) {
+      constexpr int off = C * MARCH_RW * 2 * (int)sizeof(T);
+      cp_async_elem<T, off>(dst, plane_ptr(src, plane, Grp<G>::glob(C)), nbytes);
+      cp_async_elem<T, off + (int)sizeof(T)>(dst, plane_ptr(src, plane, 11 + Grp<G>::glob(C)), nbytes);
+    }
+    cp_async_column<T, G, C + 1, XONLY>(dst, src, plane, nbytes);
+  }
 }
 TMK_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // all but the newest K groups have landed
@@ -462,13 +497,13 @@ template <int K> TMK_D void cp_async_wait() { asm volatile("cp.async.wait_group 
 // antiplane group's updated sxz, syz (stored by the antiplane kernel, which
 // has completed) and the plastic strain of the step's input, both sides.
 template <typename T>
-TMK_D void plastic_inputs(const PatchDev<T>& pp, size_t o, size_t plane, typename PairOf<T>::P* pin) {
-  pin[0] = mk2(pp.Uout[o + 7 * plane], pp.Uout[o + 18 * plane]);
-  pin[1] = mk2(pp.Uout[o + 8 * plane], pp.Uout[o + 19 * plane]);
-  pin[2] = mk2(pp.Uin[o + 10 * plane], pp.Uin[o + 21 * plane]);
+TMK_D void plastic_inputs(const T* in0, const T* out0, unsigned plane, typename PairOf<T>::P* pin) {
+  pin[0] = mk2(*plane_ptr(out0, plane, 7), *plane_ptr(out0, plane, 18));
+  pin[1] = mk2(*plane_ptr(out0, plane, 8), *plane_ptr(out0, plane, 19));
+  pin[2] = mk2(*plane_ptr(in0, plane, 10), *plane_ptr(in0, plane, 21));
 }
 
-// Stores the updated group G of one cell (flat index o of component 0).  With
+// Stores the updated group G of one cell (out0: its address in plane 0).  With
 // PL (a plastic level whose return is fused) the in-plane group first takes
 // LinElastLevelGodunov::plasticUpdate (PLASTICCORRECTION,
 // srcLinElast/PlasticPhysicsF.ChF:30-133, as the reference applies it after
@@ -477,8 +512,8 @@ TMK_D void plastic_inputs(const PatchDev<T>& pp, size_t o, size_t plane, typenam
 // return; the antiplane stresses are rewritten where the point yielded, the
 // plastic rate and strain always.
 template <typename T, int G, bool PL>
-TMK_D void store_cell(const PatchDev<T>& pp, const MarchConst<T>& mc, size_t o, size_t plane,
-                      typename PairOf<T>::P* u, const typename PairOf<T>::P* pin) {
+TMK_D void store_cell(T* out0, unsigned plane, const MarchConst<T>& mc, typename PairOf<T>::P* u,
+                      const typename PairOf<T>::P* pin) {
   constexpr int N = Grp<G>::N;
   if constexpr (G == 0 && PL) {
     T sxz[2] = {pin[0].x, pin[0].y}, syz[2] = {pin[1].x, pin[1].y}, gam[2] = {pin[2].x, pin[2].y};
@@ -490,18 +525,18 @@ TMK_D void store_cell(const PatchDev<T>& pp, const MarchConst<T>& mc, size_t o, 
       if (plastic_flow_k<T>(mc.pk, sxx, syy, szz, sxy, sxz[sd], syz[sd], lam, gam[sd], mc.pdt)) {
         if (sd) { u[2].y = sxx; u[3].y = syy; u[4].y = szz; u[5].y = sxy; }
         else { u[2].x = sxx; u[3].x = syy; u[4].x = szz; u[5].x = sxy; }
-        pp.Uout[o + (size_t)(11 * sd + 7) * plane] = sxz[sd];
-        pp.Uout[o + (size_t)(11 * sd + 8) * plane] = syz[sd];
+        *plane_ptr(out0, plane, 11 * sd + 7) = sxz[sd];
+        *plane_ptr(out0, plane, 11 * sd + 8) = syz[sd];
       }
-      pp.Uout[o + (size_t)(11 * sd + 9) * plane] = lam;
-      pp.Uout[o + (size_t)(11 * sd + 10) * plane] = gam[sd];
+      *plane_ptr(out0, plane, 11 * sd + 9) = lam;
+      *plane_ptr(out0, plane, 11 * sd + 10) = gam[sd];
     }
   }
 #pragma unroll
   for (int c = 0; c < N; ++c) {
     const int gg = Grp<G>::glob(c);
-    pp.Uout[o + (size_t)gg * plane] = u[c].x;
-    pp.Uout[o + (size_t)(11 + gg) * plane] = u[c].y;
+    *plane_ptr(out0, plane, gg) = u[c].x;
+    *plane_ptr(out0, plane, 11 + gg) = u[c].y;
   }
 }
 
@@ -551,7 +586,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   constexpr int N = Grp<G>::N, NW = kWaves<G>;
   extern __shared__ __align__(16) unsigned char march_smem[];
   P* const ring = reinterpret_cast<P*>(march_smem) + (size_t)(threadIdx.x >> 5) * march_warp_pairs<T, G>();
-  const int wid = blockIdx.x * MARCH_WARPS + (threadIdx.x >> 5);
+  const int wid = blockIdx.x * MARCH_WARPS + __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   // a later kernel of the step may be scheduled now; every warp waits for the
   // kernel before it (the fault kernel or the other component group) before
@@ -583,7 +618,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   const bool fault = pp.fault != 0;
   const bool defer0 = it.fslot >= 0;      // row 0 is finished by march_fault_row_kernel
   const bool col_valid = x >= it.x0 && x < it.x0 + MARCH_COLS && x >= pp.vlo0 && x <= pp.vhi0;
-  const size_t plane = (size_t)pp.anx * pp.any;
+  const int anx = pp.anx;
+  const unsigned plane = (unsigned)anx * (unsigned)pp.any;
   // a lane of this warp holds a cell on a domain x edge: every lane takes the
   // interior differences and face values, overwritten there by the edge's;
   // other warps (most) skip the edge code on a uniform branch
@@ -593,63 +629,58 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   const int q_s = max(it.y0 - 1, dlo1);
   const int q_e = it.y1 + 1;
 
+  // the lane's addresses in plane 0: of the next row to stage, of the row stored next
+  const T* lsrc = pp.Uin + ((long long)(q_s - pp.alo1) * anx + (x - pp.alo0));
+  T* sdst = pp.Uout + ((long long)(q_s - 1 - pp.alo1) * anx + (x - pp.alo0));
+  const T* psrc = PL ? pp.Uin + ((long long)(q_s - 1 - pp.alo1) * anx + (x - pp.alo0)) : nullptr;
+  const T* const uin = pp.Uin;
+  const unsigned ring32 = (unsigned)__cvta_generic_to_shared(ring);
+
   auto load_row = [&](int y, P* w) {
     const bool ok = lane_in && y >= dlo1 && y <= dhi1;
-    const size_t o = ok ? fab_idx(pp, 0, x, y) : 0;
+    const T* const p0 = ok ? uin + ((long long)(y - pp.alo1) * anx + (x - pp.alo0)) : uin;
 #pragma unroll
     for (int c = 0; c < N; ++c) {
       if (!live<G, 1>(c)) { w[c] = mk2(T(0), T(0)); continue; }
       const int g = Grp<G>::glob(c);
-      w[c] = ok ? mk2(pp.Uin[o + (size_t)g * plane], pp.Uin[o + (size_t)(11 + g) * plane]) : mk2(T(0), T(0));
+      w[c] = ok ? mk2(*plane_ptr(p0, plane, g), *plane_ptr(p0, plane, 11 + g)) : mk2(T(0), T(0));
     }
   };
-  // row y into its ring slot: cp.async for cells in the domain, zeros
-  // elsewhere (and for rows past the last one the item reads); the two outer
-  // columns only for the components live in x (the only ones whose neighbours
-  // are read)
+  // row y (the next one to stage) into its ring slot: cp.async for cells in
+  // the domain, zeros elsewhere (and for rows past the last one the item
+  // reads); the two outer columns only for the components live in x (the only
+  // ones whose neighbours are read)
   auto ring_row = [&](int y) -> P* { return ring + (size_t)((y & (MARCH_RING - 1)) * N) * MARCH_RW; };
+  const int y_last = min(dhi1, q_e + 2);
   auto load_row_async = [&](int y) {
-    const bool yin = y >= dlo1 && y <= dhi1 && y <= q_e + 2;
-    const bool ok = lane_in && yin;
-    const size_t o = ok ? fab_idx(pp, 0, x, y) : 0;
-    const unsigned nb = ok ? (unsigned)sizeof(T) : 0u;
-    P* const rowp = ring_row(y);
-    P* const dst = rowp + lane + 1;
-    const T* const src = pp.Uin + o;
-#pragma unroll
-    for (int c = 0; c < N; ++c) {
-      const int g = Grp<G>::glob(c);
-      T* d2 = reinterpret_cast<T*>(dst + c * MARCH_RW);
-      cp_async_elem(d2, src + (size_t)g * plane, nb);
-      cp_async_elem(d2 + 1, src + (size_t)(11 + g) * plane, nb);
-    }
-    if (lane == 0 || lane == 31) {      // the outer columns: own address -1 / +1 (oke implies ok)
+    const bool ok = lane_in && y <= y_last;       // y >= q_s >= dlo1
+    const T* const src = ok ? lsrc : uin;
+    const unsigned row32 = ring32 + (unsigned)((y & (MARCH_RING - 1)) * (N * MARCH_RW * (int)sizeof(P)));
+    cp_async_column<T, G, 0, false>(row32 + (unsigned)((lane + 1) * (int)sizeof(P)), src, plane,
+                                    ok ? (unsigned)sizeof(T) : 0u);
+    if (lane == 0 || lane == 31) {      // the outer columns: own address -1 / +1 (ext_in and ok: a cell of the FAB)
       const bool oke = ext_in && ok;
-      const unsigned nbe = oke ? (unsigned)sizeof(T) : 0u;
-      const T* const srce = oke ? src + dxe : src;
-      P* const dste = rowp + ext_pos;
-#pragma unroll
-      for (int c = 0; c < N; ++c) {
-        if (!live<G, 0>(c)) continue;
-        const int g = Grp<G>::glob(c);
-        T* d2 = reinterpret_cast<T*>(dste + c * MARCH_RW);
-        cp_async_elem(d2, srce + (size_t)g * plane, nbe);
-        cp_async_elem(d2 + 1, srce + (size_t)(11 + g) * plane, nbe);
-      }
+      cp_async_column<T, G, 0, true>(row32 + (unsigned)(ext_pos * (int)sizeof(P)), oke ? src + dxe : uin, plane,
+                                     oke ? (unsigned)sizeof(T) : 0u);
     }
     cp_async_commit();
+    lsrc += anx;
   };
 
   int cpos = it.cap0;                     // next coarse-fine face to store
-  // carried from row to row: the half slopes and the lo deltas of row q (zeroed
-  // at extrema where the limiter zeroes them), the traced x values of row q-1,
-  // the traced and corrected y values of row q-1 (An, Ap) and their jump jp
-  P n4[N], dlo[N];
-  P Anx[NW], Apx[NW], Any[NW], Apy[NW], jpy[NW], Bny[NW], Bpy[NW], jpB[NW];
+  // What a lane carries from row to row: the half slopes and lo deltas of row
+  // q, the traced x values of row q-1, the traced and corrected y values of
+  // row q-1 (An, Ap) and their jump jp.  Two sets, used in turn by two copies
+  // of the row's code: with one set each value would be moved once a row.
+  struct Carry {
+    P n4[N], dlo[N];
+    P Anx[NW], Apx[NW], Any[NW], Apy[NW], jpy[NW], Bny[NW], Bpy[NW], jpB[NW];
+  } c0, c1;
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
-    Anx[w] = mk2(T(0), T(0)); Apx[w] = Anx[w]; Any[w] = Anx[w]; Apy[w] = Anx[w]; jpy[w] = Anx[w];
-    Bny[w] = Anx[w]; Bpy[w] = Anx[w]; jpB[w] = Anx[w];
+    const P z = mk2(T(0), T(0));
+    c0.Anx[w] = z; c0.Apx[w] = z; c0.Any[w] = z; c0.Apy[w] = z; c0.jpy[w] = z;
+    c0.Bny[w] = z; c0.Bpy[w] = z; c0.jpB[w] = z;
   }
   {
 #pragma unroll
@@ -663,124 +694,151 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
     const P* r1 = ring_row(q_s + 1) + lane + 1;
 #pragma unroll
     for (int c = 0; c < N; ++c) {
-      n4[c] = mk2(T(0), T(0)); dlo[c] = n4[c];
       if (!live<G, 1>(c)) continue;
       const P W0 = r0[c * MARCH_RW];
       P nl = psub(Wb[c], W0), nr = psub(W0, r1[c * MARCH_RW]);
       if (!hl) nl = nr;
       if (!hr) nr = nl;
       if (!hl && !hr) { nl = mk2(T(0), T(0)); nr = nl; }
-      bool okx, oky, ax, ay;
-      n4[c] = half_slope(nl, nr, lim, okx, oky);
+      c0.n4[c] = half_slope(nl, nr, lim);
       if (hl) {
         P na = psub(Wa[c], Wb[c]);
         if (!hll) na = nl;
-        dlo[c] = delta_lo<T>(nl, n4[c], half_slope(na, nl, lim, ax, ay));
+        c0.dlo[c] = delta_lo<T>(nl, c0.n4[c], half_slope(na, nl, lim));
       } else {
-        dlo[c] = twice(n4[c]);
+        c0.dlo[c] = twice(c0.n4[c]);
       }
-      if (plim) dlo[c] = mk2(okx ? dlo[c].x : T(0), oky ? dlo[c].y : T(0));
     }
   }
 
-  for (int q = q_s; q <= q_e; ++q) {
+  auto row_step = [&](const int q, Carry& in, Carry& out) {
     load_row_async(q + MARCH_AHEAD);  // rows in flight while this one is computed
     // fused plastic return: its other inputs for row q-1, stored at the end of
     // this iteration, requested now so that the row's work hides their latency
     P pin[3];
     if constexpr (PL) {
-      if (col_valid && q - 1 >= it.y0 && q - 1 <= it.y1) plastic_inputs<T>(pp, fab_idx(pp, 0, x, q - 1), plane, pin);
+      if (col_valid && q - 1 >= it.y0 && q - 1 <= it.y1) plastic_inputs<T>(psrc, sdst, plane, pin);
+      psrc += anx;
     }
     cp_async_wait<MARCH_AHEAD - 2>();     // rows up to q+2 have landed
     __syncwarp();                         // ... every lane's copies, whose neighbours read them
-    P An_q[NW], Ap_q[NW], Bn_q[NW], Bp_q[NW], Anx_q[NW], Apx_q[NW];
+    P Bn_q[NW], Bp_q[NW];
     if (q <= dhi1) {
-      const P* const rw = ring_row(q);
-      P W0[N], m[N], p[N];
+      const P* const rw = ring_row(q) + lane + 1;
+      P W0[N], m[N], p[N], nl[N], nr[N];
 #pragma unroll
-      for (int c = 0; c < N; ++c) { W0[c] = rw[c * MARCH_RW + lane + 1]; m[c] = mk2(T(0), T(0)); p[c] = m[c]; }
-      // the cell's state relative to the background, for its characteristic values
+      for (int c = 0; c < N; ++c) { W0[c] = rw[c * MARCH_RW]; m[c] = mk2(T(0), T(0)); p[c] = m[c]; }
+      // the cell's stresses relative to the background, for its characteristic values
       P Wr[N];
 #pragma unroll
-      for (int c = 0; c < N; ++c) Wr[c] = padd(W0[c], kall(mc.nbg[Grp<G>::glob(c)]));
+      for (int c = 0; c < N; ++c)
+        Wr[c] = Grp<G>::glob(c) < 3 ? W0[c] : padd(W0[c], kall(mc.nbg[Grp<G>::glob(c)]));
       if (ppm) {
         // y deltas of row q; slope and lo delta of row q+1
         const P* const r1 = ring_row(q + 1) + lane + 1;
         const P* const r2 = ring_row(q + 2) + lane + 1;
-        const bool has1 = q + 1 <= dhi1, has2 = q + 2 <= dhi1;
 #pragma unroll
         for (int c = 0; c < N; ++c) {
           if (!live<G, 1>(c)) continue;
           const P W1 = r1[c * MARCH_RW];
-          const P nl = psub(W0[c], W1);
-          P nr = psub(W1, r2[c * MARCH_RW]);
-          if (!has2) nr = nl;
-          bool okx, oky;
-          const P n1 = half_slope(nl, nr, lim, okx, oky);
-          P d1 = delta_lo<T>(nl, n1, n4[c]);
-          m[c] = dlo[c];
-          p[c] = delta_hi<T>(nl, d1);
-          if (!has1) p[c] = pneg(twice(n4[c]));
-          if (plim) {
-            limit_mono(m[c], p[c]);
-            d1 = mk2(okx ? d1.x : T(0), oky ? d1.y : T(0));
-          }
-          n4[c] = n1;
-          dlo[c] = d1;
+          nl[c] = psub(W0[c], W1);
+          nr[c] = psub(W1, r2[c * MARCH_RW]);
         }
-        trace<G, 1, T>(ky, Wr, m, p, clim, An_q, Ap_q);
+        if (q + 2 > dhi1) {
+#pragma unroll
+          for (int c = 0; c < N; ++c) nr[c] = nl[c];
+        }
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+          if (!live<G, 1>(c)) continue;
+          out.n4[c] = half_slope(nl[c], nr[c], lim);
+          out.dlo[c] = delta_lo<T>(nl[c], out.n4[c], in.n4[c]);
+          p[c] = delta_hi<T>(nl[c], out.dlo[c]);
+        }
+        if (q + 1 > dhi1) {
+#pragma unroll
+          for (int c = 0; c < N; ++c)
+            if (live<G, 1>(c)) p[c] = pneg(twice(in.n4[c]));
+        }
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+          if (!live<G, 1>(c)) continue;
+          m[c] = in.dlo[c];
+          if (plim) limit_mono(m[c], p[c], in.n4[c]);
+        }
+        trace<G, 1, T>(ky, Wr, m, p, clim, out.Any, out.Apy);
         // x deltas
+        P n[N], d[N];
 #pragma unroll
         for (int c = 0; c < N; ++c) {
           if (!live<G, 0>(c)) continue;
-          P nl = psub(rw[c * MARCH_RW + lane], W0[c]), nr = psub(W0[c], rw[c * MARCH_RW + lane + 2]);
-          if (warp_xedge) {
-            const P nl0 = nl;
-            if (edge_lo) nl = nr;
-            if (edge_hi) nr = edge_lo ? mk2(T(0), T(0)) : nl0;
-            if (edge_lo && edge_hi) nl = nr;
-          }
-          bool okx, oky;
-          const P n = half_slope(nl, nr, lim, okx, oky);
-          P d = delta_lo<T>(nl, n, shfl_up2(n, 1));
-          if (warp_xedge && edge_lo) d = twice(n);
-          p[c] = delta_hi<T>(nr, shfl_dn2(d, 1));
-          if (warp_xedge && edge_hi) p[c] = pneg(twice(n));
-          if (plim) {
-            d = mk2(okx ? d.x : T(0), oky ? d.y : T(0));
-            limit_mono(d, p[c]);
-          }
-          m[c] = d;
+          nl[c] = psub(rw[c * MARCH_RW - 1], W0[c]);
+          nr[c] = psub(W0[c], rw[c * MARCH_RW + 1]);
         }
-        trace<G, 0, T>(kx, Wr, m, p, clim, Anx_q, Apx_q);
+        if (warp_xedge) {
+#pragma unroll
+          for (int c = 0; c < N; ++c) {
+            if (!live<G, 0>(c)) continue;
+            const P l = nl[c];
+            if (edge_lo) nl[c] = edge_hi ? mk2(T(0), T(0)) : nr[c];
+            if (edge_hi) nr[c] = edge_lo ? mk2(T(0), T(0)) : l;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+          if (!live<G, 0>(c)) continue;
+          n[c] = half_slope(nl[c], nr[c], lim);
+          d[c] = delta_lo<T>(nl[c], n[c], shfl_up2(n[c], 1));
+        }
+        if (warp_xedge && edge_lo) {
+#pragma unroll
+          for (int c = 0; c < N; ++c)
+            if (live<G, 0>(c)) d[c] = twice(n[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < N; ++c)
+          if (live<G, 0>(c)) p[c] = delta_hi<T>(nr[c], shfl_dn2(d[c], 1));
+        if (warp_xedge && edge_hi) {
+#pragma unroll
+          for (int c = 0; c < N; ++c)
+            if (live<G, 0>(c)) p[c] = pneg(twice(n[c]));
+        }
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+          if (!live<G, 0>(c)) continue;
+          m[c] = d[c];
+          if (plim) limit_mono(m[c], p[c], n[c]);
+        }
+        trace<G, 0, T>(kx, Wr, m, p, clim, out.Anx, out.Apx);
       } else {
-        chars<G, 1, T>(ky, Wr, An_q, Ap_q);
-        chars<G, 0, T>(kx, Wr, Anx_q, Apx_q);
+        chars<G, 1, T>(ky, Wr, out.Any, out.Apy);
+        chars<G, 0, T>(kx, Wr, out.Anx, out.Apx);
       }
       // first-pass x faces of row q, corrected y values
       P AnR[NW], ApL[NW], jn[NW], jp[NW], sum[NW], dif[NW];
 #pragma unroll
-      for (int w = 0; w < NW; ++w) { AnR[w] = shfl_dn2(Anx_q[w], 1); ApL[w] = shfl_up2(Apx_q[w], 1); }
+      for (int w = 0; w < NW; ++w) { AnR[w] = shfl_dn2(out.Anx[w], 1); ApL[w] = shfl_up2(out.Apx[w], 1); }
       if (warp_xedge) {
-        if (edge_lo) edge_value<G>(kx, kx.bgp, mc.xout_lo != 0, Anx_q, ApL);
-        if (edge_hi) edge_value<G>(kx, kx.bgn, mc.xout_hi != 0, Apx_q, AnR);
+        if (edge_lo) edge_value<G>(kx, kx.bgp, mc.xout_lo != 0, out.Anx, ApL);
+        if (edge_hi) edge_value<G>(kx, kx.bgn, mc.xout_hi != 0, out.Apx, AnR);
       }
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
-        jn[w] = psub(AnR[w], Anx_q[w]);
-        jp[w] = psub(Apx_q[w], ApL[w]);
-        Bn_q[w] = An_q[w];
-        Bp_q[w] = Ap_q[w];
+        jn[w] = psub(AnR[w], out.Anx[w]);
+        jp[w] = psub(out.Apx[w], ApL[w]);
+        Bn_q[w] = out.Any[w];
+        Bp_q[w] = out.Apy[w];
       }
       jumps<G>(jn, jp, sum, dif);
       correct<G, 0, T>(kx, sum, dif, Bn_q, Bp_q);
     } else {
       // past the domain's y-hi edge: the values arriving through it
-      edge_value<G>(ky, ky.bgn, mc.yout_hi != 0, Apy, An_q);
-      edge_value<G>(ky, ky.bgn, mc.yout_hi != 0, Bpy, Bn_q);
+      edge_value<G>(ky, ky.bgn, mc.yout_hi != 0, in.Apy, out.Any);
+      edge_value<G>(ky, ky.bgn, mc.yout_hi != 0, in.Bpy, Bn_q);
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
-        Ap_q[w] = mk2(T(0), T(0)); Bp_q[w] = Ap_q[w]; Anx_q[w] = Ap_q[w]; Apx_q[w] = Ap_q[w];
+        const P z = mk2(T(0), T(0));
+        out.Apy[w] = z; Bp_q[w] = z; out.Anx[w] = z; out.Apx[w] = z;
       }
     }
     const int yr = q - 1;
@@ -790,9 +848,9 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
       const P* wo = ring_row(yr) + lane + 1;
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
-        st[(0 * NW + w) * 32] = Anx[w]; st[(1 * NW + w) * 32] = Apx[w];
-        st[(2 * NW + w) * 32] = An_q[w]; st[(3 * NW + w) * 32] = Apy[w];
-        st[(4 * NW + w) * 32] = Bn_q[w]; st[(5 * NW + w) * 32] = Bpy[w];
+        st[(0 * NW + w) * 32] = in.Anx[w]; st[(1 * NW + w) * 32] = in.Apx[w];
+        st[(2 * NW + w) * 32] = out.Any[w]; st[(3 * NW + w) * 32] = in.Apy[w];
+        st[(4 * NW + w) * 32] = Bn_q[w]; st[(5 * NW + w) * 32] = in.Bpy[w];
       }
 #pragma unroll
       for (int c = 0; c < N; ++c) st[(6 * NW + c) * 32] = wo[c * MARCH_RW];
@@ -800,53 +858,60 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
       // row q-1: transverse correction of its x values, final x faces, update
       P jn[NW], jp[NW], sum[NW], dif[NW], BnR[NW], BpL[NW], du[N], u[N];
 #pragma unroll
-      for (int w = 0; w < NW; ++w) jn[w] = psub(An_q[w], Any[w]);
-      jumps<G>(jn, jpy, sum, dif);
-      correct<G, 1, T>(ky, sum, dif, Anx, Apx);
+      for (int w = 0; w < NW; ++w) jn[w] = psub(out.Any[w], in.Any[w]);
+      jumps<G>(jn, in.jpy, sum, dif);
+      correct<G, 1, T>(ky, sum, dif, in.Anx, in.Apx);
 #pragma unroll
-      for (int w = 0; w < NW; ++w) { BnR[w] = shfl_dn2(Anx[w], 1); BpL[w] = shfl_up2(Apx[w], 1); }
+      for (int w = 0; w < NW; ++w) { BnR[w] = shfl_dn2(in.Anx[w], 1); BpL[w] = shfl_up2(in.Apx[w], 1); }
       if (warp_xedge) {
-        if (edge_lo) edge_value<G>(kx, kx.bgp, mc.xout_lo != 0, Anx, BpL);
-        if (edge_hi) edge_value<G>(kx, kx.bgn, mc.xout_hi != 0, Apx, BnR);
+        if (edge_lo) edge_value<G>(kx, kx.bgp, mc.xout_lo != 0, in.Anx, BpL);
+        if (edge_hi) edge_value<G>(kx, kx.bgn, mc.xout_hi != 0, in.Apx, BnR);
       }
 #pragma unroll
-      for (int w = 0; w < NW; ++w) { jn[w] = psub(BnR[w], Anx[w]); jp[w] = psub(Apx[w], BpL[w]); }
+      for (int w = 0; w < NW; ++w) { jn[w] = psub(BnR[w], in.Anx[w]); jp[w] = psub(in.Apx[w], BpL[w]); }
       jumps<G>(jn, jp, sum, dif);
       add_update<G, 0, T>(kx, sum, dif, du);
 #pragma unroll
-      for (int w = 0; w < NW; ++w) jn[w] = psub(Bn_q[w], Bny[w]);
-      jumps<G>(jn, jpB, sum, dif);
+      for (int w = 0; w < NW; ++w) jn[w] = psub(Bn_q[w], in.Bny[w]);
+      jumps<G>(jn, in.jpB, sum, dif);
       add_update<G, 1, T>(ky, sum, dif, du);
       const P* wo = ring_row(yr) + lane + 1;
 #pragma unroll
       for (int c = 0; c < N; ++c) u[c] = padd(wo[c * MARCH_RW], du[c]);
-      if (col_valid && yr <= it.y1) store_cell<T, G, PL>(pp, mc, fab_idx(pp, 0, x, yr), plane, u, pin);
+      if (col_valid && yr <= it.y1) store_cell<T, G, PL>(sdst, plane, mc, u, pin);
       if (it.ncap && yr <= it.y1)
         march_capture<T, G>(pp, it, mc, yr, lane, cpos, [&](int kind, P* F) {
-          if (kind == 0) face_flux<G, 0, T>(kx, Anx, BpL, F);
-          else if (kind == 1) face_flux<G, 0, T>(kx, BnR, Apx, F);
-          else if (kind == 3) face_flux<G, 1, T>(ky, Bn_q, Bpy, F);
+          if (kind == 0) face_flux<G, 0, T>(kx, in.Anx, BpL, F);
+          else if (kind == 1) face_flux<G, 0, T>(kx, BnR, in.Apx, F);
+          else if (kind == 3) face_flux<G, 1, T>(ky, Bn_q, in.Bpy, F);
           else {
             P below[NW];
 #pragma unroll
-            for (int w = 0; w < NW; ++w) below[w] = psub(Bpy[w], jpB[w]);
-            face_flux<G, 1, T>(ky, Bny, below, F);
+            for (int w = 0; w < NW; ++w) below[w] = psub(in.Bpy[w], in.jpB[w]);
+            face_flux<G, 1, T>(ky, in.Bny, below, F);
           }
         });
     }
+    sdst += anx;
     // advance: the jumps over row q of the values from below (at the domain's
     // y-lo edge those arriving through it; a fault patch's row 0 is finished later)
     if (q == dlo1 && !fault) {
-      edge_value<G>(ky, ky.bgp, mc.yout_lo != 0, An_q, Apy);
-      edge_value<G>(ky, ky.bgp, mc.yout_lo != 0, Bn_q, Bpy);
+      edge_value<G>(ky, ky.bgp, mc.yout_lo != 0, out.Any, in.Apy);
+      edge_value<G>(ky, ky.bgp, mc.yout_lo != 0, Bn_q, in.Bpy);
     }
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
-      jpy[w] = psub(Ap_q[w], Apy[w]);
-      jpB[w] = psub(Bp_q[w], Bpy[w]);
-      Any[w] = An_q[w]; Apy[w] = Ap_q[w]; Bny[w] = Bn_q[w]; Bpy[w] = Bp_q[w];
-      Anx[w] = Anx_q[w]; Apx[w] = Apx_q[w];
+      out.jpy[w] = psub(out.Apy[w], in.Apy[w]);
+      out.jpB[w] = psub(Bp_q[w], in.Bpy[w]);
+      out.Bny[w] = Bn_q[w];
+      out.Bpy[w] = Bp_q[w];
     }
+  };
+  for (int q = q_s;; q += 2) {
+    row_step(q, c0, c1);
+    if (q + 1 > q_e) break;
+    row_step(q + 1, c1, c0);
+    if (q + 2 > q_e) break;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -923,13 +988,15 @@ TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const Ma
     add_update<G, 0, T>(mc.kx, sum, dif, du);
 #pragma unroll
     for (int c = 0; c < N; ++c) u[c] = padd(u[c], pfma(psub(Fy1[c], Fy0[c]), mc.sc, du[c]));
-    const size_t plane = (size_t)pp.anx * pp.any, o = fab_idx(pp, 0, x, dlo1);
+    const unsigned plane = (unsigned)pp.anx * (unsigned)pp.any;
+    const size_t o = fab_idx(pp, 0, x, dlo1);
+    T* const out0 = pp.Uout + o;
     P pin[3];
     if (mc.plastic) {
-      plastic_inputs<T>(pp, o, plane, pin);
-      store_cell<T, G, true>(pp, mc, o, plane, u, pin);
+      plastic_inputs<T>(pp.Uin + o, out0, plane, pin);
+      store_cell<T, G, true>(out0, plane, mc, u, pin);
     } else {
-      store_cell<T, G, false>(pp, mc, o, plane, u, pin);
+      store_cell<T, G, false>(out0, plane, mc, u, pin);
     }
   }
 }
