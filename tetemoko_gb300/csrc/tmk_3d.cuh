@@ -344,7 +344,7 @@ TMK_D double bdry_value(const DevParams& P, const Step3<T>& g, int i, int k, con
   if (P.fault_law == 1) {
     const RSFace fr = rs_face(P, nullptr, 0, 0);
     const double x = (i + 0.5) * g.dx - P.rs_x0;
-    if constexpr (!kExact<T>) return rs_setbnd_k(P, rs_face_k(P, fr, x), U22, Bi, (int)bs, dtp, 0.0, false);
+    if constexpr (!kExact<T>) return rs_setbnd_k(P, rs_face_k(P, fr, false, x, Bi[10 * bs]), U22, Bi, (int)bs, dtp, 0.0, false);
     return rs_setbnd(P, fr, U22, Bi, (int)bs, dtp, x, 0.0, false);
   }
   return sw_setbnd(P, U22, Bi, (int)bs, dtp, 0.0, false);
@@ -363,7 +363,7 @@ TMK_D void fault_face(const DevParams& P, double dx, int i, int k, const double*
   if (P.fault_law == 1) {
     const RSFace fr = rs_face(P, nullptr, 0, 0);
     int it;
-    if constexpr (!kExact<T>) it = rs_fault_k(P, rs_face_k(P, fr, xc - P.rs_x0), Wi, bval, Wg);
+    if constexpr (!kExact<T>) it = rs_fault_k(P, rs_face_k(P, fr, false, xc - P.rs_x0, bval), Wi, bval, Wg);
     else it = rs_fault(P, fr, Wi, bval, xc - P.rs_x0, Wg);
     if (it > RS_IMAX) atomicAdd(&st->newton_maxed, 1ull);
   } else {
@@ -702,7 +702,7 @@ TMK_D void bdry_final_body(const Step3<T>& g, const DevParams& P, DevStatus* st,
     const RSFace fr = rs_face(P, nullptr, 0, 0);
     const double x = (i + 0.5) * g.dx - P.rs_x0;
     double psi;
-    if constexpr (!kExact<T>) psi = rs_setbnd_k(P, rs_face_k(P, fr, x), U22, Bi, bs, g.dt, g.time + g.dt, true);
+    if constexpr (!kExact<T>) psi = rs_setbnd_k(P, rs_face_k(P, fr, false, x, Bi[10 * (long long)bs]), U22, Bi, bs, g.dt, g.time + g.dt, true);
     else psi = rs_setbnd(P, fr, U22, Bi, bs, g.dt, x, g.time + g.dt, true);
     if (isnan(psi)) report(st, ST_NAN, bo);
   } else {

@@ -1200,8 +1200,8 @@ struct tmk_graph_s {
 
 namespace {
 
-// parameter counts of fault_kernel and station_kernel
-constexpr int kFaultParams = 5;
+// parameter counts of fault_kernel, fault_ref9_kernel and station_kernel
+constexpr int kFaultParams = 6, kFaultRef9Params = 5;
 constexpr int kStationParams = 10;
 
 tmk_status graph_finish(tmk_graph_s* g) {
@@ -1212,10 +1212,11 @@ tmk_status graph_finish(tmk_graph_s* g) {
   if (n && cudaGraphGetNodes(g->graph, nodes.data(), &n) != cudaSuccess) return TMK_ERR_CUDA;
   // kernels whose fourth parameter is a time: the fault kernels (the step's
   // start) and the station kernels (the record's time)
-  const void* fe[6] = {tmk::Launch<float>::fault_entry(tmk::FAULT_SEG),
+  const void* fe[8] = {tmk::Launch<float>::fault_entry(tmk::FAULT_SEG),
                        tmk::Launch<float>::fault_entry(tmk::FAULT_SEG_SMALL),
                        tmk::Launch<double>::fault_entry(tmk::FAULT_SEG),
                        tmk::Launch<double>::fault_entry(tmk::FAULT_SEG_SMALL),
+                       tmk::Launch<float>::fault_entry(0), tmk::Launch<double>::fault_entry(0),
                        station_entry(TMK_PREC_MIXED), station_entry(TMK_PREC_FP64)};
   for (cudaGraphNode_t nd : nodes) {
     cudaGraphNodeType t;
@@ -1223,11 +1224,11 @@ tmk_status graph_finish(tmk_graph_s* g) {
     if (t != cudaGraphNodeTypeKernel) continue;
     cudaKernelNodeParams p;
     if (cudaGraphKernelNodeGetParams(nd, &p) != cudaSuccess) return TMK_ERR_CUDA;
-    const int which = (int)(std::find(fe, fe + 6, p.func) - fe);
-    if (which == 6) continue;
+    const int which = (int)(std::find(fe, fe + 8, p.func) - fe);
+    if (which == 8) continue;
     g->tnodes.push_back(nd);
     g->tbase.push_back(*(const double*)p.kernelParams[3]);
-    g->nparams.push_back(which < 4 ? kFaultParams : kStationParams);
+    g->nparams.push_back(which < 4 ? kFaultParams : which < 6 ? kFaultRef9Params : kStationParams);
   }
   return TMK_OK;
 }

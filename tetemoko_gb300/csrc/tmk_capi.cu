@@ -95,6 +95,9 @@ extern "C" tmk_status tmk_context_create(const tmk_elastic_params* e, const tmk_
   P.two_V0 = 2.0 * P.rs_V0; P.inv_2V0 = P.rs_V0 > 0 ? 1.0 / P.two_V0 : 0.0;
   P.ln_2V0 = P.rs_V0 > 0 ? std::log(P.two_V0) : 0.0;
   P.ln_halfZs = P.Zs > 0 ? std::log(0.5 * P.Zs) : 0.0;
+  P.two_inv_Zs = 2.0 / P.Zs; P.half_inv_Zp = 0.5 / P.Zp; P.inv_Zs32 = (float)P.inv_Zs;
+  P.inv_a = 1.0 / P.rs_a; P.inv_b = 1.0 / P.rs_b; P.inv_L = 1.0 / P.rs_L; P.inv_r0 = 1.0 / P.rs_r0;
+  P.inv_ramp_w = 1.0 / P.ramp_w; P.inv_dw = 1.0 / P.sw_dw;
   c->scheme = *s;
   c->nb = s->fault_law == TMK_FAULT_RS ? TMK_RS_NBDRY : (s->fault_law == TMK_FAULT_SW ? TMK_SW_NBDRY : 0);
   if (dalloc(&c->dp, 1) != cudaSuccess || dalloc(&c->dstatus, 1) != cudaSuccess) {
@@ -265,7 +268,8 @@ tmk_status build_march_lists(tmk_level_s* L) {
     int slots = L->prec == TMK_PREC_MIXED ? tmk::Launch<float>::march_slots(gk, fixed)
                                           : tmk::Launch<double>::march_slots(gk, fixed);
     slots *= tu.march_waves[g];
-    if (g == 1) slots = std::max(warps, slots - tu.fault_displace * warps * fault_ctas);
+    // the group the fault kernel runs beside leaves room for its CTAs
+    if (g == (tu.fault_first ? 0 : 1)) slots = std::max(warps, slots - tu.fault_displace * warps * fault_ctas);
     std::vector<tmk::MarchItem> items, frows;
     make_march_items(items, frows, boxes, fault_flags, slots, g == 0 && fault_ctas ? kFaultWaitRows : 0,
                      tu.min_run);
@@ -398,7 +402,8 @@ extern "C" tmk_status tmk_patch_update_state(tmk_context* c, const tmk_fab* U, c
   if (Fy) TMK_CU(cudaMemsetAsync(Fy->data, 0, (size_t)TMK_NCOMP * nvx * (nvy + 1) * sizeof(double), s));
   const PatchDev<double>* dpd = (const PatchDev<double>*)(base + off_pd);
   if (fault)
-    TMK_CU(tmk::Launch<double>::fault(dpd, (const int*)(base + off_fp), 1, nvx, c->dp, time, c->dstatus, false, tmk::FAULT_SEG, s));
+    TMK_CU(tmk::Launch<double>::fault(dpd, (const int*)(base + off_fp), 1, nvx, c->dp, c->hp, dt, dx, time, c->dstatus, false,
+                                        tmk::fault_seg_of(c->hp, tmk::FAULT_SEG), s));
   TMK_CU(tmk::Launch<double>::volume(dpd, (const TileDev*)(base + off_tl), (int)tiles.size(), c->dp, s));
   // the volume kernel writes the nine evolving components of each side;
   // lambda and gamma are left untouched, as updateState leaves them
@@ -534,6 +539,8 @@ tmk_status level_create_impl(tmk_context* const* ctxs, int nscen, const tmk_box*
   if (!L) return TMK_ERR_ALLOC;
   L->ctx = c; L->domain = pdom[0]; L->dx = dx; L->prec = c->scheme.precision;
   L->nscen = nscen;
+  for (int k = 0; k < nscen; ++k)
+    if (tmk::fault_seg_of(ctxs[k]->hp, tmk::FAULT_SEG) == 0) L->sw_ref9 = 1;
   L->dparams = c->dp;
   L->patches.resize(npatch);
   const size_t rs = real_size(L->prec);
@@ -944,11 +951,12 @@ template <typename Real>
 tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEvent_t* ev, cudaStream_t s) {
   tmk_context* c = L->ctx;
   const PatchDev<Real>* pd = (const PatchDev<Real>*)L->dpatch[par];
+  const int seg = L->sw_ref9 ? 0 : L->tune.fault_seg;
   TMK_CU(tmk::Launch<Real>::exchange(pd, L->dcopies, L->ncopies, 0, TMK_NCOMP, s));
   TMK_CU(tmk::bexchange(L->dbptr, L->dblo, L->dbnx, L->dbcopies, L->nbcopies, c->nb, s));
   if (ev) TMK_CU(cudaEventRecord(ev[1], s));
   if (!L->march) {
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, time, c->dstatus, false, L->tune.fault_seg, s));
+    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
     if (ev) TMK_CU(cudaEventRecord(ev[2], s));
     TMK_CU(tmk::Launch<Real>::volume(pd, L->dtiles, L->ntiles, L->dparams, s));
     return TMK_OK;
@@ -976,12 +984,12 @@ tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEve
       }
       TMK_CU(cudaEventRecord(L->fork_ev, s));
       TMK_CU(cudaStreamWaitEvent(L->side, L->fork_ev, 0));
-      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, time, c->dstatus, false,
-                                      L->tune.fault_seg, L->side));
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false,
+                                      seg, L->side));
       TMK_CU(cudaEventRecord(L->join_ev, L->side));
     } else {
-      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, time, c->dstatus, false,
-                                      L->tune.fault_seg, s));
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false,
+                                      seg, s));
       if (ev) TMK_CU(cudaEventRecord(ev[2], s));
     }
     TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, false, s));
@@ -992,17 +1000,17 @@ tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEve
     return TMK_OK;
   }
   if (ev) {
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, time, c->dstatus, false, L->tune.fault_seg, s));
+    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
     TMK_CU(cudaEventRecord(ev[2], s));
     TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
     TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, true, s));
   } else if (L->tune.fault_first && L->nfault) {
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, time, c->dstatus, false, L->tune.fault_seg, s));
+    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
     TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, true, s));
     TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, true, s));
   } else {
     TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, time, c->dstatus, true, L->tune.fault_seg, s));
+    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, true, seg, s));
     TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, true, s));
   }
   TMK_CU(tmk::Launch<Real>::march_fault_rows(pd, L->dfrows[0], L->nfrows[0], L->dfrows[1], L->nfrows[1], mc, s));
@@ -1253,6 +1261,7 @@ extern "C" tmk_status tmk_level_status(tmk_level* L, long long info[3]) {
 namespace tmk {
 struct CtxView {
   const DevParams* dp;
+  const DevParams* hp;
   DevStatus* st;
   int fault_law;
   int nb;
@@ -1260,7 +1269,7 @@ struct CtxView {
 };
 CtxView context_view(const tmk_context* c) {
   CtxView v;
-  v.dp = c->dp; v.st = c->dstatus; v.fault_law = c->scheme.fault_law; v.nb = c->nb;
+  v.dp = c->dp; v.hp = &c->hp; v.st = c->dstatus; v.fault_law = c->scheme.fault_law; v.nb = c->nb;
   v.max_speed = std::max(c->hp.cs, c->hp.cp);
   return v;
 }

@@ -55,6 +55,8 @@ struct DevParams {
   // FP64 operations is the fault kernel's latency; a division costs several)
   double inv_Zs, inv_Zp, lam_r, two_V0, inv_2V0;   // lam_r = lam/(lam+2G)
   double ln_2V0, ln_halfZs;                          // log(2 V0), log(Zs / 2)
+  double two_inv_Zs, half_inv_Zp, inv_a, inv_b, inv_L, inv_r0, inv_ramp_w, inv_dw;
+  float inv_Zs32;
 };
 
 // Constants of one arithmetic type.

@@ -155,199 +155,217 @@ TMK_D double rs_setbnd(const DevParams& P, const RSFace& fr, const double* U, do
   return dPsi;
 }
 
-// ------------------------------------------------ mixed-form rate-and-state
-// The same friction law for the mixed form, arranged for latency: on GB300 a
-// dependent FP64 operation takes ~70 cycles and an FP64 division or
-// transcendental several hundred, so the per-face chain of the two friction
-// solves and boundary updates is the fault kernel's run time.  Here the
-// quantities that depend only on the face (nucleation shear, ramped a, the
-// reciprocals of a, b, L) are computed once per step beside the predictors,
-// divisions by constants become products with reciprocals, reciprocals inside
-// the Newton loop are Newton-Raphson refinements of an FP32 seed, the Newton
-// step uses an FP32 reciprocal of the derivative (the iteration's fixed point
-// is unchanged), and the solve starts from the slip rate of the states it is
-// given.  Everything stays FP64; the results agree with the reference
-// ordering to rounding and are checked by the rupture metrics.
-
-// Reciprocal by two Newton-Raphson refinements r <- r + r (1 - x r) of an FP32
-// seed (x within FP32 range and nonzero).
-TMK_D double recip_nr(double x) {
-  const double r0 = (double)__frcp_rn((float)x);
-  const double r1 = fma(r0, fma(-x, r0, 1.0), r0);
-  return fma(r1, fma(-x, r1, 1.0), r1);
-}
+// ---------------------------------------------- solves on characteristic values
+// The same friction laws arranged for latency: on GB300 an FP64 instruction
+// holds its pipe for 64 cycles a warp (a division is ten of them, exp 17, log
+// 32), so a face's chain of FP64 instructions is the fault kernel's run time.
+// Quantities that depend only on the face (nucleation shear, ramped a, the
+// reciprocals of a, b, L) are computed once beside the predictors, divisions
+// by constants become products with reciprocals, the friction equation is
+// solved for a variable in which Newton converges at once, and logarithms are
+// evaluated only where a short series does not do.
 
 struct RSFaceK {
   double tau0;    // nucleation shear at the face
   double a, inv_a, b, inv_b, inv_L;
   double c_Vw;    // ramped weakening velocity (slip law with fexp > 0)
+  double eq0;     // aging law: e^-(psi - f0)/b at the stored psi
 };
 
-TMK_D RSFaceK rs_face_k(const DevParams& P, const RSFace& fr, double x) {
+// own: the face carries its own a, b, L (else the scenario's, whose reciprocals
+// come from the host)
+TMK_D RSFaceK rs_face_k(const DevParams& P, const RSFace& fr, bool own, double x, double psi) {
   RSFaceK k;
-  k.tau0 = P.rs_nsig * gaussian(P.rs_r0, x);
-  const double c_ramp = fmin(1.0, fmax(0.0, (x - P.ramp_x) / P.ramp_w));
+  const double q = x * P.inv_r0;
+  k.tau0 = P.rs_nsig * exp(-0.5 * (q * q));
+  const double c_ramp = fmin(1.0, fmax(0.0, (x - P.ramp_x) * P.inv_ramp_w));
   k.a = fr.a + P.ramp_a * c_ramp;
-  k.inv_a = 1.0 / k.a;
   k.b = fr.b;
-  k.inv_b = 1.0 / fr.b;
-  k.inv_L = 1.0 / fr.L;
+  k.inv_a = P.inv_a; k.inv_b = P.inv_b; k.inv_L = P.inv_L;
+  if (own) { k.inv_b = 1.0 / fr.b; k.inv_L = 1.0 / fr.L; }
+  if (own || P.ramp_a != 0.0) k.inv_a = 1.0 / k.a;
   k.c_Vw = P.rs_Vw + P.ramp_Vw * c_ramp;
+  k.eq0 = P.state_law == 1 ? exp((P.rs_f0 - psi) * k.inv_b) : 0.0;
   return k;
 }
+
+// State of a fault face: both sides' tangential velocities, the shared normal
+// velocity and tractions, and the slip rate.
+struct FaultFace { double vx1, vx2, vz1, vz2, vy, syy, sxy, syz, Vx, Vz, V; };
 
 // The friction equation of RSNEWTON solved for z = asinh(beta V) instead of V:
 //   f(z) = alpha z + c sinh z - phi = 0,  c = eta / beta,  V = sinh(z)/beta,  tau = alpha z.
 // f is smooth and monotone in z on the same bracket (0, asinh(beta phi/Zs)], so
 // Newton converges in a few steps where the iteration in V creeps up through
-// tens of decades; it starts from the guess V0 when that lies inside the
-// bracket.  As in the reference, a root beyond the bracket's upper end
-// V = phi/Zs yields that end.
+// tens of decades; it starts from the slip rate of the given states.  As in the
+// reference, a root beyond the bracket's upper end V = phi/Zs yields that end;
+// parameters outside the range of this form (a tensile fault, say) and, in the
+// FP64 form, roots that RSNEWTON does not reach (near or beyond the bracket's
+// end, or too far below its start) go to RSNEWTON itself.
 //
-// GB300 issues one FP64 warp instruction per 64 cycles on an SM sub-partition,
-// so the iterations run in FP32 (c e^{+-z} as e^{+-z + ln c}, whose exponent
-// stays below log(phi) inside the bracket), and one FP64 Newton step from the
-// FP32 root finishes the solve: from a start within ~1e-5 of the root the step
-// lands within ~1e-10, far below the FP32 volume arithmetic of the mixed form.
-// V is then the FP64 c sinh z of that step's start advanced to its end to
-// second order.  A step that is not small (an FP32 iteration that did not
-// converge) hands the solve to the FP64 iteration from there.
-TMK_D int rs_newton_zk(const DevParams& P, const RSFaceK& fk, double phi, double psi, double sn, double V0,
-                       double& V, double& tau) {
-  const double atolG = 2.220446049250313e-16 * 1e4;
+// The iterations run in FP32 (c e^{+-z} as e^{+-z + ln c}, whose exponent stays
+// below log(phi) inside the bracket).  The mixed form finishes with one FP64
+// Newton step from the FP32 root: from a start within ~1e-5 of the root it lands
+// within ~1e-10, far below the FP32 volume arithmetic.  The FP64 form (EXACT)
+// repeats it until the step is 1e-13 of z.  Steps are divided by the FP32
+// derivative, which leaves the fixed point as it is; e^-z is dropped past z =
+// 19, where e^-2z is below FP64 resolution; V follows the last step to first
+// order.
+template <bool EXACT, typename T>
+TMK_D int rs_solve_z(const DevParams& P, const RSFaceK& fk, double phi, double psi, double sn, T dvx, T dvz,
+                     double& V, double& tau) {
   const double alpha = sn * fk.a;
   const double lb = psi * fk.inv_a - P.ln_2V0;        // ln beta, beta = e^(psi/a) / (2 V0)
-  const double eta = 0.5 * P.Zs;
-  const double Vmax = phi * P.inv_Zs;
-  if (!(alpha > 0.0) || !(phi > 0.0) || !(lb > -600.0 && lb < 600.0) || !(P.rs_V0 > 0.0))
-    return rs_newton(P, phi, psi, sn, fk.a, V, tau);
   const double lc = P.ln_halfZs - lb;                 // ln c
-  // bracket end z_max = asinh(beta Vmax) (= ln(2 beta Vmax) to FP64 resolution past e^20)
-  const double lbv = lb + log(Vmax);
-  const double zmax = lbv > 20.0 ? 0.6931471805599453 + lbv : asinh(exp(lbv));
-  if (alpha * zmax + eta * Vmax - phi <= 0.0) {      // root beyond the reference's bracket
-    V = Vmax;
-    tau = alpha * zmax;
-    return RS_IMAX + 1;
+  const float a32 = (float)alpha, lb32 = (float)lb, lc32 = (float)lc, phi32 = (float)phi;
+  auto newton = [&]() {
+    V = sqrt((double)dvx * (double)dvx + (double)dvz * (double)dvz);
+    return rs_newton(P, phi, psi, sn, fk.a, V, tau);
+  };
+  if (!(a32 > 0.f) || !(phi32 > 0.f) || !(lb32 > -600.f && lb32 < 600.f) || !(P.rs_V0 > 0.0)) return newton();
+  // bracket end z_max = asinh(beta Vmax) (= ln(2 beta Vmax) past e^20); the
+  // root lies inside where alpha z_max > phi / 2
+  const float vmax32 = phi32 * P.inv_Zs32;
+  const float lbv = lb32 + logf(vmax32);
+  const float zmax = lbv > 20.f ? 0.6931472f + lbv : asinhf(expf(lbv));
+  if (!(a32 * zmax - 0.5f * phi32 > 1e-4f * phi32)) {
+    if (EXACT) return newton();
+    const double Vmax = phi * P.inv_Zs, l = lb + log(Vmax);
+    const double zm = l > 20.0 ? 0.6931471805599453 + l : asinh(exp(l));
+    if (alpha * zm + 0.5 * P.Zs * Vmax - phi <= 0.0) {
+      V = Vmax;
+      tau = alpha * zm;
+      return RS_IMAX + 1;
+    }
   }
-  // FP32 Newton from the guess
-  const float a32 = (float)alpha, lc32 = (float)lc, phi32 = (float)phi, zmax32 = (float)zmax;
-  float z;
-  if (V0 > 0.0 && V0 < Vmax) {
-    const float lg = (float)lb + logf((float)V0);    // ln(beta V0)
-    z = fminf(lg > 9.f ? 0.6931472f + lg : asinhf(expf(lg)), zmax32);
-  } else {
-    z = fminf(phi32 / a32, zmax32);
+  const float v0 = sqrtf((float)dvx * (float)dvx + (float)dvz * (float)dvz);
+  float z = phi32 / a32;
+  if (v0 > 0.f && v0 < vmax32) {
+    const float lg = lb32 + logf(v0);                 // ln(beta V0)
+    z = lg > 9.f ? 0.6931472f + lg : asinhf(expf(lg));
   }
+  z = fminf(z, zmax);
   int it;
   for (it = 1; it <= 30; ++it) {
-    const float ep = expf(z + lc32), em = expf(lc32 - z);
+    const float ep = __expf(z + lc32), em = __expf(lc32 - z);
     const float f = a32 * z + 0.5f * (ep - em) - phi32;
-    const float dz = -f / (a32 + 0.5f * (ep + em));
+    const float dz = __fdividef(-f, a32 + 0.5f * (ep + em));
     float zn = z + dz;
     if (zn < 0.f) zn = 0.5f * z;
-    if (zn > zmax32) zn = 0.5f * (z + zmax32);
+    if (zn > zmax) zn = 0.5f * (z + zmax);
     z = zn;
     if (fabsf(dz) <= 2e-6f * fmaxf(1.f, z)) break;
   }
-  // one FP64 Newton step
-  const double z0 = (double)z;
-  const double ep = exp(z0 + lc), em = exp(lc - z0);  // independent: issued together
-  const double sh = 0.5 * (ep - em), ch = 0.5 * (ep + em);
-  const double f = alpha * z0 + sh - phi;
-  const double dz = -f * recip_nr(alpha + ch);
-  if (fabs(dz) <= 1e-4 * fmax(1.0, z0) && z0 + dz >= 0.0 && z0 + dz <= zmax) {
-    const double z1 = z0 + dz;
-    V = (sh + ch * dz) * (2.0 * P.inv_Zs);            // c sinh(z1) / eta
-    tau = alpha * z1;
-    return it;
+  // RSNEWTON halves its way down from a slip rate far above the root and stops
+  // after RS_IMAX iterations wherever it is: the FP64 form leaves a root more
+  // than 80 halvings below the start to it
+  const float lroot = (z > 1.f ? z - 0.6931472f : logf(fmaxf(z, 1e-30f))) - lb32;       // ln V, within 0.2
+  if (EXACT && logf(v0 > 0.f && v0 <= vmax32 ? v0 : 0.5f * vmax32) - lroot > 55.45f) return newton();
+  double zz = (double)z;
+  for (int k = 0; k < 12; ++k) {
+    const float z32 = (float)zz;
+    const double ep = exp(zz + lc);
+    double sh = 0.5 * ep, ch = sh;
+    if (z32 < 19.f) {
+      const double em = 0.5 * exp(lc - zz);
+      ch = sh + em;
+      sh = sh - em;
+    }
+    const double f = alpha * zz + sh - phi;
+    const float r32 = 1.f / (a32 + (float)ch), d32 = -(float)f * r32;
+    const double dz = -f * (double)r32;
+    const float small = (EXACT || k > 0) ? 1e-13f : 1e-4f;
+    const bool done = fabsf(d32) <= small * fmaxf(1.f, z32) && z32 + d32 >= 0.f && z32 + d32 <= zmax;
+    zz = zz + dz;
+    if (done) {
+      V = (sh + ch * dz) * P.two_inv_Zs;              // c sinh(z) / eta
+      tau = alpha * zz;
+      return it + k;
+    }
+    if (!(zz > 0.0)) zz = 0.5 * (double)z32;
+    if (zz > (double)zmax) zz = 0.5 * ((double)z32 + (double)zmax);
   }
-  // the FP64 iteration from the FP32 result
-  const double c = exp(lc);
-  double zz = fmin(fmax(z0 + dz, 0.0), zmax);
-  int jt;
-  for (jt = 1; jt <= RS_IMAX; ++jt) {
-    const double e = exp(zz), ie = zz > 20.0 ? 0.0 : recip_nr(e);   // e^-2z below FP64 resolution past 20
-    const double f2 = alpha * zz + c * 0.5 * (e - ie) - phi;
-    const double d2 = -f2 * (double)__frcp_rn((float)(alpha + c * 0.5 * (e + ie)));
-    double zn = zz + d2;
-    if (zn < 0.0) zn = 0.5 * zz;
-    if (zn > zmax) zn = 0.5 * (zz + zmax);
-    zz = zn;
-    if (fabs(f2) <= atolG || fabs(d2) <= 1e-15 * fmax(1.0, zz)) break;
-  }
-  const double e = exp(zz + lc), ie = exp(lc - zz);
-  V = 0.5 * (e - ie) * (2.0 * P.inv_Zs);
-  tau = alpha * zz;
-  return it + jt;
+  return newton();
 }
 
-// RSFAULTBCF for the mixed form (same states in, same face states out).
-TMK_D int rs_fault_k(const DevParams& P, const RSFaceK& fk, const double* Wi, double psi, double* Wg) {
-  const double Zs = P.Zs, Zp = P.Zp;
-  double vx1 = Wi[0], vy1 = Wi[1], vz1 = Wi[2], sxx1 = Wi[3], syy1 = Wi[4], szz1 = Wi[5];
-  double sxy1 = Wi[6], sxz1 = Wi[7], syz1 = Wi[8];
-  double vx2 = Wi[11], vy2 = Wi[12], vz2 = Wi[13], sxx2 = Wi[14], syy2 = Wi[15], szz2 = Wi[16];
-  double sxy2 = Wi[17], sxz2 = Wi[18], syz2 = Wi[19];
-  const double wpxy1 = -sxy1 - Zs * vx1, wpyy1 = -syy1 - Zp * vy1;
-  const double wpxy2 = sxy2 - Zs * vx2, wpyy2 = syy2 - Zp * vy2;
-  const double phi_xy = 0.5 * (wpxy2 - wpxy1) + fk.tau0;
-  const double phi = fabs(phi_xy);      // the antiplane traction term is zero in 2-D
-  syy1 = -0.5 * (wpyy1 - wpyy2);
-  syy2 = syy1;
-  vy1 = -0.5 * (wpyy1 + wpyy2) * P.inv_Zp;
-  vy2 = vy1;
-  const double dvx = vx1 - vx2, dvz = vz1 - vz2;
-  double V = sqrt(dvx * dvx + dvz * dvz), tau;
-  const int it = rs_newton_zk(P, fk, phi, psi, -syy1, V, V, tau);
+// RSFAULTBCF (ibcLinElast/RSIBCF.ChF:158-323) from the values the fault sees of
+// the two sides' states: the left-going characteristic values of the P pair
+// (aP = syy + Zp rv vy) and of the S pair (aS = sxy + Zs rv vx), rv = +1, -1.
+// The antiplane traction term is zero in the law.  dvx, dvz: the states'
+// velocity differences (the first guess).  Returns the iterations used.
+template <bool EXACT, typename T>
+TMK_D int rs_face_solve(const DevParams& P, const RSFaceK& fk, double aP1, double aP2, double aS1, double aS2,
+                        double psi, T dvx, T dvz, FaultFace& f) {
+  const double phi_xy = 0.5 * (aS1 + aS2) + fk.tau0;
+  const double phi = fabs(phi_xy);
+  f.syy = 0.5 * (aP1 + aP2);
+  f.vy = (aP1 - aP2) * P.half_inv_Zp;
+  double V, tau;
+  const int it = rs_solve_z<EXACT>(P, fk, phi, psi, -f.syy, dvx, dvz, V, tau);
   // phi_xy / phi: +-1, NaN when phi is zero or NaN (as the reference's quotient)
   const double sgn = phi > 0.0 ? copysign(1.0, phi_xy) : __longlong_as_double(0x7ff8000000000000ll);
-  sxy1 = sgn * tau - fk.tau0;
-  syz1 = 0.0 * tau;                     // (phi_yz / phi) tau - tau_yz_0 with phi_yz = tau_yz_0 = 0
-  const double Vx = sgn * V, Vz = 0.0 * V;
-  vx1 = -(sxy1 + wpxy1) * P.inv_Zs;
-  vz1 = -(syz1 + 0.0) * P.inv_Zs;
-  double SHF = -(vy1 - syy1) * P.lam_r;
-  Wg[0] = vx1; Wg[1] = vy1; Wg[2] = vz1;
-  Wg[3] = sxx1 + SHF; Wg[4] = syy1; Wg[5] = szz1 + SHF;
-  Wg[6] = sxy1; Wg[7] = sxz1; Wg[8] = syz1;
-  Wg[9] = 0.0; Wg[10] = 0.0;
-  sxy2 = sxy1;
-  syz2 = syz1;
-  vx2 = vx1 - Vx;
-  vz2 = vz1 - Vz;
-  SHF = -(vy2 - syy2) * P.lam_r;
-  Wg[11] = vx2; Wg[12] = vy2; Wg[13] = vz2;
-  Wg[14] = sxx2 + SHF; Wg[15] = syy2; Wg[16] = szz2 + SHF;
-  Wg[17] = sxy2; Wg[18] = sxz2; Wg[19] = syz2;
-  Wg[20] = 0.0; Wg[21] = 0.0;
-  (void)syz2;
+  f.sxy = sgn * tau - fk.tau0;
+  f.syz = 0.0 * tau;                    // (phi_yz / phi) tau - tau_yz_0 with phi_yz = tau_yz_0 = 0
+  f.V = V;
+  f.Vx = sgn * V;
+  f.Vz = 0.0 * V;
+  f.vx1 = (aS1 - f.sxy) * P.inv_Zs;
+  f.vx2 = f.vx1 - f.Vx;
+  f.vz1 = -f.syz;
+  f.vz2 = f.vz1 - f.Vz;
   return it;
 }
 
-// RSSETBND for the mixed form (see rs_setbnd).
+// The state variable of RSSETBND (ibcLinElast/RSIBCF.ChF:61-151) after dt at
+// slip rate V: the reference's slip law, or the aging law at constant V,
+// theta' = theta e^-x + dt (1 - e^-x)/x with x = V dt / L, that is
+// psi' = psi - b x + b log(1 + r), r = (V0 dt / L) (e^x - 1)/x e^-(psi - f0)/b.
+TMK_D double rs_state_next(const DevParams& P, const RSFaceK& fk, double psi, double V, double dt) {
+  if (P.state_law == 1) {
+    const double dl = dt * fk.inv_L, x = V * dl, c = P.rs_V0 * dl;
+    double g;           // (e^x - 1)/x; the next term of the series is x^7 / 40320
+    if (x < 0.01)
+      g = 1.0 + x * (0.5 + x * (1.0 / 6.0 + x * (1.0 / 24.0 + x * (1.0 / 120.0 + x * (1.0 / 720.0 + x * (1.0 / 5040.0))))));
+    else
+      g = expm1(x) / x;
+    const double r = c * g * fk.eq0;
+    double l;           // log(1 + r); the next term of the series is r^7 / 7
+    if (r < 1e-3) {
+      l = r * (1.0 + r * (-0.5 + r * (1.0 / 3.0 + r * (-0.25 + r * (0.2 + r * (-1.0 / 6.0))))));
+    } else if (r < 1e300) {
+      l = log1p(r);
+    } else {            // out of range (or NaN): the sum itself
+      const double phi1 = -expm1(-x) / x;
+      return P.rs_f0 + fk.b * log(exp((psi - P.rs_f0) * fk.inv_b - x) + c * phi1);
+    }
+    return psi + fk.b * (l - x);
+  }
+  const double f = fk.a * asinh(V * exp(psi * fk.inv_a) * P.inv_2V0);
+  double fss = P.rs_f0 - (fk.b - fk.a) * log(V / P.rs_V0);
+  if (P.rs_fexp > 0.0) {
+    const double q = V / fk.c_Vw, q2 = q * q, q4 = q2 * q2, q8 = q4 * q4;
+    fss = P.rs_fw + (fss - P.rs_fw) / pow(1.0 + q8, 0.125);
+  }
+  return psi - dt * (V * fk.inv_L) * (f - fss);
+}
+
+// The 3-D mixed form's fault face (22-component states): RSFAULTBCF and
+// RSSETBND on the solves above.  The components that no flux, transverse term
+// or boundary value reads are left as the caller set them.
+TMK_D int rs_fault_k(const DevParams& P, const RSFaceK& fk, const double* Wi, double psi, double* Wg) {
+  FaultFace f;
+  const int it = rs_face_solve<false>(P, fk, Wi[4] + P.Zp * Wi[1], Wi[15] - P.Zp * Wi[12], Wi[6] + P.Zs * Wi[0],
+                                      Wi[17] - P.Zs * Wi[11], psi, Wi[0] - Wi[11], Wi[2] - Wi[13], f);
+  Wg[0] = f.vx1; Wg[1] = f.vy; Wg[2] = f.vz1; Wg[4] = f.syy; Wg[6] = f.sxy; Wg[8] = f.syz;
+  Wg[11] = f.vx2; Wg[12] = f.vy; Wg[13] = f.vz2; Wg[15] = f.syy; Wg[17] = f.sxy; Wg[19] = f.syz;
+  return it;
+}
 TMK_D double rs_setbnd_k(const DevParams& P, const RSFaceK& fk, const double* U, double* B, int bstride, double dt,
                          double time, bool final_) {
   const double Vx = U[0] - U[11];
   const double Vz = U[2] - U[13];
   const double V = sqrt(Vx * Vx + Vz * Vz);
-  const double psi = B[10 * bstride];
-  double dPsi;
-  if (P.state_law == 1) {
-    const double xx = V * dt * fk.inv_L;
-    const double q = (psi - P.rs_f0) * fk.inv_b - xx;
-    const double eq = exp(q), em1 = expm1(-xx);          // independent: issued together
-    const double phi1 = (xx > 1e-12) ? -em1 / xx : 1.0 - 0.5 * xx;
-    dPsi = P.rs_f0 + fk.b * log(eq + (P.rs_V0 * dt * fk.inv_L) * phi1);
-  } else {
-    const double f = fk.a * asinh(V * exp(psi * fk.inv_a) * P.inv_2V0);
-    double fss = P.rs_f0 - (fk.b - fk.a) * log(V / P.rs_V0);
-    if (P.rs_fexp > 0.0) {
-      const double q = V / fk.c_Vw, q2 = q * q, q4 = q2 * q2, q8 = q4 * q4;
-      fss = P.rs_fw + (fss - P.rs_fw) / pow(1.0 + q8, 0.125);
-    }
-    dPsi = psi - dt * (V * fk.inv_L) * (f - fss);
-  }
+  const double dPsi = rs_state_next(P, fk, B[10 * bstride], V, dt);
   if (final_) {
     const double rt = B[9 * bstride];
     B[0] = Vx;
@@ -366,17 +384,38 @@ TMK_D double rs_setbnd_k(const DevParams& P, const RSFaceK& fk, const double* U,
   return dPsi;
 }
 
-// Out-of-line copies of the mixed-form solve and boundary update for a kernel
-// that calls each twice (first pass and final): one copy of their code instead
-// of one per call site.  The fault kernel runs few warps per SM along long
-// chains of dependent FP64 operations, where instruction fetch stalls show.
-static __device__ __noinline__ int rs_fault_k_ool(const DevParams& P, const RSFaceK& fk, const double* Wi,
-                                                  double psi, double* Wg) {
-  return rs_fault_k(P, fk, Wi, psi, Wg);
+// Slip weakening on characteristic values (side 2 at component 11, the
+// corrected layout): the quantities of one face, and SWFAULTBCF
+// (ibcLinElast/SWIBCF.ChF:79-267) as rs_face_solve.  az: the values of the
+// antiplane S pair (syz + Zs rv vz).
+struct SWFaceK { double tau0, mu_s; };
+TMK_D SWFaceK sw_face_k(const DevParams& P, double xcell) {
+  const double x = xcell - P.sw_fbc0;
+  SWFaceK k;
+  k.tau0 = 0.0;
+  for (int ip = 0; ip < P.sw_np; ++ip)
+    k.tau0 = k.tau0 + P.sw_tau[ip] * smoothfn(P.sw_smooth, fabs(x - P.sw_xc[ip]) - P.sw_xw[ip]);
+  const double valx = boxcar(P.sw_fbw0, fabs(x));
+  k.mu_s = P.sw_fs * valx + (1 - valx) * P.sw_outside;
+  return k;
 }
-static __device__ __noinline__ double rs_setbnd_k_ool(const DevParams& P, const RSFaceK& fk, const double* U,
-                                                      double* B, int bstride, double dt, double time, bool final_) {
-  return rs_setbnd_k(P, fk, U, B, bstride, dt, time, final_);
+TMK_D void sw_face_solve(const DevParams& P, const SWFaceK& k, double aP1, double aP2, double aS1, double aS2,
+                         double az1, double az2, double slip, FaultFace& f) {
+  const double fx = 0.5 * (aS1 + aS2), fz = 0.5 * (az1 + az2), a1 = fx + k.tau0;
+  f.syy = 0.5 * (aP1 + aP2);
+  f.vy = (aP1 - aP2) * P.half_inv_Zp;
+  const double mu = k.mu_s - (k.mu_s - P.sw_fd) * fmin(1.0, slip * P.inv_dw);
+  const double tau = fmin(sqrt(a1 * a1 + fz * fz), -f.syy * mu) - k.tau0;
+  const double q = tau * rsqrt(fx * fx + fz * fz);
+  f.sxy = fx * q;
+  f.syz = fz * q;
+  f.vx1 = (aS1 - f.sxy) * P.inv_Zs;
+  f.vz1 = (az1 - f.syz) * P.inv_Zs;
+  f.vx2 = (f.sxy - aS2) * P.inv_Zs;
+  f.vz2 = (f.syz - az2) * P.inv_Zs;
+  f.Vx = f.vx1 - f.vx2;
+  f.Vz = f.vz1 - f.vz2;
+  f.V = sqrt(f.Vx * f.Vx + f.Vz * f.Vz);
 }
 
 // SWFAULTBCF (ibcLinElast/SWIBCF.ChF:79-267) at one fault face.  Side 2 is read

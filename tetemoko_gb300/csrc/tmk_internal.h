@@ -96,6 +96,7 @@ struct tmk_level_s {
   tmk::TileDev* dtiles = nullptr;
   int ntiles = 0;
   int march = 0;                           // column-marching volume kernel
+  int sw_ref9 = 0;                         // a scenario runs slip weakening in the reference layout
   int march_allowed = 0;                   // the scheme selects it (captures force the tile kernel)
   tmk::MarchItem* ditems[2] = {nullptr, nullptr};   // work lists of the in-plane / antiplane kernels
   int nitems[2] = {0, 0};

@@ -1,13 +1,8 @@
 // tmk_kernels.cuh -- the device kernels of one level step, templated on the
 // volume arithmetic type Real (double: plain FP64 form; float: mixed form).
 //
-//   fault_kernel   one thread per fault face (a warp per 32-face segment):
-//                  predicts the two states that meet at the fault (rows 0-2 of
-//                  the patch), runs the first-pass friction solve, the
-//                  half-step state predictor, the transverse-corrected final
-//                  solve and the boundary-data update, all friction work in FP64
-//                  (LinElastPatchGodunov::computeWHalf call order,
-//                  srcLinElast/LinElastPatchGodunov.cpp:289-452).
+//   fault_ref9_kernel  the fault row of the reference-layout slip-weakening law
+//                  (the other laws: tmk_fault_kernel.cuh)
 //   volume_kernel  one CTA per (tile, side): PPM normal predictors in x and y,
 //                  first-pass Riemann, transverse corrections, final Riemann,
 //                  fluxes and the conservative update (and, with plasticity,
@@ -68,21 +63,13 @@ TMK_D void make_sig(const DevParams& P, double dtbydx, T* sig) {
   for (int c = 0; c < 9; ++c) sig[c] = (T)(l[c] * dtbydx);
 }
 
-// =============================================================== fault kernel
+// ======================================== fault row, reference SW layout
 // Predicted state of one side's 11 components at (i, j0) in y, in arithmetic T
 // (lambda, gamma carry only their limited PPM delta: zero characteristic speed).
-// `tr` (the tracing coefficients A then B of ppm_predict_prim, mixed form with
-// PPM and primitive limiting) selects the branch-free predictor.
-template <int D, typename T>
-TMK_D void fault_pred(const DevParams& P, const Consts<T>& k, T rv, const T (*w5)[5], const bool* in, const T* sig,
-                      const T* tr, T* WM, T* WP) {
-  if (tr) ppm_predict_prim<D, T>(k, rv, w5, in, tr, tr + NSIDE, WM, WP);
-  else ppm_predict<D, T>(k, rv, w5, in, P.prim_lim != 0, P.char_lim != 0, sig, WM, WP, P.order, P.fourth != 0);
-}
 
 template <typename Real, typename T>
 TMK_D void fault_ypred_side(const PatchDev<Real>& p, const DevParams& P, const Consts<T>& k, int s, int i,
-                            const T* sig, const T* tr, bool lim, double* out11) {
+                            const T* sig, bool lim, double* out11) {
   const int j0 = p.dlo1;
   bool in[5] = {false, false, true, j0 + 1 <= p.dhi1, j0 + 2 <= p.dhi1};
   T w5[NSIDE][5];
@@ -90,7 +77,7 @@ TMK_D void fault_ypred_side(const PatchDev<Real>& p, const DevParams& P, const C
     for (int m = 0; m < 5; ++m) w5[c][m] = in[m] ? (T)p.Uin[fab_idx(p, 11 * s + c, i, j0 - 2 + m)] : T(0);
   T WM[NSIDE], WP[NSIDE];
   T rv = (s == 1) ? T(-1) : T(1);
-  fault_pred<1, T>(P, k, rv, w5, in, sig, tr, WM, WP);
+  ppm_predict<1, T>(k, rv, w5, in, P.prim_lim != 0, P.char_lim != 0, sig, WM, WP, P.order, P.fourth != 0);
   // the zero-speed components of the y direction reach no face component that
   // is read downstream (live9): not predicted
   for (int c = 0; c < NSIDE; ++c) out11[c] = live9<1>(c) ? (double)WM[c] : 0.0;
@@ -118,14 +105,14 @@ TMK_D void fault_ypred_side(const PatchDev<Real>& p, const DevParams& P, const C
 // x-direction predicted states (WM, WP) of one side at cell (i, j0)
 template <typename Real, typename T>
 TMK_D void fault_xpred_side(const PatchDev<Real>& p, const DevParams& P, const Consts<T>& k, int s, int i,
-                            const T* sig, const T* tr, T* WM, T* WP) {
+                            const T* sig, T* WM, T* WP) {
   const int j0 = p.dlo1;
   bool in[5];
   for (int m = 0; m < 5; ++m) in[m] = (i - 2 + m >= p.dlo0) && (i - 2 + m <= p.dhi0);
   T w5[NSIDE][5];
   for (int c = 0; c < NSIDE; ++c)
     for (int m = 0; m < 5; ++m) w5[c][m] = in[m] ? (T)p.Uin[fab_idx(p, 11 * s + c, i - 2 + m, j0)] : T(0);
-  fault_pred<0, T>(P, k, T(1), w5, in, sig, tr, WM, WP);
+  ppm_predict<0, T>(k, T(1), w5, in, P.prim_lim != 0, P.char_lim != 0, sig, WM, WP, P.order, P.fourth != 0);
 }
 
 // x face state (first pass) of one side at face f of row j0 from the cells
@@ -138,39 +125,28 @@ TMK_D void xface_state(const DevParams& P, const Consts<T>& k, int f, int dlo0, 
   else riemann<0, T>(k, T(1), WPl, WMr, g);
 }
 
-// One CTA of NT threads per segment of SEG fault faces of a fault patch.  The
-// predictors of the fault row are computed once per cell and side, in
-// parallel, into shared memory; one thread per face then runs the friction
-// solves, whose Newton iterations are sequential by nature.  Two variants:
-// 32 faces on 4 warps (the default) and 16 faces on 2 warps (twice the CTAs
-// for short fault rows); the level's tuning picks one.
-constexpr int FAULT_SEG = 32;
-constexpr int FAULT_THREADS = 128;
-constexpr int FAULT_SEG_SMALL = 16;
-constexpr int FAULT_THREADS_SMALL = 64;
+// The fault row under the slip-weakening law in the reference's own layout
+// (side 2 read and written at component 9, so that lambda and gamma of side 1
+// and shifted components of side 2 enter the law): the whole 11-component
+// states, in the call order of fault_kernel (tmk_fault_kernel.cuh), which
+// solves the other laws on characteristic values.  One CTA of NT threads per
+// SEG faces: the predictors once per cell and side into shared memory, then
+// one thread per face.
+constexpr int REF9_SEG = 32, REF9_THREADS = 128;
 
-template <typename Real, int SEG, int NT>
-__global__ void __launch_bounds__(NT) fault_kernel(const PatchDev<Real>* __restrict__ patches,
-                                                   const int* __restrict__ fault_patches,
-                                                   const DevParams* __restrict__ params, double time,
-                                                   DevStatus* st) {
-  static_assert(NT > SEG + 2, "the x-face threads need the threads beyond the face threads");
+template <typename Real>
+__global__ void __launch_bounds__(REF9_THREADS) fault_ref9_kernel(const PatchDev<Real>* __restrict__ patches,
+                                                                  const int* __restrict__ fault_patches,
+                                                                  const DevParams* __restrict__ params, double time,
+                                                                  DevStatus* st) {
   using T = Real;
-  // the mixed form runs the latency-arranged rate-and-state path (per-face
-  // constants, z = asinh(beta V) Newton solve); the FP64 form keeps the
-  // reference's operation order and Newton iteration on V
-  constexpr bool kZSolve = !std::is_same<Real, double>::value;
+  constexpr int SEG = REF9_SEG, NT = REF9_THREADS;
+  static_assert(NT > SEG + 2, "the x-face threads need the threads beyond the face threads");
   constexpr int NCELL = SEG + 2;             // cells / faces [s0-1, s0+SEG]
   __shared__ T xWM[2][NCELL][NSIDE], xWP[2][NCELL][NSIDE];
   __shared__ T H1x[2][SEG + 1][NSIDE];
   __shared__ double sWi[NCELL][NC];
   __shared__ double sTmp[NCELL];
-  __shared__ RSFaceK sFk[kZSolve ? NCELL : 1];   // mixed form: per-face rate-and-state constants
-  // the kernel launched after this one may be scheduled now (it reads none of
-  // this kernel's outputs before it waits for it).  When this kernel itself is
-  // a programmatic dependent of the in-plane marching kernel, it reads nothing
-  // that kernel writes (the state it reads is the step's input buffer) and it
-  // waits for it before exiting, so that the step's kernels complete in order.
   asm volatile("griddepcontrol.launch_dependents;");
   const PatchDev<Real> p = patches[fault_patches[blockIdx.y]];
   const DevParams& P = params[p.scen];
@@ -180,94 +156,52 @@ __global__ void __launch_bounds__(NT) fault_kernel(const PatchDev<Real>* __restr
     return;
   }
   const int s1 = min(s0 + SEG - 1, p.vhi0);
-  // faces whose first-pass state this segment produces: its own, plus the
-  // ghost faces lo-1 / hi+1 of the patch for the first / last segment
   const int fa = (s0 == p.vlo0) ? max(p.vlo0 - 1, p.dlo0) : s0;
   const int fb = (s1 == p.vhi0) ? min(p.vhi0 + 1, p.dhi0) : s1;
   const int tid = threadIdx.x;
   const double dt = p.dt, dx = p.dx;
-  // the constants once per CTA: computed per thread they were hundreds of FP64
-  // divisions and products queued on GB300's narrow FP64 pipe before any face
-  // could start
   __shared__ Consts<T> sk;
   __shared__ Consts<double> skd;
   __shared__ T ssig[9];
-  __shared__ T str[2 * NSIDE];     // tracing coefficients of the branch-free predictor
-  const bool fastpred = !kExact<T> && P.order == 2 && P.prim_lim && !P.char_lim;
   if (tid == 0) {
     sk.load(P);
     skd.load(P);
     make_sig(P, dt / dx, ssig);
-    if (fastpred)
-      for (int q = 0; q < NSIDE; ++q) {
-        const double sv = fabs((double)ssig[q]);
-        str[q] = (T)(0.5 * sv);
-        str[NSIDE + q] = (T)(q < 3 ? 3.0 * (0.5 * sv - sv * sv / 3.0) : 1.5 * sv * (1.0 - (2.0 / 3.0) * sv));
-      }
   }
   __syncthreads();
   const Consts<T>& k = sk;
-  const T* sig = ssig;
-  const T* tr = fastpred ? str : nullptr;
   const bool lim = P.prim_lim || P.char_lim;
   const int bs = p.bnx;
-
   // (A) x predictors of the fault-row cells [s0-1, s1+1] and y predictors of the
-  //     states entering the fault faces [fa, fb], both sides; in the mixed form
-  //     also the constants of each face
-  if constexpr (kZSolve) {
-    if (P.fault_law == 1 && tid >= NT - NCELL) {
-      const int ci = tid - (NT - NCELL), i = s0 - 1 + ci;
-      if (i >= fa && i <= fb) sFk[ci] = rs_face_k(P, rs_face(P, p.fric, i - p.blo0, bs), (i + 0.5) * dx - P.rs_x0);
-    }
-  }
+  //     states entering the fault faces [fa, fb], both sides
   for (int t = tid; t < 4 * NCELL; t += NT) {
     const int kind = t / (2 * NCELL), s = (t / NCELL) & 1, ci = t % NCELL;
     const int c = s0 - 1 + ci;
     if (kind == 0) {
       if (c >= p.dlo0 && c <= p.dhi0 && c <= s1 + 1) {
         T WM[NSIDE], WP[NSIDE];
-        fault_xpred_side(p, P, k, s, c, sig, tr, WM, WP);
-        // the x faces' zero-speed components are never read (live9): not predicted
+        fault_xpred_side(p, P, k, s, c, ssig, WM, WP);
         for (int q = 0; q < NSIDE; ++q) {
           xWM[s][ci][q] = live9<0>(q) ? WM[q] : T(0);
           xWP[s][ci][q] = live9<0>(q) ? WP[q] : T(0);
         }
       }
     } else if (c >= fa && c <= fb) {
-      fault_ypred_side(p, P, k, s, c, sig, tr, lim, &sWi[ci][11 * s]);
+      fault_ypred_side(p, P, k, s, c, ssig, lim, &sWi[ci][11 * s]);
     }
   }
   __syncthreads();
-
   if (tid < NCELL) {
-    // (B) first-pass friction solve with the persistent boundary data, and the
-    //     half-step predicted boundary data (updateBoundary, final=false)
+    // (B) first-pass solve and the half-step predicted slip
     const int i = s0 - 1 + tid;
     if (i >= fa && i <= fb) {
       double* Bi = p.B + (i - p.blo0);
-      const double xc = (i + 0.5) * dx;
       double Wg[NC];
       for (int c = 0; c < NC; ++c) Wg[c] = 0.0;
-      int it = 0;
-      const RSFace fr = rs_face(P, p.fric, i - p.blo0, bs);
-      if (P.fault_law == 1) {
-        if constexpr (kZSolve) it = rs_fault_k_ool(P, sFk[tid], sWi[tid], Bi[10 * bs], Wg);
-        else it = rs_fault(P, fr, sWi[tid], Bi[10 * bs], xc - P.rs_x0, Wg);
-      } else {
-        sw_fault(P, sWi[tid], Bi[7 * bs], xc, Wg);
-      }
-      if (it > RS_IMAX) atomicAdd(&st->newton_maxed, 1ull);
+      sw_fault(P, sWi[tid], Bi[7 * bs], (i + 0.5) * dx, Wg);
       double* first = p.first + (i - (p.vlo0 - 1));
       for (int c = 0; c < NC; ++c) first[c * p.nfirst] = Wg[c];
-      if (i >= s0 && i <= s1) {
-        if (P.fault_law == 1) {
-          if constexpr (kZSolve) sTmp[tid] = rs_setbnd_k_ool(P, sFk[tid], Wg, Bi, bs, 0.5 * dt, 0.0, false);
-          else sTmp[tid] = rs_setbnd(P, fr, Wg, Bi, bs, 0.5 * dt, xc - P.rs_x0, 0.0, false);
-        } else {
-          sTmp[tid] = sw_setbnd(P, Wg, Bi, bs, 0.5 * dt, 0.0, false);
-        }
-      }
+      if (i >= s0 && i <= s1) sTmp[tid] = sw_setbnd(P, Wg, Bi, bs, 0.5 * dt, 0.0, false);
     }
   } else {
     // (C) first-pass x faces [s0, s1+1] of the fault row, both sides
@@ -284,11 +218,9 @@ __global__ void __launch_bounds__(NT) fault_kernel(const PatchDev<Real>* __restr
     }
   }
   __syncthreads();
-
   if (tid <= s1 - s0) {
     const int i = s0 + tid, ci = tid + 1;
     double* Bi = p.B + (i - p.blo0);
-    const double xc = (i + 0.5) * dx;
     // (D) transverse correction of the fault states by the x fluxes of the row
     const double scale = -(1.0 / 2.0) * dt / dx;
     double Wi[NC];
@@ -299,36 +231,19 @@ __global__ void __launch_bounds__(NT) fault_kernel(const PatchDev<Real>* __restr
       adwdx_add<0, T>(k, T(1), (T)scale, H1x[s][tid + 1], H1x[s][tid], q);
       for (int c = 0; c < NSIDE; ++c) Wi[11 * s + c] = (double)q[c];
     }
-    // (E) final friction solve with the predicted boundary data
+    // (E) final solve with the predicted slip, (F) y fluxes through the fault
+    //     face (GETFLUXF, FP64), (G) boundary data (final, t+dt)
     double Wg[NC];
     for (int c = 0; c < NC; ++c) Wg[c] = 0.0;
-    int it = 0;
-    const RSFace fr = rs_face(P, p.fric, i - p.blo0, bs);
-    if (P.fault_law == 1) {
-      if constexpr (kZSolve) it = rs_fault_k_ool(P, sFk[ci], Wi, sTmp[ci], Wg);
-      else it = rs_fault(P, fr, Wi, sTmp[ci], xc - P.rs_x0, Wg);
-    } else {
-      sw_fault(P, Wi, sTmp[ci], xc, Wg);
-    }
-    if (it > RS_IMAX) atomicAdd(&st->newton_maxed, 1ull);
-    // (F) y fluxes through the fault face (GETFLUXF, FP64)
-    const Consts<double>& kd = skd;
+    sw_fault(P, Wi, sTmp[ci], (i + 0.5) * dx, Wg);
     double F[NSIDE];
     double* ff = p.ffault + (i - p.vlo0);
     const int nv = p.vhi0 - p.vlo0 + 1;
-    flux<1, double>(kd, 1.0, Wg, F);
+    flux<1, double>(skd, 1.0, Wg, F);
     for (int c = 0; c < NSIDE; ++c) ff[c * nv] = F[c];
-    flux<1, double>(kd, -1.0, Wg + 11, F);
+    flux<1, double>(skd, -1.0, Wg + 11, F);
     for (int c = 0; c < NSIDE; ++c) ff[(11 + c) * nv] = F[c];
-    // (G) boundary-data update with the final fault state (final=true, t+dt)
-    if (P.fault_law == 1) {
-      double np;
-      if constexpr (kZSolve) np = rs_setbnd_k_ool(P, sFk[ci], Wg, Bi, bs, dt, time + dt, true);
-      else np = rs_setbnd(P, fr, Wg, Bi, bs, dt, xc - P.rs_x0, time + dt, true);
-      if (isnan(np)) report(st, ST_NAN, (long long)i);
-    } else {
-      sw_setbnd(P, Wg, Bi, bs, dt, time + dt, true);
-    }
+    sw_setbnd(P, Wg, Bi, bs, dt, time + dt, true);
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -13,14 +13,24 @@ struct TileDev;
 struct CopyDev;
 struct MarchItem;
 
+// faces per CTA of the fault kernel: the default, and the variant for short
+// fault rows (twice the CTAs)
+constexpr int FAULT_SEG = 32;
+constexpr int FAULT_SEG_SMALL = 16;
+// seg, or 0 where slip weakening runs in the reference's layout (side 2 at
+// component 9), which needs whole states
+inline int fault_seg_of(const DevParams& p, int seg) { return p.fault_law == 2 && p.sw_off != 11 ? 0 : seg; }
+
 template <typename Real>
 struct Launch {
   static const int TX, TY;
   // one thread per fault face of every fault patch, seg faces per CTA (32 or
-  // 16); pdl as for march
+  // 16; 0: the reference-layout slip-weakening kernel, which takes either
+  // layout, scenario by scenario); hp: the level's parameters on the host (the launch constants are
+  // built from them); pdl as for march
   static cudaError_t fault(const PatchDev<Real>* patches, const int* fault_patches, int nfault, int max_faces,
-                           const DevParams* params, double time, DevStatus* st, bool pdl, int seg,
-                           cudaStream_t s);
+                           const DevParams* params, const DevParams& hp, double dt, double dx, double time,
+                           DevStatus* st, bool pdl, int seg, cudaStream_t s);
   // one CTA per (tile, side)
   static cudaError_t volume(const PatchDev<Real>* patches, const TileDev* tiles, int ntiles,
                             const DevParams* params, cudaStream_t s);
@@ -51,8 +61,9 @@ struct Launch {
   static int march_slots(int g, bool fixed);
   // warps per CTA of the marching kernels
   static int march_warps();
-  // the entry of the fault kernel variant with seg faces per CTA (to find its
-  // nodes in a captured graph); its fourth parameter is the step's start time
+  // the entry of the fault kernel variant with seg faces per CTA, or (0) of the
+  // reference-layout slip-weakening one (to find its nodes in a captured
+  // graph); its fourth parameter is the step's start time
   static const void* fault_entry(int seg);
 };
 

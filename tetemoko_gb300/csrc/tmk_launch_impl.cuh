@@ -3,6 +3,7 @@
 #pragma once
 #include "tmk_kernels.cuh"
 #include "tmk_march.cuh"
+#include "tmk_fault_kernel.cuh"
 #include "tmk_launch.h"
 
 namespace tmk {
@@ -10,24 +11,30 @@ namespace tmk {
 template <typename Real, int TX_, int TY_, int NT_>
 struct LaunchImpl {
   static cudaError_t fault(const PatchDev<Real>* patches, const int* fp, int nfault, int max_faces,
-                           const DevParams* params, double time, DevStatus* st, bool pdl, int seg,
-                           cudaStream_t s) {
+                           const DevParams* params, const DevParams& hp, double dt, double dx, double time,
+                           DevStatus* st, bool pdl, int seg, cudaStream_t s) {
     if (nfault <= 0) return cudaSuccess;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    const bool small = seg == FAULT_SEG_SMALL;
-    const int sg = small ? FAULT_SEG_SMALL : FAULT_SEG;
-    cfg.gridDim = dim3((max_faces + sg - 1) / sg, nfault);
-    cfg.blockDim = dim3(small ? FAULT_THREADS_SMALL : FAULT_THREADS);
     cfg.stream = s;
     cfg.attrs = pdl ? attr : nullptr;
     cfg.numAttrs = pdl ? 1 : 0;
+    if (seg == 0) {
+      cfg.gridDim = dim3((max_faces + REF9_SEG - 1) / REF9_SEG, nfault);
+      cfg.blockDim = dim3(REF9_THREADS);
+      return cudaLaunchKernelEx(&cfg, fault_ref9_kernel<Real>, patches, fp, params, time, st);
+    }
+    FaultConst<Real> fc;
+    fc.load(hp, dt, dx);
+    const bool small = seg == FAULT_SEG_SMALL;
+    const int sg = small ? FAULT_SEG_SMALL : FAULT_SEG;
+    cfg.gridDim = dim3((max_faces + sg - 1) / sg, nfault);
+    cfg.blockDim = dim3(fault_threads(sg));
     if (small)
-      return cudaLaunchKernelEx(&cfg, fault_kernel<Real, FAULT_SEG_SMALL, FAULT_THREADS_SMALL>, patches, fp,
-                                params, time, st);
-    return cudaLaunchKernelEx(&cfg, fault_kernel<Real, FAULT_SEG, FAULT_THREADS>, patches, fp, params, time, st);
+      return cudaLaunchKernelEx(&cfg, fault_kernel<Real, FAULT_SEG_SMALL>, patches, fp, params, time, st, fc);
+    return cudaLaunchKernelEx(&cfg, fault_kernel<Real, FAULT_SEG>, patches, fp, params, time, st, fc);
   }
   static size_t smem() { return sizeof(VolSmem<Real, TX_, TY_>); }
   static int box_x() { return VolSmem<Real, TX_, TY_>::RXP; }
@@ -146,9 +153,10 @@ struct LaunchImpl {
   template <> const int Launch<REAL>::TX = TXV;                                                             \
   template <> const int Launch<REAL>::TY = TYV;                                                             \
   template <> cudaError_t Launch<REAL>::fault(const PatchDev<REAL>* p, const int* fp, int nf, int mf,        \
-                                              const DevParams* prm, double t, DevStatus* st, bool pdl,       \
-                                              int seg, cudaStream_t s) {                                     \
-    return LaunchImpl<REAL, TXV, TYV, NTV>::fault(p, fp, nf, mf, prm, t, st, pdl, seg, s);                   \
+                                              const DevParams* prm, const DevParams& hp, double dt,          \
+                                              double dx, double t, DevStatus* st, bool pdl, int seg,         \
+                                              cudaStream_t s) {                                              \
+    return LaunchImpl<REAL, TXV, TYV, NTV>::fault(p, fp, nf, mf, prm, hp, dt, dx, t, st, pdl, seg, s);       \
   }                                                                                                          \
   template <> cudaError_t Launch<REAL>::volume(const PatchDev<REAL>* p, const TileDev* tl, int nt,          \
                                                const DevParams* prm, cudaStream_t s) {                      \
@@ -179,7 +187,8 @@ struct LaunchImpl {
   }                                                                                                          \
   template <> int Launch<REAL>::march_warps() { return MARCH_WARPS; }                                        \
   template <> const void* Launch<REAL>::fault_entry(int seg) {                                               \
-    return seg == FAULT_SEG_SMALL ? (const void*)fault_kernel<REAL, FAULT_SEG_SMALL, FAULT_THREADS_SMALL>     \
-                                  : (const void*)fault_kernel<REAL, FAULT_SEG, FAULT_THREADS>;               \
+    return seg == FAULT_SEG_SMALL ? (const void*)fault_kernel<REAL, FAULT_SEG_SMALL>                         \
+           : seg == FAULT_SEG     ? (const void*)fault_kernel<REAL, FAULT_SEG>                               \
+                                  : (const void*)fault_ref9_kernel<REAL>;                                    \
   }                                                                                                          \
   }
