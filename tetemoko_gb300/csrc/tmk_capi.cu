@@ -204,14 +204,47 @@ constexpr int kFaultDisplace = 1;
 // the marching kernels implement the PPM and CTU predictors; PLM runs the tile kernel
 bool uses_march(const tmk_scheme& s) { return s.volume_kernel != TMK_VOLUME_TILE && s.normal_pred_order != 1; }
 
-tmk_tuning default_tuning(int march_allowed) {
+// Shortest run of a level's items.  A row of a marching warp takes about the
+// same time until a sub-partition holds two warps in FP32 or one in FP64 (whose
+// pipe one warp nearly fills), and an item costs about three rows beyond its
+// own, so the time goes as (run + 3) x max(1, warps per sub-partition / 2 or 1).
+// Measured (us a step): mixed 512x256 18.7 at 4 rows and 25.8 at 16, FP64
+// 512x256 217 at 8 and 252 at 16, FP64 256x128 91 at 4 and 242 at 16, mixed
+// 1000x500 in patches of 128 65.7 at 6 and 61.5 at 16.
+int default_min_run(const tmk_level_s* L) {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int best = kMinRun;
+  double cost = 0.0;
+  for (int run : {16, 8, 4}) {
+    long long items = 0;
+    for (const LevelPatch& lp : L->patches) {
+      const int ns = (lp.valid.hi[0] - lp.valid.lo[0] + tmk::MARCH_COLS) / tmk::MARCH_COLS;
+      items += (long long)ns * ((lp.valid.hi[1] - lp.valid.lo[1] + run) / run);
+    }
+    const double per = (double)items / (4.0 * sms) / (L->prec == TMK_PREC_MIXED ? 2.0 : 1.0);
+    const double c = (run + 3) * std::max(1.0, per);
+    if (run == 16 || c < cost) { best = run; cost = c; }
+  }
+  return best;
+}
+
+// A rate-and-state fault kernel (26 us) outlasts the in-plane kernel of a
+// small level: it goes first (64x32: 22.2 against 24.9 us a step, 256x128:
+// 21.8 against 26.3; 1000x500 and above: the default order).
+constexpr long long kFaultFirstCells = 262144;
+
+tmk_tuning default_tuning(const tmk_level_s* L) {
   tmk_tuning t;
-  t.volume_kernel = march_allowed ? TMK_VOLUME_MARCH : TMK_VOLUME_TILE;
+  t.volume_kernel = L->march_allowed ? TMK_VOLUME_MARCH : TMK_VOLUME_TILE;
   t.march_waves[0] = t.march_waves[1] = 1;
-  t.min_run = kMinRun;
+  t.min_run = default_min_run(L);
   t.fault_displace = kFaultDisplace;
   t.fault_seg = tmk::FAULT_SEG;
-  t.fault_first = 0;
+  long long cells = 0;
+  for (const LevelPatch& lp : L->patches)
+    cells += (long long)(lp.valid.hi[0] - lp.valid.lo[0] + 1) * (lp.valid.hi[1] - lp.valid.lo[1] + 1);
+  t.fault_first = L->ctx->scheme.fault_law == TMK_FAULT_RS && cells <= kFaultFirstCells;
   t.plastic_fused = 0;
   return t;
 }
@@ -644,7 +677,7 @@ tmk_status level_create_impl(tmk_context* const* ctxs, int nscen, const tmk_box*
   L->htiles = tiles;
   L->march_allowed = uses_march(c->scheme) ? 1 : 0;
   L->march = L->march_allowed;
-  L->tune = default_tuning(L->march_allowed);
+  L->tune = default_tuning(L);
   if (L->march_allowed) {
     tmk_status st = build_march_lists(L);
     if (st != TMK_OK) return fail(st);
@@ -1144,19 +1177,19 @@ tmk_status time_steps(tmk_level_s* L, double time, double dt, int steps, cudaStr
 // marching choices (waves per group, shortest run, fault displacement, the
 // fault kernel's place in the step, on a plastic level the fused or separate
 // plastic return) and both fault-kernel variants, plus the
-// tile kernel; `reduced` leaves out the
-// shortest runs of 8 rows (the hierarchy autotuner times whole coarse steps).
+// tile kernel; `reduced` leaves out the shortest and longest runs (the
+// hierarchy autotuner times whole coarse steps).
 std::vector<tmk_tuning> tmk_host::tuning_candidates(const tmk_level_s* L, bool reduced) {
   std::vector<tmk_tuning> out;
-  tmk_tuning t = default_tuning(L->march_allowed);
+  tmk_tuning t = default_tuning(L);
   for (int seg : {tmk::FAULT_SEG, tmk::FAULT_SEG_SMALL}) {
     t.fault_seg = seg;
     if (L->march_allowed) {
       t.volume_kernel = TMK_VOLUME_MARCH;
       for (int w0 : {1, 2})
         for (int w1 : {1, 2})
-          for (int run : {8, 16, 32}) {
-            if (reduced && run == 8) continue;
+          for (int run : {4, 8, 16, 32}) {
+            if (reduced && (run == 4 || run == 32)) continue;
             for (int disp : {0, 1, 2})
               for (int first : {0, 1})
                 for (int fused : {0, 1}) {
@@ -1171,7 +1204,7 @@ std::vector<tmk_tuning> tmk_host::tuning_candidates(const tmk_level_s* L, bool r
                 }
           }
     }
-    tmk_tuning tt = default_tuning(L->march_allowed);
+    tmk_tuning tt = default_tuning(L);
     tt.volume_kernel = TMK_VOLUME_TILE;
     tt.fault_seg = seg;
     out.push_back(tt);

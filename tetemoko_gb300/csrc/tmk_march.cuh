@@ -58,7 +58,7 @@ TMK_D double2 padd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + 
 TMK_D double2 pmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
 TMK_D double2 pfma(double2 a, double2 b, double2 c) { return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)); }
 TMK_D double2 psub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-TMK_D float2 pneg(float2 a) { return pmul(a, make_float2(-1.f, -1.f)); }
+TMK_D float2 pneg(float2 a) { return make_float2(-a.x, -a.y); }
 TMK_D double flip(double a) { return __hiloint2double(__double2hiint(a) ^ 0x80000000, __double2loint(a)); }
 TMK_D double2 pneg(double2 a) { return make_double2(flip(a.x), flip(a.y)); }
 
@@ -129,13 +129,13 @@ template <int G, int D> TMK_HD constexpr int wave_s(int w) { return is_p<G>(w) ?
 template <typename T>
 struct MK {
   using P = typename PairOf<T>::P;
-  P Zp, Zs, nZp, nZs;  // characteristics w = s +- Z v (rv Z)
+  P Zp, Zs;            // characteristics w = s +- Z v (rv Z)
   T aP, bP, aS, bS;    // PPM tracing coefficients of the P and S speeds, halved (the deltas are kept doubled)
   // transverse term of D on the characteristic values of E: the stress part
   // from the differences jn - jp, the velocity part (times E's impedance) from
   // the sums jn + jp
   T c_lam, c_G;
-  P cvP, cvS, ncvP, ncvS;
+  P cvP, cvS;
   // update: velocities from the sums, stresses from the differences
   P e_v;
   T e_l2g, e_lam, e_G;
@@ -149,7 +149,6 @@ struct MK {
     const double s2 = (D == 1) ? -1.0 : 1.0;    // rv of side 2
     auto two = [](double a, double b) { return mk2((T)a, (T)b); };
     Zp = two(p.Zp, s2 * p.Zp); Zs = two(p.Zs, s2 * p.Zs);
-    nZp = two(-p.Zp, -s2 * p.Zp); nZs = two(-p.Zs, -s2 * p.Zs);
     const double sp = p.cp * dtdx, ss = p.cs * dtdx;
     aP = (T)(0.5 * (1.0 - sp) * (1.0 - sp)); bP = (T)(0.5 * (sp * sp - sp));
     aS = (T)(0.5 * (1.0 - ss) * (1.0 - ss)); bS = (T)(0.5 * (ss * ss - ss));
@@ -158,7 +157,7 @@ struct MK {
     c_G = (T)(0.5 * dtdx * p.G * (0.5 / p.Zs));
     // the velocity term carries the rv of y in both directions (D's or E's)
     const double vP = p.Zp * (0.25 * dtdx / p.rho), vS = p.Zs * (0.25 * dtdx / p.rho);
-    cvP = two(vP, -vP); cvS = two(vS, -vS); ncvP = two(-vP, vP); ncvS = two(-vS, vS);
+    cvP = two(vP, -vP); cvS = two(vS, -vS);
     const double ev = 0.5 * dtdx / p.rho;
     e_v = two(ev, s2 * ev);
     e_l2g = (T)(dtdx * l2g * (0.5 / p.Zp)); e_lam = (T)(dtdx * p.lam * (0.5 / p.Zp));
@@ -183,6 +182,13 @@ template <int D, typename P> TMK_D P kpair(const P& pair) {
   else return pair;
 }
 template <typename T> TMK_D auto kall(T s) { return mk2(s, s); }
+
+// position of a component among those live in y
+template <int G> TMK_HD constexpr int slope_slot(int c) {
+  int k = 0;
+  for (int q = 0; q < c; ++q) k += live<G, 1>(q) ? 1 : 0;
+  return k;
+}
 
 // Everything the marching kernel needs that is uniform over a launch (all
 // patches of a level share the scenario, dt and dx).  Built on the host and
@@ -320,15 +326,16 @@ template <typename P> TMK_D void limit2(P& m, P& p) {
 
 // The traced characteristic values of a cell in direction D (see the head of
 // the file) from its state w and its doubled deltas m (lo) and p (hi).
+// kd: the constants that are the same in both directions
 template <int G, int D, typename T>
-TMK_D void trace(const MK<T>& k, const typename PairOf<T>::P* w, const typename PairOf<T>::P* m,
+TMK_D void trace(const MK<T>& k, const MK<T>& kd, const typename PairOf<T>::P* w, const typename PairOf<T>::P* m,
                  const typename PairOf<T>::P* p, bool clim, typename PairOf<T>::P* An, typename PairOf<T>::P* Ap) {
   using P = typename PairOf<T>::P;
 #pragma unroll
   for (int q = 0; q < kWaves<G>; ++q) {
     const int v = wave_v<G, D>(q), s = wave_s<G, D>(q);
-    const P Z = kpair<D>(is_p<G>(q) ? k.Zp : k.Zs), nZ = kpair<D>(is_p<G>(q) ? k.nZp : k.nZs);
-    const P a = kall(is_p<G>(q) ? k.aP : k.aS), b = kall(is_p<G>(q) ? k.bP : k.bS);
+    const P Z = kpair<D>(is_p<G>(q) ? k.Zp : k.Zs), nZ = pneg(Z);
+    const P a = kall(is_p<G>(q) ? kd.aP : kd.aS), b = kall(is_p<G>(q) ? kd.bP : kd.bS);
     P nm = pfma(Z, m[v], m[s]), np = pfma(Z, p[v], p[s]);
     P pm = pfma(nZ, m[v], m[s]), pp = pfma(nZ, p[v], p[s]);
     if (clim) { limit2(nm, np); limit2(pm, pp); }
@@ -344,7 +351,7 @@ TMK_D void chars(const MK<T>& k, const typename PairOf<T>::P* w, typename PairOf
   for (int q = 0; q < kWaves<G>; ++q) {
     const int v = wave_v<G, D>(q), s = wave_s<G, D>(q);
     An[q] = pfma(kpair<D>(is_p<G>(q) ? k.Zp : k.Zs), w[v], w[s]);
-    Ap[q] = pfma(kpair<D>(is_p<G>(q) ? k.nZp : k.nZs), w[v], w[s]);
+    Ap[q] = pfma(pneg(kpair<D>(is_p<G>(q) ? k.Zp : k.Zs)), w[v], w[s]);
   }
 }
 
@@ -366,7 +373,8 @@ template <int G, typename P> TMK_D void jumps(const P* jn, const P* jp, P* sum, 
   for (int q = 0; q < kWaves<G>; ++q) { sum[q] = padd(jn[q], jp[q]); dif[q] = psub(jn[q], jp[q]); }
 }
 
-// Transverse term of direction D with scale -1/2 dt/dx on the characteristic
+// Transverse term of direction D with scale -1/2 dt/dx (its constants are the
+// same in both directions) on the characteristic
 // values Bn, Bp of the other direction.  E's P pair takes the normal stress
 // from D's P wave (lam) and the velocity from D's S wave; E's S pair takes the
 // shear stress from D's S wave (G) and the velocity from D's P wave; the
@@ -376,12 +384,12 @@ TMK_D void correct(const MK<T>& k, const typename PairOf<T>::P* sum, const typen
                    typename PairOf<T>::P* Bn, typename PairOf<T>::P* Bp) {
   if constexpr (G == 0) {
     Bn[0] = pfma(k.cvP, sum[1], pfma(kall(k.c_lam), dif[0], Bn[0]));
-    Bp[0] = pfma(k.ncvP, sum[1], pfma(kall(k.c_lam), dif[0], Bp[0]));
+    Bp[0] = pfma(pneg(k.cvP), sum[1], pfma(kall(k.c_lam), dif[0], Bp[0]));
     Bn[1] = pfma(k.cvS, sum[0], pfma(kall(k.c_G), dif[1], Bn[1]));
-    Bp[1] = pfma(k.ncvS, sum[0], pfma(kall(k.c_G), dif[1], Bp[1]));
+    Bp[1] = pfma(pneg(k.cvS), sum[0], pfma(kall(k.c_G), dif[1], Bp[1]));
   } else {
     Bn[0] = pfma(k.cvS, sum[0], Bn[0]);
-    Bp[0] = pfma(k.ncvS, sum[0], Bp[0]);
+    Bp[0] = pfma(pneg(k.cvS), sum[0], Bp[0]);
   }
 }
 
@@ -389,7 +397,7 @@ TMK_D void correct(const MK<T>& k, const typename PairOf<T>::P* sum, const typen
 // starts them, the y part adds to them; the state is rounded once, when they
 // are added to it.
 template <int G, int D, typename T>
-TMK_D void add_update(const MK<T>& k, const typename PairOf<T>::P* sum, const typename PairOf<T>::P* dif,
+TMK_D void add_update(const MK<T>& k, const MK<T>& kd, const typename PairOf<T>::P* sum, const typename PairOf<T>::P* dif,
                       typename PairOf<T>::P* du) {
   using P = typename PairOf<T>::P;
   using R = Role<G, D>;
@@ -397,11 +405,11 @@ TMK_D void add_update(const MK<T>& k, const typename PairOf<T>::P* sum, const ty
 #pragma unroll
   for (int q = 0; q < kWaves<G>; ++q) {
     acc(wave_v<G, D>(q), kpair<D>(k.e_v), sum[q]);
-    acc(wave_s<G, D>(q), kall(is_p<G>(q) ? k.e_l2g : k.e_G), dif[q]);
+    acc(wave_s<G, D>(q), kall(is_p<G>(q) ? kd.e_l2g : kd.e_G), dif[q]);
   }
   if constexpr (R::hasP) {
-    acc(R::zc0, kall(k.e_lam), dif[0]);
-    acc(R::zc1, kall(k.e_lam), dif[0]);
+    acc(R::zc0, kall(kd.e_lam), dif[0]);
+    acc(R::zc1, kall(kd.e_lam), dif[0]);
   }
   if constexpr (R::hasZf && D == 0) du[R::zf] = mk2(T(0), T(0));
 }
@@ -443,25 +451,33 @@ constexpr int MARCH_HALO = 2;    // halo lanes on either side (lane l holds colu
 constexpr int MARCH_WARPS = 4;   // warps per CTA
 
 // Rows q-1 (the old state of the row updated at step q) to q+2 of the rolling
-// window and the rows in flight live in a per-warp ring of shared memory
-// filled by cp.async; slot = row & 7.  A ring row holds MARCH_RW entries per
-// component: the column left of lane 0, the warp's 32 columns, the column
-// right of lane 31.  MARCH_AHEAD: the row requested at step q is q + AHEAD.
-constexpr int MARCH_RING = 8;
-constexpr int MARCH_AHEAD = 4;
+// window and the row in flight, q+3, live in a per-warp ring of five rows of
+// shared memory filled by cp.async.  A ring row holds MARCH_RW entries per
+// component: the column left of lane 0, the warp's 32 columns, the column right
+// of lane 31.
+constexpr int MARCH_RING = 5;
+constexpr int MARCH_AHEAD = 3;
 constexpr int MARCH_RW = 34;
 template <typename T, int G>
-constexpr size_t march_warp_pairs() { return (size_t)MARCH_RING * Grp<G>::N * MARCH_RW; }
+constexpr int march_row_pairs() { return Grp<G>::N * MARCH_RW; }
+// The FP32 in-plane kernel keeps the y half slopes and lo deltas of a lane (8
+// values) in shared memory, which fits its registers into four CTAs per SM.
+template <typename T, int G> constexpr bool kSlopesInSmem = sizeof(T) == 4 && G == 0;
+template <typename T, int G>
+constexpr size_t march_warp_pairs() {
+  return (size_t)MARCH_RING * march_row_pairs<T, G>() + (kSlopesInSmem<T, G> ? 8 * 32 : 0);
+}
 template <typename T, int G>
 constexpr size_t march_smem_bytes() {
   return (size_t)MARCH_WARPS * march_warp_pairs<T, G>() * sizeof(typename PairOf<T>::P);
 }
 
-// resident CTAs per SM the register allocation targets: FP32 in-plane 3 (168
-// registers, no spills, with the y-direction carries in shared memory),
-// antiplane 5 (96 registers); FP64 in-plane 2, antiplane 4
+// resident CTAs per SM the register allocation targets: FP32 in-plane 4 (128
+// registers), antiplane 6 (80); FP64 in-plane 2, antiplane 4.  FP32 with 3 / 5
+// instead: the 2048x1024 level alike (126 us a step), an ensemble of 16
+// scenarios 7.57 against 5.96 ms per 20 steps; 4 / 7 and 5 / 7 spill.
 template <typename T, int G> struct MarchMinBlocks {
-  static constexpr int value = sizeof(T) == 4 ? ((G == 0) ? 3 : 5) : ((G == 0) ? 2 : 4);
+  static constexpr int value = sizeof(T) == 4 ? ((G == 0) ? 4 : 6) : ((G == 0) ? 2 : 4);
 };
 
 // asynchronous copy of one element to shared address dst + OFF (completion
@@ -650,12 +666,14 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   // the domain, zeros elsewhere (and for rows past the last one the item
   // reads); the two outer columns only for the components live in x (the only
   // ones whose neighbours are read)
-  auto ring_row = [&](int y) -> P* { return ring + (size_t)((y & (MARCH_RING - 1)) * N) * MARCH_RW; };
+  // ring slots of rows q-1, q, q+1, q+2 and of the row in flight, handed on each row
+  constexpr int RP = march_row_pairs<T, G>();
+  int r_m1 = 4 * RP, r_0 = 0, r_1 = RP, r_2 = 2 * RP, r_3 = 3 * RP;
   const int y_last = min(dhi1, q_e + 2);
-  auto load_row_async = [&](int y) {
+  auto load_row_async = [&](int y, int slot) {
     const bool ok = lane_in && y <= y_last;       // y >= q_s >= dlo1
     const T* const src = ok ? lsrc : uin;
-    const unsigned row32 = ring32 + (unsigned)((y & (MARCH_RING - 1)) * (N * MARCH_RW * (int)sizeof(P)));
+    const unsigned row32 = ring32 + (unsigned)(slot * (int)sizeof(P));
     cp_async_column<T, G, 0, false>(row32 + (unsigned)((lane + 1) * (int)sizeof(P)), src, plane,
                                     ok ? (unsigned)sizeof(T) : 0u);
     if (lane == 0 || lane == 31) {      // the outer columns: own address -1 / +1 (ext_in and ok: a cell of the FAB)
@@ -672,6 +690,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   // q, the traced x values of row q-1, the traced and corrected y values of
   // row q-1 (An, Ap) and their jump jp.  Two sets, used in turn by two copies
   // of the row's code: with one set each value would be moved once a row.
+  constexpr bool kS = kSlopesInSmem<T, G>;
+  P* const slopes = ring + MARCH_RING * RP + lane;     // [2][4][32]
   struct Carry {
     P n4[N], dlo[N];
     P Anx[NW], Apx[NW], Any[NW], Apy[NW], jpy[NW], Bny[NW], Bpy[NW], jpB[NW];
@@ -684,14 +704,14 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   }
   {
 #pragma unroll
-    for (int y = 0; y < MARCH_AHEAD; ++y) load_row_async(q_s + y);
+    for (int y = 0; y < MARCH_AHEAD; ++y) load_row_async(q_s + y, y * RP);
     P Wa[N], Wb[N];
     load_row(q_s - 2, Wa);
     load_row(q_s - 1, Wb);
     cp_async_wait<MARCH_AHEAD - 2>();      // rows q_s, q_s + 1 have landed (a lane reads its own columns)
     const bool hl = q_s - 1 >= dlo1, hll = q_s - 2 >= dlo1, hr = q_s + 1 <= dhi1;
-    const P* r0 = ring_row(q_s) + lane + 1;
-    const P* r1 = ring_row(q_s + 1) + lane + 1;
+    const P* r0 = ring + lane + 1;
+    const P* r1 = ring + RP + lane + 1;
 #pragma unroll
     for (int c = 0; c < N; ++c) {
       if (!live<G, 1>(c)) continue;
@@ -708,11 +728,12 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
       } else {
         c0.dlo[c] = twice(c0.n4[c]);
       }
+      if (kS) { slopes[slope_slot<G>(c) * 32] = c0.n4[c]; slopes[(4 + slope_slot<G>(c)) * 32] = c0.dlo[c]; }
     }
   }
 
   auto row_step = [&](const int q, Carry& in, Carry& out) {
-    load_row_async(q + MARCH_AHEAD);  // rows in flight while this one is computed
+    load_row_async(q + MARCH_AHEAD, r_3);  // the row in flight while this one is computed
     // fused plastic return: its other inputs for row q-1, stored at the end of
     // this iteration, requested now so that the row's work hides their latency
     P pin[3];
@@ -724,8 +745,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
     __syncwarp();                         // ... every lane's copies, whose neighbours read them
     P Bn_q[NW], Bp_q[NW];
     if (q <= dhi1) {
-      const P* const rw = ring_row(q) + lane + 1;
-      P W0[N], m[N], p[N], nl[N], nr[N];
+      const P* const rw = ring + r_0 + lane + 1;
+      P W0[N], m[N], p[N], nl[N], nr[N], n4[N], dl[N];
 #pragma unroll
       for (int c = 0; c < N; ++c) { W0[c] = rw[c * MARCH_RW]; m[c] = mk2(T(0), T(0)); p[c] = m[c]; }
       // the cell's stresses relative to the background, for its characteristic values
@@ -735,8 +756,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
         Wr[c] = Grp<G>::glob(c) < 3 ? W0[c] : padd(W0[c], kall(mc.nbg[Grp<G>::glob(c)]));
       if (ppm) {
         // y deltas of row q; slope and lo delta of row q+1
-        const P* const r1 = ring_row(q + 1) + lane + 1;
-        const P* const r2 = ring_row(q + 2) + lane + 1;
+        const P* const r1 = ring + r_1 + lane + 1;
+        const P* const r2 = ring + r_2 + lane + 1;
 #pragma unroll
         for (int c = 0; c < N; ++c) {
           if (!live<G, 1>(c)) continue;
@@ -751,22 +772,23 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
 #pragma unroll
         for (int c = 0; c < N; ++c) {
           if (!live<G, 1>(c)) continue;
-          out.n4[c] = half_slope(nl[c], nr[c], lim);
-          out.dlo[c] = delta_lo<T>(nl[c], out.n4[c], in.n4[c]);
-          p[c] = delta_hi<T>(nl[c], out.dlo[c]);
+          n4[c] = kS ? slopes[slope_slot<G>(c) * 32] : in.n4[c];
+          m[c] = kS ? slopes[(4 + slope_slot<G>(c)) * 32] : in.dlo[c];
+          const P n1 = half_slope(nl[c], nr[c], lim);
+          dl[c] = delta_lo<T>(nl[c], n1, n4[c]);
+          p[c] = delta_hi<T>(nl[c], dl[c]);
+          if (kS) { slopes[slope_slot<G>(c) * 32] = n1; slopes[(4 + slope_slot<G>(c)) * 32] = dl[c]; }
+          else { out.n4[c] = n1; out.dlo[c] = dl[c]; }
         }
         if (q + 1 > dhi1) {
 #pragma unroll
           for (int c = 0; c < N; ++c)
-            if (live<G, 1>(c)) p[c] = pneg(twice(in.n4[c]));
+            if (live<G, 1>(c)) p[c] = pneg(twice(n4[c]));
         }
 #pragma unroll
-        for (int c = 0; c < N; ++c) {
-          if (!live<G, 1>(c)) continue;
-          m[c] = in.dlo[c];
-          if (plim) limit_mono(m[c], p[c], in.n4[c]);
-        }
-        trace<G, 1, T>(ky, Wr, m, p, clim, out.Any, out.Apy);
+        for (int c = 0; c < N; ++c)
+          if (live<G, 1>(c) && plim) limit_mono(m[c], p[c], n4[c]);
+        trace<G, 1, T>(ky, kx, Wr, m, p, clim, out.Any, out.Apy);
         // x deltas
         P n[N], d[N];
 #pragma unroll
@@ -809,7 +831,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
           m[c] = d[c];
           if (plim) limit_mono(m[c], p[c], n[c]);
         }
-        trace<G, 0, T>(kx, Wr, m, p, clim, out.Anx, out.Apx);
+        trace<G, 0, T>(kx, kx, Wr, m, p, clim, out.Anx, out.Apx);
       } else {
         chars<G, 1, T>(ky, Wr, out.Any, out.Apy);
         chars<G, 0, T>(kx, Wr, out.Anx, out.Apx);
@@ -845,7 +867,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
     if (defer0 && yr == dlo1) {
       // row 0 of a fault patch: keep what march_fault_row_kernel needs
       P* st = reinterpret_cast<P*>(mc.stash[G]) + (size_t)it.fslot * MARCH_STASH_VECS * N * 32 + lane;
-      const P* wo = ring_row(yr) + lane + 1;
+      const P* wo = ring + r_m1 + lane + 1;
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
         st[(0 * NW + w) * 32] = in.Anx[w]; st[(1 * NW + w) * 32] = in.Apx[w];
@@ -860,7 +882,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
 #pragma unroll
       for (int w = 0; w < NW; ++w) jn[w] = psub(out.Any[w], in.Any[w]);
       jumps<G>(jn, in.jpy, sum, dif);
-      correct<G, 1, T>(ky, sum, dif, in.Anx, in.Apx);
+      correct<G, 1, T>(kx, sum, dif, in.Anx, in.Apx);
 #pragma unroll
       for (int w = 0; w < NW; ++w) { BnR[w] = shfl_dn2(in.Anx[w], 1); BpL[w] = shfl_up2(in.Apx[w], 1); }
       if (warp_xedge) {
@@ -870,12 +892,12 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
 #pragma unroll
       for (int w = 0; w < NW; ++w) { jn[w] = psub(BnR[w], in.Anx[w]); jp[w] = psub(in.Apx[w], BpL[w]); }
       jumps<G>(jn, jp, sum, dif);
-      add_update<G, 0, T>(kx, sum, dif, du);
+      add_update<G, 0, T>(kx, kx, sum, dif, du);
 #pragma unroll
       for (int w = 0; w < NW; ++w) jn[w] = psub(Bn_q[w], in.Bny[w]);
       jumps<G>(jn, in.jpB, sum, dif);
-      add_update<G, 1, T>(ky, sum, dif, du);
-      const P* wo = ring_row(yr) + lane + 1;
+      add_update<G, 1, T>(ky, kx, sum, dif, du);
+      const P* wo = ring + r_m1 + lane + 1;
 #pragma unroll
       for (int c = 0; c < N; ++c) u[c] = padd(wo[c * MARCH_RW], du[c]);
       if (col_valid && yr <= it.y1) store_cell<T, G, PL>(sdst, plane, mc, u, pin);
@@ -893,6 +915,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
         });
     }
     sdst += anx;
+    const int freed = r_m1;
+    r_m1 = r_0; r_0 = r_1; r_1 = r_2; r_2 = r_3; r_3 = freed;
     // advance: the jumps over row q of the values from below (at the domain's
     // y-lo edge those arriving through it; a fault patch's row 0 is finished later)
     if (q == dlo1 && !fault) {
@@ -960,9 +984,9 @@ TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const Ma
       s0 = mk2((T)(pp.first[(size_t)gs * pp.nfirst + fi1] - b), (T)(pp.first[(size_t)(11 + gs) * pp.nfirst + fi1] - b));
     }
     sum[w] = psub(padd(An1[w], Ap0[w]), padd(s0, s0));
-    dif[w] = pfma(is_p<G>(w) ? mc.ky.nZp : mc.ky.nZs, padd(v0, v0), psub(An1[w], Ap0[w]));
+    dif[w] = pfma(pneg(is_p<G>(w) ? mc.ky.Zp : mc.ky.Zs), padd(v0, v0), psub(An1[w], Ap0[w]));
   }
-  correct<G, 1, T>(mc.ky, sum, dif, Bnx, Bpx);
+  correct<G, 1, T>(mc.kx, sum, dif, Bnx, Bpx);
 #pragma unroll
   for (int w = 0; w < NW; ++w) { BnR[w] = shfl_dn2(Bnx[w], 1); BpL[w] = shfl_up2(Bpx[w], 1); }
   if (x == dlo0) edge_value<G>(mc.kx, mc.kx.bgp, mc.xout_lo != 0, Bnx, BpL);
@@ -985,7 +1009,7 @@ TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const Ma
     for (int w = 0; w < NW; ++w) { jn[w] = psub(BnR[w], Bnx[w]); jp[w] = psub(Bpx[w], BpL[w]); }
     jumps<G>(jn, jp, sum, dif);
     P du[N];
-    add_update<G, 0, T>(mc.kx, sum, dif, du);
+    add_update<G, 0, T>(mc.kx, mc.kx, sum, dif, du);
 #pragma unroll
     for (int c = 0; c < N; ++c) u[c] = padd(u[c], pfma(psub(Fy1[c], Fy0[c]), mc.sc, du[c]));
     const unsigned plane = (unsigned)pp.anx * (unsigned)pp.any;
