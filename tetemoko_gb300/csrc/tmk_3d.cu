@@ -173,6 +173,62 @@ size_t layout3(Step3<T>& g, char* base) {
   return off;
 }
 
+// The step on characteristic values (tmk_3d_march.cuh) implements the decks'
+// predictor (PPM with primitive limiting) and the laws that read only those
+// values; it takes 0.57 of the time of the passes over face states (192x96x96
+// mixed: 792 against 1383 us, and 32 patches of a 96x64x64 level 984 against
+// 1116), whatever the size.  The rest (PLM, CTU, limiting of the characteristic
+// amplitudes, the reference's 9-component slip weakening) keeps those passes.
+template <typename T>
+bool march3(const tmk::DevParams& p) {
+  return std::is_same<T, float>::value && p.order == 2 && p.prim_lim && !p.char_lim &&
+         !(p.fault_law == 2 && p.sw_off != 11);
+}
+
+// its scratch of one patch: the values of the cells of S | fault-face states
+// (4 levels) | velocities | FP32 copy of U (mixed form)
+template <typename T>
+size_t layout3m(Step3<T>& g, char* base) {
+  using namespace tmk::d3;
+  constexpr bool copy = !std::is_same<T, double>::value;
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    char* p = base ? base + off : nullptr;
+    off += align_up3(bytes);
+    return p;
+  };
+  g.AF = take((size_t)18 * g.S.cells() * 2 * sizeof(T));
+  g.FA = take(g.fault ? (size_t)24 * g.fplane.cells() * 2 * sizeof(T) : 0);
+  g.FV = (T*)take(g.fault ? (size_t)4 * g.fplane.cells() * sizeof(T) : 0);
+  T* up = (T*)take(copy ? (size_t)NS * g.Ap.cells() * sizeof(T) : 0);
+  if constexpr (copy) { g.Up = up; g.Uc = up; g.uside = tmk::NSIDE; }
+  else { g.Up = (const T*)(const void*)g.U; g.Uc = nullptr; g.Ap = g.A; g.uside = 11; }
+  return off;
+}
+
+// Planes a CTA of the last pass marches over: about two planes are spent on
+// start-up, and the CTAs should come in whole waves.
+template <typename T>
+int choose_zrun(const Step3<T>* g, int np) {
+  using namespace tmk::d3;
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int best = 1 << 20;
+  double cost = 0.0;
+  for (int run : {1 << 20, 96, 64, 48, 40, 32, 28, 24, 20, 16, 14, 12, 10, 8, 6, 4}) {
+    long long n = 0;
+    int longest = 1;
+    for (int p = 0; p < np; ++p) {
+      const int nz = g[p].cur.n[2];
+      n += 2LL * cdiv(g[p].cur.n[0], STEP_COLS) * cdiv(g[p].cur.n[1], STEP_ROWS - 2) * cdiv(nz, std::min(run, nz));
+      longest = std::max(longest, std::min(run, nz));
+    }
+    const double c = (double)((n + STEP_CTAS * sms - 1) / (STEP_CTAS * sms)) * (longest + 2.5);
+    if (run == 1 << 20 || c < cost) { best = run; cost = c; }
+  }
+  return best;
+}
+
 tmk_status ensure_scratch(tmk_context* c, size_t total, cudaStream_t s) {
   if (total <= c->scratch_bytes) return TMK_OK;
   TMK_CU(cudaStreamSynchronize(s));
@@ -205,6 +261,14 @@ tmk_status patch3(tmk_context* c, const tmk_fab3* U, const tmk_fab3* B, const tm
   PlanOne<T> pl;
   tmk_status r = fill3<T>(c, U, B, Fo, valid, domain, dx, time, dt, pl.g);
   if (r != TMK_OK) return r;
+  if constexpr (std::is_same<T, float>::value) {
+    if (march3<T>(c->hp)) {
+      if ((r = ensure_scratch(c, layout3m<T>(pl.g, nullptr), s)) != TMK_OK) return r;
+      layout3m<T>(pl.g, (char*)c->scratch);
+      pl.g.zrun = choose_zrun(&pl.g, 1);
+      return launch_march_f32(pl, c->hp, c->dp, c->dstatus, dt, dx, s) == cudaSuccess ? TMK_OK : TMK_ERR_CUDA;
+    }
+  }
   if ((r = ensure_scratch(c, layout3<T>(pl.g, nullptr), s)) != TMK_OK) return r;
   layout3<T>(pl.g, (char*)c->scratch);
   Side side;
@@ -229,6 +293,10 @@ tmk_status patches3(tmk_context* c, int np, const tmk_fab3* U, const tmk_fab3* B
     const tmk_status r = fill3<T>(c, U + p, B ? B + p : nullptr, Fo, valid + p, domain, dx, time, dt, gs[p]);
     if (r != TMK_OK) return r;
   }
+  const bool mar = march3<T>(c->hp);
+  const int zrun = choose_zrun(gs.data(), np);
+  for (Step3<T>& g : gs) g.zrun = zrun;
+  auto layout = [mar](Step3<T>& g, char* base) { return mar ? layout3m<T>(g, base) : layout3<T>(g, base); };
   PlanMany<T> pl;
   pl.np = np;
   pl.copy_ = !std::is_same<T, double>::value;
@@ -245,14 +313,14 @@ tmk_status patches3(tmk_context* c, int np, const tmk_fab3* U, const tmk_fab3* B
   std::vector<size_t> offs(np);
   for (int p = 0; p < np; ++p) {
     offs[p] = total;
-    total += layout3<T>(gs[p], nullptr);
+    total += layout(gs[p], nullptr);
     pl.fault_ = pl.fault_ || gs[p].fault;
     for (int d = 0; d < 3; ++d) pl.flux_[d] = pl.flux_[d] || gs[p].F[d];
   }
   tmk_status r = ensure_scratch(c, total, s);
   if (r != TMK_OK) return r;
   char* base = (char*)c->scratch;
-  for (int p = 0; p < np; ++p) layout3<T>(gs[p], base + offs[p]);
+  for (int p = 0; p < np; ++p) layout(gs[p], base + offs[p]);
   // descriptors and prefix sums: one upload (pageable: staged before the call returns)
   std::vector<char> hbuf(head);
   std::memcpy(hbuf.data(), gs.data(), np * sizeof(Step3<T>));
@@ -261,6 +329,10 @@ tmk_status patches3(tmk_context* c, int np, const tmk_fab3* U, const tmk_fab3* B
   TMK_CU(cudaMemcpyAsync(base, hbuf.data(), head, cudaMemcpyHostToDevice, s));
   pl.dgs = (const Step3<T>*)base;
   pl.dstart = (const long long*)(base + soff);
+  if constexpr (std::is_same<T, float>::value) {
+    if (mar)
+      return launch_march_f32(pl, c->hp, c->dp, c->dstatus, dt, dx, s) == cudaSuccess ? TMK_OK : TMK_ERR_CUDA;
+  }
   Side side;
   if (pl.fault_ && (r = ensure_side(c, side)) != TMK_OK) return r;
   cudaError_t e;

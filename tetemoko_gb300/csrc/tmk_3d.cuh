@@ -100,6 +100,12 @@ struct Step3 {
   // with these tracing coefficients
   int fastpred;
   T trA[NSIDE], trB[NSIDE];
+  // the step on characteristic values (tmk_3d_march.cuh): the cells' values,
+  // the fault faces' states and velocities, planes a CTA of its last pass marches
+  void* AF;
+  void* FA;
+  T* FV;
+  int zrun;
 };
 
 template <int D> TMK_HD double rvs(int s) { return (D == 1 && s == 1) ? -1.0 : 1.0; }
@@ -716,6 +722,21 @@ __global__ void __launch_bounds__(128) bdry_final_kernel(const __grid_constant__
   bdry_final_body<T>(*gp, *Pp, st, lt);
 }
 
+// double -> float, rounded to nearest even, by the bit patterns: a conversion
+// instruction holds GB300's FP64 pipe for 64 cycles a warp (18 of them bound
+// this pass).  Numbers outside the normal float range but zero take it.
+template <typename T> TMK_D T narrow(double d) {
+  if constexpr (std::is_same<T, double>::value) {
+    return d;
+  } else {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d), a = hi & 0x7fffffffu;
+    if (a - (897u << 20) >= (253u << 20)) return (a | lo) == 0u ? __uint_as_float(hi) : (float)d;
+    const unsigned t = __funnelshift_l(lo, hi, 3);                     // exponent's low 8 bits, 23 bits of fraction
+    const unsigned f = ((t ^ 0x40000000u) & 0x7fffffffu) | (hi & 0x80000000u);
+    return __uint_as_float(f + (((lo & 0x1fffffffu) + 0x0fffffffu + (t & 1u)) >> 29));
+  }
+}
+
 // FP32 copy of the evolving components of U over Ap (mixed form)
 template <typename T>
 TMK_D void to_pred_body(const Step3<T>& g, long long t) {
@@ -727,7 +748,7 @@ TMK_D void to_pred_body(const Step3<T>& g, long long t) {
 #pragma unroll
   for (int s = 0; s < 2; ++s)
 #pragma unroll
-    for (int c = 0; c < NSIDE; ++c) out[(NSIDE * s + c) * pcs + t] = (T)g.U[(11 * s + c) * acs + o];
+    for (int c = 0; c < NSIDE; ++c) out[(NSIDE * s + c) * pcs + t] = narrow<T>(g.U[(11 * s + c) * acs + o]);
 }
 template <typename T, typename Src>
 __global__ void __launch_bounds__(128) to_pred_kernel(const __grid_constant__ Src src) {
@@ -742,8 +763,17 @@ inline unsigned blocks(long long n) { return (unsigned)((n + 127) / 128); }
 // passes also split into the bulk and the fault plane.
 enum : int {
   K_AP = 0, K_SP0, K_SP1, K_SP2, K_FL1_0, K_FL1_1, K_FL1_1B, K_FL1_1F, K_FL1_2, K_FLF_0, K_FLF_1, K_FLF_1B, K_FLF_1F, K_FLF_2,
-  K_CUR, K_BF, NKIND
+  K_CUR, K_BF,
+  K_VXY, K_VZ, K_PL, K_STEP,      // the passes of tmk_3d_march.cuh
+  NKIND
 };
+
+// Shapes of tmk_3d_march.cuh's work: warps per CTA, updated columns and halo
+// lanes of a warp that predicts x, rows or planes an item marches over; rows of
+// the last pass's tile (two of them halo) and its updated columns.
+constexpr int VAL_WARPS = 4, VAL_COLS = 28, VAL_HALO = 2, VAL_RUN_Y = 16, VAL_RUN_Z = 16;
+constexpr int STEP_ROWS = 8, STEP_COLS = 30, STEP_CTAS = 2;      // STEP_CTAS: resident per SM
+TMK_HD int cdiv(int a, int b) { return (a + b - 1) / b; }
 template <typename T>
 TMK_HD long long kind_count(const Step3<T>& g, int kind) {
   const bool f = g.fault != 0;
@@ -764,6 +794,10 @@ TMK_HD long long kind_count(const Step3<T>& g, int kind) {
     case K_FLF_2: return g.flF[2].cells();
     case K_CUR: return g.cur.cells();
     case K_BF: return f ? (long long)g.cur.n[0] * g.cur.n[2] : 0;
+    case K_VXY: return (long long)cdiv(g.S.n[0], VAL_COLS) * cdiv(g.S.n[1], VAL_RUN_Y) * g.S.n[2];
+    case K_VZ: return (long long)cdiv(g.S.n[0], 32) * g.S.n[1] * cdiv(g.S.n[2], VAL_RUN_Z);
+    case K_PL: return f ? g.fplane.cells() : 0;
+    case K_STEP: return 2LL * cdiv(g.cur.n[0], STEP_COLS) * cdiv(g.cur.n[1], STEP_ROWS - 2) * cdiv(g.cur.n[2], g.zrun);
   }
   return 0;
 }
@@ -882,6 +916,13 @@ cudaError_t launch_one_f32(const PlanOne<float>& pl, const DevParams* P, DevStat
                            const Side* side);
 cudaError_t launch_many_f32(const PlanMany<float>& pl, const DevParams* P, DevStatus* st, cudaStream_t s,
                             const Side* side);
+
+// the step on characteristic values (tmk_3d_march.cuh); hp: the context's
+// parameters on the host
+cudaError_t launch_march_f32(const PlanOne<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
+                             double dt, double dx, cudaStream_t s);
+cudaError_t launch_march_f32(const PlanMany<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
+                             double dt, double dx, cudaStream_t s);
 
 }  // namespace d3
 }  // namespace tmk

@@ -1,6 +1,7 @@
 // The mixed form of the 3-D patch step: FP32 volume arithmetic and
 // intermediates, FP64 state, friction solves and boundary data (tmk_3d.cuh).
 #include "tmk_3d.cuh"
+#include "tmk_3d_march.cuh"
 
 namespace tmk {
 namespace d3 {
@@ -12,6 +13,23 @@ cudaError_t launch_one_f32(const PlanOne<float>& pl, const DevParams* P, DevStat
 cudaError_t launch_many_f32(const PlanMany<float>& pl, const DevParams* P, DevStatus* st, cudaStream_t s,
                             const Side* side) {
   return launch_plan<float>(pl, P, st, s, side);
+}
+
+
+template <typename Plan>
+static cudaError_t march_f32(const Plan& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
+                             double dx, cudaStream_t s) {
+  K3<float> k;
+  k.load(hp, dt, dx);
+  return launch_march3<float>(pl, k, P, st, s);
+}
+cudaError_t launch_march_f32(const PlanOne<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
+                             double dt, double dx, cudaStream_t s) {
+  return march_f32(pl, hp, P, st, dt, dx, s);
+}
+cudaError_t launch_march_f32(const PlanMany<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
+                             double dt, double dx, cudaStream_t s) {
+  return march_f32(pl, hp, P, st, dt, dx, s);
 }
 
 }  // namespace d3

@@ -389,13 +389,22 @@ TMK_D double rs_setbnd_k(const DevParams& P, const RSFaceK& fk, const double* U,
 // (ibcLinElast/SWIBCF.ChF:79-267) as rs_face_solve.  az: the values of the
 // antiplane S pair (syz + Zs rv vz).
 struct SWFaceK { double tau0, mu_s; };
-TMK_D SWFaceK sw_face_k(const DevParams& P, double xcell) {
-  const double x = xcell - P.sw_fbc0;
+// The product rounds before anything is taken from it, in the units built with
+// fused multiply-adds too: whether a face on the rim of a patch or a box lies
+// inside must not depend on the precision.
+TMK_D double cell_centre(int i, double dx) { return __dmul_rn(i + 0.5, dx); }
+template <bool Z3 = false>
+TMK_D SWFaceK sw_face_k(const DevParams& P, double xcell, double zcell = 0.0) {
+  const double x = xcell - P.sw_fbc0, z = zcell - P.sw_fbc1;
   SWFaceK k;
   k.tau0 = 0.0;
-  for (int ip = 0; ip < P.sw_np; ++ip)
-    k.tau0 = k.tau0 + P.sw_tau[ip] * smoothfn(P.sw_smooth, fabs(x - P.sw_xc[ip]) - P.sw_xw[ip]);
-  const double valx = boxcar(P.sw_fbw0, fabs(x));
+  for (int ip = 0; ip < P.sw_np; ++ip) {
+    double v = P.sw_tau[ip] * smoothfn(P.sw_smooth, fabs(x - P.sw_xc[ip]) - P.sw_xw[ip]);
+    if (Z3) v = v * smoothfn(P.sw_smooth, fabs(z - P.sw_zc[ip]) - P.sw_zw[ip]);
+    k.tau0 = k.tau0 + v;
+  }
+  double valx = boxcar(P.sw_fbw0, fabs(x));
+  if (Z3) valx = valx * boxcar(P.sw_fbw1, fabs(z));
   k.mu_s = P.sw_fs * valx + (1 - valx) * P.sw_outside;
   return k;
 }
