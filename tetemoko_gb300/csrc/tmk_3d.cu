@@ -9,6 +9,7 @@
 
 #include "tmk_internal.h"
 #include "tmk_3d.cuh"
+#include "tmk_3d_march.cuh"
 
 namespace tmk {
 namespace d3 {
@@ -20,6 +21,15 @@ cudaError_t launch_one_f64(const PlanOne<double>& pl, const DevParams* P, DevSta
 cudaError_t launch_many_f64(const PlanMany<double>& pl, const DevParams* P, DevStatus* st, cudaStream_t s,
                             const Side* side) {
   return launch_plan<double>(pl, P, st, s, side);
+}
+
+cudaError_t launch_march(const PlanOne<double>& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
+                         double dx, cudaStream_t s) {
+  return launch_march3<double>(pl, hp, P, st, dt, dx, s);
+}
+cudaError_t launch_march(const PlanMany<double>& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
+                         double dx, cudaStream_t s) {
+  return launch_march3<double>(pl, hp, P, st, dt, dx, s);
 }
 
 __global__ void plastic3_kernel(double* U, Bx A, Bx box, const DevParams* P, double dt) {
@@ -177,12 +187,10 @@ size_t layout3(Step3<T>& g, char* base) {
 // predictor (PPM with primitive limiting) and the laws that read only those
 // values; it takes 0.57 of the time of the passes over face states (192x96x96
 // mixed: 792 against 1383 us, and 32 patches of a 96x64x64 level 984 against
-// 1116), whatever the size.  The rest (PLM, CTU, limiting of the characteristic
+// 1116; 64x48x48 FP64: 795 against 2703), whatever the size.  The rest (PLM, CTU, limiting of the characteristic
 // amplitudes, the reference's 9-component slip weakening) keeps those passes.
-template <typename T>
 bool march3(const tmk::DevParams& p) {
-  return std::is_same<T, float>::value && p.order == 2 && p.prim_lim && !p.char_lim &&
-         !(p.fault_law == 2 && p.sw_off != 11);
+  return p.order == 2 && p.prim_lim && !p.char_lim && !(p.fault_law == 2 && p.sw_off != 11);
 }
 
 // its scratch of one patch: the values of the cells of S | fault-face states
@@ -220,10 +228,10 @@ int choose_zrun(const Step3<T>* g, int np) {
     int longest = 1;
     for (int p = 0; p < np; ++p) {
       const int nz = g[p].cur.n[2];
-      n += 2LL * cdiv(g[p].cur.n[0], STEP_COLS) * cdiv(g[p].cur.n[1], STEP_ROWS - 2) * cdiv(nz, std::min(run, nz));
+      n += 2LL * cdiv(g[p].cur.n[0], STEP_COLS) * cdiv(g[p].cur.n[1], step_rows<T> - 2) * cdiv(nz, std::min(run, nz));
       longest = std::max(longest, std::min(run, nz));
     }
-    const double c = (double)((n + STEP_CTAS * sms - 1) / (STEP_CTAS * sms)) * (longest + 2.5);
+    const double c = (double)((n + step_ctas<T> * sms - 1) / (step_ctas<T> * sms)) * (longest + 2.5);
     if (run == 1 << 20 || c < cost) { best = run; cost = c; }
   }
   return best;
@@ -261,13 +269,11 @@ tmk_status patch3(tmk_context* c, const tmk_fab3* U, const tmk_fab3* B, const tm
   PlanOne<T> pl;
   tmk_status r = fill3<T>(c, U, B, Fo, valid, domain, dx, time, dt, pl.g);
   if (r != TMK_OK) return r;
-  if constexpr (std::is_same<T, float>::value) {
-    if (march3<T>(c->hp)) {
-      if ((r = ensure_scratch(c, layout3m<T>(pl.g, nullptr), s)) != TMK_OK) return r;
-      layout3m<T>(pl.g, (char*)c->scratch);
-      pl.g.zrun = choose_zrun(&pl.g, 1);
-      return launch_march_f32(pl, c->hp, c->dp, c->dstatus, dt, dx, s) == cudaSuccess ? TMK_OK : TMK_ERR_CUDA;
-    }
+  if (march3(c->hp)) {
+    if ((r = ensure_scratch(c, layout3m<T>(pl.g, nullptr), s)) != TMK_OK) return r;
+    layout3m<T>(pl.g, (char*)c->scratch);
+    pl.g.zrun = choose_zrun(&pl.g, 1);
+    return launch_march(pl, c->hp, c->dp, c->dstatus, dt, dx, s) == cudaSuccess ? TMK_OK : TMK_ERR_CUDA;
   }
   if ((r = ensure_scratch(c, layout3<T>(pl.g, nullptr), s)) != TMK_OK) return r;
   layout3<T>(pl.g, (char*)c->scratch);
@@ -293,7 +299,7 @@ tmk_status patches3(tmk_context* c, int np, const tmk_fab3* U, const tmk_fab3* B
     const tmk_status r = fill3<T>(c, U + p, B ? B + p : nullptr, Fo, valid + p, domain, dx, time, dt, gs[p]);
     if (r != TMK_OK) return r;
   }
-  const bool mar = march3<T>(c->hp);
+  const bool mar = march3(c->hp);
   const int zrun = choose_zrun(gs.data(), np);
   for (Step3<T>& g : gs) g.zrun = zrun;
   auto layout = [mar](Step3<T>& g, char* base) { return mar ? layout3m<T>(g, base) : layout3<T>(g, base); };
@@ -329,10 +335,7 @@ tmk_status patches3(tmk_context* c, int np, const tmk_fab3* U, const tmk_fab3* B
   TMK_CU(cudaMemcpyAsync(base, hbuf.data(), head, cudaMemcpyHostToDevice, s));
   pl.dgs = (const Step3<T>*)base;
   pl.dstart = (const long long*)(base + soff);
-  if constexpr (std::is_same<T, float>::value) {
-    if (mar)
-      return launch_march_f32(pl, c->hp, c->dp, c->dstatus, dt, dx, s) == cudaSuccess ? TMK_OK : TMK_ERR_CUDA;
-  }
+  if (mar) return launch_march(pl, c->hp, c->dp, c->dstatus, dt, dx, s) == cudaSuccess ? TMK_OK : TMK_ERR_CUDA;
   Side side;
   if (pl.fault_ && (r = ensure_side(c, side)) != TMK_OK) return r;
   cudaError_t e;

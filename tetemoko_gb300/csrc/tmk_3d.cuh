@@ -772,7 +772,9 @@ enum : int {
 // lanes of a warp that predicts x, rows or planes an item marches over; rows of
 // the last pass's tile (two of them halo) and its updated columns.
 constexpr int VAL_WARPS = 4, VAL_COLS = 28, VAL_HALO = 2, VAL_RUN_Y = 16, VAL_RUN_Z = 16;
-constexpr int STEP_ROWS = 8, STEP_COLS = 30, STEP_CTAS = 2;      // STEP_CTAS: resident per SM
+constexpr int STEP_COLS = 30;
+template <typename T> constexpr int step_rows = sizeof(T) == 4 ? 8 : 12;
+template <typename T> constexpr int step_ctas = sizeof(T) == 4 ? 2 : 1;   // resident per SM
 TMK_HD int cdiv(int a, int b) { return (a + b - 1) / b; }
 template <typename T>
 TMK_HD long long kind_count(const Step3<T>& g, int kind) {
@@ -797,7 +799,7 @@ TMK_HD long long kind_count(const Step3<T>& g, int kind) {
     case K_VXY: return (long long)cdiv(g.S.n[0], VAL_COLS) * cdiv(g.S.n[1], VAL_RUN_Y) * g.S.n[2];
     case K_VZ: return (long long)cdiv(g.S.n[0], 32) * g.S.n[1] * cdiv(g.S.n[2], VAL_RUN_Z);
     case K_PL: return f ? g.fplane.cells() : 0;
-    case K_STEP: return 2LL * cdiv(g.cur.n[0], STEP_COLS) * cdiv(g.cur.n[1], STEP_ROWS - 2) * cdiv(g.cur.n[2], g.zrun);
+    case K_STEP: return 2LL * cdiv(g.cur.n[0], STEP_COLS) * cdiv(g.cur.n[1], step_rows<T> - 2) * cdiv(g.cur.n[2], g.zrun);
   }
   return 0;
 }
@@ -919,10 +921,10 @@ cudaError_t launch_many_f32(const PlanMany<float>& pl, const DevParams* P, DevSt
 
 // the step on characteristic values (tmk_3d_march.cuh); hp: the context's
 // parameters on the host
-cudaError_t launch_march_f32(const PlanOne<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
-                             double dt, double dx, cudaStream_t s);
-cudaError_t launch_march_f32(const PlanMany<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
-                             double dt, double dx, cudaStream_t s);
+cudaError_t launch_march(const PlanOne<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
+                         double dx, cudaStream_t s);
+cudaError_t launch_march(const PlanMany<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
+                         double dx, cudaStream_t s);
 
 }  // namespace d3
 }  // namespace tmk

@@ -15,21 +15,13 @@ cudaError_t launch_many_f32(const PlanMany<float>& pl, const DevParams* P, DevSt
   return launch_plan<float>(pl, P, st, s, side);
 }
 
-
-template <typename Plan>
-static cudaError_t march_f32(const Plan& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
-                             double dx, cudaStream_t s) {
-  K3<float> k;
-  k.load(hp, dt, dx);
-  return launch_march3<float>(pl, k, P, st, s);
+cudaError_t launch_march(const PlanOne<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
+                         double dx, cudaStream_t s) {
+  return launch_march3<float>(pl, hp, P, st, dt, dx, s);
 }
-cudaError_t launch_march_f32(const PlanOne<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
-                             double dt, double dx, cudaStream_t s) {
-  return march_f32(pl, hp, P, st, dt, dx, s);
-}
-cudaError_t launch_march_f32(const PlanMany<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st,
-                             double dt, double dx, cudaStream_t s) {
-  return march_f32(pl, hp, P, st, dt, dx, s);
+cudaError_t launch_march(const PlanMany<float>& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt,
+                         double dx, cudaStream_t s) {
+  return launch_march3<float>(pl, hp, P, st, dt, dx, s);
 }
 
 }  // namespace d3

@@ -27,7 +27,8 @@
 // the step (about 450 us) issue, 500 instructions a cell and side, with L2 close
 // behind (144 B of values read, 144 B of FP64 state read and written a cell and
 // side, plus the tile's halo).  The whole step 792 us; one pass per term, each
-// through memory, took 1383 us.
+// through memory, took 1383 us.  FP64 (64x48x48): every kernel the FP64 pipe,
+// which the first two keep 70 % and the last 82 % busy; 795 us, was 2703 us.
 #pragma once
 
 #include "tmk_3d.cuh"
@@ -414,12 +415,14 @@ TMK_D void store_flux(const Step3<T>& g, const K3<T>& k, T rvs, int s, int i, in
 // plane m arrives, the stages that need nothing above it are done for m, then
 // plane m - 1 is finished.  8 rows at two CTAs per SM (128 registers, a few
 // spilled): the whole step of a 192x96x96 patch took 792 us, against 828 us with
-// 16 rows and 1015 us with 12 rows at one CTA (no spills, too few warps).
+// 16 rows and 1015 us with 12 rows at one CTA (no spills, too few warps).  FP64
+// 12 rows, one CTA: 795 us for a 64x48x48 patch, 814 with 8 rows (more halo) and
+// 834 with 16 (spills).
 template <typename T, typename Src>
-__global__ void __launch_bounds__(32 * STEP_ROWS, STEP_CTAS)
+__global__ void __launch_bounds__(32 * step_rows<T>, step_ctas<T>)
 step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
   using V = typename PairOf<T>::P;
-  constexpr int NR = STEP_ROWS;
+  constexpr int NR = step_rows<T>;
   // [9] A_y, WHalf2[1][0] of plane m, WHalf2[1][2] of plane m - 1; [3] the final y values of plane m - 1
   extern __shared__ __align__(16) unsigned char step_smem[];
   V (*const s1)[NR + 2][32] = reinterpret_cast<V (*)[NR + 2][32]>(step_smem);
@@ -859,11 +862,15 @@ __global__ void __launch_bounds__(64) plane_kernel(const __grid_constant__ Src s
 template <typename T, int DM> constexpr size_t val_smem_bytes() {
   return (size_t)VAL_WARPS * 4 * kValComps<DM> * 32 * 2 * sizeof(T);
 }
-template <typename T> constexpr size_t step_smem_bytes() { return (size_t)12 * (STEP_ROWS + 2) * 32 * 2 * sizeof(T); }
+template <typename T> constexpr size_t step_smem_bytes() { return (size_t)12 * (step_rows<T> + 2) * 32 * 2 * sizeof(T); }
 
-// The whole step on stream s (One: one patch, Many: a batch).
+// The whole step on stream s (One: one patch, Many: a batch); hp: the context's
+// parameters on the host.
 template <typename T, typename Plan>
-cudaError_t launch_march3(const Plan& pl, const K3<T>& k, const DevParams* P, DevStatus* st, cudaStream_t s) {
+cudaError_t launch_march3(const Plan& pl, const DevParams& hp, const DevParams* P, DevStatus* st, double dt, double dx,
+                          cudaStream_t s) {
+  K3<T> k;
+  k.load(hp, dt, dx);
   using Src = typename Plan::Src;
   static const cudaError_t configured = [] {
     cudaError_t e = cudaFuncSetAttribute(values_kernel<T, 1, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -885,7 +892,7 @@ cudaError_t launch_march3(const Plan& pl, const K3<T>& k, const DevParams* P, De
       pl.src(K_VZ), k, nz);
   if (pl.fault())
     plane_kernel<T, Src><<<(unsigned)((pl.n(K_PL) + 63) / 64), 64, 0, s>>>(pl.src(K_PL), k, P, st);
-  step_kernel<T, Src><<<(unsigned)pl.n(K_STEP), 32 * STEP_ROWS, step_smem_bytes<T>(), s>>>(pl.src(K_STEP), k);
+  step_kernel<T, Src><<<(unsigned)pl.n(K_STEP), 32 * step_rows<T>, step_smem_bytes<T>(), s>>>(pl.src(K_STEP), k);
   return cudaGetLastError();
 }
 

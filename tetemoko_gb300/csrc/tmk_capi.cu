@@ -383,18 +383,21 @@ extern "C" tmk_status tmk_patch_update_state(tmk_context* c, const tmk_fab* U, c
   cudaStream_t s = (cudaStream_t)stream;
   const int anx = U->hi[0] - U->lo[0] + 1, any = U->hi[1] - U->lo[1] + 1;
   const size_t ucount = (size_t)TMK_NCOMP * anx * any;
+  // the marching kernels (128x128 with fluxes: 83 us against the tile kernel's
+  // 557) find their items by index; PLM runs the tile kernel
+  const bool march = uses_march(c->scheme);
   std::vector<TileDev> tiles;
-  make_tiles(tiles, 0, *valid, tmk::Launch<double>::TX, tmk::Launch<double>::TY);
+  if (!march) make_tiles(tiles, 0, *valid, tmk::Launch<double>::TX, tmk::Launch<double>::TY);
   const int nfirst = nvx + 2;
-  // scratch: Uout | first | ffault | PatchDev | tiles | fault patch index
+  // scratch: Uout | first | ffault | PatchDev and fault patch index | tiles | tensor map
+  struct Head { PatchDev<double> pd; int fault_patch; };
   size_t off_u = 0;
   size_t off_first = align_up(off_u + ucount * sizeof(double));
   size_t off_ff = align_up(off_first + (size_t)TMK_NCOMP * nfirst * sizeof(double));
   size_t off_pd = align_up(off_ff + (size_t)TMK_NCOMP * nvx * sizeof(double));
-  size_t off_tl = align_up(off_pd + sizeof(PatchDev<double>));
-  size_t off_fp = align_up(off_tl + tiles.size() * sizeof(TileDev));
-  size_t off_tm = align_up(off_fp + sizeof(int));
-  size_t total = align_up(off_tm + sizeof(CUtensorMap));
+  size_t off_tl = align_up(off_pd + sizeof(Head));
+  size_t off_tm = align_up(off_tl + tiles.size() * sizeof(TileDev));
+  size_t total = align_up(off_tm + (march ? 0 : sizeof(CUtensorMap)));
   if (total > c->scratch_bytes) {
     TMK_CU(cudaStreamSynchronize(s));
     cudaFree(c->scratch);
@@ -403,8 +406,9 @@ extern "C" tmk_status tmk_patch_update_state(tmk_context* c, const tmk_fab* U, c
     c->scratch_bytes = total;
   }
   char* base = (char*)c->scratch;
-  PatchDev<double> pd;
-  std::memset(&pd, 0, sizeof(pd));
+  Head head;
+  std::memset(&head, 0, sizeof(head));
+  PatchDev<double>& pd = head.pd;
   pd.Uin = U->data;
   pd.Uout = (double*)(base + off_u);
   pd.alo0 = U->lo[0]; pd.alo1 = U->lo[1]; pd.anx = anx; pd.any = any;
@@ -422,22 +426,25 @@ extern "C" tmk_status tmk_patch_update_state(tmk_context* c, const tmk_fab* U, c
   pd.status = c->dstatus;
   // the tile kernel stages its tiles with TMA when U's layout allows a tensor map
   alignas(64) unsigned char tmap[sizeof(CUtensorMap)];
-  const bool use_tma = encode_fab_map(tmap, U->data, (int)sizeof(double), anx, any,
-                                      tmk::Launch<double>::volume_box_x(), tmk::Launch<double>::volume_box_y());
+  const bool use_tma = !march && encode_fab_map(tmap, U->data, (int)sizeof(double), anx, any,
+                                                tmk::Launch<double>::volume_box_x(), tmk::Launch<double>::volume_box_y());
   pd.tmap = use_tma ? (const void*)(base + off_tm) : nullptr;
-  const int zero = 0;
   // descriptors are staged through pageable memory: synchronous with respect to the host
-  TMK_CU(cudaMemcpyAsync(base + off_pd, &pd, sizeof(pd), cudaMemcpyHostToDevice, s));
-  TMK_CU(cudaMemcpyAsync(base + off_tl, tiles.data(), tiles.size() * sizeof(TileDev), cudaMemcpyHostToDevice, s));
-  TMK_CU(cudaMemcpyAsync(base + off_fp, &zero, sizeof(int), cudaMemcpyHostToDevice, s));
-  if (use_tma) TMK_CU(cudaMemcpyAsync(base + off_tm, tmap, sizeof(tmap), cudaMemcpyHostToDevice, s));
-  if (Fx) TMK_CU(cudaMemsetAsync(Fx->data, 0, (size_t)TMK_NCOMP * (nvx + 1) * nvy * sizeof(double), s));
-  if (Fy) TMK_CU(cudaMemsetAsync(Fy->data, 0, (size_t)TMK_NCOMP * nvx * (nvy + 1) * sizeof(double), s));
+  TMK_CU(cudaMemcpyAsync(base + off_pd, &head, sizeof(head), cudaMemcpyHostToDevice, s));
   const PatchDev<double>* dpd = (const PatchDev<double>*)(base + off_pd);
+  const int* dfp = (const int*)(base + off_pd + offsetof(Head, fault_patch));
   if (fault)
-    TMK_CU(tmk::Launch<double>::fault(dpd, (const int*)(base + off_fp), 1, nvx, c->dp, c->hp, dt, dx, time, c->dstatus, false,
+    TMK_CU(tmk::Launch<double>::fault(dpd, dfp, 1, nvx, c->dp, c->hp, dt, dx, time, c->dstatus, false,
                                         tmk::fault_seg_of(c->hp, tmk::FAULT_SEG), s));
-  TMK_CU(tmk::Launch<double>::volume(dpd, (const TileDev*)(base + off_tl), (int)tiles.size(), c->dp, s));
+  if (march) {
+    TMK_CU(tmk::patch_march(dpd, nvx, nvy, fault, c->hp, dt, dx, s));
+  } else {
+    TMK_CU(cudaMemcpyAsync(base + off_tl, tiles.data(), tiles.size() * sizeof(TileDev), cudaMemcpyHostToDevice, s));
+    if (use_tma) TMK_CU(cudaMemcpyAsync(base + off_tm, tmap, sizeof(tmap), cudaMemcpyHostToDevice, s));
+    if (Fx) TMK_CU(cudaMemsetAsync(Fx->data, 0, (size_t)TMK_NCOMP * (nvx + 1) * nvy * sizeof(double), s));
+    if (Fy) TMK_CU(cudaMemsetAsync(Fy->data, 0, (size_t)TMK_NCOMP * nvx * (nvy + 1) * sizeof(double), s));
+    TMK_CU(tmk::Launch<double>::volume(dpd, (const TileDev*)(base + off_tl), (int)tiles.size(), c->dp, s));
+  }
   // the volume kernel writes the nine evolving components of each side;
   // lambda and gamma are left untouched, as updateState leaves them
   for (int sd = 0; sd < 2; ++sd)
@@ -1299,11 +1306,12 @@ struct CtxView {
   int fault_law;
   int nb;
   double max_speed;
+  bool march;
 };
 CtxView context_view(const tmk_context* c) {
   CtxView v;
   v.dp = c->dp; v.hp = &c->hp; v.st = c->dstatus; v.fault_law = c->scheme.fault_law; v.nb = c->nb;
-  v.max_speed = std::max(c->hp.cs, c->hp.cp);
+  v.max_speed = std::max(c->hp.cs, c->hp.cp); v.march = uses_march(c->scheme);
   return v;
 }
 }  // namespace tmk

@@ -5,6 +5,55 @@ TMK_INSTANTIATE_LAUNCH(double, 16, 8, 256)
 
 namespace tmk {
 
+// ---- one patch by itself on the marching kernels
+template <int G, int SCH>
+static cudaError_t patch_group(const PatchDev<double>* dpd, int nx, int ny, MarchConst<double>& mc, bool pdl,
+                               cudaStream_t s) {
+  constexpr size_t smem = march_smem_bytes<double, G, true>();
+  auto* const kernel = march_kernel<double, G, false, SCH, true>;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (configured != cudaSuccess) return configured;
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // One FP64 warp nearly fills a sub-partition's pipe, an item costs about
+  // three rows beyond its own, and the other group's items (half the work) run
+  // beside these: the shortest run that leaves no sub-partition with two.
+  const int ns = (nx + MARCH_COLS - 1) / MARCH_COLS;
+  double cost = 0.0;
+  for (int run = 64; run >= 1; run /= 2) {
+    const double per = 1.5 * ns * ((ny + run - 1) / run) / (4.0 * sms);
+    const double c = (run + 3) * (per > 1.0 ? per : 1.0);
+    if (run == 64 || c < cost) { mc.patch_run = run; cost = c; }
+  }
+  const int nitems = ns * ((ny + mc.patch_run - 1) / mc.patch_run);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(32 * MARCH_WARPS);
+  cfg.gridDim = dim3((nitems + MARCH_WARPS - 1) / MARCH_WARPS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = pdl ? attr : nullptr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, dpd, (const MarchItem*)nullptr, nitems, mc);
+}
+
+cudaError_t patch_march(const PatchDev<double>* dpd, int nx, int ny, bool fault, const DevParams& hp, double dt,
+                        double dx, cudaStream_t s) {
+  MarchConst<double> mc;
+  mc.load(hp, dt, dx);
+  mc.stash[0] = mc.stash[1] = nullptr;
+  mc.caps[0] = mc.caps[1] = nullptr;
+  const bool fx = march_scheme_fixed(mc);
+  cudaError_t e = fx ? patch_group<0, MARCH_SCH_PPM_PRIM>(dpd, nx, ny, mc, fault, s)
+                     : patch_group<0, MARCH_SCH_RUNTIME>(dpd, nx, ny, mc, fault, s);
+  if (e != cudaSuccess) return e;
+  return fx ? patch_group<1, MARCH_SCH_PPM_PRIM>(dpd, nx, ny, mc, true, s)
+            : patch_group<1, MARCH_SCH_RUNTIME>(dpd, nx, ny, mc, true, s);
+}
+
 __global__ void plastic_fab_kernel(double* U, int alo0, int alo1, int anx, int any, int lo0, int lo1, int hi0,
                                    int hi1, const DevParams* P, double dt) {
   const int nx = hi0 - lo0 + 1, ny = hi1 - lo1 + 1;

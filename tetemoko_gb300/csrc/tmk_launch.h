@@ -67,6 +67,13 @@ struct Launch {
   static const void* fault_entry(int seg);
 };
 
+// The volume update of one FP64 patch (dpd: its descriptor on the device, nx by
+// ny valid cells) by the marching kernels, fluxes of all its faces included
+// where it has arrays for them; with a fault the fault kernel is the launch
+// before it in the stream.
+cudaError_t patch_march(const PatchDev<double>* dpd, int nx, int ny, bool fault, const DevParams& hp, double dt,
+                        double dx, cudaStream_t s);
+
 // FP64 <-> Real conversion of a FAB on the device
 cudaError_t convert_d2f(const double* src, float* dst, size_t n, cudaStream_t s);
 cudaError_t convert_f2d(const float* src, double* dst, size_t n, cudaStream_t s);

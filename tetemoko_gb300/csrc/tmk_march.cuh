@@ -211,6 +211,7 @@ struct MarchConst {
   PlasticK<T> pk;
   T pdt;
   int plastic;
+  int patch_run;     // rows of an item of the patch form, which has no work list
   TMK_HD void load(const DevParams& p, double dt, double dx) {
     kx.load(p, 0, dt / dx);
     ky.load(p, 1, dt / dx);
@@ -218,7 +219,7 @@ struct MarchConst {
     for (int c = 0; c < 9; ++c) nbg[c] = (T)-p.bg[c];
     plim = p.prim_lim != 0; clim = p.char_lim != 0; lim = plim || clim; ppm = p.order != 0;
     xout_lo = p.bc[0] == 0; xout_hi = p.bc[1] == 0; yout_lo = p.bc[2] == 0; yout_hi = p.bc[3] == 0;
-    plastic = 0;
+    plastic = 0; patch_run = 0;
     pk.load(p);
     pdt = (T)dt;
   }
@@ -467,9 +468,10 @@ template <typename T, int G>
 constexpr size_t march_warp_pairs() {
   return (size_t)MARCH_RING * march_row_pairs<T, G>() + (kSlopesInSmem<T, G> ? 8 * 32 : 0);
 }
-template <typename T, int G>
+template <typename T, int G, bool PATCH = false>
 constexpr size_t march_smem_bytes() {
-  return (size_t)MARCH_WARPS * march_warp_pairs<T, G>() * sizeof(typename PairOf<T>::P);
+  const size_t stash = PATCH ? (size_t)MARCH_STASH_VECS * Grp<G>::N * 32 : 0;
+  return (size_t)MARCH_WARPS * (march_warp_pairs<T, G>() + stash) * sizeof(typename PairOf<T>::P);
 }
 
 // resident CTAs per SM the register allocation targets: FP32 in-plane 4 (128
@@ -591,10 +593,42 @@ constexpr int MARCH_SCH_RUNTIME = 0, MARCH_SCH_PPM_PRIM = 1;
 template <typename T>
 TMK_HD bool march_scheme_fixed(const MarchConst<T>& mc) { return mc.ppm && mc.plim && !mc.clim; }
 
+// Fluxes of the patch form (GETFLUXF over all faces of the valid box): a cell
+// of row `row` stores its lo faces, the last one of a row or column its hi face
+// too; the antiplane group also zeroes the components without a flux (plastic
+// rate and strain).
+template <typename T, int G, int D>
+TMK_D void store_face(const PatchDev<T>& pp, int x, int row, const typename PairOf<T>::P* F) {
+  constexpr int N = Grp<G>::N;
+  const int nx = pp.vhi0 - pp.vlo0 + (D == 0 ? 2 : 1), ny = pp.vhi1 - pp.vlo1 + (D == 0 ? 1 : 2);
+  const unsigned plane = (unsigned)nx * (unsigned)ny;
+  T* const f = (D == 0 ? pp.Fx : pp.Fy) + ((long long)(row - pp.vlo1) * nx + (x - pp.vlo0));
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    *plane_ptr(f, plane, Grp<G>::glob(c)) = F[c].x;
+    *plane_ptr(f, plane, 11 + Grp<G>::glob(c)) = F[c].y;
+  }
+  if constexpr (G == 1) {
+#pragma unroll
+    for (int c = 9; c < 11; ++c) { *plane_ptr(f, plane, c) = T(0); *plane_ptr(f, plane, 11 + c) = T(0); }
+  }
+}
+
+template <typename T, int G>
+TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const MarchConst<T>& mc, int lane,
+                            const typename PairOf<T>::P* st, bool faces);
+
 // PL: a plastic level with the fused return (in-plane group only): every
 // stored cell takes the plastic return, and the kernel runs after the
 // antiplane one.
-template <typename T, int G, bool PL = false, int SCH = MARCH_SCH_RUNTIME>
+// PATCH: one patch by itself (patches[0]), items by index (strips of columns
+// fastest, runs of mc.patch_run rows), the fluxes of all faces where the patch
+// has arrays for them; an item on the fault keeps its row 0 in shared memory,
+// waits for the fault kernel when the rest of its rows are done and finishes it.
+// FP64 128x128 with fluxes: 83 us a call (in-plane 74, beside it the antiplane
+// kernel and the fault kernel's 48), bound by the FP64 pipe of the one warp a
+// sub-partition holds; the tile kernel, which forms face states, 557 us.
+template <typename T, int G, bool PL = false, int SCH = MARCH_SCH_RUNTIME, bool PATCH = false>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value) march_kernel(const PatchDev<T>* __restrict__ patches,
                                                                  const MarchItem* __restrict__ items, int nitems,
                                                                  const __grid_constant__ MarchConst<T> mc) {
@@ -614,7 +648,20 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   }
   // the fused plastic return reads the antiplane kernel's stresses: wait for it
   if (PL) asm volatile("griddepcontrol.wait;" ::: "memory");
-  const MarchItem it = items[wid];
+  MarchItem it;
+  if constexpr (PATCH) {
+    const PatchDev<T>& p0 = patches[0];
+    const unsigned ns = (unsigned)(p0.vhi0 - p0.vlo0 + MARCH_COLS) / MARCH_COLS, r = (unsigned)wid / ns;
+    it.patch = 0;
+    it.x0 = p0.vlo0 + (int)((unsigned)wid - r * ns) * MARCH_COLS;
+    it.y0 = p0.vlo1 + (int)r * mc.patch_run;
+    it.y1 = min(it.y0 + mc.patch_run - 1, p0.vhi1);
+    it.fslot = p0.fault && it.y0 == p0.dlo1 ? 0 : -1;
+    it.cap0 = 0;
+    it.ncap = 0;
+  } else {
+    it = items[wid];
+  }
   const PatchDev<T>& pp = patches[it.patch];
   const int x = it.x0 - MARCH_HALO + lane;
   const int dlo0 = pp.dlo0, dhi0 = pp.dhi0, dlo1 = pp.dlo1, dhi1 = pp.dhi1;
@@ -632,7 +679,14 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   const MK<T>& kx = mc.kx;
   const MK<T>& ky = mc.ky;
   const bool fault = pp.fault != 0;
-  const bool defer0 = it.fslot >= 0;      // row 0 is finished by march_fault_row_kernel
+  const bool defer0 = it.fslot >= 0;      // row 0 is finished by march_fault_row_kernel (PATCH: at the end)
+  // what a fault-row item keeps for its row 0
+  P* stash0 = nullptr;
+  if constexpr (PATCH)
+    stash0 = reinterpret_cast<P*>(march_smem) + (size_t)MARCH_WARPS * march_warp_pairs<T, G>() +
+             (size_t)(threadIdx.x >> 5) * MARCH_STASH_VECS * N * 32 + lane;
+  else if (defer0)
+    stash0 = reinterpret_cast<P*>(mc.stash[G]) + (size_t)it.fslot * MARCH_STASH_VECS * N * 32 + lane;
   const bool col_valid = x >= it.x0 && x < it.x0 + MARCH_COLS && x >= pp.vlo0 && x <= pp.vhi0;
   const int anx = pp.anx;
   const unsigned plane = (unsigned)anx * (unsigned)pp.any;
@@ -865,8 +919,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
     }
     const int yr = q - 1;
     if (defer0 && yr == dlo1) {
-      // row 0 of a fault patch: keep what march_fault_row_kernel needs
-      P* st = reinterpret_cast<P*>(mc.stash[G]) + (size_t)it.fslot * MARCH_STASH_VECS * N * 32 + lane;
+      // row 0 of a fault patch: keep what fault_row_finish needs
+      P* const st = stash0;
       const P* wo = ring + r_m1 + lane + 1;
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
@@ -913,6 +967,24 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
             face_flux<G, 1, T>(ky, in.Bny, below, F);
           }
         });
+      if constexpr (PATCH) {
+        if (col_valid && yr <= it.y1) {
+          P F[N];
+          if (pp.Fx) {
+            face_flux<G, 0, T>(kx, in.Anx, BpL, F);
+            store_face<T, G, 0>(pp, x, yr, F);
+            if (x == pp.vhi0) { face_flux<G, 0, T>(kx, BnR, in.Apx, F); store_face<T, G, 0>(pp, x + 1, yr, F); }
+          }
+          if (pp.Fy) {
+            P below[NW];
+#pragma unroll
+            for (int w = 0; w < NW; ++w) below[w] = psub(in.Bpy[w], in.jpB[w]);
+            face_flux<G, 1, T>(ky, in.Bny, below, F);
+            store_face<T, G, 1>(pp, x, yr, F);
+            if (yr == pp.vhi1) { face_flux<G, 1, T>(ky, Bn_q, in.Bpy, F); store_face<T, G, 1>(pp, x, yr + 1, F); }
+          }
+        }
+      }
     }
     sdst += anx;
     const int freed = r_m1;
@@ -939,19 +1011,23 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if constexpr (PATCH) {
+    if (defer0) fault_row_finish<T, G>(pp, it, mc, lane, stash0, true);
+  }
 }
 
 // Row 0 of a fault-row strip of group G once the fault kernel has produced the
 // first-pass fault states and the fault-face fluxes: the transverse correction
 // of the row's x values, its final x faces and its update (the same steps as
-// the marching loop, with the stashed row-0 values).
+// the marching loop, with the stashed row-0 values; st: the lane's).  faces: the
+// patch form's fluxes too.
 template <typename T, int G>
-TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const MarchConst<T>& mc, int lane) {
+TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const MarchConst<T>& mc, int lane,
+                            const typename PairOf<T>::P* st, bool faces) {
   using P = typename PairOf<T>::P;
   constexpr int N = Grp<G>::N, NW = kWaves<G>;
   const int x = it.x0 - MARCH_HALO + lane;
   const int dlo0 = pp.dlo0, dhi0 = pp.dhi0, dlo1 = pp.dlo1;
-  const P* st = reinterpret_cast<const P*>(mc.stash[G]) + (size_t)it.fslot * MARCH_STASH_VECS * N * 32 + lane;
   P Bnx[NW], Bpx[NW], An1[NW], Ap0[NW], Bn1[NW], Bp0[NW], u[N], Fy0[N], Fy1[N];
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
@@ -1004,6 +1080,18 @@ TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const Ma
     });
   }
   const bool col_valid = x >= it.x0 && x < it.x0 + MARCH_COLS && x >= pp.vlo0 && x <= pp.vhi0;
+  if (faces && col_valid) {
+    P F[N];
+    if (pp.Fx) {
+      face_flux<G, 0, T>(mc.kx, Bnx, BpL, F);
+      store_face<T, G, 0>(pp, x, dlo1, F);
+      if (x == pp.vhi0) { face_flux<G, 0, T>(mc.kx, BnR, Bpx, F); store_face<T, G, 0>(pp, x + 1, dlo1, F); }
+    }
+    if (pp.Fy) {
+      store_face<T, G, 1>(pp, x, dlo1, Fy0);
+      if (pp.vhi1 == dlo1) store_face<T, G, 1>(pp, x, dlo1 + 1, Fy1);
+    }
+  }
   if (col_valid) {
 #pragma unroll
     for (int w = 0; w < NW; ++w) { jn[w] = psub(BnR[w], Bnx[w]); jp[w] = psub(Bpx[w], BpL[w]); }
@@ -1035,12 +1123,15 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS) march_fault_row_kernel(const
                                                                            const __grid_constant__ MarchConst<T> mc) {
   const int wid = blockIdx.x * MARCH_WARPS + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  auto stash = [&](const MarchItem& it, int g, int n) {
+    return reinterpret_cast<const typename PairOf<T>::P*>(mc.stash[g]) + (size_t)it.fslot * MARCH_STASH_VECS * n * 32 + lane;
+  };
   if (wid < n0) {
     const MarchItem it = rows0[wid];
-    fault_row_finish<T, 0>(patches[it.patch], it, mc, lane);
+    fault_row_finish<T, 0>(patches[it.patch], it, mc, lane, stash(it, 0, Grp<0>::N), false);
   } else if (wid < n0 + n1) {
     const MarchItem it = rows1[wid - n0];
-    fault_row_finish<T, 1>(patches[it.patch], it, mc, lane);
+    fault_row_finish<T, 1>(patches[it.patch], it, mc, lane, stash(it, 1, Grp<1>::N), false);
   }
 }
 

@@ -21,6 +21,7 @@ struct CtxView {
   int fault_law;
   int nb;
   double max_speed;
+  bool march;
 };
 CtxView context_view(const tmk_context* c);
 }  // namespace tmk
@@ -86,15 +87,14 @@ tmk_status scratch_address(void** out) {
 
 size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-// Writes the patch descriptor, the fault-patch index and the tile list of the
-// valid box into the scratch (replacing the host-to-device copies of the
+// Writes the patch descriptor, the fault-patch index and (the tile kernel's) the
+// tile list of the valid box into the scratch (replacing the host-to-device copies of the
 // allocating entry point).
 __global__ void noalloc_setup_kernel(tmk::PatchDev<double> pd, tmk::PatchDev<double>* dpd, int* fault_idx,
-                                     tmk::TileDev* tiles, int TX, int TY) {
-  const int nx = pd.vhi0 - pd.vlo0 + 1, ny = pd.vhi1 - pd.vlo1 + 1;
-  const int ntx = (nx + TX - 1) / TX, nty = (ny + TY - 1) / TY;
+                                     tmk::TileDev* tiles, int ntiles, int TX, int TY) {
+  const int ntx = (pd.vhi0 - pd.vlo0 + TX) / TX;
   if (blockIdx.x == 0 && threadIdx.x == 0) { *dpd = pd; *fault_idx = 0; }
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntx * nty; t += gridDim.x * blockDim.x) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
     tmk::TileDev tl;
     tl.patch = 0;
     tl.x0 = pd.vlo0 + (t % ntx) * TX;
@@ -139,7 +139,9 @@ extern "C" tmk_status tmk_patch_update_state_noalloc(tmk_context* c, const tmk_f
              Fy->lo[1] != v.lo[1] || Fy->hi[1] != v.hi[1] + 1))
     return TMK_ERR_BAD_DESC;
 
-  // layout of the scratch: descriptor | fault index | tiles | updated state | fault buffers
+  // layout of the scratch: descriptor | fault index | tiles (room for them in
+  // either form: which patches fit does not depend on the scheme) | updated
+  // state | fault buffers
   const int TX = tmk::Launch<double>::TX, TY = tmk::Launch<double>::TY;
   const int ntiles = ((nvx + TX - 1) / TX) * ((nvy + TY - 1) / TY);
   const int anx = U->hi[0] - U->lo[0] + 1, any = U->hi[1] - U->lo[1] + 1;
@@ -179,14 +181,19 @@ extern "C" tmk_status tmk_patch_update_state_noalloc(tmk_context* c, const tmk_f
   tmk::PatchDev<double>* dpd = (tmk::PatchDev<double>*)(base + off_pd);
   int* dfi = (int*)(base + off_fi);
   tmk::TileDev* dtl = (tmk::TileDev*)(base + off_tl);
-  const int sblocks = std::min(1024, std::max(1, (ntiles + 255) / 256));
-  noalloc_setup_kernel<<<sblocks, 256, 0, s>>>(pd, dpd, dfi, dtl, TX, TY);
+  const int listed = cv.march ? 0 : ntiles;
+  const int sblocks = std::min(1024, std::max(1, (listed + 255) / 256));
+  noalloc_setup_kernel<<<sblocks, 256, 0, s>>>(pd, dpd, dfi, dtl, listed, TX, TY);
   TMK_CU(cudaGetLastError());
-  if (Fx) TMK_CU(cudaMemsetAsync(Fx->data, 0, (size_t)TMK_NCOMP * (nvx + 1) * nvy * sizeof(double), s));
-  if (Fy) TMK_CU(cudaMemsetAsync(Fy->data, 0, (size_t)TMK_NCOMP * nvx * (nvy + 1) * sizeof(double), s));
   if (fault) TMK_CU(tmk::Launch<double>::fault(dpd, dfi, 1, nvx, cv.dp, *cv.hp, dt, dx, time, cv.st, false,
                                               tmk::fault_seg_of(*cv.hp, tmk::FAULT_SEG), s));
-  TMK_CU(tmk::Launch<double>::volume(dpd, dtl, ntiles, cv.dp, s));
+  if (cv.march) {
+    TMK_CU(tmk::patch_march(dpd, nvx, nvy, fault, *cv.hp, dt, dx, s));
+  } else {
+    if (Fx) TMK_CU(cudaMemsetAsync(Fx->data, 0, (size_t)TMK_NCOMP * (nvx + 1) * nvy * sizeof(double), s));
+    if (Fy) TMK_CU(cudaMemsetAsync(Fy->data, 0, (size_t)TMK_NCOMP * nvx * (nvy + 1) * sizeof(double), s));
+    TMK_CU(tmk::Launch<double>::volume(dpd, dtl, ntiles, cv.dp, s));
+  }
   for (int sd = 0; sd < 2; ++sd)
     TMK_CU(tmk::copy_valid(pd.Uout, U->data, pd.alo0, pd.alo1, anx, any, pd.vlo0, pd.vlo1, pd.vhi0, pd.vhi1,
                            11 * sd, tmk::NSIDE, s));
