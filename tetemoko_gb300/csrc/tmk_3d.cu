@@ -185,10 +185,11 @@ size_t layout3(Step3<T>& g, char* base) {
 
 // The step on characteristic values (tmk_3d_march.cuh) implements the decks'
 // predictor (PPM with primitive limiting) and the laws that read only those
-// values; it takes 0.57 of the time of the passes over face states (192x96x96
-// mixed: 792 against 1383 us, and 32 patches of a 96x64x64 level 984 against
-// 1116; 64x48x48 FP64: 795 against 2703), whatever the size.  The rest (PLM, CTU, limiting of the characteristic
-// amplitudes, the reference's 9-component slip weakening) keeps those passes.
+// values; whatever the size it beats the passes over face states (192x96x96
+// mixed: 778 against 1383 us, the 32-cell patches of a 96x64x64 level 837
+// against 1100; 64x48x48 FP64: 595 against 2703).  The rest (PLM, CTU, limiting
+// of the characteristic amplitudes, the reference's 9-component slip weakening)
+// keeps those passes.
 bool march3(const tmk::DevParams& p) {
   return p.order == 2 && p.prim_lim && !p.char_lim && !(p.fault_law == 2 && p.sw_off != 11);
 }
@@ -214,27 +215,40 @@ size_t layout3m(Step3<T>& g, char* base) {
   return off;
 }
 
-// Planes a CTA of the last pass marches over: about two planes are spent on
-// start-up, and the CTAs should come in whole waves.
+// Rows and planes an item of the predictor (vrun) and a CTA of the last pass
+// (zrun) march over.  An item costs about three rows beyond its own (a CTA two
+// and a half planes), so runs are long, but not so long that sub-partitions
+// (SMs) idle: one FP64 warp nearly fills its sub-partition's pipe, two FP32
+// warps the issue, and CTAs of the last pass come in waves.
 template <typename T>
-int choose_zrun(const Step3<T>* g, int np) {
+void choose_runs(Step3<T>* g, int np) {
   using namespace tmk::d3;
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int best = 1 << 20;
+  int vrun = 16, zrun = 1 << 20;
   double cost = 0.0;
-  for (int run : {1 << 20, 96, 64, 48, 40, 32, 28, 24, 20, 16, 14, 12, 10, 8, 6, 4}) {
+  for (int run : {16, 8, 4}) {
+    long long n = 0;
+    for (int p = 0; p < np; ++p) {
+      const int* m = g[p].S.n;
+      n += val_xy_items(m[0], m[1], m[2], run) + val_z_items(m[0], m[1], m[2], run) / 2;
+    }
+    const double c = std::max(1.0, n / (4.0 * sms * (sizeof(T) == 4 ? 2 : 1))) * (run + 3);
+    if (run == 16 || c < cost) { vrun = run; cost = c; }
+  }
+  for (int run : {1 << 20, 96, 64, 48, 40, 32, 28, 24, 20, 16, 14, 12, 10, 8, 6, 4, 2}) {
     long long n = 0;
     int longest = 1;
     for (int p = 0; p < np; ++p) {
       const int nz = g[p].cur.n[2];
-      n += 2LL * cdiv(g[p].cur.n[0], STEP_COLS) * cdiv(g[p].cur.n[1], step_rows<T> - 2) * cdiv(nz, std::min(run, nz));
+      n += 2LL * step_tiles<T>(g[p].cur.n[0], g[p].cur.n[1]) * cdiv(nz, std::min(run, nz));
       longest = std::max(longest, std::min(run, nz));
     }
-    const double c = (double)((n + step_ctas<T> * sms - 1) / (step_ctas<T> * sms)) * (longest + 2.5);
-    if (run == 1 << 20 || c < cost) { best = run; cost = c; }
+    const int slots = step_ctas<T> * sms;
+    const double c = (double)((n + slots - 1) / slots) * (longest + 2.5);
+    if (run == 1 << 20 || c < cost) { zrun = run; cost = c; }
   }
-  return best;
+  for (int p = 0; p < np; ++p) { g[p].vrun = vrun; g[p].zrun = zrun; }
 }
 
 tmk_status ensure_scratch(tmk_context* c, size_t total, cudaStream_t s) {
@@ -272,7 +286,7 @@ tmk_status patch3(tmk_context* c, const tmk_fab3* U, const tmk_fab3* B, const tm
   if (march3(c->hp)) {
     if ((r = ensure_scratch(c, layout3m<T>(pl.g, nullptr), s)) != TMK_OK) return r;
     layout3m<T>(pl.g, (char*)c->scratch);
-    pl.g.zrun = choose_zrun(&pl.g, 1);
+    choose_runs(&pl.g, 1);
     return launch_march(pl, c->hp, c->dp, c->dstatus, dt, dx, s) == cudaSuccess ? TMK_OK : TMK_ERR_CUDA;
   }
   if ((r = ensure_scratch(c, layout3<T>(pl.g, nullptr), s)) != TMK_OK) return r;
@@ -300,8 +314,7 @@ tmk_status patches3(tmk_context* c, int np, const tmk_fab3* U, const tmk_fab3* B
     if (r != TMK_OK) return r;
   }
   const bool mar = march3(c->hp);
-  const int zrun = choose_zrun(gs.data(), np);
-  for (Step3<T>& g : gs) g.zrun = zrun;
+  choose_runs(gs.data(), np);
   auto layout = [mar](Step3<T>& g, char* base) { return mar ? layout3m<T>(g, base) : layout3<T>(g, base); };
   PlanMany<T> pl;
   pl.np = np;

@@ -101,11 +101,12 @@ struct Step3 {
   int fastpred;
   T trA[NSIDE], trB[NSIDE];
   // the step on characteristic values (tmk_3d_march.cuh): the cells' values,
-  // the fault faces' states and velocities, planes a CTA of its last pass marches
+  // the fault faces' states and velocities, rows or planes an item of the
+  // predictor marches over, planes a CTA of the last pass does
   void* AF;
   void* FA;
   T* FV;
-  int zrun;
+  int vrun, zrun;
 };
 
 template <int D> TMK_HD double rvs(int s) { return (D == 1 && s == 1) ? -1.0 : 1.0; }
@@ -768,14 +769,33 @@ enum : int {
   NKIND
 };
 
-// Shapes of tmk_3d_march.cuh's work: warps per CTA, updated columns and halo
-// lanes of a warp that predicts x, rows or planes an item marches over; rows of
-// the last pass's tile (two of them halo) and its updated columns.
-constexpr int VAL_WARPS = 4, VAL_COLS = 28, VAL_HALO = 2, VAL_RUN_Y = 16, VAL_RUN_Z = 16;
-constexpr int STEP_COLS = 30;
-template <typename T> constexpr int step_rows = sizeof(T) == 4 ? 8 : 12;
-template <typename T> constexpr int step_ctas = sizeof(T) == 4 ? 2 : 1;   // resident per SM
+// Shapes of tmk_3d_march.cuh's work.  A warp's lanes hold the columns of a strip
+// of x: the predictor's 28 between two halo lanes on either side, the last
+// pass's 30 between one.  What is left of a row after whole strips takes lane
+// groups of 16, 8 or 4, several planes (rows of a tile) to a warp: a 32-cell row
+// as two whole strips would leave two thirds of the lanes idle.
+constexpr int VAL_WARPS = 4, VAL_HALO = 2;
+template <typename T> constexpr int step_rows = 8;      // warps of a tile
+template <typename T> constexpr int step_ctas = sizeof(T) == 4 ? 2 : 1;       // resident per SM
 TMK_HD int cdiv(int a, int b) { return (a + b - 1) / b; }
+TMK_HD int lane_group(int cols) { return cols <= 4 ? 4 : cols <= 8 ? 8 : cols <= 16 ? 16 : 32; }
+// strips of `n` columns: whole ones, the lanes of a group of the rest (0: none)
+struct Strips { int whole, group; };
+TMK_HD Strips strips(int n, int halo) {
+  const int cols = 32 - 2 * halo, whole = n / cols, rest = n - whole * cols;
+  return Strips{whole, rest ? lane_group(rest + 2 * halo) : 0};
+}
+// tiles of the last pass in x and y
+template <typename T> TMK_HD int step_tiles(int n0, int n1) {
+  const Strips st = strips(n0, 1);
+  return st.whole * cdiv(n1, step_rows<T> - 2) + (st.group ? cdiv(n1, step_rows<T> * (32 / st.group) - 2) : 0);
+}
+// items of the x and y predictor along one row of planes
+TMK_HD long long val_xy_items(int n0, int n1, int n2, int run) {
+  const Strips st = strips(n0, VAL_HALO);
+  return (long long)cdiv(n1, run) * ((long long)st.whole * n2 + (st.group ? cdiv(n2, 32 / st.group) : 0));
+}
+TMK_HD long long val_z_items(int n0, int n1, int n2, int run) { return (long long)cdiv(n0 * n1, 32) * cdiv(n2, run); }
 template <typename T>
 TMK_HD long long kind_count(const Step3<T>& g, int kind) {
   const bool f = g.fault != 0;
@@ -796,10 +816,10 @@ TMK_HD long long kind_count(const Step3<T>& g, int kind) {
     case K_FLF_2: return g.flF[2].cells();
     case K_CUR: return g.cur.cells();
     case K_BF: return f ? (long long)g.cur.n[0] * g.cur.n[2] : 0;
-    case K_VXY: return (long long)cdiv(g.S.n[0], VAL_COLS) * cdiv(g.S.n[1], VAL_RUN_Y) * g.S.n[2];
-    case K_VZ: return (long long)cdiv(g.S.n[0], 32) * g.S.n[1] * cdiv(g.S.n[2], VAL_RUN_Z);
+    case K_VXY: return val_xy_items(g.S.n[0], g.S.n[1], g.S.n[2], g.vrun);
+    case K_VZ: return val_z_items(g.S.n[0], g.S.n[1], g.S.n[2], g.vrun);
     case K_PL: return f ? g.fplane.cells() : 0;
-    case K_STEP: return 2LL * cdiv(g.cur.n[0], STEP_COLS) * cdiv(g.cur.n[1], step_rows<T> - 2) * cdiv(g.cur.n[2], g.zrun);
+    case K_STEP: return 2LL * step_tiles<T>(g.cur.n[0], g.cur.n[1]) * cdiv(g.cur.n[2], g.zrun);
   }
   return 0;
 }

@@ -22,13 +22,16 @@
 // WHalf[1] and the boundary data of one face are one thread's work.
 //
 // What bounds them, at 192x96x96 mixed (rate and state): the FP32 copy of the
-// state (79 us) and the z values (38 us) DRAM; the x and y values (70 us) the
-// issue of the limiters; the plane (48 us) the latency of four dependent solves;
-// the step (about 450 us) issue, 500 instructions a cell and side, with L2 close
-// behind (144 B of values read, 144 B of FP64 state read and written a cell and
-// side, plus the tile's halo).  The whole step 792 us; one pass per term, each
-// through memory, took 1383 us.  FP64 (64x48x48): every kernel the FP64 pipe,
-// which the first two keep 70 % and the last 82 % busy; 795 us, was 2703 us.
+// state (78 us) and the z values (35 us) DRAM; the x and y values (70 us) the
+// issue of the limiters; the plane (48 us) the latency of four dependent solves,
+// beside which the step's tiles away from the fault run; the step (about 420 us)
+// issue, 500 instructions a cell and side, with L2 close behind (144 B of values
+// read, 144 B of FP64 state read and written a cell and side, plus the tile's
+// halo).  A call 778 us; one pass per term, each through memory, took 1383 us.
+// FP64 (64x48x48): every kernel the FP64 pipe; 595 us, was 2703 us.  32-cell
+// boxes of a 96x64x64 level, mixed: 837 us, was 1100 (half of either is reading
+// the state back), of which the step 141 (231 before a row's last columns took
+// lane groups).
 #pragma once
 
 #include "tmk_3d.cuh"
@@ -144,9 +147,9 @@ TMK_D void stage_column(unsigned dst, const T* src, const T* src2, unsigned plan
 
 // A warp marches along DM over a run of rows (planes) with x in its lanes: the
 // limited deltas of DM from a rolling window of rows in shared memory, and
-// (DM = 1) those of x from its neighbour lanes.  28 of 32 lanes hold values
-// where x is predicted (a delta reads the slopes of both neighbours), all 32
-// otherwise.
+// (DM = 1) those of x from its neighbour lanes, where a delta reads the slopes
+// of both neighbours (two halo lanes on either side of a strip).  For z the
+// lanes hold 32 consecutive cells of the plane, across the ends of rows.
 template <typename T, int DM, typename Src>
 __global__ void __launch_bounds__(32 * VAL_WARPS, sizeof(T) == 4 ? 4 : 2)
 values_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k, long long nitems) {
@@ -154,34 +157,56 @@ values_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k, 
   constexpr int NC8 = kValComps<DM>, RP = NC8 * 32;
   constexpr bool X = DM == 1;
   extern __shared__ __align__(16) unsigned char val_smem[];
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const unsigned lane = threadIdx.x & 31u;
+  // the z kernel, scheduled beside the x and y one, completes after it
+  if constexpr (X) asm volatile("griddepcontrol.launch_dependents;");
   const long long item = (long long)blockIdx.x * VAL_WARPS + warp;
-  if (item >= nitems) return;
-  long long lt;
-  const Step3<T>* gp = find_item<T>(src, item, lt);
-  if (!gp) return;
+  long long lt = 0;
+  const Step3<T>* gp = item < nitems ? find_item<T>(src, item, lt) : nullptr;
+  if (!gp) {
+    if constexpr (!X) asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   const Step3<T>& g = *gp;
-  // item -> strip of columns, run along DM, the third coordinate
-  const unsigned u = (unsigned)lt, ns = (unsigned)cdiv(g.S.n[0], X ? VAL_COLS : 32);
-  const unsigned rest = u / ns, strip = u - rest * ns;
-  const unsigned nr = X ? (unsigned)cdiv(g.S.n[1], VAL_RUN_Y) : (unsigned)g.S.n[1];
-  const unsigned third = rest / nr, second = rest - third * nr;
-  const int x = g.S.lo[0] + (int)strip * (X ? VAL_COLS : 32) + lane - (X ? VAL_HALO : 0);
-  const int run = X ? VAL_RUN_Y : VAL_RUN_Z;
-  const int q0 = X ? g.S.lo[1] + (int)second * run : g.S.lo[2] + (int)third * run;
+  // item -> cell of the lane, run along DM
+  const unsigned u = (unsigned)lt;
+  const int run = g.vrun;
+  int x, y, z;
+  bool own = true;                      // not a halo lane
+  if constexpr (X) {
+    const Strips st = strips(g.S.n[0], VAL_HALO);
+    const unsigned nr = (unsigned)cdiv(g.S.n[1], run), nw = nr * (unsigned)(st.whole * g.S.n[2]);
+    const bool rest = u >= nw;
+    const unsigned gl = rest ? (unsigned)st.group : 32u, per = 32u / gl, ns = rest ? 1u : (unsigned)st.whole;
+    const unsigned v = rest ? u - nw : u, t = v / ns, strip = rest ? (unsigned)st.whole : v - t * ns;
+    const unsigned third = t / nr, second = t - third * nr, cx = lane & (gl - 1u);
+    x = g.S.lo[0] + (int)(strip * (32 - 2 * VAL_HALO) + cx) - VAL_HALO;
+    y = g.S.lo[1] + (int)second * run;
+    z = g.S.lo[2] + (int)(third * per + lane / gl);
+    own = cx >= VAL_HALO && cx < gl - VAL_HALO && z < g.S.lo[2] + g.S.n[2];
+  } else {
+    const unsigned ns = (unsigned)cdiv(g.S.n[0] * g.S.n[1], 32), third = u / ns;
+    const unsigned cell = (u - third * ns) * 32u + lane, cy = cell / (unsigned)g.S.n[0];
+    x = g.S.lo[0] + (int)(cell - cy * (unsigned)g.S.n[0]);
+    y = g.S.lo[1] + (int)cy;
+    z = g.S.lo[2] + (int)third * run;
+    own = (int)cy < g.S.n[1];
+  }
+  const int q0 = X ? y : z;             // the same for all lanes
   const int q1 = min(q0 + run - 1, g.S.lo[DM] + g.S.n[DM] - 1);
-  const int y = X ? q0 : g.S.lo[1] + (int)second, z = X ? g.S.lo[2] + (int)third : q0;   // of row q0
   const int dloq = g.dlo[DM], dhiq = g.dhi[DM];
   const Bx& A = g.Ap;
-  const bool lane_in = x >= g.dlo[0] && x <= g.dhi[0] && x >= A.lo[0] && x < A.lo[0] + A.n[0];
-  const bool store = lane_in && x < g.S.lo[0] + g.S.n[0] && x >= g.S.lo[0] && (!X || (lane >= VAL_HALO && lane < 32 - VAL_HALO));
+  const bool lane_in = x >= g.dlo[0] && x <= g.dhi[0] && x >= A.lo[0] && x < A.lo[0] + A.n[0] &&
+                       (X ? z < g.S.lo[2] + g.S.n[2] : own);
+  const bool store = lane_in && own && x < g.S.lo[0] + g.S.n[0] && x >= g.S.lo[0];
   const long long pcs = A.cells(), dq = X ? A.n[0] : (long long)A.n[0] * A.n[1];
   const T* const safe = g.Up;
   // the lane's address in component 0 of the next row to stage
   const T* lsrc = g.Up + A.at(x, y, z);
   const long long side2 = (long long)g.uside * pcs;
   P* const ring = reinterpret_cast<P*>(val_smem) + warp * 4 * RP;
-  const unsigned ring32 = (unsigned)__cvta_generic_to_shared(ring) + (unsigned)(lane * (int)sizeof(P));
+  const unsigned ring32 = (unsigned)__cvta_generic_to_shared(ring) + lane * (unsigned)sizeof(P);
   const int q_last = min(dhiq, q1 + 2);
   auto stage = [&](int q) {
     const bool ok = lane_in && q <= q_last;
@@ -331,6 +356,7 @@ values_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k, 
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
+  if constexpr (!X) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ------------------------------------------------------------ linear stages
@@ -410,45 +436,50 @@ TMK_D void store_flux(const Step3<T>& g, const K3<T>& k, T rvs, int s, int i, in
 
 // ------------------------------------------------------------ the step
 // One CTA per tile of 30 x (NR - 2) cells, run of planes and side; a warp per
-// row of y, x in the lanes, marching in z.  Neighbours: x by lane, y through
+// row of y, x in the lanes, marching in z.  (The columns left over by whole
+// tiles: 14 x (2 NR - 2), 6 x (4 NR - 2) or 2 x (8 NR - 2) cells, two to eight
+// rows to a warp.)  Neighbours: x by lane, y through
 // shared memory (two exchanges a plane), z carried from plane to plane.  When
 // plane m arrives, the stages that need nothing above it are done for m, then
-// plane m - 1 is finished.  8 rows at two CTAs per SM (128 registers, a few
-// spilled): the whole step of a 192x96x96 patch took 792 us, against 828 us with
-// 16 rows and 1015 us with 12 rows at one CTA (no spills, too few warps).  FP64
-// 12 rows, one CTA: 795 us for a 64x48x48 patch, 814 with 8 rows (more halo) and
-// 834 with 16 (spills).
-template <typename T, typename Src>
-__global__ void __launch_bounds__(32 * step_rows<T>, step_ctas<T>)
-step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
+// plane m - 1 is finished.  8 rows, FP32 at two CTAs per SM (128 registers, some
+// spilled), FP64 one: a 192x96x96 mixed patch took 778 us, 823 with 16 rows and
+// 785 with 10 at one CTA (no spills, but the 32-cell boxes 931 against 852); a
+// 64x48x48 FP64 patch 595 us, 629 with 10 rows and 612 with 12.
+// GL: lanes of a row, 32 or (0) fewer, from the strips; FLUX: a patch has flux
+// arrays.  Both fixed at compile time: the common form spills least.
+template <typename T, int GL, bool FLUX>
+TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
   using V = typename PairOf<T>::P;
   constexpr int NR = step_rows<T>;
   // [9] A_y, WHalf2[1][0] of plane m, WHalf2[1][2] of plane m - 1; [3] the final y values of plane m - 1
   extern __shared__ __align__(16) unsigned char step_smem[];
-  V (*const s1)[NR + 2][32] = reinterpret_cast<V (*)[NR + 2][32]>(step_smem);
-  V (*const s2)[NR + 2][32] = s1 + 9;
-  long long lt;
-  const Step3<T>* gp = find_item<T>(src, blockIdx.x, lt);
-  if (!gp) return;
-  const Step3<T>& g = *gp;
-  const int row = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const unsigned u = (unsigned)lt, side = u & 1u;
-  const unsigned nx = (unsigned)cdiv(g.cur.n[0], STEP_COLS), ny = (unsigned)cdiv(g.cur.n[1], NR - 2);
-  const unsigned t1 = (u >> 1) / nx, tx = (u >> 1) - t1 * nx, tz = t1 / ny, ty = t1 - tz * ny;
+  constexpr int PL = (NR + 2) * 32;       // entries of one value; rows of a lane group each
+  V* const s1 = reinterpret_cast<V*>(step_smem);
+  V* const s2 = s1 + 9 * PL;
+  const unsigned side = u & 1u;
+  const Strips st = strips(g.cur.n[0], 1);
+  const unsigned nw = (unsigned)st.whole * (unsigned)cdiv(g.cur.n[1], NR - 2);
+  const unsigned nt = (unsigned)step_tiles<T>(g.cur.n[0], g.cur.n[1]), tz = (u >> 1) / nt, t1 = (u >> 1) - tz * nt;
+  const unsigned gl = GL ? GL : (unsigned)st.group;            // lanes of a group, that is of a row
+  const unsigned ty = GL && st.whole ? t1 / (unsigned)st.whole : t1 - nw;
+  const unsigned tx = GL && st.whole ? t1 - ty * (unsigned)st.whole : (unsigned)st.whole;
+  const int cx = (int)(threadIdx.x & (gl - 1u)), row = (int)(threadIdx.x / gl), rows = (int)(32u * NR / gl);
+  const int at = (int)gl + (int)threadIdx.x;                   // the thread's entry: row + 1, column cx
   const int s = (int)side;
   const T rv = s ? T(-1) : T(1);
-  const int x = g.cur.lo[0] + (int)tx * STEP_COLS - 1 + lane, y = g.cur.lo[1] + (int)ty * (NR - 2) - 1 + row;
+  const int x = g.cur.lo[0] + (int)tx * 30 - 1 + cx, y = g.cur.lo[1] + (int)ty * (rows - 2) - 1 + row;
   const int z0 = g.cur.lo[2] + (int)tz * g.zrun, z1 = min(z0 + g.zrun, g.cur.lo[2] + g.cur.n[2]) - 1;
   const bool in = x >= g.S.lo[0] && x < g.S.lo[0] + g.S.n[0] && y >= g.S.lo[1] && y < g.S.lo[1] + g.S.n[1];
-  const bool upd = lane >= 1 && lane <= STEP_COLS && row >= 1 && row <= NR - 2 && x < g.cur.lo[0] + g.cur.n[0] &&
+  const bool upd = cx >= 1 && cx <= (int)gl - 2 && row >= 1 && row <= rows - 2 && x < g.cur.lo[0] + g.cur.n[0] &&
                    y < g.cur.lo[1] + g.cur.n[1];
   const bool xlo = x == g.dlo[0], xhi = x == g.dhi[0];
   const bool warp_x = __any_sync(0xffffffffu, xlo || xhi);
   const bool ylo = y == g.dlo[1], yhi = y == g.dhi[1], yfault = ylo && g.fault != 0;
+  // the fault plane's states: the kernel before this one in the stream
+  if (__any_sync(0xffffffffu, yfault)) asm volatile("griddepcontrol.wait;" ::: "memory");
   const int zlo = g.dlo[2], zhi = g.dhi[2];
   const unsigned scs = (unsigned)g.S.cells();
   const unsigned dz = (unsigned)g.S.n[0] * (unsigned)g.S.n[1];
-  const bool wants_flux = g.F[0] || g.F[1] || g.F[2];
   const int ms = max(z0 - 1, zlo);
   const V* vp = reinterpret_cast<const V*>(g.AF) + (unsigned long long)scs * (unsigned)(s * 9) + (in ? g.S.at(x, y, ms) : 0);
   const V zero = mk2(T(0), T(0));
@@ -474,11 +505,11 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
     for (int w = 0; w < 3; ++w) jump(hn[w], a[w].y, a[w].x, lp[w], sum[w], dif[w]);
   };
   // the lo face values of a cell in y: the row below, the edge, or the fault's
-  // state of level l in plane kz (ylo, yhi: uniform over the warp)
+  // state of level l in plane kz
   const bool on_plane = yfault && in && x >= g.fplane.lo[0] && x < g.fplane.lo[0] + g.fplane.n[0];
-  auto ylo_face = [&](const V (*sm)[NR + 2][32], const V* a, int l, int kz, T* ln, T* lp) {
+  auto ylo_face = [&](const V* sm, const V* a, int l, int kz, T* ln, T* lp) {
 #pragma unroll
-    for (int w = 0; w < 3; ++w) { ln[w] = a[w].x; lp[w] = sm[w][row][lane].y; }
+    for (int w = 0; w < 3; ++w) { ln[w] = a[w].x; lp[w] = sm[w * PL + at - (int)gl].y; }
     if (ylo) {
       if (yfault) {
         const bool have = on_plane && kz >= g.fplane.lo[2] && kz < g.fplane.lo[2] + g.fplane.n[2];
@@ -496,11 +527,11 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
       }
     }
   };
-  auto yjump = [&](const V (*sm)[NR + 2][32], const V* a, int l, int kz, T* sum, T* dif) {
+  auto yjump = [&](const V* sm, const V* a, int l, int kz, T* sum, T* dif) {
     T ln[3], lp[3], hn[3];
     ylo_face(sm, a, l, kz, ln, lp);
 #pragma unroll
-    for (int w = 0; w < 3; ++w) hn[w] = sm[w][row + 2][lane].x;
+    for (int w = 0; w < 3; ++w) hn[w] = sm[w * PL + at + (int)gl].x;
     if (yhi) {
 #pragma unroll
       for (int w = 0; w < 3; ++w) hn[w] = arriving(k.out[3] != 0, a[w].y, k.nbg[ws<1>(w)]);
@@ -552,7 +583,7 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
       correct3<0, 1, 1, T>(k, rv, sum, dif, yx);
       correct3<0, 2, 1, T>(k, rv, sum, dif, nzx);
 #pragma unroll
-      for (int w = 0; w < 3; ++w) { s1[w][row + 1][lane] = by[w]; s1[3 + w][row + 1][lane] = yx[w]; }
+      for (int w = 0; w < 3; ++w) { s1[w * PL + at] = by[w]; s1[(3 + w) * PL + at] = yx[w]; }
     }
     if (fin) {
 #pragma unroll
@@ -565,7 +596,7 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
       correct3<2, 0, 1, T>(k, rv, sum, dif, xz);
       correct3<2, 1, 1, T>(k, rv, sum, dif, yz);
 #pragma unroll
-      for (int w = 0; w < 3; ++w) s1[6 + w][row + 1][lane] = yz[w];
+      for (int w = 0; w < 3; ++w) s1[(6 + w) * PL + at] = yz[w];
     }
     __syncthreads();
     V xy[3], fx[3], fy[3];
@@ -578,14 +609,14 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
       // the final z values of plane m: jumps of WHalf2[0][1] in x and WHalf2[1][0] in y
       xjump(xy, sum, dif);
       correct3<0, 2, 0, T>(k, rv, sum, dif, nfz);
-      yjump(s1 + 3, yx, 1, m, sum, dif);
+      yjump(s1 + 3 * PL, yx, 1, m, sum, dif);
       correct3<1, 2, 0, T>(k, rv, sum, dif, nfz);
     }
     if (fin) {
       // the final x and y values of plane m - 1
 #pragma unroll
       for (int w = 0; w < 3; ++w) { fx[w] = ax[w]; fy[w] = ay[w]; }
-      yjump(s1 + 6, yz, 2, m - 1, sum, dif);
+      yjump(s1 + 6 * PL, yz, 2, m - 1, sum, dif);
       correct3<1, 0, 0, T>(k, rv, sum, dif, fx);
 #pragma unroll
       for (int w = 0; w < 3; ++w) {
@@ -604,7 +635,7 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
       }
       correct3<2, 1, 0, T>(k, rv, sum, dif, fy);
 #pragma unroll
-      for (int w = 0; w < 3; ++w) s2[w][row + 1][lane] = fy[w];
+      for (int w = 0; w < 3; ++w) s2[w * PL + at] = fy[w];
     }
     __syncthreads();
     if (fin) {
@@ -626,7 +657,7 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
         dif[w] = jn - jfz[w];
       }
       update3<2, T>(k, rv, sum, dif, du);
-      if (wants_flux) {
+      if (FLUX && (g.F[0] || g.F[1] || g.F[2])) {
         // the lo faces of this cell, and the hi face of the last one
         T n[3], p[3], hn[3];
 #pragma unroll
@@ -651,7 +682,7 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
           if (y == g.cur.lo[1] + g.cur.n[1] - 1) {
 #pragma unroll
             for (int w = 0; w < 3; ++w) {
-              hn[w] = yhi ? arriving(k.out[3] != 0, fy[w].y, k.nbg[ws<1>(w)]) : s2[w][row + 2][lane].x;
+              hn[w] = yhi ? arriving(k.out[3] != 0, fy[w].y, k.nbg[ws<1>(w)]) : s2[w * PL + at + (int)gl].x;
               p[w] = fy[w].y;
             }
             store_flux<1, T>(g, k, rv, s, x, y + 1, kz, hn, p);
@@ -697,6 +728,21 @@ step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
   }
 }
 
+template <typename T, bool FLUX, typename Src>
+__global__ void __launch_bounds__(32 * step_rows<T>, step_ctas<T>)
+step_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k) {
+  long long lt;
+  const Step3<T>* gp = find_item<T>(src, blockIdx.x, lt);
+  if (!gp) return;
+  const Step3<T>& g = *gp;
+  // a tile of whole strips or of the columns left over
+  const Strips st = strips(g.cur.n[0], 1);
+  const unsigned nt = (unsigned)step_tiles<T>(g.cur.n[0], g.cur.n[1]), u = (unsigned)lt;
+  const bool whole = (u >> 1) % nt < (unsigned)st.whole * (unsigned)cdiv(g.cur.n[1], step_rows<T> - 2);
+  if (whole) step_tile<T, 32, FLUX>(g, k, u);
+  else step_tile<T, 0, FLUX>(g, k, u);
+}
+
 // ------------------------------------------------------------ the fault plane
 // One thread per fault face (x, z) of the first pass: the four friction solves
 // of the face from the predictors' values around it, and on valid faces the
@@ -706,6 +752,9 @@ template <typename T, typename Src>
 __global__ void __launch_bounds__(64) plane_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k,
                                                    const DevParams* Pp, DevStatus* st) {
   using V = typename PairOf<T>::P;
+  // the step's tiles away from the fault may start (the values they read were
+  // complete before this kernel started)
+  asm volatile("griddepcontrol.launch_dependents;");
   TMK3_FIND(T)
   const Step3<T>& g = *gp;
   const DevParams& P = *Pp;
@@ -879,20 +928,44 @@ cudaError_t launch_march3(const Plan& pl, const DevParams& hp, const DevParams* 
       e = cudaFuncSetAttribute(values_kernel<T, 2, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)val_smem_bytes<T, 2>());
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(step_kernel<T, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      e = cudaFuncSetAttribute(step_kernel<T, false, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)step_smem_bytes<T>());
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(step_kernel<T, true, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)step_smem_bytes<T>());
     return e;
   }();
   if (configured != cudaSuccess) return configured;
   if (pl.copy() && pl.n(K_AP)) to_pred_kernel<T, Src><<<blocks(pl.n(K_AP)), 128, 0, s>>>(pl.src(K_AP));
+  // The z predictor does not wait for the x and y one, nor the step's tiles away
+  // from the fault for the plane kernel (launch attribute; the kernels still
+  // complete in order, since every z warp and the tiles on the fault wait).
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  auto config = [&](long long ctas, int threads, size_t smem, bool beside) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = beside ? attr : nullptr;
+    cfg.numAttrs = beside ? 1 : 0;
+    return cfg;
+  };
   const long long nxy = pl.n(K_VXY), nz = pl.n(K_VZ);
-  values_kernel<T, 1, Src><<<(unsigned)((nxy + VAL_WARPS - 1) / VAL_WARPS), 32 * VAL_WARPS, val_smem_bytes<T, 1>(), s>>>(
-      pl.src(K_VXY), k, nxy);
-  values_kernel<T, 2, Src><<<(unsigned)((nz + VAL_WARPS - 1) / VAL_WARPS), 32 * VAL_WARPS, val_smem_bytes<T, 2>(), s>>>(
-      pl.src(K_VZ), k, nz);
+  cudaLaunchConfig_t cfg = config((nxy + VAL_WARPS - 1) / VAL_WARPS, 32 * VAL_WARPS, val_smem_bytes<T, 1>(), false);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, values_kernel<T, 1, Src>, pl.src(K_VXY), k, nxy);
+  if (e != cudaSuccess) return e;
+  cfg = config((nz + VAL_WARPS - 1) / VAL_WARPS, 32 * VAL_WARPS, val_smem_bytes<T, 2>(), true);
+  if ((e = cudaLaunchKernelEx(&cfg, values_kernel<T, 2, Src>, pl.src(K_VZ), k, nz)) != cudaSuccess) return e;
   if (pl.fault())
     plane_kernel<T, Src><<<(unsigned)((pl.n(K_PL) + 63) / 64), 64, 0, s>>>(pl.src(K_PL), k, P, st);
-  step_kernel<T, Src><<<(unsigned)pl.n(K_STEP), 32 * step_rows<T>, step_smem_bytes<T>(), s>>>(pl.src(K_STEP), k);
+  cfg = config(pl.n(K_STEP), 32 * step_rows<T>, step_smem_bytes<T>(), pl.fault());
+  const bool flux = pl.flux(0) || pl.flux(1) || pl.flux(2);
+  e = flux ? cudaLaunchKernelEx(&cfg, step_kernel<T, true, Src>, pl.src(K_STEP), k)
+           : cudaLaunchKernelEx(&cfg, step_kernel<T, false, Src>, pl.src(K_STEP), k);
+  if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 
