@@ -204,47 +204,84 @@ constexpr int kFaultDisplace = 1;
 // the marching kernels implement the PPM and CTU predictors; PLM runs the tile kernel
 bool uses_march(const tmk_scheme& s) { return s.volume_kernel != TMK_VOLUME_TILE && s.normal_pred_order != 1; }
 
+// The fault kernel first and both component groups in one launch that finishes
+// the fault rows (one_launch), or the groups' kernels with the fault kernel
+// between them and a launch for the fault rows.  Mixed, us a step, first against
+// second: slip weakening 64x32 12.0 / 13.7, 512x256 16.5 / 18.8, 1000x1000 64.8 /
+// 66.5, 2048x1024 118 / 123; rate and state, whose fault kernel holds its SMs
+// longer, 64x32 20.6 / 23.5, 512x256 20.9 / 25.1, but 1000x500 in patches of 128
+// 64.1 / 63.0 and 2048x1024 alike.  FP64 64x32 80 / 82, 512x256 198 / 217,
+// 2048x1024 2258 / 2223.  Without a fault the groups share one launch too.
+constexpr long long kOneLaunchCells = 450000;
+bool one_launch(const tmk_level_s* L) {
+  long long cells = 0;
+  bool rs = false;
+  for (const LevelPatch& lp : L->patches) {
+    cells += (long long)(lp.valid.hi[0] - lp.valid.lo[0] + 1) * (lp.valid.hi[1] - lp.valid.lo[1] + 1);
+    rs = rs || (lp.fault && L->ctx->scheme.fault_law == TMK_FAULT_RS);
+  }
+  return cells <= kOneLaunchCells || (L->prec == TMK_PREC_MIXED && !rs);
+}
+
 // Shortest run of a level's items.  A row of a marching warp takes about the
 // same time until a sub-partition holds two warps in FP32 or one in FP64 (whose
-// pipe one warp nearly fills), and an item costs about three rows beyond its
-// own, so the time goes as (run + 3) x max(1, warps per sub-partition / 2 or 1).
-// Measured (us a step): mixed 512x256 18.7 at 4 rows and 25.8 at 16, FP64
-// 512x256 217 at 8 and 252 at 16, FP64 256x128 91 at 4 and 242 at 16, mixed
-// 1000x500 in patches of 128 65.7 at 6 and 61.5 at 16.
-int default_min_run(const tmk_level_s* L) {
+// pipe one warp nearly fills), and an item costs two to three rows beyond its
+// own.
+// In one launch, FP32: the shortest run whose CTAs and the fault kernel's (each
+// takes the room of two) are resident at once with a tenth to spare, since a
+// second wave costs more than shorter runs gain (us a step: 512x256 16.5 at 5
+// rows, 19.3 at 4, 18.8 at 8; 512x512 25.1 at 10, 26.7 at 7); where none of 16
+// rows is, 16 (1024x512 38.7, 40 at 8).  FP64: (run + 2.2) x the CTAs per SM,
+// of which the ones beyond the first cost half (512x256 198 at 4, 218 at 8;
+// 256x128 98 at 5, 101 at 4, 118 at 8).
+// In two launches: (run + 3) x max(1, warps per sub-partition / 2 or 1) (mixed
+// 1000x500 in patches of 128 61.5 at 16 rows, 65.7 at 6).
+int default_min_run(const tmk_level_s* L, bool both) {
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const bool mixed = L->prec == TMK_PREC_MIXED;
+  auto count = [&](int run, long long& fault_ctas) {
+    long long items = 0;
+    fault_ctas = 0;
+    for (const LevelPatch& lp : L->patches) {
+      const int nx = lp.valid.hi[0] - lp.valid.lo[0] + 1, ny = lp.valid.hi[1] - lp.valid.lo[1] + 1;
+      items += (long long)((nx + tmk::MARCH_COLS - 1) / tmk::MARCH_COLS) * ((ny + run - 1) / run);
+      if (lp.fault) fault_ctas += (nx + tmk::FAULT_SEG - 1) / tmk::FAULT_SEG;
+    }
+    return items;
+  };
+  long long fc = 0;
+  if (both && mixed) {
+    for (int run = 4; run < kMinRun; ++run) {
+      const long long ctas = 2 * ((count(run, fc) + 3) / 4);
+      if (10 * (ctas + 2 * fc) <= 9 * 4LL * sms) return run;
+    }
+    return kMinRun;
+  }
   int best = kMinRun;
   double cost = 0.0;
-  for (int run : {16, 8, 4}) {
-    long long items = 0;
-    for (const LevelPatch& lp : L->patches) {
-      const int ns = (lp.valid.hi[0] - lp.valid.lo[0] + tmk::MARCH_COLS) / tmk::MARCH_COLS;
-      items += (long long)ns * ((lp.valid.hi[1] - lp.valid.lo[1] + run) / run);
+  for (int run = kMinRun; run >= 4; run -= both ? 1 : run / 2) {
+    const long long items = count(run, fc);
+    double c;
+    if (both) {
+      const double per = (2.0 * ((items + 3) / 4) + fc) / sms;
+      c = (run + 2.2) * (per > 1.0 ? 0.65 + 0.5 * per : 1.0);
+    } else {
+      c = (run + 3) * std::max(1.0, items / (4.0 * sms) / (mixed ? 2.0 : 1.0));
     }
-    const double per = (double)items / (4.0 * sms) / (L->prec == TMK_PREC_MIXED ? 2.0 : 1.0);
-    const double c = (run + 3) * std::max(1.0, per);
-    if (run == 16 || c < cost) { best = run; cost = c; }
+    if (run == kMinRun || c < cost) { best = run; cost = c; }
   }
   return best;
 }
-
-// A rate-and-state fault kernel (26 us) outlasts the in-plane kernel of a
-// small level: it goes first (64x32: 22.2 against 24.9 us a step, 256x128:
-// 21.8 against 26.3; 1000x500 and above: the default order).
-constexpr long long kFaultFirstCells = 262144;
 
 tmk_tuning default_tuning(const tmk_level_s* L) {
   tmk_tuning t;
   t.volume_kernel = L->march_allowed ? TMK_VOLUME_MARCH : TMK_VOLUME_TILE;
   t.march_waves[0] = t.march_waves[1] = 1;
-  t.min_run = default_min_run(L);
+  t.fault_first = one_launch(L);
+  t.min_run = default_min_run(L, t.fault_first != 0);
   t.fault_displace = kFaultDisplace;
   t.fault_seg = tmk::FAULT_SEG;
-  long long cells = 0;
-  for (const LevelPatch& lp : L->patches)
-    cells += (long long)(lp.valid.hi[0] - lp.valid.lo[0] + 1) * (lp.valid.hi[1] - lp.valid.lo[1] + 1);
-  t.fault_first = L->ctx->scheme.fault_law == TMK_FAULT_RS && cells <= kFaultFirstCells;
   t.plastic_fused = 0;
   return t;
 }
@@ -979,6 +1016,12 @@ extern "C" tmk_status tmk_level_take_valid(tmk_level* L, int p, double* U, doubl
 
 namespace {
 
+// With the fault kernel first, both groups run in one launch whose fault-row
+// items finish row 0 themselves.
+bool both_groups(const tmk_level_s* L) {
+  return L->march && L->tune.fault_first && !(L->ctx->scheme.plasticity && L->tune.plastic_fused);
+}
+
 // The kernels of one level step after the coarse-fine fill.  Marching form:
 // the in-plane kernel, then the fault kernel (scheduled as in-plane CTAs
 // retire, reading only the step's input state), then the antiplane kernel
@@ -1039,21 +1082,23 @@ tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEve
     TMK_CU(tmk::Launch<Real>::march_fault_rows(pd, L->dfrows[0], L->nfrows[0], nullptr, 0, mc, s));
     return TMK_OK;
   }
-  if (ev) {
+  if (both_groups(L)) {
     TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
-    TMK_CU(cudaEventRecord(ev[2], s));
-    TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
-    TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, true, s));
-  } else if (L->tune.fault_first && L->nfault) {
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
-    TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, true, s));
-    TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, true, s));
+    if (ev) TMK_CU(cudaEventRecord(ev[2], s));
+    TMK_CU(tmk::Launch<Real>::march_both(pd, L->ditems[0], L->nitems[0], L->ditems[1], L->nitems[1], mc,
+                                         L->nfault && !ev, s));
   } else {
-    TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, true, seg, s));
+    if (ev) {
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
+      TMK_CU(cudaEventRecord(ev[2], s));
+      TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
+    } else {
+      TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, true, seg, s));
+    }
     TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, true, s));
+    TMK_CU(tmk::Launch<Real>::march_fault_rows(pd, L->dfrows[0], L->nfrows[0], L->dfrows[1], L->nfrows[1], mc, s));
   }
-  TMK_CU(tmk::Launch<Real>::march_fault_rows(pd, L->dfrows[0], L->nfrows[0], L->dfrows[1], L->nfrows[1], mc, s));
   // the plastic return as a pass over the level (PLASTICCORRECTION after the update)
   if (c->scheme.plasticity) TMK_CU(tmk::Launch<Real>::plastic(pd, L->dtiles, L->ntiles, L->dparams, s));
   return TMK_OK;
@@ -1277,13 +1322,13 @@ extern "C" tmk_status tmk_level_autotune(tmk_level* L, double time, double dt, i
 
 extern "C" int tmk_level_launches_per_step(const tmk_level* L) {
   if (!L) return 0;
-  // marching form: the two groups' kernels, the fault-row finisher (two
-  // launches with the fused plastic return) and the plastic pass
+  // marching form: the two groups' kernels and the fault-row finisher (two
+  // launches with the fused plastic return), or one kernel of both groups that
+  // finishes the fault rows, and the plastic pass
   const bool plastic = L->ctx->scheme.plasticity != 0, fused = plastic && L->tune.plastic_fused;
   const int frows = fused ? (L->nfrows[0] ? 1 : 0) + (L->nfrows[1] ? 1 : 0) : (L->nfrows[0] + L->nfrows[1] ? 1 : 0);
-  const int vol = L->march ? (L->nitems[0] ? 1 : 0) + (L->nitems[1] ? 1 : 0) + frows +
-                                 (plastic && !fused && L->ntiles ? 1 : 0)
-                           : (L->ntiles ? 1 : 0);
+  const int groups = both_groups(L) ? 1 : (L->nitems[0] ? 1 : 0) + (L->nitems[1] ? 1 : 0) + frows;
+  const int vol = L->march ? groups + (plastic && !fused && L->ntiles ? 1 : 0) : (L->ntiles ? 1 : 0);
   return (L->ncopies ? 1 : 0) + (L->nbcopies ? 1 : 0) + (L->nfault ? 1 : 0) + vol + amr_launches(L);
 }
 

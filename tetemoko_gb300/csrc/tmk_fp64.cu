@@ -6,25 +6,26 @@ TMK_INSTANTIATE_LAUNCH(double, 16, 8, 256)
 namespace tmk {
 
 // ---- one patch by itself on the marching kernels
-template <int G, int SCH>
-static cudaError_t patch_group(const PatchDev<double>* dpd, int nx, int ny, MarchConst<double>& mc, bool pdl,
-                               cudaStream_t s) {
-  constexpr size_t smem = march_smem_bytes<double, G, true>();
-  auto* const kernel = march_kernel<double, G, false, SCH, true>;
+template <int SCH>
+static cudaError_t patch_scheme(const PatchDev<double>* dpd, int nx, int ny, MarchConst<double>& mc, bool pdl,
+                                cudaStream_t s) {
+  constexpr size_t smem = std::max(march_smem_bytes<double, 0, true>(), march_smem_bytes<double, 1, true>());
+  auto* const kernel = march_both_kernel<double, SCH, MARCH_PATCH>;
   static const cudaError_t configured =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (configured != cudaSuccess) return configured;
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // One FP64 warp nearly fills a sub-partition's pipe, an item costs about
-  // three rows beyond its own, and the other group's items (half the work) run
-  // beside these: the shortest run that leaves no sub-partition with two.
-  const int ns = (nx + MARCH_COLS - 1) / MARCH_COLS;
+  // An item costs 2.6 rows beyond its own; CTAs of both groups beyond one per SM
+  // fill the gaps of its FP64 pipe (one warp a sub-partition leaves it 44 % idle)
+  // until it is full at about two (128x128, us a call: runs of 1 row 83, 2 rows
+  // 89, 3 rows 94, 4 rows 111).
+  const int ns = (nx + MARCH_COLS - 1) / MARCH_COLS, fc = pdl ? (nx + FAULT_SEG - 1) / FAULT_SEG : 0;
   double cost = 0.0;
-  for (int run = 64; run >= 1; run /= 2) {
-    const double per = 1.5 * ns * ((ny + run - 1) / run) / (4.0 * sms);
-    const double c = (run + 3) * (per > 1.0 ? per : 1.0);
-    if (run == 64 || c < cost) { mc.patch_run = run; cost = c; }
+  for (int run = 16; run >= 1; --run) {
+    const double n = (2.0 * ((ns * ((ny + run - 1) / run) + 3) / 4) + fc) / sms;
+    const double c = (run + 2.6) * (n > 1.0 ? std::max(0.9 + 0.23 * n, 0.35 + 0.5 * n) : 1.0);
+    if (run == 16 || c < cost) { mc.patch_run = run; cost = c; }
   }
   const int nitems = ns * ((ny + mc.patch_run - 1) / mc.patch_run);
   cudaLaunchAttribute attr[1];
@@ -32,12 +33,13 @@ static cudaError_t patch_group(const PatchDev<double>* dpd, int nx, int ny, Marc
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(32 * MARCH_WARPS);
-  cfg.gridDim = dim3((nitems + MARCH_WARPS - 1) / MARCH_WARPS);
+  cfg.gridDim = dim3(2 * ((nitems + MARCH_WARPS - 1) / MARCH_WARPS));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = pdl ? attr : nullptr;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, dpd, (const MarchItem*)nullptr, nitems, mc);
+  const MarchItem* const none = nullptr;
+  return cudaLaunchKernelEx(&cfg, kernel, dpd, none, nitems, none, nitems, mc);
 }
 
 cudaError_t patch_march(const PatchDev<double>* dpd, int nx, int ny, bool fault, const DevParams& hp, double dt,
@@ -46,12 +48,8 @@ cudaError_t patch_march(const PatchDev<double>* dpd, int nx, int ny, bool fault,
   mc.load(hp, dt, dx);
   mc.stash[0] = mc.stash[1] = nullptr;
   mc.caps[0] = mc.caps[1] = nullptr;
-  const bool fx = march_scheme_fixed(mc);
-  cudaError_t e = fx ? patch_group<0, MARCH_SCH_PPM_PRIM>(dpd, nx, ny, mc, fault, s)
-                     : patch_group<0, MARCH_SCH_RUNTIME>(dpd, nx, ny, mc, fault, s);
-  if (e != cudaSuccess) return e;
-  return fx ? patch_group<1, MARCH_SCH_PPM_PRIM>(dpd, nx, ny, mc, true, s)
-            : patch_group<1, MARCH_SCH_RUNTIME>(dpd, nx, ny, mc, true, s);
+  return march_scheme_fixed(mc) ? patch_scheme<MARCH_SCH_PPM_PRIM>(dpd, nx, ny, mc, fault, s)
+                                : patch_scheme<MARCH_SCH_RUNTIME>(dpd, nx, ny, mc, fault, s);
 }
 
 __global__ void plastic_fab_kernel(double* U, int alo0, int alo1, int anx, int any, int lo0, int lo1, int hi0,

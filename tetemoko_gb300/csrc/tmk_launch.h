@@ -51,6 +51,11 @@ struct Launch {
   // launch; it waits for that kernel before it exits)
   static cudaError_t march(int g, const PatchDev<Real>* patches, const MarchItem* items, int nitems,
                            const MarchConst<Real>& mc, bool pdl, cudaStream_t s);
+  // both groups in one launch, fault-row items finishing their row 0 (after the
+  // fault kernel)
+  static cudaError_t march_both(const PatchDev<Real>* patches, const MarchItem* items0, int n0,
+                                const MarchItem* items1, int n1, const MarchConst<Real>& mc, bool pdl,
+                                cudaStream_t s);
   // row 0 of the fault-row strips of both groups, after the fault kernel
   static cudaError_t march_fault_rows(const PatchDev<Real>* patches, const MarchItem* rows0, int n0,
                                       const MarchItem* rows1, int n1, const MarchConst<Real>& mc,

@@ -88,17 +88,42 @@ struct LaunchImpl {
     cfg.stream = s;
     cfg.attrs = pdl ? attr : nullptr;
     cfg.numAttrs = pdl ? 1 : 0;
-    if (g == 0) {
-      cfg.dynamicSmemBytes = march_smem_bytes<Real, 0>();
-      if (mc.plastic)
-        return fx ? cudaLaunchKernelEx(&cfg, march_kernel<Real, 0, true, MARCH_SCH_PPM_PRIM>, patches, items, nitems, mc)
-                  : cudaLaunchKernelEx(&cfg, march_kernel<Real, 0, true>, patches, items, nitems, mc);
-      return fx ? cudaLaunchKernelEx(&cfg, march_kernel<Real, 0, false, MARCH_SCH_PPM_PRIM>, patches, items, nitems, mc)
-                : cudaLaunchKernelEx(&cfg, march_kernel<Real, 0>, patches, items, nitems, mc);
-    }
-    cfg.dynamicSmemBytes = march_smem_bytes<Real, 1>();
-    return fx ? cudaLaunchKernelEx(&cfg, march_kernel<Real, 1, false, MARCH_SCH_PPM_PRIM>, patches, items, nitems, mc)
-              : cudaLaunchKernelEx(&cfg, march_kernel<Real, 1>, patches, items, nitems, mc);
+    cfg.dynamicSmemBytes = g == 0 ? march_smem_bytes<Real, 0>() : march_smem_bytes<Real, 1>();
+    auto* const kernel = fx ? march_entry<MARCH_SCH_PPM_PRIM>(g, mc) : march_entry<MARCH_SCH_RUNTIME>(g, mc);
+    return cudaLaunchKernelEx(&cfg, kernel, patches, items, nitems, mc);
+  }
+  template <int SCH>
+  static auto march_entry(int g, const MarchConst<Real>& mc) {
+    if (g == 0) return mc.plastic ? march_kernel<Real, 0, true, SCH> : march_kernel<Real, 0, false, SCH>;
+    return march_kernel<Real, 1, false, SCH>;
+  }
+  template <int SCH>
+  static cudaError_t march_both_scheme(const PatchDev<Real>* patches, const MarchItem* items0, int n0,
+                                       const MarchItem* items1, int n1, const MarchConst<Real>& mc, bool pdl,
+                                       cudaStream_t s) {
+    auto* const kernel = march_both_kernel<Real, SCH, MARCH_OWN>;
+    constexpr size_t smem = std::max(march_smem_bytes<Real, 0>(), march_smem_bytes<Real, 1>());
+    static const cudaError_t configured =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (configured != cudaSuccess) return configured;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(32 * MARCH_WARPS);
+    cfg.gridDim = dim3((n0 + MARCH_WARPS - 1) / MARCH_WARPS + (n1 + MARCH_WARPS - 1) / MARCH_WARPS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = pdl ? attr : nullptr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, patches, items0, n0, items1, n1, mc);
+  }
+  static cudaError_t march_both(const PatchDev<Real>* patches, const MarchItem* items0, int n0,
+                                const MarchItem* items1, int n1, const MarchConst<Real>& mc, bool pdl,
+                                cudaStream_t s) {
+    if (n0 + n1 <= 0) return cudaSuccess;
+    return march_scheme_fixed(mc) ? march_both_scheme<MARCH_SCH_PPM_PRIM>(patches, items0, n0, items1, n1, mc, pdl, s)
+                                  : march_both_scheme<MARCH_SCH_RUNTIME>(patches, items0, n0, items1, n1, mc, pdl, s);
   }
   // the dynamic shared memory limit of the marching kernels of one scheme form
   template <int SCH>
@@ -176,6 +201,11 @@ struct LaunchImpl {
   template <> cudaError_t Launch<REAL>::march(int g, const PatchDev<REAL>* p, const MarchItem* it, int n,    \
                                               const MarchConst<REAL>& mc, bool pdl, cudaStream_t s) {      \
     return LaunchImpl<REAL, TXV, TYV, NTV>::march(g, p, it, n, mc, pdl, s);                                  \
+  }                                                                                                          \
+  template <> cudaError_t Launch<REAL>::march_both(const PatchDev<REAL>* p, const MarchItem* i0, int n0,       \
+                                                   const MarchItem* i1, int n1, const MarchConst<REAL>& mc,   \
+                                                   bool pdl, cudaStream_t s) {                                \
+    return LaunchImpl<REAL, TXV, TYV, NTV>::march_both(p, i0, n0, i1, n1, mc, pdl, s);                        \
   }                                                                                                          \
   template <> cudaError_t Launch<REAL>::march_fault_rows(const PatchDev<REAL>* p, const MarchItem* r0,      \
                                                          int n0, const MarchItem* r1, int n1,              \

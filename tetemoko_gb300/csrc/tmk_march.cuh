@@ -621,22 +621,24 @@ TMK_D void fault_row_finish(const PatchDev<T>& pp, const MarchItem& it, const Ma
 // PL: a plastic level with the fused return (in-plane group only): every
 // stored cell takes the plastic return, and the kernel runs after the
 // antiplane one.
-// PATCH: one patch by itself (patches[0]), items by index (strips of columns
-// fastest, runs of mc.patch_run rows), the fluxes of all faces where the patch
-// has arrays for them; an item on the fault keeps its row 0 in shared memory,
-// waits for the fault kernel when the rest of its rows are done and finishes it.
-// FP64 128x128 with fluxes: 83 us a call (in-plane 74, beside it the antiplane
-// kernel and the fault kernel's 48), bound by the FP64 pipe of the one warp a
-// sub-partition holds; the tile kernel, which forms face states, 557 us.
-template <typename T, int G, bool PL = false, int SCH = MARCH_SCH_RUNTIME, bool PATCH = false>
-__global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value) march_kernel(const PatchDev<T>* __restrict__ patches,
-                                                                 const MarchItem* __restrict__ items, int nitems,
-                                                                 const __grid_constant__ MarchConst<T> mc) {
+// FORM: how the items of the fault row end.  MARCH_LEVEL leaves row 0 to
+// march_fault_row_kernel.  The other two run when the fault kernel is the launch
+// before: an item keeps its row 0, waits for the fault kernel when the rest of
+// its rows are done and finishes it, MARCH_OWN on a level (row 0 kept in the
+// level's stash), MARCH_PATCH on one patch by itself (patches[0]; row 0 kept in
+// shared memory, items by index with the strips of columns fastest and runs of
+// mc.patch_run rows, and the fluxes of all faces where the patch has arrays for
+// them).
+constexpr int MARCH_LEVEL = 0, MARCH_PATCH = 1, MARCH_OWN = 2;
+template <typename T, int G, bool PL, int SCH, int FORM>
+TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem* __restrict__ items, int nitems,
+                       const MarchConst<T>& mc, int block) {
   using P = typename PairOf<T>::P;
   constexpr int N = Grp<G>::N, NW = kWaves<G>;
+  constexpr bool PATCH = FORM == MARCH_PATCH;
   extern __shared__ __align__(16) unsigned char march_smem[];
   P* const ring = reinterpret_cast<P*>(march_smem) + (size_t)(threadIdx.x >> 5) * march_warp_pairs<T, G>();
-  const int wid = blockIdx.x * MARCH_WARPS + __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int wid = block * MARCH_WARPS + __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   // a later kernel of the step may be scheduled now; every warp waits for the
   // kernel before it (the fault kernel or the other component group) before
@@ -679,7 +681,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   const MK<T>& kx = mc.kx;
   const MK<T>& ky = mc.ky;
   const bool fault = pp.fault != 0;
-  const bool defer0 = it.fslot >= 0;      // row 0 is finished by march_fault_row_kernel (PATCH: at the end)
+  const bool defer0 = it.fslot >= 0;      // row 0 is finished by march_fault_row_kernel (PATCH, OWN: at the end)
   // what a fault-row item keeps for its row 0
   P* stash0 = nullptr;
   if constexpr (PATCH)
@@ -1011,9 +1013,31 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if constexpr (PATCH) {
-    if (defer0) fault_row_finish<T, G>(pp, it, mc, lane, stash0, true);
+  if constexpr (FORM != MARCH_LEVEL) {
+    if (defer0) fault_row_finish<T, G>(pp, it, mc, lane, stash0, PATCH);
   }
+}
+
+template <typename T, int G, bool PL = false, int SCH = MARCH_SCH_RUNTIME>
+__global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, G>::value)
+march_kernel(const PatchDev<T>* __restrict__ patches, const MarchItem* __restrict__ items, int nitems,
+             const __grid_constant__ MarchConst<T> mc) {
+  march_items<T, G, PL, SCH, MARCH_LEVEL>(patches, items, nitems, mc, (int)blockIdx.x);
+}
+
+// Both groups in one launch, the in-plane CTAs first, where the launches and
+// their order are what a step waits for: after the fault kernel one launch
+// finishes the step, and the groups share the SMs that either leaves idle (mixed
+// 512x256, slip weakening: 16.5 us a step, 18.8 as separate launches).  The
+// patch form, FP64 128x128 with fluxes: 83 us, bound by the FP64 pipe; the tile
+// kernel, which forms face states, 557 us.
+template <typename T, int SCH, int FORM>
+__global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, 0>::value)
+march_both_kernel(const PatchDev<T>* __restrict__ patches, const MarchItem* __restrict__ items0, int n0,
+                  const MarchItem* __restrict__ items1, int n1, const __grid_constant__ MarchConst<T> mc) {
+  const int b0 = (n0 + MARCH_WARPS - 1) / MARCH_WARPS;
+  if ((int)blockIdx.x < b0) march_items<T, 0, false, SCH, FORM>(patches, items0, n0, mc, (int)blockIdx.x);
+  else march_items<T, 1, false, SCH, FORM>(patches, items1, n1, mc, (int)blockIdx.x - b0);
 }
 
 // Row 0 of a fault-row strip of group G once the fault kernel has produced the
