@@ -34,6 +34,8 @@ using tmk::PatchDev;
 using tmk::TileDev;
 using tmk::CopyDev;
 using tmk::fab_idx;
+using tmk::pdl_trigger;
+using tmk::pdl_wait;
 using namespace tmk_host;
 
 namespace {
@@ -115,7 +117,9 @@ __device__ __forceinline__ double bval(const double* B, int blo, int bnx, int c,
 template <typename Real>
 __global__ void cf_sites_kernel(const PatchDev<Real>* __restrict__ cp, const SiteU* __restrict__ su, int nsu,
                                 const SiteB* __restrict__ sb, int nsb, int nb, double a,
-                                Real* __restrict__ svu, double* __restrict__ svb) {
+                                Real* svu, double* svb) {
+  pdl_trigger();
+  pdl_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < nsu * NC) {                      // component-major: neighbouring threads, neighbouring sites
     const SiteU s = su[t % nsu];
@@ -163,7 +167,9 @@ __global__ void cf_sites_kernel(const PatchDev<Real>* __restrict__ cp, const Sit
 template <typename Real>
 __global__ void cf_apply_kernel(const PatchDev<Real>* __restrict__ fp, const FineU* __restrict__ fu, int nfu,
                                 const FineB* __restrict__ fb, int nfb, int nb,
-                                const Real* __restrict__ svu, const double* __restrict__ svb) {
+                                const Real* svu, const double* svb) {
+  pdl_trigger();
+  pdl_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < nfu * NC) {
     const FineU e = fu[t % nfu];
@@ -191,14 +197,18 @@ __global__ void cf_apply_kernel(const PatchDev<Real>* __restrict__ fp, const Fin
 // fault data at the start of a step (AMRLevelLinElast::advance m_BOld.copy)
 template <typename Real>
 __global__ void bsnap_kernel(const PatchDev<Real>* __restrict__ pd, const int* __restrict__ fpatches, int nb) {
+  pdl_trigger();
+  pdl_wait();
   const PatchDev<Real>& P = pd[fpatches[blockIdx.x]];
   const int n = nb * P.bnx;
   for (int k = threadIdx.x; k < n; k += blockDim.x) P.Bold[k] = P.B[k];
 }
 
 // LevelFluxRegister::incrementCoarse: R = -dt * F_coarse
-__global__ void reg_coarse_kernel(const double* __restrict__ cap, const int* __restrict__ cslot, int nent, double dt,
-                                  double* __restrict__ R) {
+__global__ void reg_coarse_kernel(const double* cap, const int* __restrict__ cslot, int nent, double dt,
+                                  double* R) {
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nent * NC) return;
   const int e = t / NC, c = t % NC;
@@ -206,8 +216,10 @@ __global__ void reg_coarse_kernel(const double* __restrict__ cap, const int* __r
 }
 
 // LevelFluxRegister::incrementFine: R += (dt / r) * F_fine over the r fine faces
-__global__ void reg_fine_kernel(const double* __restrict__ cap, const int* __restrict__ fslot, int nent, int r,
-                                double s, double* __restrict__ R) {
+__global__ void reg_fine_kernel(const double* cap, const int* __restrict__ fslot, int nent, int r,
+                                double s, double* R) {
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nent * NC) return;
   const int e = t / NC, c = t % NC;
@@ -220,7 +232,9 @@ __global__ void reg_fine_kernel(const double* __restrict__ cap, const int* __res
 template <typename Real>
 __global__ void reflux_kernel(const PatchDev<Real>* __restrict__ cp, const RefluxCell* __restrict__ cells, int ncells,
                               const int* __restrict__ list, const double* __restrict__ sc,
-                              const double* __restrict__ R) {
+                              const double* R) {
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ncells * NC) return;
   const RefluxCell cl = cells[t % ncells];
@@ -241,6 +255,8 @@ template <typename Real>
 __global__ void avgdown_kernel(const PatchDev<Real>* __restrict__ cp, const PatchDev<Real>* __restrict__ fp,
                                const AvgU* __restrict__ au, int nau, const AvgB* __restrict__ ab, int nab, int nb,
                                int r, double sU, double sB, int both) {
+  pdl_trigger();
+  pdl_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < nau) {                           // one coarse cell, all components: neighbouring threads, neighbouring cells
     const AvgU e = au[t];
@@ -482,6 +498,9 @@ tmk_status rebuild_captures_impl(tmk_level_s* L) {
   for (int g = 0; g < 2 && L->march_allowed; ++g) {
     std::vector<tmk::MarchItem>& items = L->hitems[g];
     std::vector<std::vector<int4>> per(items.size());
+    // items come patch by patch
+    std::vector<size_t> first(L->patches.size() + 1, items.size());
+    for (size_t k = items.size(); k-- > 0;) first[items[k].patch] = k;
     for (const auto& kv : slot) {
       const int p = std::get<0>(kv.first), d = std::get<1>(kv.first);
       const int i = std::get<2>(kv.first), j = std::get<3>(kv.first);
@@ -490,9 +509,9 @@ tmk_status rebuild_captures_impl(tmk_level_s* L) {
       if (d == 0) { kind = i <= v.hi[0] ? 0 : 1; if (kind == 1) ci = i - 1; }
       else { kind = j <= v.hi[1] ? 2 : 3; if (kind == 3) cj = j - 1; }
       int owner = -1;
-      for (size_t k = 0; k < items.size(); ++k) {
+      for (size_t k = first[p]; k < items.size() && items[k].patch == p; ++k) {
         const tmk::MarchItem& m = items[k];
-        if (m.patch == p && ci >= m.x0 && ci < m.x0 + tmk::MARCH_COLS && cj >= m.y0 && cj <= m.y1) { owner = (int)k; break; }
+        if (ci >= m.x0 && ci < m.x0 + tmk::MARCH_COLS && cj >= m.y0 && cj <= m.y1) { owner = (int)k; break; }
       }
       if (owner < 0) return TMK_ERR_BAD_DESC;
       per[owner].push_back(make_int4(cj, kind, ci - items[owner].x0 + tmk::MARCH_HALO, kv.second));
@@ -504,9 +523,8 @@ tmk_status rebuild_captures_impl(tmk_level_s* L) {
       items[k].ncap = (int)per[k].size();
       caps.insert(caps.end(), per[k].begin(), per[k].end());
     }
-    for (tmk::MarchItem& f : L->hfrows[g])
-      for (const tmk::MarchItem& m : items)
-        if (m.patch == f.patch && m.x0 == f.x0 && m.y0 == f.y0) { f.cap0 = m.cap0; f.ncap = m.ncap; break; }
+    for (const tmk::MarchItem& m : items)
+      if (m.fslot >= 0) { L->hfrows[g][m.fslot].cap0 = m.cap0; L->hfrows[g][m.fslot].ncap = m.ncap; }
     L->dmcap[g] = nullptr;
     if (!caps.empty()) {
       if (dalloc(&L->dmcap[g], caps.size()) != cudaSuccess) return TMK_ERR_ALLOC;
@@ -782,12 +800,10 @@ tmk_status launch_fill(CFLink* k, double alpha, cudaStream_t s) {
   if (ns == 0) return TMK_OK;
   const PatchDev<Real>* cp = (const PatchDev<Real>*)k->C->dpatch[k->C->parity];
   const PatchDev<Real>* fp = (const PatchDev<Real>*)k->F->dpatch[k->F->parity];
-  cf_sites_kernel<Real><<<blocks_for(ns, 128), 128, 0, s>>>(cp, k->dsu, k->nsu, k->dsb, k->nsb, nb, alpha,
-                                                             (Real*)k->dsvu, k->dsvb);
-  TMK_CU(cudaGetLastError());
-  cf_apply_kernel<Real><<<blocks_for(nf, 128), 128, 0, s>>>(fp, k->dfu, k->nfu, k->dfb, k->nfb, nb,
-                                                             (const Real*)k->dsvu, k->dsvb);
-  TMK_CU(cudaGetLastError());
+  TMK_CU(tmk::launch_chained(cf_sites_kernel<Real>, dim3(blocks_for(ns, 128)), 128, 0, true, s, cp, k->dsu, k->nsu, k->dsb,
+                             k->nsb, nb, alpha, (Real*)k->dsvu, k->dsvb));
+  TMK_CU(tmk::launch_chained(cf_apply_kernel<Real>, dim3(blocks_for(nf, 128)), 128, 0, true, s, fp, k->dfu, k->nfu, k->dfb,
+                             k->nfb, nb, (const Real*)k->dsvu, k->dsvb));
   return TMK_OK;
 }
 
@@ -799,9 +815,8 @@ template <typename Real>
 tmk_status launch_reflux(CFLink* k, cudaStream_t s) {
   if (!k->ncells) return TMK_OK;
   const PatchDev<Real>* cp = (const PatchDev<Real>*)k->C->dpatch[k->C->parity];
-  reflux_kernel<Real><<<blocks_for((long long)k->ncells * NC, 128), 128, 0, s>>>(cp, k->dcells, k->ncells,
-                                                                                   k->dlist, k->dsc, k->dR);
-  TMK_CU(cudaGetLastError());
+  TMK_CU(tmk::launch_chained(reflux_kernel<Real>, dim3(blocks_for((long long)k->ncells * NC, 128)), 128, 0, true, s, cp,
+                             k->dcells, k->ncells, k->dlist, k->dsc, k->dR));
   return TMK_OK;
 }
 
@@ -814,9 +829,8 @@ tmk_status launch_avgdown(CFLink* k, cudaStream_t s) {
   const PatchDev<Real>* fp = (const PatchDev<Real>*)k->F->dpatch[k->F->parity];
   const int r = k->r;
   const int both = k->C->ctx->scheme.plasticity ? 0 : 1;
-  avgdown_kernel<Real><<<blocks_for(n, 128), 128, 0, s>>>(cp, fp, k->dau, k->nau, k->dab, k->nab, nb, r,
-                                                          1.0 / (double)(r * r), 1.0 / (double)r, both);
-  TMK_CU(cudaGetLastError());
+  TMK_CU(tmk::launch_chained(avgdown_kernel<Real>, dim3(blocks_for(n, 128)), 128, 0, true, s, cp, fp, k->dau, k->nau, k->dab,
+                             k->nab, nb, r, 1.0 / (double)(r * r), 1.0 / (double)r, both));
   return TMK_OK;
 }
 
@@ -850,12 +864,11 @@ tmk_status rebuild_captures(tmk_level_s* L) { return rebuild_captures_impl(L); }
 tmk_status amr_pre_step(tmk_level_s* L, double time, double dt, double tco, double tcn, cudaStream_t s) {
   if (L->finer && L->nfault && L->ctx->nb > 0) {
     if (L->prec == TMK_PREC_MIXED)
-      bsnap_kernel<float><<<L->nfault, 256, 0, s>>>((const PatchDev<float>*)L->dpatch[L->parity], L->dfault,
-                                                     L->ctx->nb);
+      TMK_CU(tmk::launch_chained(bsnap_kernel<float>, dim3(L->nfault), 256, 0, true, s,
+                                 (const PatchDev<float>*)L->dpatch[L->parity], L->dfault, L->ctx->nb));
     else
-      bsnap_kernel<double><<<L->nfault, 256, 0, s>>>((const PatchDev<double>*)L->dpatch[L->parity], L->dfault,
-                                                      L->ctx->nb);
-    TMK_CU(cudaGetLastError());
+      TMK_CU(tmk::launch_chained(bsnap_kernel<double>, dim3(L->nfault), 256, 0, true, s,
+                                 (const PatchDev<double>*)L->dpatch[L->parity], L->dfault, L->ctx->nb));
   }
   if (L->coarser) {
     const double alpha = snap_alpha(time, dt, tco, tcn, L->coarser->r);
@@ -868,14 +881,13 @@ tmk_status amr_pre_step(tmk_level_s* L, double time, double dt, double tco, doub
 tmk_status amr_post_step(tmk_level_s* L, double dt, cudaStream_t s) {
   if (L->finer && L->finer->nent) {
     CFLink* k = L->finer;
-    reg_coarse_kernel<<<blocks_for((long long)k->nent * NC, 128), 128, 0, s>>>(L->cap, k->dcslot, k->nent, dt, k->dR);
-    TMK_CU(cudaGetLastError());
+    TMK_CU(tmk::launch_chained(reg_coarse_kernel, dim3(blocks_for((long long)k->nent * NC, 128)), 128, 0, true, s, L->cap,
+                               k->dcslot, k->nent, dt, k->dR));
   }
   if (L->coarser && L->coarser->nent) {
     CFLink* k = L->coarser;
-    reg_fine_kernel<<<blocks_for((long long)k->nent * NC, 128), 128, 0, s>>>(L->cap, k->dfslot, k->nent, k->r,
-                                                                             dt / (double)k->r, k->dR);
-    TMK_CU(cudaGetLastError());
+    TMK_CU(tmk::launch_chained(reg_fine_kernel, dim3(blocks_for((long long)k->nent * NC, 128)), 128, 0, true, s, L->cap,
+                               k->dfslot, k->nent, k->r, dt / (double)k->r, k->dR));
   }
   return TMK_OK;
 }
@@ -1201,7 +1213,7 @@ struct tmk_graph_s {
 namespace {
 
 // parameter counts of fault_kernel, fault_ref9_kernel and station_kernel
-constexpr int kFaultParams = 6, kFaultRef9Params = 5;
+constexpr int kFaultParams = 7, kFaultRef9Params = 5;
 constexpr int kStationParams = 10;
 
 tmk_status graph_finish(tmk_graph_s* g) {

@@ -471,7 +471,7 @@ extern "C" tmk_status tmk_patch_update_state(tmk_context* c, const tmk_fab* U, c
   const PatchDev<double>* dpd = (const PatchDev<double>*)(base + off_pd);
   const int* dfp = (const int*)(base + off_pd + offsetof(Head, fault_patch));
   if (fault)
-    TMK_CU(tmk::Launch<double>::fault(dpd, dfp, 1, nvx, c->dp, c->hp, dt, dx, time, c->dstatus, false,
+    TMK_CU(tmk::Launch<double>::fault(dpd, dfp, 1, nvx, c->dp, c->hp, dt, dx, time, c->dstatus, tmk::FAULT_ALONE,
                                         tmk::fault_seg_of(c->hp, tmk::FAULT_SEG), s));
   if (march) {
     TMK_CU(tmk::patch_march(dpd, nvx, nvy, fault, c->hp, dt, dx, s));
@@ -738,18 +738,9 @@ tmk_status level_create_impl(tmk_context* const* ctxs, int nscen, const tmk_box*
     TMK_CU(cudaMemcpy(L->dcopies, copies.data(), copies.size() * sizeof(CopyDev), cudaMemcpyHostToDevice));
   }
   if (L->nbcopies) {
-    std::vector<double*> bp(npatch, nullptr);
-    std::vector<int> blo(npatch, 0), bnx(npatch, 0);
-    for (int p = 0; p < npatch; ++p) { bp[p] = L->patches[p].B; blo[p] = L->patches[p].blo; bnx[p] = L->patches[p].bnx; }
-    if (dalloc(&L->dbcopies, bcopies.size()) != cudaSuccess || dalloc(&L->dbptr, npatch) != cudaSuccess ||
-        dalloc(&L->dblo, npatch) != cudaSuccess || dalloc(&L->dbnx, npatch) != cudaSuccess)
-      return fail(TMK_ERR_ALLOC);
-    L->allocs.push_back(L->dbcopies); L->allocs.push_back(L->dbptr);
-    L->allocs.push_back(L->dblo); L->allocs.push_back(L->dbnx);
+    if (dalloc(&L->dbcopies, bcopies.size()) != cudaSuccess) return fail(TMK_ERR_ALLOC);
+    L->allocs.push_back(L->dbcopies);
     TMK_CU(cudaMemcpy(L->dbcopies, bcopies.data(), bcopies.size() * sizeof(CopyDev), cudaMemcpyHostToDevice));
-    TMK_CU(cudaMemcpy(L->dbptr, bp.data(), npatch * sizeof(double*), cudaMemcpyHostToDevice));
-    TMK_CU(cudaMemcpy(L->dblo, blo.data(), npatch * sizeof(int), cudaMemcpyHostToDevice));
-    TMK_CU(cudaMemcpy(L->dbnx, bnx.data(), npatch * sizeof(int), cudaMemcpyHostToDevice));
   }
   if (L->prec == TMK_PREC_MIXED) {
     if (dalloc(&L->stage, max_count) != cudaSuccess) return fail(TMK_ERR_ALLOC);
@@ -1035,11 +1026,10 @@ tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEve
   tmk_context* c = L->ctx;
   const PatchDev<Real>* pd = (const PatchDev<Real>*)L->dpatch[par];
   const int seg = L->sw_ref9 ? 0 : L->tune.fault_seg;
-  TMK_CU(tmk::Launch<Real>::exchange(pd, L->dcopies, L->ncopies, 0, TMK_NCOMP, s));
-  TMK_CU(tmk::bexchange(L->dbptr, L->dblo, L->dbnx, L->dbcopies, L->nbcopies, c->nb, s));
+  TMK_CU(tmk::Launch<Real>::exchange(pd, L->dcopies, L->ncopies, 0, TMK_NCOMP, L->dbcopies, L->nbcopies, c->nb, s));
   if (ev) TMK_CU(cudaEventRecord(ev[1], s));
   if (!L->march) {
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
+    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, tmk::FAULT_ALONE, seg, s));
     if (ev) TMK_CU(cudaEventRecord(ev[2], s));
     TMK_CU(tmk::Launch<Real>::volume(pd, L->dtiles, L->ntiles, L->dparams, s));
     return TMK_OK;
@@ -1067,11 +1057,11 @@ tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEve
       }
       TMK_CU(cudaEventRecord(L->fork_ev, s));
       TMK_CU(cudaStreamWaitEvent(L->side, L->fork_ev, 0));
-      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false,
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, tmk::FAULT_ALONE,
                                       seg, L->side));
       TMK_CU(cudaEventRecord(L->join_ev, L->side));
     } else {
-      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false,
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, tmk::FAULT_ALONE,
                                       seg, s));
       if (ev) TMK_CU(cudaEventRecord(ev[2], s));
     }
@@ -1083,18 +1073,19 @@ tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEve
     return TMK_OK;
   }
   if (both_groups(L)) {
-    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
+    TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus,
+                                    ev ? tmk::FAULT_ALONE : tmk::FAULT_AFTER, seg, s));
     if (ev) TMK_CU(cudaEventRecord(ev[2], s));
     TMK_CU(tmk::Launch<Real>::march_both(pd, L->ditems[0], L->nitems[0], L->ditems[1], L->nitems[1], mc,
                                          L->nfault && !ev, s));
   } else {
     if (ev) {
-      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, false, seg, s));
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, tmk::FAULT_ALONE, seg, s));
       TMK_CU(cudaEventRecord(ev[2], s));
       TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
     } else {
       TMK_CU(tmk::Launch<Real>::march(0, pd, L->ditems[0], L->nitems[0], mc, false, s));
-      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, true, seg, s));
+      TMK_CU(tmk::Launch<Real>::fault(pd, L->dfault, L->nfault, L->max_faces, L->dparams, c->hp, dt, L->dx, time, c->dstatus, tmk::FAULT_BESIDE, seg, s));
     }
     TMK_CU(tmk::Launch<Real>::march(1, pd, L->ditems[1], L->nitems[1], mc, true, s));
     TMK_CU(tmk::Launch<Real>::march_fault_rows(pd, L->dfrows[0], L->nfrows[0], L->dfrows[1], L->nfrows[1], mc, s));
@@ -1329,7 +1320,7 @@ extern "C" int tmk_level_launches_per_step(const tmk_level* L) {
   const int frows = fused ? (L->nfrows[0] ? 1 : 0) + (L->nfrows[1] ? 1 : 0) : (L->nfrows[0] + L->nfrows[1] ? 1 : 0);
   const int groups = both_groups(L) ? 1 : (L->nitems[0] ? 1 : 0) + (L->nitems[1] ? 1 : 0) + frows;
   const int vol = L->march ? groups + (plastic && !fused && L->ntiles ? 1 : 0) : (L->ntiles ? 1 : 0);
-  return (L->ncopies ? 1 : 0) + (L->nbcopies ? 1 : 0) + (L->nfault ? 1 : 0) + vol + amr_launches(L);
+  return (L->ncopies + L->nbcopies ? 1 : 0) + (L->nfault ? 1 : 0) + vol + amr_launches(L);
 }
 
 extern "C" tmk_status tmk_level_status(tmk_level* L, long long info[3]) {

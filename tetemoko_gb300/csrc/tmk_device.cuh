@@ -22,6 +22,30 @@
 
 namespace tmk {
 
+// Programmatic dependent launch.  The small kernels of a step are chained by it:
+// each lets the next one be scheduled when all its CTAs have started, and waits
+// for the one before it to complete before it touches what earlier kernels
+// write, so they still run in order but without the gaps between them (about
+// a microsecond each).  Data that an earlier kernel of the chain wrote is read
+// with plain loads: a read-only load could move above the wait.
+TMK_D void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+TMK_D void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... K, typename... A>
+cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, int threads, size_t smem, bool chained, cudaStream_t s,
+                           A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = chained ? attr : nullptr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 constexpr int NC = 22;
 constexpr int NSIDE = 9;          // evolving components per side
 constexpr int NGHOST = 4;

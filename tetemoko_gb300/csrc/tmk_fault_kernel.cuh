@@ -148,7 +148,8 @@ __global__ void __launch_bounds__(fault_threads(SEG)) fault_kernel(const PatchDe
                                                                    const int* __restrict__ fault_patches,
                                                                    const DevParams* __restrict__ params, double time,
                                                                    DevStatus* st,
-                                                                   const __grid_constant__ FaultConst<Real> fc) {
+                                                                   const __grid_constant__ FaultConst<Real> fc,
+                                                                   int after) {
   using T = Real;
   constexpr bool kFp64 = std::is_same<Real, double>::value;
   constexpr int NCELL = SEG + 2;             // cells / faces [s0-1, s0+SEG]
@@ -157,11 +158,14 @@ __global__ void __launch_bounds__(fault_threads(SEG)) fault_kernel(const PatchDe
   __shared__ T sVc[2][2][SEG];                          // ... velocities corrected by the x fluxes
   __shared__ double sA[2][3][NCELL], sB[2][3][SEG];     // the whole values (with the background) in FP64, both passes
   // The kernel launched after this one may be scheduled now (it reads none of
-  // this kernel's outputs before it waits for it).  When this kernel itself is
-  // a programmatic dependent of the in-plane marching kernel, it reads nothing
-  // that kernel writes (the state it reads is the step's input buffer) and it
-  // waits for it before exiting, so that the step's kernels complete in order.
-  asm volatile("griddepcontrol.launch_dependents;");
+  // this kernel's outputs before it waits for it).  As a programmatic dependent
+  // of the in-plane marching kernel this one reads nothing that kernel writes
+  // (the state it reads is the step's input buffer) and waits for it before
+  // exiting, so that the step's kernels complete in order.  As the step's first
+  // kernel after its ghost cells (`after`) it waits for what is before it, also
+  // for the kernel it lets start, which reads those cells.
+  if (after) pdl_wait();
+  pdl_trigger();
   const PatchDev<Real>& p = patches[fault_patches[blockIdx.y]];
   const DevParams& P = params[p.scen];
   const int s0 = p.vlo0 + blockIdx.x * SEG;

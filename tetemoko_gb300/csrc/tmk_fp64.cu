@@ -28,18 +28,9 @@ static cudaError_t patch_scheme(const PatchDev<double>* dpd, int nx, int ny, Mar
     if (run == 16 || c < cost) { mc.patch_run = run; cost = c; }
   }
   const int nitems = ns * ((ny + mc.patch_run - 1) / mc.patch_run);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(32 * MARCH_WARPS);
-  cfg.gridDim = dim3(2 * ((nitems + MARCH_WARPS - 1) / MARCH_WARPS));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = pdl ? attr : nullptr;
-  cfg.numAttrs = pdl ? 1 : 0;
   const MarchItem* const none = nullptr;
-  return cudaLaunchKernelEx(&cfg, kernel, dpd, none, nitems, none, nitems, mc);
+  return launch_chained(kernel, dim3(2 * ((nitems + MARCH_WARPS - 1) / MARCH_WARPS)), 32 * MARCH_WARPS, smem, pdl, s, dpd,
+                        none, nitems, none, nitems, mc);
 }
 
 cudaError_t patch_march(const PatchDev<double>* dpd, int nx, int ny, bool fault, const DevParams& hp, double dt,
@@ -217,24 +208,5 @@ cudaError_t copy_valid_comps(const double* src, double* dst, int alo0, int alo1,
 cudaError_t convert_d2f(const double* src, float* dst, size_t n, cudaStream_t s) { return convert_launch(src, dst, n, s); }
 cudaError_t convert_f2d(const float* src, double* dst, size_t n, cudaStream_t s) { return convert_launch(src, dst, n, s); }
 cudaError_t copy_fab(const double* src, double* dst, size_t n, cudaStream_t s) { return convert_launch(src, dst, n, s); }
-
-// Fault-row exchange: copy boundary data faces [lo0, hi0] from src to dst patch.
-__global__ void bexchange_kernel(double* const* __restrict__ bptr, const int* __restrict__ blo,
-                                 const int* __restrict__ bnx, const CopyDev* __restrict__ copies, int nb) {
-  const CopyDev cp = copies[blockIdx.x];
-  const int n = cp.hi0 - cp.lo0 + 1;
-  for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
-    int c = idx / n, i = cp.lo0 + idx % n;
-    bptr[cp.dst][(size_t)c * bnx[cp.dst] + (i - blo[cp.dst])] = bptr[cp.src][(size_t)c * bnx[cp.src] + (i - blo[cp.src])];
-  }
-}
-
-
-cudaError_t bexchange(double* const* bptr, const int* blo, const int* bnx, const CopyDev* copies, int ncopies,
-                      int nb, cudaStream_t s) {
-  if (ncopies <= 0) return cudaSuccess;
-  bexchange_kernel<<<ncopies, 128, 0, s>>>(bptr, blo, bnx, copies, nb);
-  return cudaGetLastError();
-}
 
 }  // namespace tmk

@@ -111,9 +111,6 @@ struct tmk_level_s {
   int ncopies = 0;
   tmk::CopyDev* dbcopies = nullptr;
   int nbcopies = 0;
-  double** dbptr = nullptr;
-  int* dblo = nullptr;
-  int* dbnx = nullptr;
   double* stage = nullptr;                 // FP64 staging for set/get of the mixed form
   size_t stage_count = 0;
   // put/take of a pinned host FAB in the mixed form: the copy-engine stream

@@ -544,6 +544,7 @@ __global__ void __launch_bounds__(256) plastic_tiles_kernel(const PatchDev<Real>
                                                             const TileDev* __restrict__ tiles,
                                                             const DevParams* __restrict__ params) {
   using T = Real;
+  pdl_trigger();
   const TileDev tl = tiles[blockIdx.x];
   const PatchDev<Real>& p = patches[tl.patch];
   // the parameters in T once per CTA (FP64-to-FP32 conversions use GB300's
@@ -555,6 +556,7 @@ __global__ void __launch_bounds__(256) plastic_tiles_kernel(const PatchDev<Real>
     sdt = (T)p.dt;
   }
   __syncthreads();
+  pdl_wait();
   const T dt = sdt;
   for (int idx = threadIdx.x; idx < tl.nx * tl.ny; idx += blockDim.x) {
     const int x = tl.x0 + idx % tl.nx, y = tl.y0 + idx / tl.nx;
@@ -589,13 +591,26 @@ struct CopyDev { int src, dst; int lo0, lo1, hi0, hi1; };
 
 template <typename Real>
 __global__ void exchange_kernel(const PatchDev<Real>* __restrict__ patches, const CopyDev* __restrict__ copies,
-                                int c0, int ncomp, int to_in) {
+                                int ncopies, int c0, int ncomp, const CopyDev* __restrict__ bcopies, int nb) {
+  pdl_trigger();
+  if ((int)blockIdx.x >= ncopies) {        // fault data: nb planes of a run of faces
+    const CopyDev cp = bcopies[blockIdx.x - ncopies];
+    const PatchDev<Real>& ps = patches[cp.src];
+    const PatchDev<Real>& pd = patches[cp.dst];
+    const int n = cp.hi0 - cp.lo0 + 1;
+    pdl_wait();
+    for (int idx = threadIdx.x + blockIdx.y * blockDim.x; idx < nb * n; idx += blockDim.x * gridDim.y) {
+      const int c = idx / n, i = cp.lo0 + idx % n;
+      pd.B[(size_t)c * pd.bnx + (i - pd.blo0)] = ps.B[(size_t)c * ps.bnx + (i - ps.blo0)];
+    }
+    return;
+  }
   const CopyDev cp = copies[blockIdx.x];
   const PatchDev<Real>& ps = patches[cp.src];
   const PatchDev<Real>& pd = patches[cp.dst];
   const int nx = cp.hi0 - cp.lo0 + 1, ny = cp.hi1 - cp.lo1 + 1;
-  const Real* src = (to_in ? ps.Uout : ps.Uin) + fab_idx(ps, c0, cp.lo0, cp.lo1);
-  Real* dst = (to_in ? (Real*)pd.Uout : (Real*)pd.Uin) + fab_idx(pd, c0, cp.lo0, cp.lo1);
+  const Real* src = ps.Uin + fab_idx(ps, c0, cp.lo0, cp.lo1);
+  Real* dst = (Real*)pd.Uin + fab_idx(pd, c0, cp.lo0, cp.lo1);
   const size_t splane = (size_t)ps.any * ps.anx, dplane = (size_t)pd.any * pd.anx;
   const int nrow = ncomp * ny;
   const int step = blockDim.x * gridDim.y, t0 = threadIdx.x + blockIdx.y * blockDim.x;
@@ -603,6 +618,7 @@ __global__ void exchange_kernel(const PatchDev<Real>* __restrict__ patches, cons
   constexpr int W = 16 / sizeof(Real);
   const bool vec = nx % W == 0 && ps.anx % W == 0 && pd.anx % W == 0 && splane % W == 0 && dplane % W == 0 &&
                    ((uintptr_t)src & 15) == 0 && ((uintptr_t)dst & 15) == 0;
+  pdl_wait();
   if (vec) {
     // four vectors per thread in flight: all loads, then all stores
     constexpr int U = 4;
@@ -615,7 +631,7 @@ __global__ void exchange_kernel(const PatchDev<Real>* __restrict__ patches, cons
         const int idx = base + u * step;
         if (idx < n) {
           const int row = idx / nv, k = idx - row * nv, c = row / ny, j = row - c * ny;
-          v[u] = __ldg((const float4*)(src + c * splane + (size_t)j * ps.anx + k * W));
+          v[u] = *(const float4*)(src + c * splane + (size_t)j * ps.anx + k * W);
           o[u] = c * dplane + (size_t)j * pd.anx + k * W;
         }
       }

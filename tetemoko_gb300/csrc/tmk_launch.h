@@ -21,25 +21,30 @@ constexpr int FAULT_SEG_SMALL = 16;
 // component 9), which needs whole states
 inline int fault_seg_of(const DevParams& p, int seg) { return p.fault_law == 2 && p.sw_off != 11 ? 0 : seg; }
 
+enum : int { FAULT_ALONE = 0, FAULT_BESIDE, FAULT_AFTER };
+
 template <typename Real>
 struct Launch {
   static const int TX, TY;
   // one thread per fault face of every fault patch, seg faces per CTA (32 or
   // 16; 0: the reference-layout slip-weakening kernel, which takes either
-  // layout, scenario by scenario); hp: the level's parameters on the host (the launch constants are
-  // built from them); pdl as for march
+  // layout, scenario by scenario); hp: the level's parameters on the host (the
+  // launch constants are built from them); place: FAULT_ALONE a plain launch,
+  // FAULT_BESIDE scheduled beside the in-plane kernel before it, FAULT_AFTER
+  // chained to whatever is before it
   static cudaError_t fault(const PatchDev<Real>* patches, const int* fault_patches, int nfault, int max_faces,
                            const DevParams* params, const DevParams& hp, double dt, double dx, double time,
-                           DevStatus* st, bool pdl, int seg, cudaStream_t s);
+                           DevStatus* st, int place, int seg, cudaStream_t s);
   // one CTA per (tile, side)
   static cudaError_t volume(const PatchDev<Real>* patches, const TileDev* tiles, int ntiles,
                             const DevParams* params, cudaStream_t s);
   // plastic correction of every tile's cells after the marching kernels
   static cudaError_t plastic(const PatchDev<Real>* patches, const TileDev* tiles, int ntiles,
                              const DevParams* params, cudaStream_t s);
-  // same-level ghost exchange of components [c0, c0+ncomp) into the input buffers
+  // same-level ghost exchange of components [c0, c0+ncomp) into the input
+  // buffers, and of the fault data (bcopies, nb planes)
   static cudaError_t exchange(const PatchDev<Real>* patches, const CopyDev* copies, int ncopies, int c0,
-                              int ncomp, cudaStream_t s);
+                              int ncomp, const CopyDev* bcopies, int nbcopies, int nb, cudaStream_t s);
   static size_t volume_smem();
   // the tile kernel's staged box (columns, rows) of one component: the TMA
   // tensor maps of the FABs it reads are encoded with it
@@ -97,8 +102,6 @@ cudaError_t copy_valid_comps(const double* src, double* dst, int alo0, int alo1,
 // copy components [c0, c0+ncomp) of the valid box of a FAB into another FAB of the same shape
 cudaError_t copy_valid(const double* src, double* dst, int alo0, int alo1, int anx, int any, int vlo0, int vlo1,
                        int vhi0, int vhi1, int c0, int ncomp, cudaStream_t s);
-cudaError_t bexchange(double* const* bptr, const int* blo, const int* bnx, const CopyDev* copies, int ncopies,
-                      int nb, cudaStream_t s);
 // PLASTICCORRECTION over a box of an FP64 FAB
 cudaError_t plastic_fab(double* U, int alo0, int alo1, int anx, int any, int lo0, int lo1, int hi0, int hi1,
                         const DevParams* P, double dt, cudaStream_t s);

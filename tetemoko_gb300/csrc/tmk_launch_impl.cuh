@@ -12,29 +12,17 @@ template <typename Real, int TX_, int TY_, int NT_>
 struct LaunchImpl {
   static cudaError_t fault(const PatchDev<Real>* patches, const int* fp, int nfault, int max_faces,
                            const DevParams* params, const DevParams& hp, double dt, double dx, double time,
-                           DevStatus* st, bool pdl, int seg, cudaStream_t s) {
+                           DevStatus* st, int place, int seg, cudaStream_t s) {
     if (nfault <= 0) return cudaSuccess;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.stream = s;
-    cfg.attrs = pdl ? attr : nullptr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    if (seg == 0) {
-      cfg.gridDim = dim3((max_faces + REF9_SEG - 1) / REF9_SEG, nfault);
-      cfg.blockDim = dim3(REF9_THREADS);
-      return cudaLaunchKernelEx(&cfg, fault_ref9_kernel<Real>, patches, fp, params, time, st);
-    }
+    if (seg == 0)
+      return launch_chained(fault_ref9_kernel<Real>, dim3((max_faces + REF9_SEG - 1) / REF9_SEG, nfault), REF9_THREADS, 0,
+                            place == FAULT_BESIDE, s, patches, fp, params, time, st);
     FaultConst<Real> fc;
     fc.load(hp, dt, dx);
-    const bool small = seg == FAULT_SEG_SMALL;
-    const int sg = small ? FAULT_SEG_SMALL : FAULT_SEG;
-    cfg.gridDim = dim3((max_faces + sg - 1) / sg, nfault);
-    cfg.blockDim = dim3(fault_threads(sg));
-    if (small)
-      return cudaLaunchKernelEx(&cfg, fault_kernel<Real, FAULT_SEG_SMALL>, patches, fp, params, time, st, fc);
-    return cudaLaunchKernelEx(&cfg, fault_kernel<Real, FAULT_SEG>, patches, fp, params, time, st, fc);
+    const int sg = seg == FAULT_SEG_SMALL ? FAULT_SEG_SMALL : FAULT_SEG;
+    auto* const kernel = sg == FAULT_SEG_SMALL ? fault_kernel<Real, FAULT_SEG_SMALL> : fault_kernel<Real, FAULT_SEG>;
+    return launch_chained(kernel, dim3((max_faces + sg - 1) / sg, nfault), fault_threads(sg), 0, place != FAULT_ALONE, s,
+                          patches, fp, params, time, st, fc, place == FAULT_AFTER ? 1 : 0);
   }
   static size_t smem() { return sizeof(VolSmem<Real, TX_, TY_>); }
   static int box_x() { return VolSmem<Real, TX_, TY_>::RXP; }
@@ -57,16 +45,15 @@ struct LaunchImpl {
   static cudaError_t plastic(const PatchDev<Real>* patches, const TileDev* tiles, int ntiles,
                              const DevParams* params, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
-    plastic_tiles_kernel<Real><<<ntiles, 256, 0, s>>>(patches, tiles, params);
-    return cudaGetLastError();
+    return launch_chained(plastic_tiles_kernel<Real>, dim3(ntiles), 256, 0, true, s, patches, tiles, params);
   }
   static cudaError_t exchange(const PatchDev<Real>* patches, const CopyDev* copies, int ncopies, int c0,
-                              int ncomp, cudaStream_t s) {
-    if (ncopies <= 0) return cudaSuccess;
+                              int ncomp, const CopyDev* bcopies, int nbcopies, int nb, cudaStream_t s) {
+    if (ncopies + nbcopies <= 0) return cudaSuccess;
     // about two waves of 256-thread CTAs: each copy box spread over up to 8 CTAs
-    const int chunks = std::max(1, std::min(8, (2 * 8 * 152 + ncopies - 1) / ncopies));
-    exchange_kernel<Real><<<dim3(ncopies, chunks), 256, 0, s>>>(patches, copies, c0, ncomp, 0);
-    return cudaGetLastError();
+    const int chunks = std::max(1, std::min(8, (2 * 8 * 152 + ncopies) / (ncopies + 1)));
+    return launch_chained(exchange_kernel<Real>, dim3(ncopies + nbcopies, chunks), 256, 0, true, s, patches, copies,
+                          ncopies, c0, ncomp, bcopies, nb);
   }
   static cudaError_t march(int g, const PatchDev<Real>* patches, const MarchItem* items, int nitems,
                            const MarchConst<Real>& mc, bool pdl, cudaStream_t s) {
@@ -79,18 +66,10 @@ struct LaunchImpl {
       configured = true;
     }
     const bool fx = march_scheme_fixed(mc);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(32 * MARCH_WARPS);
-    cfg.gridDim = dim3((nitems + MARCH_WARPS - 1) / MARCH_WARPS);
-    cfg.stream = s;
-    cfg.attrs = pdl ? attr : nullptr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cfg.dynamicSmemBytes = g == 0 ? march_smem_bytes<Real, 0>() : march_smem_bytes<Real, 1>();
     auto* const kernel = fx ? march_entry<MARCH_SCH_PPM_PRIM>(g, mc) : march_entry<MARCH_SCH_RUNTIME>(g, mc);
-    return cudaLaunchKernelEx(&cfg, kernel, patches, items, nitems, mc);
+    return launch_chained(kernel, dim3((nitems + MARCH_WARPS - 1) / MARCH_WARPS), 32 * MARCH_WARPS,
+                          g == 0 ? march_smem_bytes<Real, 0>() : march_smem_bytes<Real, 1>(), pdl, s, patches, items,
+                          nitems, mc);
   }
   template <int SCH>
   static auto march_entry(int g, const MarchConst<Real>& mc) {
@@ -106,17 +85,8 @@ struct LaunchImpl {
     static const cudaError_t configured =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (configured != cudaSuccess) return configured;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(32 * MARCH_WARPS);
-    cfg.gridDim = dim3((n0 + MARCH_WARPS - 1) / MARCH_WARPS + (n1 + MARCH_WARPS - 1) / MARCH_WARPS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = pdl ? attr : nullptr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, patches, items0, n0, items1, n1, mc);
+    return launch_chained(kernel, dim3((n0 + MARCH_WARPS - 1) / MARCH_WARPS + (n1 + MARCH_WARPS - 1) / MARCH_WARPS),
+                          32 * MARCH_WARPS, smem, pdl, s, patches, items0, n0, items1, n1, mc);
   }
   static cudaError_t march_both(const PatchDev<Real>* patches, const MarchItem* items0, int n0,
                                 const MarchItem* items1, int n1, const MarchConst<Real>& mc, bool pdl,
@@ -179,17 +149,18 @@ struct LaunchImpl {
   template <> const int Launch<REAL>::TY = TYV;                                                             \
   template <> cudaError_t Launch<REAL>::fault(const PatchDev<REAL>* p, const int* fp, int nf, int mf,        \
                                               const DevParams* prm, const DevParams& hp, double dt,          \
-                                              double dx, double t, DevStatus* st, bool pdl, int seg,         \
+                                              double dx, double t, DevStatus* st, int place, int seg,        \
                                               cudaStream_t s) {                                              \
-    return LaunchImpl<REAL, TXV, TYV, NTV>::fault(p, fp, nf, mf, prm, hp, dt, dx, t, st, pdl, seg, s);       \
+    return LaunchImpl<REAL, TXV, TYV, NTV>::fault(p, fp, nf, mf, prm, hp, dt, dx, t, st, place, seg, s);     \
   }                                                                                                          \
   template <> cudaError_t Launch<REAL>::volume(const PatchDev<REAL>* p, const TileDev* tl, int nt,          \
                                                const DevParams* prm, cudaStream_t s) {                      \
     return LaunchImpl<REAL, TXV, TYV, NTV>::volume(p, tl, nt, prm, s);                                       \
   }                                                                                                          \
   template <> cudaError_t Launch<REAL>::exchange(const PatchDev<REAL>* p, const CopyDev* c, int n, int c0,  \
-                                                 int nc, cudaStream_t s) {                                   \
-    return LaunchImpl<REAL, TXV, TYV, NTV>::exchange(p, c, n, c0, nc, s);                                    \
+                                                 int nc, const CopyDev* bc, int nbc, int nb,                 \
+                                                 cudaStream_t s) {                                           \
+    return LaunchImpl<REAL, TXV, TYV, NTV>::exchange(p, c, n, c0, nc, bc, nbc, nb, s);                       \
   }                                                                                                          \
   template <> size_t Launch<REAL>::volume_smem() { return LaunchImpl<REAL, TXV, TYV, NTV>::smem(); }         \
   template <> int Launch<REAL>::volume_box_x() { return LaunchImpl<REAL, TXV, TYV, NTV>::box_x(); }          \

@@ -185,7 +185,7 @@ extern "C" tmk_status tmk_patch_update_state_noalloc(tmk_context* c, const tmk_f
   const int sblocks = std::min(1024, std::max(1, (listed + 255) / 256));
   noalloc_setup_kernel<<<sblocks, 256, 0, s>>>(pd, dpd, dfi, dtl, listed, TX, TY);
   TMK_CU(cudaGetLastError());
-  if (fault) TMK_CU(tmk::Launch<double>::fault(dpd, dfi, 1, nvx, cv.dp, *cv.hp, dt, dx, time, cv.st, false,
+  if (fault) TMK_CU(tmk::Launch<double>::fault(dpd, dfi, 1, nvx, cv.dp, *cv.hp, dt, dx, time, cv.st, tmk::FAULT_ALONE,
                                               tmk::fault_seg_of(*cv.hp, tmk::FAULT_SEG), s));
   if (cv.march) {
     TMK_CU(tmk::patch_march(dpd, nvx, nvy, fault, *cv.hp, dt, dx, s));

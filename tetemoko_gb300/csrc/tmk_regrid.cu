@@ -107,7 +107,7 @@ tmk_status tag_launch(tmk_level_s* L, const TagConst& tc, unsigned char* raw, cu
   for (const LevelPatch& lp : L->patches)
     maxc = std::max(maxc, (lp.valid.hi[0] - lp.valid.lo[0] + 1) * (lp.valid.hi[1] - lp.valid.lo[1] + 1));
   const PatchDev<Real>* pd = (const PatchDev<Real>*)L->dpatch[L->parity];
-  if (!tc.initial) TMK_CU(Launch<Real>::exchange(pd, L->dcopies, L->ncopies, 0, TMK_NCOMP, s));
+  if (!tc.initial) TMK_CU(Launch<Real>::exchange(pd, L->dcopies, L->ncopies, 0, TMK_NCOMP, nullptr, 0, 0, s));
   dim3 grid(std::min(64, (maxc + 255) / 256), (unsigned)L->patches.size());
   tag_kernel<Real><<<grid, 256, 0, s>>>(pd, tc, raw);
   TMK_CU(cudaGetLastError());
