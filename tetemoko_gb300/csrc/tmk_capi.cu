@@ -151,31 +151,33 @@ void make_tiles(std::vector<TileDev>& out, int patch, const tmk_box& v, int TX, 
 size_t align_up(size_t n) { return (n + 255) & ~(size_t)255; }
 
 // Work items of one component group's marching kernel: strips of MARCH_COLS
-// columns by runs of rows.  Each warp marches one item; the runs are sized so
-// that all items fit in one wave of resident warps (`slots`): a strip gets
-// max(1, floor(slots * rows / total strip-rows)) runs (at least kMinRun rows
-// each, which bounds the 2-row start-up overhead).  The first run of a strip
-// on the fault row waits for the fault kernel before it starts; it counts
-// `wait_rows` extra rows and is shortened by as many.
+// columns by runs of rows, one warp each.  All patches' runs are about as long
+// as the shortest length (of min_run or more) whose items fit into `slots`
+// warps: a run is what a warp's time goes by, and patches of different heights
+// that took their share of the slots each, rounded down, ran longest where the
+// rounding lost most.
 constexpr int kMinRun = 16;
 void make_march_items(std::vector<tmk::MarchItem>& out, std::vector<tmk::MarchItem>& fault_rows,
-                      const std::vector<tmk_box>& boxes, const std::vector<int>& fault, int slots, int wait_rows,
-                      int min_run) {
-  long long strip_rows = 0;
-  for (size_t p = 0; p < boxes.size(); ++p) {
-    const tmk_box& v = boxes[p];
-    const int ns = (v.hi[0] - v.lo[0] + tmk::MARCH_COLS) / tmk::MARCH_COLS;
-    strip_rows += (long long)ns * (v.hi[1] - v.lo[1] + 1 + (fault[p] ? wait_rows : 0));
+                      const std::vector<tmk_box>& boxes, const std::vector<int>& fault, int slots, int min_run) {
+  auto runs = [](const tmk_box& v, int run) { return (v.hi[1] - v.lo[1] + run) / run; };
+  auto items = [&](int run) {
+    long long n = 0;
+    for (const tmk_box& v : boxes)
+      n += (long long)((v.hi[0] - v.lo[0] + tmk::MARCH_COLS) / tmk::MARCH_COLS) * runs(v, run);
+    return n;
+  };
+  int rows = 1;
+  for (const tmk_box& v : boxes) rows = std::max(rows, v.hi[1] - v.lo[1] + 1);
+  int lo = min_run, hi = std::max(rows, min_run);      // the shortest that fits, else the tallest patch's rows
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    if (items(mid) <= slots) hi = mid;
+    else lo = mid + 1;
   }
-  if (slots <= 0) slots = 1;
   for (size_t p = 0; p < boxes.size(); ++p) {
     const tmk_box& v = boxes[p];
-    const int rows = v.hi[1] - v.lo[1] + 1;
-    const int w = fault[p] ? wait_rows : 0;
-    int k = (int)((long long)slots * (rows + w) / std::max(1LL, strip_rows));
-    k = std::max(1, std::min(k, (rows + w + min_run - 1) / min_run));
-    const int run = (rows + w + k - 1) / k;
-    const int first = std::min(rows, std::max(4, run - w));
+    const int rows = v.hi[1] - v.lo[1] + 1, k = runs(v, lo), run = (rows + k - 1) / k;
+    const int first = std::min(rows, std::max(4, run));
     for (int x0 = v.lo[0]; x0 <= v.hi[0]; x0 += tmk::MARCH_COLS)
       for (int y0 = v.lo[1]; y0 <= v.hi[1];) {
         const int len = (y0 == v.lo[1]) ? first : run;
@@ -194,92 +196,82 @@ void make_march_items(std::vector<tmk::MarchItem>& out, std::vector<tmk::MarchIt
   }
 }
 
-// Row-equivalents a fault-row item waits for the fault kernel (0: no marching
-// item waits, row 0 of the fault patches is finished after the fault kernel),
-// and the antiplane CTAs each fault-kernel CTA keeps from being resident (the
-// fault kernel runs beside the antiplane kernel; measured best at 1).
-constexpr int kFaultWaitRows = 0;
+// The CTAs each fault-kernel CTA keeps from being resident, in the group it runs
+// beside (measured best at 1).
 constexpr int kFaultDisplace = 1;
 
 // the marching kernels implement the PPM and CTU predictors; PLM runs the tile kernel
 bool uses_march(const tmk_scheme& s) { return s.volume_kernel != TMK_VOLUME_TILE && s.normal_pred_order != 1; }
 
-// The fault kernel first and both component groups in one launch that finishes
-// the fault rows (one_launch), or the groups' kernels with the fault kernel
-// between them and a launch for the fault rows.  Mixed, us a step, first against
-// second: slip weakening 64x32 12.0 / 13.7, 512x256 16.5 / 18.8, 1000x1000 64.8 /
-// 66.5, 2048x1024 118 / 123; rate and state, whose fault kernel holds its SMs
-// longer, 64x32 20.6 / 23.5, 512x256 20.9 / 25.1, but 1000x500 in patches of 128
-// 64.1 / 63.0 and 2048x1024 alike.  FP64 64x32 80 / 82, 512x256 198 / 217,
-// 2048x1024 2258 / 2223.  Without a fault the groups share one launch too.
-constexpr long long kOneLaunchCells = 450000;
-bool one_launch(const tmk_level_s* L) {
-  long long cells = 0;
-  bool rs = false;
-  for (const LevelPatch& lp : L->patches) {
-    cells += (long long)(lp.valid.hi[0] - lp.valid.lo[0] + 1) * (lp.valid.hi[1] - lp.valid.lo[1] + 1);
-    rs = rs || (lp.fault && L->ctx->scheme.fault_law == TMK_FAULT_RS);
-  }
-  return cells <= kOneLaunchCells || (L->prec == TMK_PREC_MIXED && !rs);
+// Resident warps of group g's marching kernel under the level's scheme.
+int march_slots_of(const tmk_level_s* L, int gk) {
+  const tmk::DevParams& hp = L->ctx->hp;
+  const bool fixed = hp.order != 0 && hp.prim_lim && !hp.char_lim;   // march_scheme_fixed of the launches
+  return L->prec == TMK_PREC_MIXED ? tmk::Launch<float>::march_slots(gk, fixed)
+                                   : tmk::Launch<double>::march_slots(gk, fixed);
+}
+long long march_item_count(const tmk_level_s* L, int run) {
+  long long items = 0;
+  for (const LevelPatch& lp : L->patches)
+    items += (long long)((lp.valid.hi[0] - lp.valid.lo[0] + tmk::MARCH_COLS) / tmk::MARCH_COLS) *
+             ((lp.valid.hi[1] - lp.valid.lo[1] + run) / run);
+  return items;
 }
 
-// Shortest run of a level's items.  A row of a marching warp takes about the
-// same time until a sub-partition holds two warps in FP32 or one in FP64 (whose
-// pipe one warp nearly fills), and an item costs two to three rows beyond its
-// own.
-// In one launch, FP32: the shortest run whose CTAs and the fault kernel's (each
-// takes the room of two) are resident at once with a tenth to spare, since a
-// second wave costs more than shorter runs gain (us a step: 512x256 16.5 at 5
-// rows, 19.3 at 4, 18.8 at 8; 512x512 25.1 at 10, 26.7 at 7); where none of 16
-// rows is, 16 (1024x512 38.7, 40 at 8).  FP64: (run + 2.2) x the CTAs per SM,
-// of which the ones beyond the first cost half (512x256 198 at 4, 218 at 8;
-// 256x128 98 at 5, 101 at 4, 118 at 8).
-// In two launches: (run + 3) x max(1, warps per sub-partition / 2 or 1) (mixed
-// 1000x500 in patches of 128 61.5 at 16 rows, 65.7 at 6).
-int default_min_run(const tmk_level_s* L, bool both) {
+// Shortest run of a level's items with both groups in one launch.  A row of a
+// marching warp takes about the same time until a sub-partition holds two warps
+// in FP32 or one in FP64 (whose pipe one warp nearly fills), and an item costs
+// two to three rows beyond its own.
+// FP32: the shortest run whose CTAs and the fault kernel's (each takes the room
+// of two) are resident at once with a tenth to spare, since a second wave costs
+// more than shorter runs gain (us a step: 512x256 16.5 at 5 rows, 19.3 at 4, 18.8
+// at 8; 512x512 25.1 at 10, 30.4 at 8); where none of 16 rows is, 16 (1024x512
+// 38.8, 40.3 at 8).  FP64: 4 rows (512x256 198, 217 at 8), up to 6 where that
+// keeps the CTAs at one per SM (256x128 97 at 5, 101 at 4).
+int default_min_run(const tmk_level_s* L) {
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool mixed = L->prec == TMK_PREC_MIXED;
-  auto count = [&](int run, long long& fault_ctas) {
-    long long items = 0;
-    fault_ctas = 0;
-    for (const LevelPatch& lp : L->patches) {
-      const int nx = lp.valid.hi[0] - lp.valid.lo[0] + 1, ny = lp.valid.hi[1] - lp.valid.lo[1] + 1;
-      items += (long long)((nx + tmk::MARCH_COLS - 1) / tmk::MARCH_COLS) * ((ny + run - 1) / run);
-      if (lp.fault) fault_ctas += (nx + tmk::FAULT_SEG - 1) / tmk::FAULT_SEG;
-    }
-    return items;
-  };
   long long fc = 0;
-  if (both && mixed) {
-    for (int run = 4; run < kMinRun; ++run) {
-      const long long ctas = 2 * ((count(run, fc) + 3) / 4);
-      if (10 * (ctas + 2 * fc) <= 9 * 4LL * sms) return run;
-    }
+  for (const LevelPatch& lp : L->patches)
+    if (lp.fault) fc += (lp.valid.hi[0] - lp.valid.lo[0] + tmk::FAULT_SEG) / tmk::FAULT_SEG;
+  if (L->prec == TMK_PREC_MIXED) {
+    for (int run = 4; run < kMinRun; ++run)
+      if (10 * (2 * ((march_item_count(L, run) + 3) / 4) + 2 * fc) <= 9 * 4LL * sms) return run;
     return kMinRun;
   }
-  int best = kMinRun;
+  int best = 4;
   double cost = 0.0;
-  for (int run = kMinRun; run >= 4; run -= both ? 1 : run / 2) {
-    const long long items = count(run, fc);
-    double c;
-    if (both) {
-      const double per = (2.0 * ((items + 3) / 4) + fc) / sms;
-      c = (run + 2.2) * (per > 1.0 ? 0.65 + 0.5 * per : 1.0);
-    } else {
-      c = (run + 3) * std::max(1.0, items / (4.0 * sms) / (mixed ? 2.0 : 1.0));
-    }
-    if (run == kMinRun || c < cost) { best = run; cost = c; }
+  for (int run = 4; run <= 6; ++run) {
+    const double n = (2.0 * ((march_item_count(L, run) + 3) / 4) + fc) / sms;
+    const double c = (run + 2.2) * (n > 1.0 ? 0.65 + 0.5 * n : 1.0);
+    if (run == 4 || c < cost) { best = run; cost = c; }
   }
   return best;
 }
 
+// Longest run by default: beyond it more, shorter items balance better than one
+// wave of long ones (us a step: an ensemble of 16 scenarios, 3.5 M cells, 202 at
+// runs of 28 in two waves, 272 at 57 in one; mixed 4096x1024 218 / 221; FP64
+// 2048x1024 2160 at 32, 2209 at 64).
+constexpr int kMaxRun = 48;
+
 tmk_tuning default_tuning(const tmk_level_s* L) {
   tmk_tuning t;
   t.volume_kernel = L->march_allowed ? TMK_VOLUME_MARCH : TMK_VOLUME_TILE;
+  // The fault kernel first and both component groups in one launch that finishes
+  // the fault rows, rather than the groups' kernels with the fault kernel between
+  // them and a launch for the fault rows.  Mixed, us a step, first against second:
+  // slip weakening 64x32 12.0 / 13.7, 512x256 16.5 / 18.8, 2048x1024 117 / 123;
+  // rate and state 64x32 20.6 / 23.5, 512x256 20.9 / 25.1, 1000x500 in patches of
+  // 128 61.7 / 61.7, 2048x1024 117 / 124.  FP64 512x256 198 / 217, 2048x1024
+  // 2160 / 2178.
+  t.fault_first = 1;
+  t.min_run = default_min_run(L);
   t.march_waves[0] = t.march_waves[1] = 1;
-  t.fault_first = one_launch(L);
-  t.min_run = default_min_run(L, t.fault_first != 0);
+  if (L->march_allowed) {
+    const long long n = march_item_count(L, kMaxRun), slots = std::max(1, march_slots_of(L, 0));
+    t.march_waves[0] = t.march_waves[1] = (int)std::min(8LL, std::max(1LL, (n + slots - 1) / slots));
+  }
   t.fault_displace = kFaultDisplace;
   t.fault_seg = tmk::FAULT_SEG;
   t.plastic_fused = 0;
@@ -328,21 +320,22 @@ tmk_status build_march_lists(tmk_level_s* L) {
   const size_t rs = real_size(L->prec);
   const int warps = L->prec == TMK_PREC_MIXED ? tmk::Launch<float>::march_warps()
                                                : tmk::Launch<double>::march_warps();
+  const bool fused = L->ctx->scheme.plasticity && tu.plastic_fused;
   for (int g = 0; g < 2; ++g) {
     level_free(L, L->ditems[g]);
     level_free(L, L->dfrows[g]);
     level_free(L, L->stash[g]);
-    const int gk = (g == 0 && L->ctx->scheme.plasticity && tu.plastic_fused) ? 2 : g;   // the kernel of group g
-    const tmk::DevParams& hp = L->ctx->hp;
-    const bool fixed = hp.order != 0 && hp.prim_lim && !hp.char_lim;   // march_scheme_fixed of the launches
-    int slots = L->prec == TMK_PREC_MIXED ? tmk::Launch<float>::march_slots(gk, fixed)
-                                          : tmk::Launch<double>::march_slots(gk, fixed);
-    slots *= tu.march_waves[g];
-    // the group the fault kernel runs beside leaves room for its CTAs
-    if (g == (tu.fault_first ? 0 : 1)) slots = std::max(warps, slots - tu.fault_displace * warps * fault_ctas);
+    // The group whose CTAs start beside the fault kernel's leaves room for them:
+    // the antiplane one as a launch of its own, the in-plane one in one launch
+    // (2048x1024 mixed, rate and state, 117 us a step, 124 without).  In one
+    // launch of the FP64 form they share the pipe rather than the room, and the
+    // antiplane runs are as long as the in-plane ones (1024x512 579 us, 617 with
+    // room left).
+    const bool both = tu.fault_first && !fused, fp64 = L->prec != TMK_PREC_MIXED;
+    int slots = march_slots_of(L, fused && g == 0 ? 2 : both && fp64 ? 0 : g) * tu.march_waves[g];
+    if (g == (both ? 0 : 1) && !(both && fp64)) slots = std::max(warps, slots - tu.fault_displace * warps * fault_ctas);
     std::vector<tmk::MarchItem> items, frows;
-    make_march_items(items, frows, boxes, fault_flags, slots, g == 0 && fault_ctas ? kFaultWaitRows : 0,
-                     tu.min_run);
+    make_march_items(items, frows, boxes, fault_flags, slots, tu.min_run);
     L->nitems[g] = (int)items.size();
     L->hitems[g] = items;
     L->hfrows[g] = frows;

@@ -389,10 +389,6 @@ TMK_D double rs_setbnd_k(const DevParams& P, const RSFaceK& fk, const double* U,
 // (ibcLinElast/SWIBCF.ChF:79-267) as rs_face_solve.  az: the values of the
 // antiplane S pair (syz + Zs rv vz).
 struct SWFaceK { double tau0, mu_s; };
-// The product rounds before anything is taken from it, in the units built with
-// fused multiply-adds too: whether a face on the rim of a patch or a box lies
-// inside must not depend on the precision.
-TMK_D double cell_centre(int i, double dx) { return __dmul_rn(i + 0.5, dx); }
 template <bool Z3 = false>
 TMK_D SWFaceK sw_face_k(const DevParams& P, double xcell, double zcell = 0.0) {
   const double x = xcell - P.sw_fbc0, z = zcell - P.sw_fbc1;

@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(fault_threads(SEG)) fault_kernel(const PatchDe
         b_s1 = Bi[(rs ? 7 : 6) * bs];
         if (rs) b_s2 = Bi[8 * bs];
       }
-      if (rs) fk = rs_face_k(P, rs_face(P, p.fric, i - p.blo0, bs), p.fric != nullptr, cell_centre(i, dx) - P.rs_x0, b_state);
-      else wk = sw_face_k(P, cell_centre(i, dx));
+      if (rs) fk = rs_face_k(P, rs_face(P, p.fric, i - p.blo0, bs), p.fric != nullptr, (i + 0.5) * dx - P.rs_x0, b_state);
+      else wk = sw_face_k(P, (i + 0.5) * dx);
     }
   } else if (role == 0 && ci >= 0) {
     if (i >= p.dlo0 && i <= p.dhi0 && i <= s1 + 1) {
