@@ -218,7 +218,8 @@ values_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k, 
   };
   auto row = [&](int q) -> const P* { return ring + ((q - q0) & 3) * RP + lane; };
   stage(q0); stage(q0 + 1); stage(q0 + 2);
-  P n4[NC8], dlo[NC8];
+  constexpr bool kD = kDiffsOnce<T>;
+  P n4[NC8], dlo[NC8], nd[NC8];         // nd (FP64): the difference to the next row
   {
     const bool hl = q0 - 1 >= dloq, hll = q0 - 2 >= dloq, hr = q0 + 1 <= dhiq;
     P Wa[NC8], Wb[NC8];
@@ -237,6 +238,7 @@ values_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k, 
       n4[c] = mk2(T(0), T(0)); dlo[c] = n4[c];
       if (!wave_comp<DM>(val_comp<DM>(c))) continue;
       P nl = psub(Wb[c], r0[c * 32]), nr2 = psub(r0[c * 32], r1[c * 32]);
+      if (kD) nd[c] = nr2;
       if (!hl) nl = nr2;
       if (!hr) nr2 = nl;
       if (!hl && !hr) { nl = mk2(T(0), T(0)); nr2 = nl; }
@@ -272,8 +274,9 @@ values_kernel(const __grid_constant__ Src src, const __grid_constant__ K3<T> k, 
     for (int c = 0; c < NC8; ++c) {
       if (!wave_comp<DM>(val_comp<DM>(c))) continue;
       const P W1 = r1[c * 32];
-      nl[c] = psub(W[c], W1);
+      nl[c] = kD ? nd[c] : psub(W[c], W1);
       nr[c] = psub(W1, r2[c * 32]);
+      if (kD) nd[c] = nr[c];
     }
     if (q + 2 > dhiq) {
 #pragma unroll

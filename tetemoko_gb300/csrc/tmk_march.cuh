@@ -183,11 +183,17 @@ template <int D, typename P> TMK_D P kpair(const P& pair) {
 }
 template <typename T> TMK_D auto kall(T s) { return mk2(s, s); }
 
-// position of a component among those live in y
-template <int G> TMK_HD constexpr int slope_slot(int c) {
+// position of a component among those live in y; of those live in x, and the
+// component at a position
+template <int G, int D = 1> TMK_HD constexpr int slope_slot(int c) {
   int k = 0;
-  for (int q = 0; q < c; ++q) k += live<G, 1>(q) ? 1 : 0;
+  for (int q = 0; q < c; ++q) k += live<G, D>(q) ? 1 : 0;
   return k;
+}
+template <int G, int D> TMK_HD constexpr int slot_comp(int k) {
+  int c = 0;
+  while (!live<G, D>(c) || slope_slot<G, D>(c) != k) ++c;
+  return c;
 }
 
 // Everything the marching kernel needs that is uniform over a launch (all
@@ -464,9 +470,15 @@ constexpr int march_row_pairs() { return Grp<G>::N * MARCH_RW; }
 // The FP32 in-plane kernel keeps the y half slopes and lo deltas of a lane (8
 // values) in shared memory, which fits its registers into four CTAs per SM.
 template <typename T, int G> constexpr bool kSlopesInSmem = sizeof(T) == 4 && G == 0;
+// The FP64 form computes each difference of two cells once, since a sum holds
+// its pipe for 64 cycles: a row's difference to the next one is kept for the
+// next row (in shared memory, its registers being full), and the one to the
+// right comes from the neighbour lane (2048x1024 2160 -> 2080 us a step).
+template <typename T> constexpr bool kDiffsOnce = sizeof(T) == 8;
 template <typename T, int G>
 constexpr size_t march_warp_pairs() {
-  return (size_t)MARCH_RING * march_row_pairs<T, G>() + (kSlopesInSmem<T, G> ? 8 * 32 : 0);
+  return (size_t)MARCH_RING * march_row_pairs<T, G>() + (kSlopesInSmem<T, G> ? 8 * 32 : 0) +
+         (kDiffsOnce<T> ? (G == 0 ? 4 : 2) * 32 : 0);
 }
 template <typename T, int G, bool PATCH = false>
 constexpr size_t march_smem_bytes() {
@@ -748,6 +760,8 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
   // of the row's code: with one set each value would be moved once a row.
   constexpr bool kS = kSlopesInSmem<T, G>;
   P* const slopes = ring + MARCH_RING * RP + lane;     // [2][4][32]
+  constexpr bool kD = kDiffsOnce<T>;
+  P* const diffs = slopes;                             // [4 or 2][32] (FP64, which keeps no slopes there)
   struct Carry {
     P n4[N], dlo[N];
     P Anx[NW], Apx[NW], Any[NW], Apy[NW], jpy[NW], Bny[NW], Bpy[NW], jpB[NW];
@@ -773,6 +787,7 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
       if (!live<G, 1>(c)) continue;
       const P W0 = r0[c * MARCH_RW];
       P nl = psub(Wb[c], W0), nr = psub(W0, r1[c * MARCH_RW]);
+      if (kD) diffs[slope_slot<G>(c) * 32] = nr;
       if (!hl) nl = nr;
       if (!hr) nr = nl;
       if (!hl && !hr) { nl = mk2(T(0), T(0)); nr = nl; }
@@ -818,8 +833,9 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
         for (int c = 0; c < N; ++c) {
           if (!live<G, 1>(c)) continue;
           const P W1 = r1[c * MARCH_RW];
-          nl[c] = psub(W0[c], W1);
+          nl[c] = kD ? diffs[slope_slot<G>(c) * 32] : psub(W0[c], W1);
           nr[c] = psub(W1, r2[c * MARCH_RW]);
+          if (kD) diffs[slope_slot<G>(c) * 32] = nr[c];
         }
         if (q + 2 > dhi1) {
 #pragma unroll
@@ -851,7 +867,26 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
         for (int c = 0; c < N; ++c) {
           if (!live<G, 0>(c)) continue;
           nl[c] = psub(rw[c * MARCH_RW - 1], W0[c]);
-          nr[c] = psub(W0[c], rw[c * MARCH_RW + 1]);
+          if (!kD) nr[c] = psub(W0[c], rw[c * MARCH_RW + 1]);
+        }
+        if constexpr (kD) {
+          // lane 31's differences to the column right of it, one per lane for
+          // all components and sides in one instruction
+          constexpr int NX = slope_slot<G, 0>(N);
+          int cc = slot_comp<G, 0>(0);
+#pragma unroll
+          for (int k = 1; k < NX; ++k)
+            if ((lane >> 1) == k) cc = slot_comp<G, 0>(k);
+          const T* const last = reinterpret_cast<const T*>(ring + r_0 + cc * MARCH_RW + 32) + (lane & 1);
+          const T e = last[0] - last[2];
+#pragma unroll
+          for (int c = 0; c < N; ++c) {
+            if (!live<G, 0>(c)) continue;
+            const int k = 2 * slope_slot<G, 0>(c);
+            const P r = shfl_dn2(nl[c], 1);
+            const T ex = __shfl_sync(0xffffffffu, e, k), ey = __shfl_sync(0xffffffffu, e, k + 1);
+            nr[c] = lane == 31 ? mk2(ex, ey) : r;
+          }
         }
         if (warp_xedge) {
 #pragma unroll
@@ -1029,7 +1064,7 @@ march_kernel(const PatchDev<T>* __restrict__ patches, const MarchItem* __restric
 // their order are what a step waits for: after the fault kernel one launch
 // finishes the step, and the groups share the SMs that either leaves idle (mixed
 // 512x256, slip weakening: 16.5 us a step, 18.8 as separate launches).  The
-// patch form, FP64 128x128 with fluxes: 83 us, bound by the FP64 pipe; the tile
+// patch form, FP64 128x128 with fluxes: 81 us, bound by the FP64 pipe; the tile
 // kernel, which forms face states, 557 us.
 template <typename T, int SCH, int FORM>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, MarchMinBlocks<T, 0>::value)
