@@ -732,9 +732,8 @@ def three_d_measurement(steps, warmup, stream, fp64_steps=3, cpu_seconds=5.0, si
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                          "frac": achieved / hbm_peak, "traffic": traffic,
                          "algorithmic_bytes_per_step": BYTES_PER_CELL_3D * nx * ny * nz,
-                         "kernel": "the whole 3-D step (18 launches: FP32 copy, 3 predictors, 4 first-pass, "
-                                   "3 paired second-pass + 1 fault-plane and 4 final face passes, update, "
-                                   "boundary data)",
+                         "kernel": "the whole 3-D step (5 launches: FP32 copy, x and y values, z values, fault plane, "
+                                   "transverse stages and update)",
                          "timing": f"CUDA events on the launch stream around {mixed['steps']} steps"},
             "cpu_baseline": cpu,
             "patches_32": tiles,
@@ -966,7 +965,7 @@ def main():
             traffic = None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved / hbm_peak, "traffic": traffic,
-                "kernel": "volume update: march_kernel<float,0> (in-plane) + march_kernel<float,1> (antiplane)",
+                "kernel": "volume update: march_both_kernel<float> (both component groups), or one launch a group",
                 "algorithmic_bytes_per_launch": BYTES_PER_CELL_MIXED * cells, "peak_source": peak_src,
                 "kernel_ms": vol_ms, "fault_kernel_ms": fault_ms, "step_ms_profiled": step_ms,
                 "timing": f"average over a second timed pass of {nprof} steps with CUDA events on the launch "

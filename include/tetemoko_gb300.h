@@ -135,19 +135,19 @@ typedef struct {
 typedef struct { int lo[2], hi[2]; } tmk_box;   /* cell-centred, inclusive */
 
 /* How a level's step is cut into work (an extension: the reference's patch
- * loop has no such choices).  Defaults: the scheme's volume kernel, one wave
- * per marching group, runs of at least 16 rows, one antiplane slot per
- * fault-kernel CTA, 32 fault faces per fault-kernel CTA, the fault kernel
- * after the in-plane marching kernel, the plastic return as a pass. */
+ * loop has no such choices).  Defaults: the scheme's volume kernel, the fault
+ * kernel first, runs of 4 to 16 rows or more by the level's size in as many
+ * waves as keep them below 48, one CTA slot per fault-kernel CTA, 32 fault
+ * faces per fault-kernel CTA, the plastic return as a pass. */
 typedef struct {
   int volume_kernel;    /* TMK_VOLUME_MARCH or TMK_VOLUME_TILE (march only if the scheme allows it) */
   int march_waves[2];   /* marching items of the in-plane / antiplane group, in waves of resident CTAs: 1..8 */
   int min_run;          /* fewest rows of a marching item: 4..4096 */
-  int fault_displace;   /* antiplane CTA slots left free per fault-kernel CTA: 0..4 */
-  int fault_seg;        /* fault faces per fault-kernel CTA: 32 (4 warps) or 16 (2 warps) */
-  int fault_first;      /* 1: the fault kernel first, running beside the in-plane marching kernel
-                           (2-warp CTAs fit in the registers two in-plane CTAs leave free);
-                           0: after it, beside the antiplane kernel */
+  int fault_displace;   /* CTA slots left free per fault-kernel CTA in the group it runs beside: 0..4 */
+  int fault_seg;        /* fault faces per fault-kernel CTA: 32 (6 warps) or 16 (3 warps) */
+  int fault_first;      /* 1: the fault kernel first, then both component groups in one launch that
+                           finishes the fault rows; 0: after the in-plane marching kernel, beside
+                           the antiplane one, then a launch for the fault rows */
   int plastic_fused;    /* plastic levels of the marching form: 1: the Drucker-Prager return is
                            applied by the in-plane marching kernel as it stores each cell (the
                            antiplane kernel runs first, the fault kernel on a side stream beside

@@ -1,5 +1,7 @@
 // The 3-D patch step (CH_SPACEDIM == 3): kernels, templated on the arithmetic
-// of the volume stencil T.
+// of the volume stencil T.  The decks' scheme (PPM with primitive limiting) runs
+// the passes of tmk_3d_march.cuh; the ones below carry the other predictors and
+// limiters and the reference's 9-component slip weakening.
 //
 // LinElastPatchGodunov::updateState in 3-D (srcLinElast/LinElastPatchGodunov.cpp:
 // 101-129, 174-469) as five kinds of passes over one patch, each a grid of one

@@ -8,7 +8,10 @@
 //                  fluxes and the conservative update (and, with plasticity,
 //                  the Drucker-Prager return) of a TX x TY tile, every stage
 //                  in shared memory; the fault faces come from fault_kernel.
-//   exchange_kernel  same-level ghost copy between patches (LevelData::exchange).
+//                  For the PLM predictor and as a tuning choice: the others run
+//                  the marching kernels (tmk_march.cuh), also on one patch.
+//   exchange_kernel  same-level ghost copy of state and fault data between
+//                  patches (LevelData::exchange).
 #pragma once
 #include "tmk_device.cuh"
 #include "tmk_fault.cuh"
