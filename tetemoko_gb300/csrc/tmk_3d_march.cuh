@@ -22,16 +22,13 @@
 // WHalf[1] and the boundary data of one face are one thread's work.
 //
 // What bounds them, at 192x96x96 mixed (rate and state): the FP32 copy of the
-// state (78 us) and the z values (35 us) DRAM; the x and y values (70 us) the
+// state (80 us) and the z values (40 us) DRAM; the x and y values (73 us) the
 // issue of the limiters; the plane (48 us) the latency of four dependent solves,
-// beside which the step's tiles away from the fault run; the step (about 420 us)
-// issue, 500 instructions a cell and side, with L2 close behind (144 B of values
-// read, 144 B of FP64 state read and written a cell and side, plus the tile's
-// halo).  A call 778 us; one pass per term, each through memory, took 1383 us.
-// FP64 (64x48x48): every kernel the FP64 pipe; 595 us, was 2703 us.  32-cell
-// boxes of a 96x64x64 level, mixed: 837 us, was 1100 (half of either is reading
-// the state back), of which the step 141 (231 before a row's last columns took
-// lane groups).
+// beside which the step's tiles away from the fault run; the step (294 us)
+// issue, 48 % of slots, and its last wave of CTAs.  A call 685 us; one pass per
+// term, each through memory, took 1383 us.  FP64 (64x48x48): every kernel the
+// FP64 pipe; 581 us, was 2703 us.  32-cell boxes of a 96x64x64 level, mixed: 807
+// us, was 1097 (520 of either is reading the state back).
 #pragma once
 
 #include "tmk_3d.cuh"
@@ -437,6 +434,17 @@ TMK_D void store_flux(const Step3<T>& g, const K3<T>& k, T rvs, int s, int i, in
   out[10 * cs] = 0.0;
 }
 
+// asynchronous copies of one thread's element of nine planes to shared entries NT apart
+template <typename E, int NT, int C>
+TMK_D void stage_plane(unsigned dst, const E* src, unsigned plane, unsigned nbytes) {
+  if constexpr (C < 9) {
+    asm volatile("cp.async.ca.shared.global [%0 + %4], [%1], %2, %3;" ::"r"(dst), "l"(plane_ptr(src, plane, C)),
+                 "n"(sizeof(E)), "r"(nbytes), "n"(C * NT * (int)sizeof(E))
+                 : "memory");
+    stage_plane<E, NT, C + 1>(dst, src, plane, nbytes);
+  }
+}
+
 // ------------------------------------------------------------ the step
 // One CTA per tile of 30 x (NR - 2) cells, run of planes and side; a warp per
 // row of y, x in the lanes, marching in z.  (The columns left over by whole
@@ -444,10 +452,13 @@ TMK_D void store_flux(const Step3<T>& g, const K3<T>& k, T rvs, int s, int i, in
 // rows to a warp.)  Neighbours: x by lane, y through
 // shared memory (two exchanges a plane), z carried from plane to plane.  When
 // plane m arrives, the stages that need nothing above it are done for m, then
-// plane m - 1 is finished.  8 rows, FP32 at two CTAs per SM (128 registers, some
-// spilled), FP64 one: a 192x96x96 mixed patch took 778 us, 823 with 16 rows and
-// 785 with 10 at one CTA (no spills, but the 32-cell boxes 931 against 852); a
-// 64x48x48 FP64 patch 595 us, 629 with 10 rows and 612 with 12.
+// plane m - 1 is finished.  8 rows, FP32 at two CTAs per SM (128 registers), FP64
+// at one.  What a thread carries of the first values and the z jumps stays in its
+// own shared memory slots, where cp.async puts the next plane's values: kept in
+// registers they spilled, and the loads of the spills, not those of the values,
+// were what warps waited for (192x96x96 mixed 394 us, 294 now).  Measured with
+// the spills: 16 rows 823 us a call against 778, 10 rows at one CTA 785 (32-cell
+// boxes 931 against 852); FP64 64x48x48 10 rows 629 against 595, 12 rows 612.
 // GL: lanes of a row, 32 or (0) fewer, from the strips; FLUX: a patch has flux
 // arrays.  Both fixed at compile time: the common form spills least.
 template <typename T, int GL, bool FLUX>
@@ -457,8 +468,17 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
   // [9] A_y, WHalf2[1][0] of plane m, WHalf2[1][2] of plane m - 1; [3] the final y values of plane m - 1
   extern __shared__ __align__(16) unsigned char step_smem[];
   constexpr int PL = (NR + 2) * 32;       // entries of one value; rows of a lane group each
+  constexpr int NT = 32 * NR;
   V* const s1 = reinterpret_cast<V*>(step_smem);
   V* const s2 = s1 + 9 * PL;
+  // the thread's values of two planes and the state it updates, copied in by
+  // cp.async: the values of plane m + 1 land where those of m - 1 were
+  V* const vals = s2 + 3 * PL + threadIdx.x;                                // [2][9][NT]
+  double* const unext = reinterpret_cast<double*>(s2 + 3 * PL + 18 * NT) + threadIdx.x;
+  // and its p jumps of the z values, kept from plane to plane ([4][3][NT]: of A_z,
+  // WHalf2[2][0], WHalf2[2][1], the final values): registers here would spill
+  T* const js = reinterpret_cast<T*>(reinterpret_cast<double*>(s2 + 3 * PL + 18 * NT) + 9 * NT) + threadIdx.x;
+  const unsigned v32 = (unsigned)__cvta_generic_to_shared(vals), u32 = (unsigned)__cvta_generic_to_shared(unext);
   const unsigned side = u & 1u;
   const Strips st = strips(g.cur.n[0], 1);
   const unsigned nw = (unsigned)st.whole * (unsigned)cdiv(g.cur.n[1], NR - 2);
@@ -543,26 +563,22 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
     for (int w = 0; w < 3; ++w) jump(hn[w], a[w].y, ln[w], lp[w], sum[w], dif[w]);
   };
 
-  // carried from plane to plane (plane k = m - 1): the values of x and y, and of
-  // z, WHalf2[2][0], WHalf2[2][1] and the final z values with their p jumps
-  V ax[3], ay[3], az[3], zx[3], zy[3], fz[3];
-  T jz[3], jzx[3], jzy[3], jfz[3];
+  // carried from plane to plane (plane k = m - 1): WHalf2[2][0], WHalf2[2][1] and
+  // the final z values (their p jumps and the first values are in shared memory)
+  V zx[3], zy[3], fz[3];
 #pragma unroll
-  for (int w = 0; w < 3; ++w) {
-    ax[w] = zero; ay[w] = zero; az[w] = zero; zx[w] = zero; zy[w] = zero; fz[w] = zero;
-    jz[w] = T(0); jzx[w] = T(0); jzy[w] = T(0); jfz[w] = T(0);
-  }
+  for (int w = 0; w < 3; ++w) { zx[w] = zero; zy[w] = zero; fz[w] = zero; }
+  constexpr unsigned VSLOT = 9 * NT;
+  stage_plane<V, NT, 0>(v32 + (ms & 1) * VSLOT * (unsigned)sizeof(V), vp, scs, in ? (unsigned)sizeof(V) : 0u);
+  cp_async_commit();
   for (int m = ms; m <= z1 + 1; ++m) {
     const bool have = m <= zhi, fin = m > ms && m - 1 >= z0;      // uniform over the CTA
     V bx[3], by[3], bz[3], nzx[3], nzy[3], nfz[3];
+    const V *const vm = vals + (m & 1) * VSLOT, *const vb = vals + ((m + 1) & 1) * VSLOT;      // planes m and m - 1
+    cp_async_wait<0>();                   // the thread's values of plane m
     if (have) {
 #pragma unroll
-      for (int w = 0; w < 3; ++w) {
-        bx[w] = in ? *plane_ptr(vp, scs, w) : zero;
-        by[w] = in ? *plane_ptr(vp, scs, 3 + w) : zero;
-        bz[w] = in ? *plane_ptr(vp, scs, 6 + w) : zero;
-      }
-      vp += dz;
+      for (int w = 0; w < 3; ++w) { bx[w] = vm[w * NT]; by[w] = vm[(3 + w) * NT]; bz[w] = vm[(6 + w) * NT]; }
     } else {
       // past the domain's z-hi edge: only the values arriving through it
 #pragma unroll
@@ -570,12 +586,14 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
         const bool o = k.out[5] != 0;
         const T b = k.nbg[ws<2>(w)];
         bx[w] = zero; by[w] = zero;
-        bz[w] = mk2(arriving(o, az[w].y, b), T(0));
+        bz[w] = mk2(arriving(o, vb[(6 + w) * NT].y, b), T(0));
         nzx[w] = mk2(arriving(o, zx[w].y, b), T(0));
         nzy[w] = mk2(arriving(o, zy[w].y, b), T(0));
         nfz[w] = mk2(arriving(o, fz[w].y, b), T(0));
       }
     }
+    if (fin && upd) stage_plane<double, NT, 0>(u32, up, acs, 8u);
+    cp_async_commit();
     // ---- first exchange: A_y and WHalf2[1][0] of plane m, WHalf2[1][2] of plane m - 1
     V yx[3], yz[3], xz[3];
     T sum[3], dif[3];
@@ -591,16 +609,20 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
     if (fin) {
 #pragma unroll
       for (int w = 0; w < 3; ++w) {
-        xz[w] = ax[w]; yz[w] = ay[w];
-        const T jn = bz[w].x - az[w].x;
-        sum[w] = jn + jz[w];
-        dif[w] = jn - jz[w];
+        xz[w] = vb[w * NT]; yz[w] = vb[(3 + w) * NT];
+        const T jn = bz[w].x - vb[(6 + w) * NT].x;
+        sum[w] = jn + js[w * NT];
+        dif[w] = jn - js[w * NT];
       }
       correct3<2, 0, 1, T>(k, rv, sum, dif, xz);
       correct3<2, 1, 1, T>(k, rv, sum, dif, yz);
 #pragma unroll
       for (int w = 0; w < 3; ++w) s1[(6 + w) * PL + at] = yz[w];
     }
+    // the p jump of A_z over plane m; at the domain's z-lo edge the value from below arrives through it
+#pragma unroll
+    for (int w = 0; w < 3; ++w)
+      js[w * NT] = bz[w].y - (m == zlo ? arriving(k.out[4] != 0, bz[w].x, k.nbg[ws<2>(w)]) : vb[(6 + w) * NT].y);
     __syncthreads();
     V xy[3], fx[3], fy[3];
     if (have) {
@@ -618,14 +640,14 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
     if (fin) {
       // the final x and y values of plane m - 1
 #pragma unroll
-      for (int w = 0; w < 3; ++w) { fx[w] = ax[w]; fy[w] = ay[w]; }
+      for (int w = 0; w < 3; ++w) { fx[w] = vb[w * NT]; fy[w] = vb[(3 + w) * NT]; }
       yjump(s1 + 6 * PL, yz, 2, m - 1, sum, dif);
       correct3<1, 0, 0, T>(k, rv, sum, dif, fx);
 #pragma unroll
       for (int w = 0; w < 3; ++w) {
         const T jn = nzy[w].x - zy[w].x;
-        sum[w] = jn + jzy[w];
-        dif[w] = jn - jzy[w];
+        sum[w] = jn + js[(6 + w) * NT];
+        dif[w] = jn - js[(6 + w) * NT];
       }
       correct3<2, 0, 0, T>(k, rv, sum, dif, fx);
       xjump(xz, sum, dif);
@@ -633,19 +655,22 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
 #pragma unroll
       for (int w = 0; w < 3; ++w) {
         const T jn = nzx[w].x - zx[w].x;
-        sum[w] = jn + jzx[w];
-        dif[w] = jn - jzx[w];
+        sum[w] = jn + js[(3 + w) * NT];
+        dif[w] = jn - js[(3 + w) * NT];
       }
       correct3<2, 1, 0, T>(k, rv, sum, dif, fy);
 #pragma unroll
       for (int w = 0; w < 3; ++w) s2[w * PL + at] = fy[w];
     }
     __syncthreads();
+    // plane m - 1's values have been used: those of plane m + 1 may land
+    if (m < zhi && m <= z1) {
+      vp += dz;
+      stage_plane<V, NT, 0>(v32 + ((m + 1) & 1) * VSLOT * (unsigned)sizeof(V), vp, scs, in ? (unsigned)sizeof(V) : 0u);
+    }
+    cp_async_commit();
     if (fin) {
       const int kz = m - 1;
-      double uo[9];
-#pragma unroll
-      for (int c = 0; c < 9; ++c) uo[c] = upd ? *plane_ptr(up, acs, c) : 0.0;
       T du[9];
 #pragma unroll
       for (int c = 0; c < 9; ++c) du[c] = T(0);
@@ -656,8 +681,8 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
 #pragma unroll
       for (int w = 0; w < 3; ++w) {
         const T jn = nfz[w].x - fz[w].x;
-        sum[w] = jn + jfz[w];
-        dif[w] = jn - jfz[w];
+        sum[w] = jn + js[(9 + w) * NT];
+        dif[w] = jn - js[(9 + w) * NT];
       }
       update3<2, T>(k, rv, sum, dif, du);
       if (FLUX && (g.F[0] || g.F[1] || g.F[2])) {
@@ -693,7 +718,7 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
         }
         if (upd && g.F[2]) {
 #pragma unroll
-          for (int w = 0; w < 3; ++w) { n[w] = fz[w].x; p[w] = fz[w].y - jfz[w]; }
+          for (int w = 0; w < 3; ++w) { n[w] = fz[w].x; p[w] = fz[w].y - js[(9 + w) * NT]; }
           store_flux<2, T>(g, k, rv, s, x, y, kz, n, p);
           if (kz == g.cur.lo[2] + g.cur.n[2] - 1) {
 #pragma unroll
@@ -702,9 +727,10 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
           }
         }
       }
+      cp_async_wait<1>();                 // the state; the next plane's values may still be on their way
       if (upd) {
 #pragma unroll
-        for (int c = 0; c < 9; ++c) *plane_ptr(up, acs, c) = uo[c] + widen(du[c]);
+        for (int c = 0; c < 9; ++c) *plane_ptr(up, acs, c) = unext[c * NT] + widen(du[c]);
       }
       up += adz;
     }
@@ -714,7 +740,6 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
       for (int w = 0; w < 3; ++w) {
         const bool o = k.out[4] != 0;
         const T b = k.nbg[ws<2>(w)];
-        az[w].y = arriving(o, bz[w].x, b);
         zx[w].y = arriving(o, nzx[w].x, b);
         zy[w].y = arriving(o, nzy[w].x, b);
         fz[w].y = arriving(o, nfz[w].x, b);
@@ -722,11 +747,10 @@ TMK_D void step_tile(const Step3<T>& g, const K3<T>& k, unsigned u) {
     }
 #pragma unroll
     for (int w = 0; w < 3; ++w) {
-      jz[w] = bz[w].y - az[w].y;
-      jzx[w] = nzx[w].y - zx[w].y;
-      jzy[w] = nzy[w].y - zy[w].y;
-      jfz[w] = nfz[w].y - fz[w].y;
-      ax[w] = bx[w]; ay[w] = by[w]; az[w] = bz[w]; zx[w] = nzx[w]; zy[w] = nzy[w]; fz[w] = nfz[w];
+      js[(3 + w) * NT] = nzx[w].y - zx[w].y;
+      js[(6 + w) * NT] = nzy[w].y - zy[w].y;
+      js[(9 + w) * NT] = nfz[w].y - fz[w].y;
+      zx[w] = nzx[w]; zy[w] = nzy[w]; fz[w] = nfz[w];
     }
   }
 }
@@ -919,7 +943,9 @@ __global__ void __launch_bounds__(64) plane_kernel(const __grid_constant__ Src s
 template <typename T, int DM> constexpr size_t val_smem_bytes() {
   return (size_t)VAL_WARPS * 4 * kValComps<DM> * 32 * 2 * sizeof(T);
 }
-template <typename T> constexpr size_t step_smem_bytes() { return (size_t)12 * (step_rows<T> + 2) * 32 * 2 * sizeof(T); }
+template <typename T> constexpr size_t step_smem_bytes() {
+  return (size_t)12 * (step_rows<T> + 2) * 32 * 2 * sizeof(T) + (size_t)step_rows<T> * 32 * (9 * (4 * sizeof(T) + 8) + 12 * sizeof(T));
+}
 
 // The whole step on stream s (One: one patch, Many: a batch); hp: the context's
 // parameters on the host.
