@@ -456,9 +456,9 @@ TMK_D void stage_plane(unsigned dst, const E* src, unsigned plane, unsigned nbyt
 // at one.  What a thread carries of the first values and the z jumps stays in its
 // own shared memory slots, where cp.async puts the next plane's values: kept in
 // registers they spilled, and the loads of the spills, not those of the values,
-// were what warps waited for (192x96x96 mixed 394 us, 294 now).  Measured with
-// the spills: 16 rows 823 us a call against 778, 10 rows at one CTA 785 (32-cell
-// boxes 931 against 852); FP64 64x48x48 10 rows 629 against 595, 12 rows 612.
+// were what warps waited for (192x96x96 mixed 394 us, 294 now).  A call there took
+// 738 us with 16 rows, 708 with 14 and 906 with 12 (at one CTA), 694 with 8; a
+// 64x48x48 FP64 patch 602 with 10 rows and 582 with 8.
 // GL: lanes of a row, 32 or (0) fewer, from the strips; FLUX: a patch has flux
 // arrays.  Both fixed at compile time: the common form spills least.
 template <typename T, int GL, bool FLUX>
