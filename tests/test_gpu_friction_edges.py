@@ -1,0 +1,102 @@
+"""Rate-and-state faces at the ends of what the friction laws meet == the oracle:
+slip rates below the last bit of the sides' velocities, faces without traction,
+states so low that the aging law's exponential overflows, and the lines between
+the forms of the solve and of the state evolution.  Through every form that
+solves them: the 2-D patch step, the 2-D level and the 3-D patch step, FP64 and
+mixed."""
+import numpy as np
+import pytest
+
+import oracle as O
+from tetemoko_gb300 import _capi as A, scenarios as S
+from tests.helpers import perturbed_state
+
+pytestmark = pytest.mark.gpu
+
+G = A.TMK_NGHOST
+NX, NY, NZ = 37, 5, 3
+FORMS = ["patch_fp64", "level_fp64", "level_mixed", "patch3_fp64", "patch3_mixed"]
+
+
+def _sc(form, law, **rs):
+    prec = A.TMK_PREC_MIXED if form.endswith("mixed") else A.TMK_PREC_FP64
+    sc = S.rate_state(nx=NX, ny=NY, dx=0.1, precision=prec, state_law=law)
+    for k, v in rs.items():
+        setattr(sc.rs, k, v)
+    return sc
+
+
+def _step(form, sc, U, B, dt):
+    """One step of the 2-D state U, B (uniform in z for the 3-D forms): the GPU's and
+    the oracle's (status or None, U, B) with the fault data over the valid faces."""
+    import torch
+    from tetemoko_gb300.level import Context, LinElastLevelGodunov, LinElastPatchGodunov, LinElastPatchGodunov3D
+    ctx = Context(sc)
+    Uo, Bo = U.copy(), B.copy()
+    v = slice(G, -G)
+    if form.startswith("patch3"):
+        rep = lambda a: np.ascontiguousarray(np.repeat(a[:, None], NZ + 2 * G, axis=1))
+        Uo, Bo = rep(U), rep(B)
+        lo, hi = (0, 0, 0), (NX - 1, NY - 1, NZ - 1)
+        Ud, Bd = torch.from_numpy(Uo.copy()).cuda(), torch.from_numpy(Bo.copy()).cuda()
+        rc, _ = O.patch_update_state_3d(sc, Uo, (-G, -G, -G), lo, hi, lo, hi, Bo, (-G, -G), 0.1, 0.0, dt)
+        pg = LinElastPatchGodunov3D(ctx, (lo, hi))
+        pg.set_current_box((lo, hi))
+        pg.update_state(Ud, (-G, -G, -G), dt, B=Bd, blo=(-G, -G))
+        out = None, Ud.cpu().numpy()[:, v, v, v], Bd.cpu().numpy()[:, v, v]
+        ref = rc, Uo[:, v, v, v], Bo[:, v, v]
+    else:
+        rc, _, _ = O.patch_update_state(sc, Uo, (-G, -G), (0, 0), (NX - 1, NY - 1), Bo, -G, 0.0, dt)
+        ref = rc, Uo[:, v, v], Bo[:, v]
+        if form.startswith("patch"):
+            Ud, Bd = torch.from_numpy(U.copy()).cuda(), torch.from_numpy(B.copy()).cuda()
+            pg = LinElastPatchGodunov(ctx)
+            pg.set_current_box((0, 0, NX - 1, NY - 1))
+            pg.update_state(Ud, (-G, -G), dt, B=Bd, bxlo=-G)
+            out = None, Ud.cpu().numpy()[:, v, v], Bd.cpu().numpy()[:, v]
+        else:
+            lv = LinElastLevelGodunov(ctx, [(0, 0, NX - 1, NY - 1)])
+            lv.set_level(U, B)
+            lv.step(0.0, dt)
+            Ug, Bg = U.copy(), B.copy()
+            lv.get_level(Ug, Bg)
+            out = lv.status()[0], Ug[:, v, v], Bg[:, v]
+            lv.close()
+    ctx.close()
+    return out, ref
+
+
+@pytest.mark.parametrize("law", [A.TMK_RS_SLIP_LAW, A.TMK_RS_AGING_LAW], ids=["slip", "aging"])
+@pytest.mark.parametrize("form", FORMS)
+def test_slip_rate_below_the_velocities_last_bit_is_zero(cuda_lib, form, law):
+    """psi = 1.5 holds the fault at about 1e-55 m/s while its sides move at 0.1 m/s
+    or so: the difference of the sides' velocities is exactly zero, so the slip law's
+    logarithm makes the half-step state NaN, the final slip rate with it, and the
+    step reports it; the aging law goes on."""
+    sc = _sc(form, law)
+    U = perturbed_state(sc, np.random.default_rng(2), amp_v=0.5, amp_s=2.0)
+    B = sc.initial_B()
+    B[10] = 1.5
+    (rc, Ug, Bg), (rco, Uo, Bo) = _step(form, sc, U, B, sc.dt() / 2)
+    nan = law == A.TMK_RS_SLIP_LAW
+    assert np.isnan(Bo[10]).all() == nan and (nan or not Bo[:3].any())
+    assert np.array_equal(Bg[:3], Bo[:3], equal_nan=True)
+    assert np.array_equal(np.isnan(Bg), np.isnan(Bo))
+    if rc is not None:
+        assert rc == rco == (2 if nan else 0)
+    if not nan:
+        assert np.abs(Bg[10] - Bo[10]).max() <= 1e-12 * 1.5
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_a_face_without_traction_is_reported(cuda_lib, form):
+    """No shear on the fault and none to nucleate: the direction of slip is 0/0, the
+    slip rate and the state NaN, and the step reports it."""
+    sc = _sc(form, A.TMK_RS_AGING_LAW, nsig=0.0)
+    sc.elastic.sxy0 = 0.0
+    U, B = sc.initial_U(), sc.initial_B()
+    B[10] = 0.6
+    (rc, Ug, Bg), (rco, Uo, Bo) = _step(form, sc, U, B, sc.dt() / 2)
+    assert np.isnan(Bo[[0, 2, 10]]).all()
+    assert np.array_equal(np.isnan(Bg), np.isnan(Bo))
+    assert rc is None or rc == rco == 2

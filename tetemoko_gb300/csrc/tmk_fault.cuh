@@ -292,7 +292,10 @@ TMK_D int rs_solve_z(const DevParams& P, const RSFaceK& fk, double phi, double p
 // the two sides' states: the left-going characteristic values of the P pair
 // (aP = syy + Zp rv vy) and of the S pair (aS = sxy + Zs rv vx), rv = +1, -1.
 // The antiplane traction term is zero in the law.  dvx, dvz: the states'
-// velocity differences (the first guess).  Returns the iterations used.
+// velocity differences (the first guess).  The slip rates are those of RSSETBND,
+// the differences of the two sides' velocities: zero where V is below their last
+// bit and NaN without a traction, on which the state evolution's NaN, and with it
+// the status of the step, depends.  Returns the iterations used.
 template <bool EXACT, typename T>
 TMK_D int rs_face_solve(const DevParams& P, const RSFaceK& fk, double aP1, double aP2, double aS1, double aS2,
                         double psi, T dvx, T dvz, FaultFace& f) {
@@ -306,13 +309,13 @@ TMK_D int rs_face_solve(const DevParams& P, const RSFaceK& fk, double aP1, doubl
   const double sgn = phi > 0.0 ? copysign(1.0, phi_xy) : __longlong_as_double(0x7ff8000000000000ll);
   f.sxy = sgn * tau - fk.tau0;
   f.syz = 0.0 * tau;                    // (phi_yz / phi) tau - tau_yz_0 with phi_yz = tau_yz_0 = 0
-  f.V = V;
-  f.Vx = sgn * V;
-  f.Vz = 0.0 * V;
   f.vx1 = (aS1 - f.sxy) * P.inv_Zs;
-  f.vx2 = f.vx1 - f.Vx;
+  f.vx2 = __dsub_rn(f.vx1, sgn * V);
   f.vz1 = -f.syz;
-  f.vz2 = f.vz1 - f.Vz;
+  f.vz2 = f.vz1 - 0.0 * V;
+  f.Vx = __dsub_rn(f.vx1, f.vx2);       // of the rounded velocities: not fused with vx1's product
+  f.Vz = f.vz1 - f.vz2;
+  f.V = fabs(f.Vx);                     // Vz is zero, or NaN as Vx is
   return it;
 }
 
