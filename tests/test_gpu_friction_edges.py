@@ -100,3 +100,22 @@ def test_a_face_without_traction_is_reported(cuda_lib, form):
     assert np.isnan(Bo[[0, 2, 10]]).all()
     assert np.array_equal(np.isnan(Bg), np.isnan(Bo))
     assert rc is None or rc == rco == 2
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_aging_law_at_rest_far_below_steady_state(cuda_lib, form):
+    """b = 5e-5 and psi 0.05 below f0: e^(1000) overflows, on a fault that stands
+    still (slip rate exactly zero): the state is f0 + b log(V0 dt / L)."""
+    sc = _sc(form, A.TMK_RS_AGING_LAW, a=0.001, b=5e-5)
+    sc.elastic.sxy0 = 50.0
+    sc.rs.nsig = 0.0
+    U = perturbed_state(sc, np.random.default_rng(2), amp_v=0.5, amp_s=2.0)
+    B = sc.initial_B()
+    B[10] = 0.55
+    dt = sc.dt() / 2
+    (rc, Ug, Bg), (rco, Uo, Bo) = _step(form, sc, U, B, dt)
+    assert rco == 0 and not Bo[:3].any()
+    assert rc in (0, None) and not Bg[:3].any()
+    known = sc.rs.f0 + sc.rs.b * np.log(sc.rs.V0 * dt / sc.rs.L)
+    assert np.abs(Bo[10] - known).max() <= 1e-14
+    assert np.abs(Bg[10] - known).max() <= 1e-14

@@ -338,7 +338,7 @@ TMK_D double rs_state_next(const DevParams& P, const RSFaceK& fk, double psi, do
     } else if (r < 1e300) {
       l = log1p(r);
     } else {            // out of range (or NaN): the sum itself
-      const double phi1 = -expm1(-x) / x;
+      const double phi1 = x > 1e-12 ? -expm1(-x) / x : 1.0 - 0.5 * x;
       return P.rs_f0 + fk.b * log(exp((psi - P.rs_f0) * fk.inv_b - x) + c * phi1);
     }
     return psi + fk.b * (l - x);
