@@ -1,0 +1,41 @@
+"""The autotuners leave a level no slower than they find it: the tuning it has and
+the default are among the candidates.  A slip-weakening level of 512x256, whose
+default runs of 5 rows are on no grid of the tuner's (without it the tuned level
+took 1.11 times as long; the times of one tuning differ by 1.5 %)."""
+import numpy as np
+import pytest
+
+from tetemoko_gb300 import _capi as A, scenarios as S
+
+pytestmark = pytest.mark.gpu
+
+
+def test_a_tuned_level_is_no_slower_than_the_default(cuda_lib):
+    import torch
+    from tetemoko_gb300.level import Context, LinElastLevelGodunov
+    sc = S.slip_weakening(nx=512, ny=256, dx=0.1, precision=A.TMK_PREC_MIXED)
+    dt = sc.dt()
+    ctx = Context(sc)
+    lv = LinElastLevelGodunov(ctx, [(0, 0, 511, 255)])
+    lv.set_level(sc.initial_U(), sc.initial_B())
+    default = lv.tuning()
+    tuned, _ = lv.autotune(0.0, dt, steps=8)
+
+    def step_us(t):
+        lv.set_tuning(t)
+        g = lv.graph(10, 0.0, dt)
+        us = []
+        for k in range(24):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            g.launch(0.0)
+            b.record()
+            torch.cuda.synchronize()
+            us.append(a.elapsed_time(b) * 100.0)
+        g.close()
+        return float(np.median(us[4:]))
+
+    ratios = [step_us(tuned) / step_us(default) for _ in range(5)]
+    lv.close()
+    ctx.close()
+    assert float(np.median(ratios)) <= 1.05, (ratios, tuned.as_dict())
