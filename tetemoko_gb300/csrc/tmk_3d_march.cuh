@@ -955,21 +955,15 @@ cudaError_t launch_march3(const Plan& pl, const DevParams& hp, const DevParams* 
   K3<T> k;
   k.load(hp, dt, dx);
   using Src = typename Plan::Src;
-  static const cudaError_t configured = [] {
-    cudaError_t e = cudaFuncSetAttribute(values_kernel<T, 1, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)val_smem_bytes<T, 1>());
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(values_kernel<T, 2, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)val_smem_bytes<T, 2>());
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(step_kernel<T, false, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)step_smem_bytes<T>());
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(step_kernel<T, true, Src>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)step_smem_bytes<T>());
-    return e;
-  }();
-  if (configured != cudaSuccess) return configured;
+  static DeviceOnce once;
+  cudaError_t e = once_per_device(once, [] {
+    cudaError_t r = allow_smem(values_kernel<T, 1, Src>, val_smem_bytes<T, 1>());
+    if (r == cudaSuccess) r = allow_smem(values_kernel<T, 2, Src>, val_smem_bytes<T, 2>());
+    if (r == cudaSuccess) r = allow_smem(step_kernel<T, false, Src>, step_smem_bytes<T>());
+    if (r == cudaSuccess) r = allow_smem(step_kernel<T, true, Src>, step_smem_bytes<T>());
+    return r;
+  });
+  if (e != cudaSuccess) return e;
   if (pl.copy() && pl.n(K_AP)) to_pred_kernel<T, Src><<<blocks(pl.n(K_AP)), 128, 0, s>>>(pl.src(K_AP));
   // The z predictor does not wait for the x and y one, nor the step's tiles away
   // from the fault for the plane kernel (launch attribute; the kernels still
@@ -989,8 +983,7 @@ cudaError_t launch_march3(const Plan& pl, const DevParams& hp, const DevParams* 
   };
   const long long nxy = pl.n(K_VXY), nz = pl.n(K_VZ);
   cudaLaunchConfig_t cfg = config((nxy + VAL_WARPS - 1) / VAL_WARPS, 32 * VAL_WARPS, val_smem_bytes<T, 1>(), false);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, values_kernel<T, 1, Src>, pl.src(K_VXY), k, nxy);
-  if (e != cudaSuccess) return e;
+  if ((e = cudaLaunchKernelEx(&cfg, values_kernel<T, 1, Src>, pl.src(K_VXY), k, nxy)) != cudaSuccess) return e;
   cfg = config((nz + VAL_WARPS - 1) / VAL_WARPS, 32 * VAL_WARPS, val_smem_bytes<T, 2>(), true);
   if ((e = cudaLaunchKernelEx(&cfg, values_kernel<T, 2, Src>, pl.src(K_VZ), k, nz)) != cudaSuccess) return e;
   if (pl.fault())

@@ -14,6 +14,7 @@
 //     reciprocals, for the mixed-precision volume kernel.
 #pragma once
 #include <cuda_runtime.h>
+#include "tmk_once.h"
 #include <stdint.h>
 #include <type_traits>
 
@@ -44,6 +45,17 @@ cudaError_t launch_chained(void (*kernel)(K...), dim3 grid, int threads, size_t 
   cfg.attrs = chained ? attr : nullptr;
   cfg.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
+// The dynamic shared memory limit of a kernel on the current device.
+template <typename... K>
+cudaError_t allow_smem(void (*kernel)(K...), size_t smem) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+template <typename Set> cudaError_t once_per_device(DeviceOnce& once, Set&& set) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  return e == cudaSuccess ? once(dev, set) : e;
 }
 
 constexpr int NC = 22;

@@ -11,9 +11,9 @@ static cudaError_t patch_scheme(const PatchDev<double>* dpd, int nx, int ny, Mar
                                 cudaStream_t s) {
   constexpr size_t smem = std::max(march_smem_bytes<double, 0, true>(), march_smem_bytes<double, 1, true>());
   auto* const kernel = march_both_kernel<double, SCH, MARCH_PATCH>;
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (configured != cudaSuccess) return configured;
+  static DeviceOnce once;
+  const cudaError_t e = once_per_device(once, [=] { return allow_smem(kernel, smem); });
+  if (e != cudaSuccess) return e;
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // An item costs 2.6 rows beyond its own; CTAs of both groups beyond one per SM

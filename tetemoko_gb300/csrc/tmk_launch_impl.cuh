@@ -30,14 +30,10 @@ struct LaunchImpl {
   static cudaError_t volume(const PatchDev<Real>* patches, const TileDev* tiles, int ntiles,
                             const DevParams* params, cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
-    static bool configured = false;
+    static DeviceOnce once;
     const size_t sm = smem();
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(volume_kernel<Real, TX_, TY_, NT_>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    const cudaError_t e = once_per_device(once, [&] { return allow_smem(volume_kernel<Real, TX_, TY_, NT_>, sm); });
+    if (e != cudaSuccess) return e;
     dim3 grid(ntiles, 2);
     volume_kernel<Real, TX_, TY_, NT_><<<grid, NT_, sm, s>>>(patches, tiles, params);
     return cudaGetLastError();
@@ -58,13 +54,12 @@ struct LaunchImpl {
   static cudaError_t march(int g, const PatchDev<Real>* patches, const MarchItem* items, int nitems,
                            const MarchConst<Real>& mc, bool pdl, cudaStream_t s) {
     if (nitems <= 0) return cudaSuccess;
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = march_configure<MARCH_SCH_RUNTIME>();
-      if (e == cudaSuccess) e = march_configure<MARCH_SCH_PPM_PRIM>();
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    static DeviceOnce once;
+    const cudaError_t e = once_per_device(once, [] {
+      const cudaError_t r = march_configure<MARCH_SCH_RUNTIME>();
+      return r == cudaSuccess ? march_configure<MARCH_SCH_PPM_PRIM>() : r;
+    });
+    if (e != cudaSuccess) return e;
     const bool fx = march_scheme_fixed(mc);
     auto* const kernel = fx ? march_entry<MARCH_SCH_PPM_PRIM>(g, mc) : march_entry<MARCH_SCH_RUNTIME>(g, mc);
     return launch_chained(kernel, dim3((nitems + MARCH_WARPS - 1) / MARCH_WARPS), 32 * MARCH_WARPS,
@@ -82,9 +77,9 @@ struct LaunchImpl {
                                        cudaStream_t s) {
     auto* const kernel = march_both_kernel<Real, SCH, MARCH_OWN>;
     constexpr size_t smem = std::max(march_smem_bytes<Real, 0>(), march_smem_bytes<Real, 1>());
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (configured != cudaSuccess) return configured;
+    static DeviceOnce once;
+    const cudaError_t e = once_per_device(once, [=] { return allow_smem(kernel, smem); });
+    if (e != cudaSuccess) return e;
     return launch_chained(kernel, dim3((n0 + MARCH_WARPS - 1) / MARCH_WARPS + (n1 + MARCH_WARPS - 1) / MARCH_WARPS),
                           32 * MARCH_WARPS, smem, pdl, s, patches, items0, n0, items1, n1, mc);
   }
@@ -98,21 +93,15 @@ struct LaunchImpl {
   // the dynamic shared memory limit of the marching kernels of one scheme form
   template <int SCH>
   static cudaError_t march_configure() {
-    cudaError_t e = cudaFuncSetAttribute(march_kernel<Real, 0, false, SCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)march_smem_bytes<Real, 0>());
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(march_kernel<Real, 1, false, SCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)march_smem_bytes<Real, 1>());
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(march_kernel<Real, 0, true, SCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)march_smem_bytes<Real, 0>());
+    cudaError_t e = allow_smem(march_kernel<Real, 0, false, SCH>, march_smem_bytes<Real, 0>());
+    if (e == cudaSuccess) e = allow_smem(march_kernel<Real, 1, false, SCH>, march_smem_bytes<Real, 1>());
+    if (e == cudaSuccess) e = allow_smem(march_kernel<Real, 0, true, SCH>, march_smem_bytes<Real, 0>());
     return e;
   }
   template <int G, bool PL, int SCH>
   static int march_blocks() {
     int b = 0;
-    cudaFuncSetAttribute(march_kernel<Real, G, PL, SCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)march_smem_bytes<Real, G>());
+    allow_smem(march_kernel<Real, G, PL, SCH>, march_smem_bytes<Real, G>());
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, march_kernel<Real, G, PL, SCH>, 32 * MARCH_WARPS,
                                                       march_smem_bytes<Real, G>()) != cudaSuccess)
       return 0;
