@@ -257,8 +257,11 @@ TMK_D double clip_mag(double a, double b, double c) {
   const unsigned long long m = mb < mc ? mb : mc;
   return with_sign(ma < m ? ma : m, a);
 }
-// x * 2^K by the exponent bits (|K| <= 3); zeros, denormals and numbers near
-// the overflow limit, which only serve as bounds here, are returned as they are
+// x * 2^K by the exponent bits (|K| <= 3), for the limiters' bounds alone: zeros,
+// numbers below 2^-1020 and numbers near the overflow limit are returned as they
+// are (limited slopes down there are of no account: the product of two differences
+// below 1e-154, which a limiter by products tests, is zero).  Unlimited slopes and
+// deltas take the product and the sum.
 template <int K> TMK_D double mul_pow2(double x) {
   const int hi = __double2hiint(x);
   const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
@@ -289,12 +292,14 @@ TMK_D void same_sign(double2 a, double2 b, bool& x, bool& y) { x = same_sign1(a.
 // dl dr > 0, else 0.
 template <typename P> TMK_D P half_slope(P nl, P nr, bool limit) {
   using T = decltype(nl.x);
+  if (!limit) return pmul(padd(nl, nr), kall(T(0.25)));     // the slope itself: exact down to the smallest numbers
   const P q = quarter(padd(nl, nr));
-  if (!limit) return q;
   bool x, y;
   same_sign(nl, nr, x, y);
   return mk2(x ? clip_mag(q.x, nl.x, nr.x) : T(0), y ? clip_mag(q.y, nl.y, nr.y) : T(0));
 }
+// the doubled lo delta of a cell at a domain edge
+template <typename P> TMK_D P edge_delta(P n, bool limit) { return limit ? twice(n) : padd(n, n); }
 
 // Twice the PPM delta (lo face value - w) of a cell from its negated
 // difference to the cell below and both cells' half slopes:
@@ -797,7 +802,7 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
         if (!hll) na = nl;
         c0.dlo[c] = delta_lo<T>(nl, c0.n4[c], half_slope(na, nl, lim));
       } else {
-        c0.dlo[c] = twice(c0.n4[c]);
+        c0.dlo[c] = edge_delta(c0.n4[c], lim);
       }
       if (kS) { slopes[slope_slot<G>(c) * 32] = c0.n4[c]; slopes[(4 + slope_slot<G>(c)) * 32] = c0.dlo[c]; }
     }
@@ -855,7 +860,7 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
         if (q + 1 > dhi1) {
 #pragma unroll
           for (int c = 0; c < N; ++c)
-            if (live<G, 1>(c)) p[c] = pneg(twice(n4[c]));
+            if (live<G, 1>(c)) p[c] = pneg(edge_delta(n4[c], lim));
         }
 #pragma unroll
         for (int c = 0; c < N; ++c)
@@ -906,7 +911,7 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
         if (warp_xedge && edge_lo) {
 #pragma unroll
           for (int c = 0; c < N; ++c)
-            if (live<G, 0>(c)) d[c] = twice(n[c]);
+            if (live<G, 0>(c)) d[c] = edge_delta(n[c], lim);
         }
 #pragma unroll
         for (int c = 0; c < N; ++c)
@@ -914,7 +919,7 @@ TMK_D void march_items(const PatchDev<T>* __restrict__ patches, const MarchItem*
         if (warp_xedge && edge_hi) {
 #pragma unroll
           for (int c = 0; c < N; ++c)
-            if (live<G, 0>(c)) p[c] = pneg(twice(n[c]));
+            if (live<G, 0>(c)) p[c] = pneg(edge_delta(n[c], lim));
         }
 #pragma unroll
         for (int c = 0; c < N; ++c) {
