@@ -807,15 +807,11 @@ __global__ void __launch_bounds__(64) plane_kernel(const __grid_constant__ Src s
   double* const Bi = g.B + g.bb.at(i, j, kz);
   const long long bs = g.bb.cells();
   const double b0 = Bi[(rs ? 10 : 7) * bs];
-  // A face exactly on the rim of a slip-weakening patch is inside or outside by
-  // rounding: a batch rounds the face's position first, a mixed patch by itself
-  // lets it fuse with the difference from the patch's centre, and either keeps
-  // the side it has always had.
+  constexpr bool kFused = !kExact<T> && std::is_same<Src, One<T>>::value;       // cell_from
   RSFaceK fk;
   SWFaceK wk;
   if (rs) fk = rs_face_k(P, rs_face(P, nullptr, 0, 0), false, (i + 0.5) * g.dx - P.rs_x0, b0);
-  else if constexpr (std::is_same<Src, One<T>>::value) wk = sw_face_k<true>(P, (i + 0.5) * g.dx, (kz + 0.5) * g.dx);
-  else wk = sw_face_k<true>(P, __dmul_rn(i + 0.5, g.dx), __dmul_rn(kz + 0.5, g.dx));
+  else wk = sw_face_k<true>(P, cell_from<kFused>(i, g.dx, P.sw_fbc0), cell_from<kFused>(kz, g.dx, P.sw_fbc1));
   auto inS = [&](int a, int c) { return g.S.has(a, j, c); };
   auto val = [&](int s, int D, int w, int a, int c) { return val_plane(g, s, D, w)[g.S.at(a, j, c)]; };
   // jumps of the first-pass values of x (or z) over cell (a, c); false outside ccBox

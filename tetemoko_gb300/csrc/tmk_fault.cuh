@@ -398,9 +398,19 @@ TMK_D double rs_setbnd_k(const DevParams& P, const RSFaceK& fk, const double* U,
 // (ibcLinElast/SWIBCF.ChF:79-267) as rs_face_solve.  az: the values of the
 // antiplane S pair (syz + Zs rv vz).
 struct SWFaceK { double tau0, mu_s; };
+
+// Centre of cell i relative to c.  A face exactly on the rim of a nucleation
+// patch or friction box (odd nx, box at the grid's middle) is inside or outside
+// by the rounding of this number, with a jump of the whole patch: the 2-D mixed
+// form and a mixed 3-D patch by itself round it once (FUSED), FP64, as the
+// reference's Fortran, and the mixed batch round the product first.  Each form
+// keeps the side it has always had; written out, not left to the compiler.
+template <bool FUSED> TMK_D double cell_from(int i, double dx, double c) {
+  return FUSED ? __fma_rn(i + 0.5, dx, -c) : __dsub_rn(__dmul_rn(i + 0.5, dx), c);
+}
+// x, z: the face's position relative to the friction box's centre
 template <bool Z3 = false>
-TMK_D SWFaceK sw_face_k(const DevParams& P, double xcell, double zcell = 0.0) {
-  const double x = xcell - P.sw_fbc0, z = zcell - P.sw_fbc1;
+TMK_D SWFaceK sw_face_k(const DevParams& P, double x, double z = 0.0) {
   SWFaceK k;
   k.tau0 = 0.0;
   for (int ip = 0; ip < P.sw_np; ++ip) {

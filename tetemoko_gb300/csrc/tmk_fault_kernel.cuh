@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(fault_threads(SEG)) fault_kernel(const PatchDe
         if (rs) b_s2 = Bi[8 * bs];
       }
       if (rs) fk = rs_face_k(P, rs_face(P, p.fric, i - p.blo0, bs), p.fric != nullptr, (i + 0.5) * dx - P.rs_x0, b_state);
-      else wk = sw_face_k(P, (i + 0.5) * dx);
+      else wk = sw_face_k(P, cell_from<!kFp64>(i, dx, P.sw_fbc0));
     }
   } else if (role == 0 && ci >= 0) {
     if (i >= p.dlo0 && i <= p.dhi0 && i <= s1 + 1) {
