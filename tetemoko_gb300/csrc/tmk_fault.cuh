@@ -201,7 +201,7 @@ struct FaultFace { double vx1, vx2, vz1, vz2, vy, syy, sxy, syz, Vx, Vz, V; };
 // reference, a root beyond the bracket's upper end V = phi/Zs yields that end;
 // parameters outside the range of this form (a tensile fault, say) and, in the
 // FP64 form, roots that RSNEWTON does not reach (near or beyond the bracket's
-// end, or too far below its start) go to RSNEWTON itself.
+// end, too far below its start, or where beta^2 is out of range) go to RSNEWTON itself.
 //
 // The iterations run in FP32 (c e^{+-z} as e^{+-z + ln c}, whose exponent stays
 // below log(phi) inside the bracket).  The mixed form finishes with one FP64
@@ -226,7 +226,9 @@ TMK_D int rs_solve_z(const DevParams& P, const RSFaceK& fk, double phi, double p
     V = sqrt((double)dvx * (double)dvx + (double)dvz * (double)dvz);
     return rs_newton(P, phi, psi, sn, fk.a, V, tau);
   };
-  if (!(a32 > 0.f) || !(phi32 > 0.f) || !(lb32 > -600.f && lb32 < 600.f) || !(P.rs_V0 > 0.0)) return newton();
+  // RSNEWTON's derivative squares beta, which overflows past e^354.9
+  if (!(a32 > 0.f) || !(phi32 > 0.f) || !(lb32 > -600.f && lb32 < (EXACT ? 354.f : 600.f)) || !(P.rs_V0 > 0.0))
+    return newton();
   // bracket end z_max = asinh(beta Vmax) (= ln(2 beta Vmax) past e^20); the
   // root lies inside where alpha z_max > phi / 2
   const float vmax32 = phi32 * P.inv_Zs32;
