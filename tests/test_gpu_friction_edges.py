@@ -201,3 +201,41 @@ def test_the_lines_between_the_forms_of_the_solve(cuda_lib, form, name, law):
     dpsi = 1e-13 + 4.0 * (a + b) * (x + 1.0 * (law == A.TMK_RS_SLIP_LAW) * x * 60.0) * rel
     dpsi = dpsi + 4.0 * (a + b) * dt / sc.rs.L * 1e-14 * phi / Zs * 60.0
     assert (np.abs(Bg[10] - Bo[10])[ok] <= dpsi[ok]).all()
+
+
+@pytest.mark.parametrize("form", ["level", "patch3"])
+def test_mixed_shear_holds_the_velocities_by_the_whole_impedance(cuda_lib, form):
+    """600 faces whose sides move at +-2 m/s, varying slowly along the fault, weak
+    enough to slip: the shear they carry, tau + Zs/2 V, mixed less FP64.  The rounding
+    of the entering values (18.5 MPa in FP32) is 4e-7 a face, 1.6e-8 in the mean; the
+    impedance rounded to FP32 would shift the mean by 4.2e-8 Zs v = 7.7e-7.  Bound 2e-7."""
+    import torch
+    from tetemoko_gb300.level import Context, LinElastLevelGodunov, LinElastPatchGodunov3D
+    nx, shear = 600, []
+    for prec in (A.TMK_PREC_FP64, A.TMK_PREC_MIXED):
+        sc = S.rate_state(nx=nx, ny=NY, dx=0.1, precision=prec)
+        sc.rs.nsig = 0.0
+        U, B, dt = sc.initial_U(), sc.initial_B(), sc.dt() / 2
+        v = 2.0 + 0.1 * np.sin(np.arange(nx + 2 * G) * 0.011)
+        U[0], U[11] = v, -v
+        B[10] = 0.4
+        ctx = Context(sc)
+        if form == "level":
+            lv = LinElastLevelGodunov(ctx, [(0, 0, nx - 1, NY - 1)])
+            lv.set_level(U, B)
+            lv.step(0.0, dt)
+            lv.get_level(U, B)
+            lv.close()
+            Bv = B[:, G:-G]
+        else:
+            rep = lambda a: torch.from_numpy(np.repeat(a[:, None], NZ + 2 * G, axis=1).copy()).cuda()
+            dom = ((0, 0, 0), (nx - 1, NY - 1, NZ - 1))
+            Ud, Bd = rep(U), rep(B)
+            pg = LinElastPatchGodunov3D(ctx, dom)
+            pg.set_current_box(dom)
+            pg.update_state(Ud, (-G,) * 3, dt, B=Bd, blo=(-G, -G))
+            Bv = Bd.cpu().numpy()[:, G + 1, G:-G]
+        shear.append(Bv[3] + 0.5 * sc.constants()["Zs"] * Bv[2])
+        assert (Bv[2] > 0.5).all()
+        ctx.close()
+    assert abs(np.mean(shear[1] - shear[0])) <= 2e-7

@@ -53,24 +53,27 @@ struct K3 {
   T e_v, e_l2g, e_lam, e_G;               // update
   T hZp, hZs, irho, l2g, lam, G;          // face states and fluxes
   T nbg[9];                               // minus the background
+  float lZs;                              // what Zs loses in T
   double s0[3];                           // background syy, sxy, syz (the fault's tractions)
   int out[6];                             // absorbing edge (else free)
   void load(const DevParams& p, double dt, double dx) {
     const double r = dt / dx, sp = p.cp * r, ss = p.cs * r;
     Zp = (T)p.Zp; Zs = (T)p.Zs;
+    const double zp = (double)Zp, zs = (double)Zs;         // the rounded ones (MK)
+    lZs = (float)(p.Zs - zs);
     aP = (T)(0.5 * (1.0 - sp) * (1.0 - sp)); bP = (T)(0.5 * (sp * sp - sp));
     aS = (T)(0.5 * (1.0 - ss) * (1.0 - ss)); bS = (T)(0.5 * (ss * ss - ss));
     for (int k = 0; k < 2; ++k) {
       const double sc = k == 0 ? 0.5 : 1.0 / 3.0;
-      c_lam[k] = (T)(sc * r * p.lam * (0.5 / p.Zp));
-      c_G[k] = (T)(sc * r * p.G * (0.5 / p.Zs));
-      c_vP[k] = (T)(p.Zp * (0.5 * sc * r / p.rho));
-      c_vS[k] = (T)(p.Zs * (0.5 * sc * r / p.rho));
+      c_lam[k] = (T)(sc * r * p.lam * (0.5 / zp));
+      c_G[k] = (T)(sc * r * p.G * (0.5 / zs));
+      c_vP[k] = (T)(zp * (0.5 * sc * r / p.rho));
+      c_vS[k] = (T)(zs * (0.5 * sc * r / p.rho));
     }
     const double l = p.lam + 2.0 * p.G;
     e_v = (T)(0.5 * r / p.rho);
-    e_l2g = (T)(r * l * (0.5 / p.Zp)); e_lam = (T)(r * p.lam * (0.5 / p.Zp)); e_G = (T)(r * p.G * (0.5 / p.Zs));
-    hZp = (T)(0.5 / p.Zp); hZs = (T)(0.5 / p.Zs); irho = (T)(1.0 / p.rho);
+    e_l2g = (T)(r * l * (0.5 / zp)); e_lam = (T)(r * p.lam * (0.5 / zp)); e_G = (T)(r * p.G * (0.5 / zs));
+    hZp = (T)(0.5 / zp); hZs = (T)(0.5 / zs); irho = (T)(1.0 / p.rho);
     l2g = (T)l; lam = (T)p.lam; G = (T)p.G;
     for (int c = 0; c < 9; ++c) nbg[c] = (T)-p.bg[c];
     s0[0] = p.bg[4]; s0[1] = p.bg[6]; s0[2] = p.bg[8];
@@ -910,9 +913,15 @@ __global__ void __launch_bounds__(64) plane_kernel(const __grid_constant__ Src s
     }
     int it = 0;
     const double aP1 = (double)a[0][0].x + k.s0[0], aP2 = (double)a[1][0].x + k.s0[0];
-    const double aS1 = (double)a[0][1].x + k.s0[1], aS2 = (double)a[1][1].x + k.s0[1];
+    // the laws take the unrounded Zs: the rest of its product with the velocities
+    auto whole = [&](int s, int w) {
+      const double d = (double)a[s][w].x + k.s0[w];
+      if constexpr (kExact<T>) return d;
+      else return d + widen((s ? -k.lZs : k.lZs) * v[s][w - 1]);
+    };
+    const double aS1 = whole(0, 1), aS2 = whole(1, 1);
     if (rs) it = rs_face_solve<kExact<T>>(P, fk, aP1, aP2, aS1, aS2, bval, v[0][0] - v[1][0], v[0][1] - v[1][1], f);
-    else sw_face_solve(P, wk, aP1, aP2, aS1, aS2, (double)a[0][2].x + k.s0[2], (double)a[1][2].x + k.s0[2], bval, f);
+    else sw_face_solve(P, wk, aP1, aP2, aS1, aS2, whole(0, 2), whole(1, 2), bval, f);
     if (it > RS_IMAX) atomicAdd(&st->newton_maxed, 1ull);
     const T sP = (T)(f.syy - k.s0[0]), sS = (T)(f.sxy - k.s0[1]), sz = (T)(f.syz - k.s0[2]), vy = (T)f.vy;
     plane_face(g, l, 0, 0)[fo] = mk2(sP, vy);

@@ -30,6 +30,7 @@ template <typename T>
 struct FaultConst {
   MK<T> kx, ky;
   T nbg[9];                 // minus the background
+  typename PairOf<T>::P lZp, lZs;       // what the impedances lose in T (rv Z in y)
   T sig[9];                 // characteristic Courant numbers (general predictor)
   Consts<T> k;
   int fast;                 // PPM with primitive limiting: the deltas of tmk_march.cuh
@@ -43,6 +44,8 @@ struct FaultConst {
     const double l[9] = {-p.cp, -p.cs, -p.cs, 0.0, 0.0, 0.0, p.cs, p.cs, p.cp};
     for (int c = 0; c < 9; ++c) sig[c] = (T)(l[c] * (dt / dx));
     k.load(p);
+    const T lp = (T)(p.Zp - (double)(T)p.Zp), ls = (T)(p.Zs - (double)(T)p.Zs);
+    lZp = mk2(lp, -lp); lZs = mk2(ls, -ls);
     fast = p.order == 2 && p.prim_lim && !p.char_lim;
     xout_lo = p.bc[0] == 0; xout_hi = p.bc[1] == 0;
     s0[0] = p.bg[4]; s0[1] = p.bg[6]; s0[2] = p.bg[8];
@@ -115,7 +118,9 @@ TMK_D void fault_chars(const PatchDev<T>& p, const FaultConst<T>& fc, const DevP
       const T v = w[q][2], sr = w[3 + q][2] + fc.nbg[pair_s<D>(q)];
       const T nm = fma(Z, dm[q], dm[3 + q]), np = fma(Z, dp[q], dp[3 + q]);
       const T dn = fma(b, np, a * nm);          // the traced left-going delta at the lo face
-      An[q] = fma(Z, v, sr) + dn;
+      // the friction laws take the unrounded Z: the rest of its product with v
+      if constexpr (D == 1 && !kExact<T>) An[q] = fma(Z, v, fma(side_of(q == 0 ? fc.lZp : fc.lZs, s), v, sr + dn));
+      else An[q] = fma(Z, v, sr) + dn;
       const T pm = fma(-Z, dm[q], dm[3 + q]);
       if (D == 0) {
         const T pp = fma(-Z, dp[q], dp[3 + q]);
@@ -136,7 +141,9 @@ TMK_D void fault_chars(const PatchDev<T>& p, const FaultConst<T>& fc, const DevP
     for (int q = 0; q < 3; ++q) {
       const T Z = side_of(q == 0 ? k.Zp : k.Zs, D == 0 ? 0 : s);
       const T n0 = fc.nbg[pair_s<D>(q)];
-      An[q] = fma(Z, WM[pair_v<D>(q)], WM[pair_s<D>(q)] + n0);
+      const T v = WM[pair_v<D>(q)], sr = WM[pair_s<D>(q)] + n0;
+      if constexpr (D == 1 && !kExact<T>) An[q] = fma(Z, v, fma(side_of(q == 0 ? fc.lZp : fc.lZs, s), v, sr));
+      else An[q] = fma(Z, v, sr);
       if (D == 0) Ap[q] = fma(-Z, WP[pair_v<D>(q)], WP[pair_s<D>(q)] + n0);
       else if (q > 0) vlo[q - 1] = WM[pair_v<D>(q)];
     }

@@ -148,21 +148,25 @@ struct MK {
   TMK_HD void load(const DevParams& p, int D, double dtdx) {
     const double s2 = (D == 1) ? -1.0 : 1.0;    // rv of side 2
     auto two = [](double a, double b) { return mk2((T)a, (T)b); };
+    // An and Ap carry the velocity times the rounded impedances: what undoes or
+    // matches that product takes them too, or FP32 would scale every velocity by
+    // Z's rounding (4e-8)
+    const double zp = (double)(T)p.Zp, zs = (double)(T)p.Zs;
     Zp = two(p.Zp, s2 * p.Zp); Zs = two(p.Zs, s2 * p.Zs);
     const double sp = p.cp * dtdx, ss = p.cs * dtdx;
     aP = (T)(0.5 * (1.0 - sp) * (1.0 - sp)); bP = (T)(0.5 * (sp * sp - sp));
     aS = (T)(0.5 * (1.0 - ss) * (1.0 - ss)); bS = (T)(0.5 * (ss * ss - ss));
     const double l2g = p.lam + 2.0 * p.G;
-    c_lam = (T)(0.5 * dtdx * p.lam * (0.5 / p.Zp));
-    c_G = (T)(0.5 * dtdx * p.G * (0.5 / p.Zs));
+    c_lam = (T)(0.5 * dtdx * p.lam * (0.5 / zp));
+    c_G = (T)(0.5 * dtdx * p.G * (0.5 / zs));
     // the velocity term carries the rv of y in both directions (D's or E's)
-    const double vP = p.Zp * (0.25 * dtdx / p.rho), vS = p.Zs * (0.25 * dtdx / p.rho);
+    const double vP = zp * (0.25 * dtdx / p.rho), vS = zs * (0.25 * dtdx / p.rho);
     cvP = two(vP, -vP); cvS = two(vS, -vS);
     const double ev = 0.5 * dtdx / p.rho;
     e_v = two(ev, s2 * ev);
-    e_l2g = (T)(dtdx * l2g * (0.5 / p.Zp)); e_lam = (T)(dtdx * p.lam * (0.5 / p.Zp));
-    e_G = (T)(dtdx * p.G * (0.5 / p.Zs));
-    hZp = two(0.5 / p.Zp, s2 * 0.5 / p.Zp); hZs = two(0.5 / p.Zs, s2 * 0.5 / p.Zs);
+    e_l2g = (T)(dtdx * l2g * (0.5 / zp)); e_lam = (T)(dtdx * p.lam * (0.5 / zp));
+    e_G = (T)(dtdx * p.G * (0.5 / zs));
+    hZp = two(0.5 / zp, s2 * 0.5 / zp); hZs = two(0.5 / zs, s2 * 0.5 / zs);
     f_irho = two(-1.0 / p.rho, -s2 / p.rho);
     f_l2g = two(-l2g, -s2 * l2g); f_lam = two(-p.lam, -s2 * p.lam); f_G = two(-p.G, -s2 * p.G);
     const int v[3] = {D, 1 - D, 2}, s[3] = {3 + D, 6, 7 + D};
