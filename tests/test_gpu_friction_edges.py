@@ -150,19 +150,22 @@ def test_mixed_solve_is_fp64_to_the_last_digits(cuda_lib):
     assert np.median(np.abs(tau[1] - tau[0]) / tau[0]) <= 3e-16
 
 
-# (a, b, psi from, psi to): what the sweep of the state over the faces crosses.
-# With 70 MPa of shear on 120 MPa, f0 = 0.6, L = 0.02 m, V0 = 1e-6 m/s and dt = 7.5 ms:
+# (a, b, psi from, psi to, the sides' velocity difference if not 0): what the sweep of
+# the state over the faces crosses.  With 70 MPa of shear on 120 MPa, f0 = 0.6, L = 0.02 m, V0 = 1e-6 m/s and dt = 7.5 ms:
 SWEEPS = {
     "slip_in_a_step": (0.008, 0.012, 0.40, 0.75),    # V dt / L = 0.01 (psi near 0.50) and r = 1e-3 (psi = 0.505)
     "sum_in_range": (0.010, 4e-4, 0.312, 0.324),     # r = 1e300, where log1p gives way to the sum itself
     "exp_of_minus_z": (0.0305, 0.036, 0.20, 0.90),   # z = 19, past which e^-z is dropped
     "bracket_end": (0.008, 0.012, 0.160, 0.170),     # the root at V = phi / Zs
     "bracket_far": (0.008, 0.012, 0.00, 0.30),
-    "halvings": (0.008, 0.012, 0.85, 0.97),          # 80 halvings from the bracket's middle to the root
+    "tiny_rate": (0.008, 0.012, 0.85, 0.97),         # V = 1e-21 to 1e-27 from rest
+    "halvings": (0.008, 0.012, 0.93, 0.99, 1.0),     # 80 halvings from 1 m/s to the root (psi = 0.957)
 }
 # what RSNEWTON itself does not solve, and FP64 leaves to it:
 UNSOLVED = {
-    "unreached": (0.008, 0.012, 0.97, 1.05),         # 100 halvings end above the root
+    "tiniest_rate": (0.008, 0.012, 0.97, 1.05),      # below the velocities' last bit at RSNEWTON's residual
+    "unreached": (0.008, 0.012, 0.99, 1.15, 1.0),    # 100 halvings from 1 m/s end above the root (psi = 1.07)
+    "unreached_from_above": (0.008, 0.012, 0.99, 1.15, 40.0),     # ... from the bracket's middle
     "beta_squared": (0.0015, 0.004, 0.40, 0.60),     # beta^2 overflows past psi = 0.513: NaN from V = 0
 }
 CASES = [(f, n) for n in SWEEPS for f in FORMS] + [(f, n) for n in UNSOLVED for f in FORMS if f.endswith("fp64")]
@@ -171,32 +174,37 @@ CASES = [(f, n) for n in SWEEPS for f in FORMS] + [(f, n) for n in UNSOLVED for 
 @pytest.mark.parametrize("law", [A.TMK_RS_SLIP_LAW, A.TMK_RS_AGING_LAW], ids=["slip", "aging"])
 @pytest.mark.parametrize("form,name", CASES, ids=["%s-%s" % c for c in CASES])
 def test_the_lines_between_the_forms_of_the_solve(cuda_lib, form, name, law):
-    """241 faces of a uniform state (which the mixed form holds exactly) whose psi
-    crosses a line.  RSNEWTON stops at a residual of 2.2e-12 MPa: a relative error of
-    the slip rate of 2.2e-12 / (a sn), or of FP64's rounding of phi where that is more;
+    """241 faces of a uniform state (which the mixed form holds exactly, but for the FP32
+    rounding of a moving fault's shear, 1e-7 of it) whose psi crosses a line.
+    RSNEWTON stops at a residual of 2.2e-12 MPa: a relative error of the slip rate of 2.2e-12 / (a sn), or of FP64's rounding of phi where that is more;
     the mixed form's accepted step is at most 1e-8 of the slip rate off.  The slip rate
     is the difference of two velocities of phi / Zs: 1e-14 of that.  Each bound twice,
     for the two or four solves in turn; the state moves by b, or the slip law's
     a + (b - a), times V dt / L for a relative change of V."""
     nx = 241
-    a, b, p0, p1 = {**SWEEPS, **UNSOLVED}[name]
+    a, b, p0, p1, *move = {**SWEEPS, **UNSOLVED}[name]
     sc = _sc(form, law, nx=nx, a=a, b=b, nsig=0.0)
     if law == A.TMK_RS_SLIP_LAW:
         sc.rs.L = 2.0           # the explicit step is stable
     U, B, dt = sc.initial_U(), sc.initial_B(), sc.dt() / 2
     B[10] = np.linspace(p0, p1, nx + 2 * G)
+    alpha, phi, Zs = 120.0 * a, 70.0, sc.constants()["Zs"]
+    if move:
+        U[0], U[11] = 0.5 * move[0], -0.5 * move[0]
+        phi += 0.5 * Zs * move[0]
     (rc, Ug, Bg), (rco, Uo, Bo) = _step(form, sc, U, B, dt)
     nan = np.isnan(Bo[10])
     assert np.array_equal(np.isnan(Bg), np.isnan(Bo)) and (rc is None or rc == rco)
     assert name in UNSOLVED or not nan.any()
-    alpha, phi, Zs = 120.0 * a, 70.0, sc.constants()["Zs"]
     V = np.where(nan, 0.0, Bo[2])
-    rel = max(2.2e-12 / alpha, 1e-15 * phi / alpha) + (1e-8 if form.endswith("mixed") else 0.0)
+    mixed = form.endswith("mixed")
+    shear = 1e-7 * phi if mixed and move else 0.0
+    rel = max(2.2e-12 / alpha, 1e-15 * phi / alpha) + (1e-8 if mixed else 0.0) + shear / alpha
     dV = 2.0 * (rel * V + 1e-14 * phi / Zs)
     ok = ~nan
     assert (np.abs(Bg[2] - Bo[2])[ok] <= dV[ok]).all()
     # alpha z: z moves by the relative change of V; never less than FP64's rounding
-    assert (np.abs(Bg[3] - Bo[3])[ok] <= 2.0 * alpha * rel + 1e-12 * phi).all()
+    assert (np.abs(Bg[3] - Bo[3])[ok] <= 2.0 * alpha * rel + 2.0 * shear + 1e-12 * phi).all()
     x = V * dt / sc.rs.L
     dpsi = 1e-13 + 4.0 * (a + b) * (x + 1.0 * (law == A.TMK_RS_SLIP_LAW) * x * 60.0) * rel
     dpsi = dpsi + 4.0 * (a + b) * dt / sc.rs.L * 1e-14 * phi / Zs * 60.0

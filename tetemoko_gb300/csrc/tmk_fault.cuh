@@ -31,18 +31,20 @@ TMK_D RSFace rs_face(const DevParams& P, const double* fric, int off, int stride
 
 // RSNEWTON (ibcLinElast/RSIBCF.ChF:336-401): bracketed Newton on the slip rate
 // for  sn a asinh(V exp(psi/a)/(2V0)) + Zs/2 V = phi  on (0, phi/Zs).  The loop
-// is bounded by IMAX; returns the iterations used.
+// is bounded by IMAX; returns the iterations used.  halve: the first iterations,
+// known to halve V without a look at the function, done at once (same bits).
 TMK_D int rs_newton(const DevParams& P, double phi, double psi, double sn, double c_rs_a, double& V,
-                    double& tau) {
+                    double& tau, int halve = 0) {
   const double atolG = 2.220446049250313e-16 * 1e4;
   double Vmin = 0.0, Vmax = phi / P.Zs;
   if (V < Vmin || V > Vmax) V = (Vmin + Vmax) / 2.0;
+  if (halve > 0) { V = V * __hiloint2double((1023 - halve) << 20, 0); Vmax = 2.0 * V; }
   double alpha = sn * c_rs_a;
   double beta = exp(psi / c_rs_a) / (2.0 * P.rs_V0);
   double eta = 0.5 * P.Zs;
   double fval = alpha * asinh(beta * V) + eta * V - phi;
   int it;
-  for (it = 1; it <= RS_IMAX; ++it) {
+  for (it = halve + 1; it <= RS_IMAX; ++it) {
     if (fval < 0) Vmin = V; else Vmax = V;
     double dfval = alpha * beta / sqrt((beta * beta) * (V * V) + 1) + eta;
     double dV = -fval / dfval;
@@ -222,9 +224,9 @@ TMK_D int rs_solve_z(const DevParams& P, const RSFaceK& fk, double phi, double p
   const double lb = psi * fk.inv_a - P.ln_2V0;        // ln beta, beta = e^(psi/a) / (2 V0)
   const double lc = P.ln_halfZs - lb;                 // ln c
   const float a32 = (float)alpha, lb32 = (float)lb, lc32 = (float)lc, phi32 = (float)phi;
-  auto newton = [&]() {
+  auto newton = [&](int halve = 0) {
     V = sqrt((double)dvx * (double)dvx + (double)dvz * (double)dvz);
-    return rs_newton(P, phi, psi, sn, fk.a, V, tau);
+    return rs_newton(P, phi, psi, sn, fk.a, V, tau, halve);
   };
   // RSNEWTON's derivative squares beta, which overflows past e^354.9
   if (!(a32 > 0.f) || !(phi32 > 0.f) || !(lb32 > -600.f && lb32 < (EXACT ? 354.f : 600.f)) || !(P.rs_V0 > 0.0))
@@ -262,11 +264,24 @@ TMK_D int rs_solve_z(const DevParams& P, const RSFaceK& fk, double phi, double p
     z = zn;
     if (fabsf(dz) <= 2e-6f * fmaxf(1.f, z)) break;
   }
-  // RSNEWTON halves its way down from a slip rate far above the root and stops
+  // RSNEWTON halves its way down from a slip rate V far above the root and stops
   // after RS_IMAX iterations wherever it is: the FP64 form leaves a root more
-  // than 80 halvings below the start to it
-  const float lroot = (z > 1.f ? z - 0.6931472f : logf(fmaxf(z, 1e-30f))) - lb32;       // ln V, within 0.2
-  if (EXACT && logf(v0 > 0.f && v0 <= vmax32 ? v0 : 0.5f * vmax32) - lroot > 55.45f) return newton();
+  // than 80 halvings below the start (or, from rest, the bracket's middle) to it,
+  // beginning where the halvings end.  A step leaves the bracket while
+  // asinh(beta V) is above the root's z by more than 1 (+ eta V_root / alpha,
+  // nothing here); 2.5 allows for the FP32 root and for a start that FP64 puts at
+  // the bracket's middle.  (An iteration takes 3 us and holds up the step: a plastic
+  // FP64 level of 512x256 whose fault heals 298 us a step, 837 with every
+  // halving; from rest there are none.)
+  if (EXACT) {
+    const bool from = v0 > 0.f && v0 <= vmax32;
+    const float lv0 = logf(from ? v0 : 0.5f * vmax32);
+    const float lroot = (z > 1.f ? z - 0.6931472f : logf(fmaxf(z, 1e-30f))) - lb32;       // ln V, within 0.2
+    if (lv0 - lroot > 55.45f) {
+      const float h = (0.6931472f + lb32 + lv0 - z - 2.5f) * 1.442695f;
+      return newton(v0 > 0.f && a32 > 1e-6f ? min(max((int)h, 0), RS_IMAX) : 0);
+    }
+  }
   double zz = (double)z;
   for (int k = 0; k < 12; ++k) {
     const float z32 = (float)zz;
