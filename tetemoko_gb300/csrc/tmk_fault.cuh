@@ -33,8 +33,10 @@ TMK_D RSFace rs_face(const DevParams& P, const double* fric, int off, int stride
 // for  sn a asinh(V exp(psi/a)/(2V0)) + Zs/2 V = phi  on (0, phi/Zs).  The loop
 // is bounded by IMAX; returns the iterations used.  halve: the first iterations,
 // known to halve V without a look at the function, done at once (same bits).
+// climb: the root lies beyond phi/Zs; f and f' fall towards that end, so once
+// f(end) / f'(V) reaches past it every further step only halves the distance.
 TMK_D int rs_newton(const DevParams& P, double phi, double psi, double sn, double c_rs_a, double& V,
-                    double& tau, int halve = 0) {
+                    double& tau, int halve = 0, bool climb = false) {
   const double atolG = 2.220446049250313e-16 * 1e4;
   double Vmin = 0.0, Vmax = phi / P.Zs;
   if (V < Vmin || V > Vmax) V = (Vmin + Vmax) / 2.0;
@@ -43,10 +45,16 @@ TMK_D int rs_newton(const DevParams& P, double phi, double psi, double sn, doubl
   double beta = exp(psi / c_rs_a) / (2.0 * P.rs_V0);
   double eta = 0.5 * P.Zs;
   double fval = alpha * asinh(beta * V) + eta * V - phi;
+  const double fend = climb ? alpha * asinh(beta * Vmax) + eta * Vmax - phi : 0.0;
+  climb = fend < -1e-6;
   int it;
   for (it = halve + 1; it <= RS_IMAX; ++it) {
     if (fval < 0) Vmin = V; else Vmax = V;
     double dfval = alpha * beta / sqrt((beta * beta) * (V * V) + 1) + eta;
+    if (climb && -0.999 * fend > (Vmax - V) * dfval) {
+      for (; it <= RS_IMAX; ++it) V = (V + Vmax) / 2.0;
+      break;
+    }
     double dV = -fval / dfval;
     V = V + dV;
     if (V < Vmin || V > Vmax) V = (Vmin + Vmax) / 2.0;
@@ -224,9 +232,9 @@ TMK_D int rs_solve_z(const DevParams& P, const RSFaceK& fk, double phi, double p
   const double lb = psi * fk.inv_a - P.ln_2V0;        // ln beta, beta = e^(psi/a) / (2 V0)
   const double lc = P.ln_halfZs - lb;                 // ln c
   const float a32 = (float)alpha, lb32 = (float)lb, lc32 = (float)lc, phi32 = (float)phi;
-  auto newton = [&](int halve = 0) {
+  auto newton = [&](int halve = 0, bool climb = false) {
     V = sqrt((double)dvx * (double)dvx + (double)dvz * (double)dvz);
-    return rs_newton(P, phi, psi, sn, fk.a, V, tau, halve);
+    return rs_newton(P, phi, psi, sn, fk.a, V, tau, halve, climb);
   };
   // RSNEWTON's derivative squares beta, which overflows past e^354.9
   if (!(a32 > 0.f) || !(phi32 > 0.f) || !(lb32 > -600.f && lb32 < (EXACT ? 354.f : 600.f)) || !(P.rs_V0 > 0.0))
@@ -237,7 +245,7 @@ TMK_D int rs_solve_z(const DevParams& P, const RSFaceK& fk, double phi, double p
   const float lbv = lb32 + logf(vmax32);
   const float zmax = lbv > 20.f ? 0.6931472f + lbv : asinhf(expf(lbv));
   if (!(a32 * zmax - 0.5f * phi32 > 1e-4f * phi32)) {
-    if (EXACT) return newton();
+    if (EXACT) return newton(0, true);
     const double Vmax = phi * P.inv_Zs, l = lb + log(Vmax);
     const double zm = l > 20.0 ? 0.6931471805599453 + l : asinh(exp(l));
     if (alpha * zm + 0.5 * P.Zs * Vmax - phi <= 0.0) {
