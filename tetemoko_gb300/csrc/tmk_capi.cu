@@ -91,9 +91,9 @@ extern "C" tmk_status tmk_context_create(const tmk_elastic_params* e, const tmk_
     P.sw_off = sw->layout == TMK_SW_LAYOUT_OFFSET11 ? 11 : 9;
   }
   if (pl) { P.p_mu = pl->mu; P.p_beta = pl->beta; P.p_eta = pl->eta; P.p_b = pl->b; P.p_h = pl->h; }
-  P.inv_Zs = 1.0 / P.Zs; P.inv_Zp = 1.0 / P.Zp; P.lam_r = P.lam / (P.lam + 2.0 * P.G);
-  P.two_V0 = 2.0 * P.rs_V0; P.inv_2V0 = P.rs_V0 > 0 ? 1.0 / P.two_V0 : 0.0;
-  P.ln_2V0 = P.rs_V0 > 0 ? std::log(P.two_V0) : 0.0;
+  P.inv_Zs = 1.0 / P.Zs;
+  P.inv_2V0 = P.rs_V0 > 0 ? 1.0 / (2.0 * P.rs_V0) : 0.0;
+  P.ln_2V0 = P.rs_V0 > 0 ? std::log(2.0 * P.rs_V0) : 0.0;
   P.ln_halfZs = P.Zs > 0 ? std::log(0.5 * P.Zs) : 0.0;
   P.two_inv_Zs = 2.0 / P.Zs; P.half_inv_Zp = 0.5 / P.Zp; P.inv_Zs32 = (float)P.inv_Zs;
   P.inv_a = 1.0 / P.rs_a; P.inv_b = 1.0 / P.rs_b; P.inv_L = 1.0 / P.rs_L; P.inv_r0 = 1.0 / P.rs_r0;
@@ -251,8 +251,8 @@ int default_min_run(const tmk_level_s* L) {
 
 // Longest run by default: beyond it more, shorter items balance better than one
 // wave of long ones (us a step: an ensemble of 16 scenarios, 3.5 M cells, 202 at
-// runs of 28 in two waves, 272 at 57 in one; mixed 4096x1024 218 / 221; FP64
-// 2048x1024 2160 at 32, 2209 at 64).
+// runs of 28 in two waves, 272 at 57 in one; mixed 4096x1024 222 in two waves,
+// 225 in one; FP64 2048x1024 alike).
 constexpr int kMaxRun = 48;
 
 tmk_tuning default_tuning(const tmk_level_s* L) {
@@ -263,8 +263,8 @@ tmk_tuning default_tuning(const tmk_level_s* L) {
   // them and a launch for the fault rows.  Mixed, us a step, first against second:
   // slip weakening 64x32 12.0 / 13.7, 512x256 16.5 / 18.8, 2048x1024 117 / 123;
   // rate and state 64x32 20.6 / 23.5, 512x256 20.9 / 25.1, 1000x500 in patches of
-  // 128 61.7 / 61.7, 2048x1024 117 / 124.  FP64 512x256 198 / 217, 2048x1024
-  // 2160 / 2178.
+  // 128 52 / 49, 2048x1024 117 / 124.  FP64 512x256 198 / 217, 2048x1024
+  // 2090 / 2170.
   t.fault_first = 1;
   t.min_run = default_min_run(L);
   t.march_waves[0] = t.march_waves[1] = 1;
@@ -301,8 +301,9 @@ void level_free(tmk_level_s* L, T*& p) {
 
 // The marching work lists of both component groups under the level's tuning:
 // group g's list holds about march_waves[g] waves of its kernel's resident
-// warps; the antiplane kernel shares the SMs with the fault kernel, leaving
-// fault_displace CTA slots per fault-kernel CTA.
+// warps.  The group that starts beside the fault kernel leaves fault_displace
+// CTA slots per fault-kernel CTA: the in-plane one in the joint launch, the
+// antiplane one as a launch of its own.
 tmk_status build_march_lists(tmk_level_s* L) {
   const int npatch = (int)L->patches.size();
   const tmk_tuning& tu = L->tune;
@@ -325,12 +326,14 @@ tmk_status build_march_lists(tmk_level_s* L) {
     level_free(L, L->ditems[g]);
     level_free(L, L->dfrows[g]);
     level_free(L, L->stash[g]);
-    // The group whose CTAs start beside the fault kernel's leaves room for them:
-    // the antiplane one as a launch of its own, the in-plane one in one launch
-    // (2048x1024 mixed, rate and state, 117 us a step, 124 without).  In one
-    // launch of the FP64 form they share the pipe rather than the room, and the
-    // antiplane runs are as long as the in-plane ones (1024x512 579 us, 617 with
-    // room left).
+    // Room beside the fault kernel: rate and state 2048x1024 mixed 117 us a step,
+    // 124 without.  In the joint launch of the FP64 form the groups share the pipe
+    // rather than the room, and the antiplane runs are as long as the in-plane ones
+    // (1024x512 579 us, 617 with room left).  In the mixed form the antiplane runs
+    // are those of its own kernel, six CTAs per SM, although the joint launch holds
+    // four: its rows are half the work of in-plane ones, and shorter items after
+    // them even out the launch's end (2048x1024 118 us, sized for four 122; other sizes
+    // alike).
     const bool both = tu.fault_first && !fused, fp64 = L->prec != TMK_PREC_MIXED;
     int slots = march_slots_of(L, fused && g == 0 ? 2 : both && fp64 ? 0 : g) * tu.march_waves[g];
     if (g == (both ? 0 : 1) && !(both && fp64)) slots = std::max(warps, slots - tu.fault_displace * warps * fault_ctas);
@@ -1006,14 +1009,15 @@ bool both_groups(const tmk_level_s* L) {
   return L->march && L->tune.fault_first && !(L->ctx->scheme.plasticity && L->tune.plastic_fused);
 }
 
-// The kernels of one level step after the coarse-fine fill.  Marching form:
-// the in-plane kernel, then the fault kernel (scheduled as in-plane CTAs
-// retire, reading only the step's input state), then the antiplane kernel
-// beside it, then row 0 of the fault patches, which alone needs the fault
-// results.  With the tuning's fault_first the fault kernel comes first and the
-// in-plane kernel is its programmatic dependent, so that the fault kernel's
-// CTAs run beside the in-plane ones.  With per-launch timing the fault kernel
-// runs first and alone.
+// The kernels of one level step after the coarse-fine fill.  Marching form, by
+// default (fault_first): the fault kernel, which waits for what is before it, then
+// both component groups in one launch, its programmatic dependent, so that the
+// first marching CTAs run beside the fault kernel's; its fault-row items wait for
+// the fault kernel before they finish row 0, which alone needs its results.
+// With fault_first 0: the in-plane kernel, then the fault kernel (scheduled as
+// in-plane CTAs retire, reading only the step's input state), then the antiplane
+// kernel beside it, then row 0 of the fault patches.  With per-launch timing the
+// fault kernel runs first and alone.
 template <typename Real>
 tmk_status step_kernels(tmk_level_s* L, int par, double time, double dt, cudaEvent_t* ev, cudaStream_t s) {
   tmk_context* c = L->ctx;

@@ -87,9 +87,9 @@ struct DevParams {
   double sw_zc[SW_MAXP], sw_zw[SW_MAXP], sw_fbc1, sw_fbw1;   // z profiles (3-D)
   // plasticity (PLASTICSETF)
   double p_mu, p_beta, p_eta, p_b, p_h;
-  // reciprocals the mixed form's friction solve multiplies by (its chain of
-  // FP64 operations is the fault kernel's latency; a division costs several)
-  double inv_Zs, inv_Zp, lam_r, two_V0, inv_2V0;   // lam_r = lam/(lam+2G)
+  // reciprocals the friction solves multiply by (their chain of FP64 operations
+  // is the fault kernel's latency; a division costs several)
+  double inv_Zs, inv_2V0;
   double ln_2V0, ln_halfZs;                          // log(2 V0), log(Zs / 2)
   double two_inv_Zs, half_inv_Zp, inv_a, inv_b, inv_L, inv_r0, inv_ramp_w, inv_dw;
   float inv_Zs32;

@@ -497,8 +497,8 @@ constexpr size_t march_smem_bytes() {
 
 // resident CTAs per SM the register allocation targets: FP32 in-plane 4 (128
 // registers), antiplane 6 (80); FP64 in-plane 2, antiplane 4.  FP32 with 3 / 5
-// instead: the 2048x1024 level alike (126 us a step), an ensemble of 16
-// scenarios 7.57 against 5.96 ms per 20 steps; 4 / 7 and 5 / 7 spill.
+// instead, us a step: slip weakening 512x256 19.2 against 17.0, rate and state
+// 512x512 32.7 against 25.7, 2048x1024 121 against 118; 4 / 7 and 5 / 7 spill.
 template <typename T, int G> struct MarchMinBlocks {
   static constexpr int value = sizeof(T) == 4 ? ((G == 0) ? 4 : 6) : ((G == 0) ? 2 : 4);
 };
