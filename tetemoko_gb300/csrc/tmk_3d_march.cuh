@@ -417,8 +417,8 @@ TMK_D double widen(double f) { return f; }
 TMK_D bool has_denormal(const float* f) {
   unsigned least = ~0u;
 #pragma unroll
-  for (int c = 0; c < 9; ++c) least = min(least, (__float_as_uint(f[c]) & 0x7fffffffu) - 1u);
-  return least < 0x007fffffu;
+  for (int c = 0; c < 9; ++c) least = min(least, (__float_as_uint(f[c]) << 1) - 1u);      // zeros wrap around
+  return least < 0x00ffffffu;
 }
 TMK_D bool has_denormal(const double*) { return false; }
 
