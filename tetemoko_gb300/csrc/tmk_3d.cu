@@ -186,7 +186,7 @@ size_t layout3(Step3<T>& g, char* base) {
 // The step on characteristic values (tmk_3d_march.cuh) implements the decks'
 // predictor (PPM with primitive limiting) and the laws that read only those
 // values; whatever the size it beats the passes over face states (192x96x96
-// mixed: 685 against 1383 us, the 32-cell patches of a 96x64x64 level 807
+// mixed: 690 against 1383 us, the 32-cell patches of a 96x64x64 level 807
 // against 1097; 64x48x48 FP64: 581 against 2703).  The rest (PLM, CTU, limiting
 // of the characteristic amplitudes, the reference's 9-component slip weakening)
 // keeps those passes.

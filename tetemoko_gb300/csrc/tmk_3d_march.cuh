@@ -25,7 +25,7 @@
 // state (80 us) and the z values (40 us) DRAM; the x and y values (73 us) the
 // issue of the limiters; the plane (48 us) the latency of four dependent solves,
 // beside which the step's tiles away from the fault run; the step (294 us)
-// issue, 48 % of slots, and its last wave of CTAs.  A call 685 us; one pass per
+// issue, 48 % of slots, and its last wave of CTAs.  A call 690 us; one pass per
 // term, each through memory, took 1383 us.  FP64 (64x48x48): every kernel the
 // FP64 pipe; 581 us, was 2703 us.  32-cell boxes of a 96x64x64 level, mixed: 807
 // us, was 1097 (520 of either is reading the state back).
