@@ -1,7 +1,7 @@
 """The autotuners leave a level no slower than they find it: the tuning it has and
 the default are among the candidates.  A slip-weakening level of 512x256, whose
 default runs of 5 rows are on no grid of the tuner's (without it the tuned level
-took 1.11 times as long; the times of one tuning differ by 1.5 %)."""
+took 1.07 to 1.11 times as long; the times of one tuning differ by 0.3 %)."""
 import numpy as np
 import pytest
 
